@@ -134,6 +134,7 @@ struct crt_bvh {
     // neither compute nor store them.
     mutable bool wide4_ready = false;
     mutable bool cwide_ready = false;  // the compressed 4-wide nodes, derived likewise
+    uint32_t* cw_bad() const { return reinterpret_cast<uint32_t*>(cwide.as<char>() + 64ull * n); }
     // Refit topology of the last build (crt_refit, derived on its first call).
     DevBuf refit_link, refit_leaf, refit_dfs, refit_cnt;
     bool refit_ready = false;
@@ -195,7 +196,7 @@ struct crt_ctx {
     DevBuf mesh_vertices, mesh_indices, mesh_out;  // crt_triangles_from_indexed staging
     DevBuf probe_flag;                             // crt_selftest_wait
     DevBuf step_in, step_out;                      // crt_radix_digit_counts / _offsets
-    DevBuf pool_counter;                           // persistent traversal: next ray to take
+    DevBuf pool;                                   // persistent traversal: its counters and left-over rays
     DevBuf opt_scratch;                            // crt_optimize
     uint64_t last_trace_stats[2] = {0, 0};
     // pinned host staging
@@ -326,7 +327,7 @@ crt_status crt_destroy(crt_ctx* x) {
                       &x->ray_order, &x->ray_order_scratch, &x->shade_models, &x->shade_materials,
                       &x->shade_rays, &x->shade_hits, &x->image, &x->refit_state, &x->xtri_sorted,
                       &x->mesh_vertices, &x->mesh_indices, &x->mesh_out, &x->probe_flag, &x->step_in,
-                      &x->step_out, &x->pool_counter};
+                      &x->step_out, &x->pool};
     for (DevBuf* b : bufs) b->release();
     for (auto& e : x->ev)
         if (e) cudaEventDestroy(e);
@@ -712,12 +713,11 @@ crt_status ensure_wide4(crt_ctx* x, const crt_bvh* b) {
 }
 
 // Derives the compressed 4-wide traversal nodes of b on x's stream if the
-// last build (or refit) has not yet done so.
+// last build (or refit) has not yet done so; their bad flag follows them.
 crt_status ensure_cwide(crt_ctx* x, const crt_bvh* b) {
     if (b->cwide_ready || b->n <= 1) return CRT_OK;
-    CRT_TRY(b->cwide.reserve(64ull * b->n));
-    crt::launch_cwide(b->wide.as<float4>(), b->depth_odd.as<uint8_t>(), b->n - 1, b->cwide.as<uint4>(),
-                      x->err.as<uint32_t>(), x->stream);
+    CRT_TRY(b->cwide.reserve(64ull * b->n + 16));
+    crt::launch_cwide(b->wide.as<float4>(), b->n - 1, b->abs_eps, b->cwide.as<uint4>(), b->cw_bad(), x->stream);
     CRT_CUDA(cudaGetLastError());
     b->cwide_ready = true;
     return CRT_OK;
@@ -725,6 +725,7 @@ crt_status ensure_cwide(crt_ctx* x, const crt_bvh* b) {
 
 // Enqueues one traversal launch on device-resident rays/hits (no sync).
 constexpr uint32_t kPoolMinRays = 65536;  // below this a launch of one thread per ray fills the GPU as well
+                                          // (measured sides at the kernel, crt_walk4.cuh)
 constexpr uint32_t kChunkedCopyMinRays = 1u << 20;  // crt_trace: smaller host batches copy in one piece
 
 // classes_ready: the predictor's classes of these rays are already in its
@@ -735,7 +736,11 @@ crt_status trace_device(crt_ctx* x, const crt_bvh* b, const crt_ray* d_rays, uin
                         bool classes_ready = false) {
     if (n_rays == 0) return CRT_OK;
     if (flags & CRT_TRACE_WIDE) CRT_TRY(ensure_wide4(x, b));
-    if (flags & CRT_TRACE_COMPRESSED) CRT_TRY(ensure_cwide(x, b));
+    // Large batches over one scene: persistent warps over the compressed nodes;
+    // pixels in 8x4 tiles, seeded, 4-wide and counting walks keep one thread per ray.
+    const bool pool = !(flags & (CRT_TRACE_WIDE | CRT_TRACE_PER_RAY_THREADS | CRT_TRACE_USE_PREDICTOR | CRT_TRACE_STATS)) &&
+                      !seed_classes && tile_width == 0 && n_rays >= kPoolMinRays && b->n > 1;
+    if (pool || (flags & CRT_TRACE_COMPRESSED)) CRT_TRY(ensure_cwide(x, b));
     x->tev_valid = false;
     CRT_CUDA(cudaEventRecord(x->tev[0], x->stream));
     crt::TraceParams p{};
@@ -743,7 +748,10 @@ crt_status trace_device(crt_ctx* x, const crt_bvh* b, const crt_ray* d_rays, uin
     p.xtri = b->xtri.as<float4>();
     p.wide = (flags & CRT_TRI_WATERTIGHT) ? b->wide_wt.as<float4>() : b->wide.as<float4>();
     p.wide4 = (b->n > 1) ? b->wide4.as<float4>() : nullptr;
-    p.cwide = (b->n > 1 && (flags & CRT_TRACE_COMPRESSED)) ? b->cwide.as<uint4>() : nullptr;
+    if (b->n > 1 && (pool || (flags & CRT_TRACE_COMPRESSED))) {
+        p.cwide = b->cwide.as<uint4>();
+        p.cw_bad = b->cw_bad();
+    }
     p.rays = d_rays;
     p.hits = d_hits;
     p.n_rays = n_rays;
@@ -802,15 +810,9 @@ crt_status trace_device(crt_ctx* x, const crt_bvh* b, const crt_ray* d_rays, uin
     const bool deep = (b->depth_bound + 2 > 64) || (3 * ((b->depth_bound + 2) / 2) + 3 > 96);
     const uint32_t launch_flags =
         (flags & (CRT_TRACE_ANY | CRT_TRI_WATERTIGHT | CRT_TRACE_WIDE | CRT_TRACE_COMPRESSED)) | (deep ? (1u << 16) : 0u);
-    // Large closest-hit batches over the binary nodes: persistent warps that
-    // refill finished lanes (the rays of a batch differ widely in walk
-    // length); pixels in 8x4 tiles, any-hit, seeded and wide walks keep one
-    // thread per ray, which shares node fetches between a tile's rays.
-    const bool pool = !(flags & (CRT_TRACE_ANY | CRT_TRACE_WIDE | CRT_TRACE_COMPRESSED | CRT_TRACE_PER_RAY_THREADS)) &&
-                      !p.pred_class && tile_width == 0 && n_rays >= kPoolMinRays;
-    if (pool) CRT_TRY(x->pool_counter.reserve(16));
+    if (pool) CRT_TRY(x->pool.reserve(crt::trace_pool_bytes(n_rays)));
     CRT_CUDA(cudaEventRecord(x->tev[1], x->stream));
-    if (pool) crt::launch_trace_pool(p, launch_flags, x->pool_counter.as<uint32_t>(), x->stream);
+    if (pool) crt::launch_trace_pool(p, launch_flags, x->pool.as<uint32_t>(), x->stream);
     else crt::launch_trace(p, launch_flags, static_cast<int>(x->cfg.trace_block), x->stream);
     CRT_CUDA(cudaGetLastError());
     CRT_CUDA(cudaEventRecord(x->tev[2], x->stream));
@@ -1808,7 +1810,11 @@ struct crt_batch {
     DevBuf node_box, node_kids, pf, clus_a, clus_b, it, ploc_lb, hist, sort_lb;
     DevBuf nodes, wide, wide_wt, depth_odd, xtri, xtri_sorted, inv_perm;
     DevBuf ray_order, ray_order_scratch;  // CRT_TRACE_SORT_RAYS
-    DevBuf pool_counter;                  // the persistent trace's ray counter
+    DevBuf pool;                          // the persistent trace's counters and left-over rays
+    DevBuf cwide;                         // compressed 4-wide nodes (and their bad flag) of the scenes' current trees
+    bool cwide_ready = false;
+    bool g_cwide = false;                 // the captured graph derives them
+    uint32_t* cw_bad() const { return reinterpret_cast<uint32_t*>(cwide.as<char>() + 64ull * n_tris); }
     bool models_set = false;
     cudaGraphExec_t graph = nullptr;
     const void* g_tris = nullptr;
@@ -1846,6 +1852,11 @@ crt_status batch_upload_models(crt_ctx* x, crt_batch* bt, const crt_mesh_model* 
     bt->models_set = true;
     (void)x;
     return CRT_OK;
+}
+
+// Whether a batch's trace runs on the persistent ray pool.
+bool batch_pool(const crt_batch* bt, uint32_t flags) {
+    return !(flags & CRT_TRACE_USE_PREDICTOR) && bt->n_rays >= kPoolMinRays;
 }
 
 // Enqueue build (and trace when rays != null) without synchronising.
@@ -1888,12 +1899,18 @@ crt_status batch_trace_enqueue(crt_ctx* x, crt_batch* bt, const crt_ray* rays, u
                               s);
         p.order = bt->ray_order.as<uint32_t>();
     }
-    // large closest-hit batches: the persistent ray pool, each lane walking
-    // its ray's scene (as trace_device does for one scene)
-    if (!(flags & CRT_TRACE_ANY) && !p.pred_class && bt->n_rays >= kPoolMinRays)
-        crt::launch_trace_batch_pool(p, bt->scenes.as<crt::BatchScene>(), bt->n_scenes, flags & CRT_TRI_WATERTIGHT, deep,
-                                     bt->pool_counter.as<uint32_t>(), s);
-    else
+    // large batches: the persistent ray pool, each lane walking its ray's scene
+    // (as trace_device does for one scene)
+    if (batch_pool(bt, flags)) {
+        if (!bt->cwide_ready)
+            crt::launch_cwide_batch(bt->wide.as<float4>(), bt->scenes.as<crt::BatchScene>(), bt->n_scenes, bt->n_tris,
+                                    bt->cwide.as<uint4>(), bt->cw_bad(), s);
+        bt->cwide_ready = true;
+        p.cwide = bt->cwide.as<uint4>();
+        p.cw_bad = bt->cw_bad();
+        crt::launch_trace_batch_pool(p, bt->scenes.as<crt::BatchScene>(), bt->n_scenes,
+                                     flags & (CRT_TRACE_ANY | CRT_TRI_WATERTIGHT), deep, bt->pool.as<uint32_t>(), s);
+    } else
         crt::launch_trace_batch(p, bt->scenes.as<crt::BatchScene>(), bt->n_scenes, bt->n_rays,
                                 flags & (CRT_TRACE_ANY | CRT_TRI_WATERTIGHT), static_cast<int>(bt->cfg.trace_block), deep,
                                 s);
@@ -1920,6 +1937,7 @@ crt_status batch_enqueue(crt_ctx* x, crt_batch* bt, const crt_triangle* tris, co
     const uint32_t tiles = (bt->n_tris + crt::sort_tile_keys(bits) - 1) / crt::sort_tile_keys(bits);
     const size_t lb_words = static_cast<size_t>(tiles) * 256 + 1;  // per pass (room for 256-digit scene pass)
     uint32_t* err = bt->err.as<uint32_t>();
+    bt->cwide_ready = false;
     CRT_CUDA(cudaMemsetAsync(bt->err.p, 0, 16, s));
     CRT_CUDA(cudaMemsetAsync(bt->states.p, 0, crt::batch_box_state_bytes() * bt->n_scenes, s));
     CRT_CUDA(cudaMemsetAsync(bt->hist.p, 0, 4ull * passes * radix, s));
@@ -1969,8 +1987,13 @@ crt_status batch_enqueue(crt_ctx* x, crt_batch* bt, const crt_triangle* tris, co
     return CRT_OK;
 }
 
-// Scratch of CRT_TRACE_SORT_RAYS for a batch, reserved outside graph capture.
-crt_status batch_order_buffers(crt_batch* bt, uint32_t flags) {
+// Buffers of a batch's trace (compressed nodes, the scratch of CRT_TRACE_SORT_RAYS),
+// reserved outside graph capture.
+crt_status batch_trace_buffers(crt_batch* bt, uint32_t flags) {
+    if (batch_pool(bt, flags)) {
+        CRT_TRY(bt->cwide.reserve(64ull * bt->n_tris + 16));
+        CRT_TRY(bt->pool.reserve(crt::trace_pool_bytes(bt->ray_cap)));
+    }
     // sized for the batch's ray capacity, so a later crt_batch_set_ray_counts
     // never moves a buffer that a captured graph points at
     if (!(flags & CRT_TRACE_SORT_RAYS) || bt->ray_cap <= 1) return CRT_OK;
@@ -2073,7 +2096,6 @@ crt_status crt_batch_create(crt_ctx* x, const uint32_t* tri_counts, const uint32
     R(bt->depth_odd, N);
     R(bt->xtri, 48ull * N);
     R(bt->xtri_sorted, 48ull * N);
-    R(bt->pool_counter, 16);
     if (st != CRT_OK) { crt_batch_free(bt); return st; }
     std::vector<uint32_t> seg(n_scenes + 1), segh(256, 0);
     for (uint32_t k = 0; k < n_scenes; ++k) { seg[k] = hs[k].tri_off; segh[k] = hs[k].n_tris; }
@@ -2105,7 +2127,7 @@ crt_status crt_batch_free(crt_batch* bt) {
                       &bt->codes_a, &bt->codes_b, &bt->vals_a, &bt->vals_b, &bt->codes, &bt->perm_global,
                       &bt->perm_local, &bt->node_box, &bt->node_kids, &bt->pf, &bt->clus_a, &bt->clus_b, &bt->it,
                       &bt->ploc_lb, &bt->hist, &bt->sort_lb, &bt->nodes, &bt->wide, &bt->wide_wt, &bt->depth_odd, &bt->xtri, &bt->ray_order, &bt->ray_order_scratch,
-                      &bt->inv_perm, &bt->xtri_sorted, &bt->pool_counter};
+                      &bt->inv_perm, &bt->xtri_sorted, &bt->pool, &bt->cwide};
     for (DevBuf* b : bufs) b->release();
     delete bt;
     return CRT_OK;
@@ -2195,7 +2217,7 @@ crt_status crt_batch_trace(crt_ctx* x, crt_batch* bt, const crt_ray* rays, uint3
     CRT_TRY(check_aligned16(rays, "crt_batch_trace: rays"));
     CRT_TRY(check_aligned16(hits, "crt_batch_trace: hits"));
     CRT_CUDA(cudaSetDevice(x->device));
-    CRT_TRY(batch_order_buffers(bt, flags));
+    CRT_TRY(batch_trace_buffers(bt, flags));
     CRT_CUDA(cudaMemsetAsync(bt->err.p, 0, 16, x->stream));
     const bool deep = bt->cfg.stack_depth > 64 || bt->max_iters + 2 > 64;
     CRT_TRY(batch_trace_enqueue(x, bt, rays, flags, hits, deep));
@@ -2208,7 +2230,7 @@ crt_status crt_batch_run(crt_ctx* x, crt_batch* bt, const crt_triangle* tris, co
     CRT_TRY(batch_trace_flags(bt, flags, "crt_batch_run"));
     CRT_TRY(check_batch_buffers(tris, rays, hits, "crt_batch_run"));
     CRT_CUDA(cudaSetDevice(x->device));
-    CRT_TRY(batch_order_buffers(bt, flags));  // before any graph capture: no allocation inside it
+    CRT_TRY(batch_trace_buffers(bt, flags));  // before any graph capture: no allocation inside it
     if (graph_used) *graph_used = 0;
     if (bt->max_iters + 2 > 64) bt->cfg.stack_depth = 1024;
     if (use_graph) {
@@ -2234,9 +2256,11 @@ crt_status crt_batch_run(crt_ctx* x, crt_batch* bt, const crt_triangle* tris, co
             } else {
                 bt->g_tris = tris; bt->g_rays = rays; bt->g_hits = hits; bt->g_flags = flags; bt->g_cfg = bt->cfg;
                 bt->g_counts = bt->ray_counts();
+                bt->g_cwide = bt->cwide_ready;
             }
         }
         if (bt->graph) {
+            bt->cwide_ready = bt->g_cwide;
             CRT_CUDA(cudaGraphLaunch(bt->graph, x->stream));
             if (graph_used) *graph_used = 1;
             CRT_TRY(batch_check(x, bt));
@@ -2318,7 +2342,7 @@ crt_status crt_batch_autotune(crt_ctx* x, crt_batch* bt, const crt_triangle* tri
     if (!x || !bt || !tris || !rays || !hits) return fail(CRT_ERR_INVALID_ARG, "crt_batch_autotune: null argument");
     CRT_TRY(check_batch_buffers(tris, rays, hits, "crt_batch_autotune"));
     CRT_CUDA(cudaSetDevice(x->device));
-    CRT_TRY(batch_order_buffers(bt, flags));
+    CRT_TRY(batch_trace_buffers(bt, flags));
     cudaEvent_t e0, e1, e2;
     CRT_CUDA(cudaEventCreate(&e0));
     CRT_CUDA(cudaEventCreate(&e1));

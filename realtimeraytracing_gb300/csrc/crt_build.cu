@@ -1384,101 +1384,138 @@ __global__ void __launch_bounds__(256) wide4_kernel(const float4* __restrict__ w
 }
 
 // ================================= K4c: compressed 4-wide traversal nodes
-// The same four children as wide4_kernel, in 64 bytes: the node's origin
-// (the minimum corner over its children), one power-of-two step per axis
-// (the least with 255 steps covering the node's extent, biased exponent in a
-// byte) and each child box as 8-bit step counts, the minimum rounded down
-// and the maximum up.  The traversal decodes origin + q * step; rounding to
-// nearest is monotone, so the decoded box encloses the exact one.  Record:
-// (origin xyz, exponents | child count << 24), (qlo x, y, z, qhi x), (qhi y,
-// z, 0, 0), four child references; byte c of each q word belongs to child c.
-__device__ __forceinline__ uint32_t quant_step_exp(double extent) {
-    int e = -126;
-    if (extent > 0.0) {
-        int k = 0;
-        frexp(extent / 255.0, &k);  // extent / 255 < 2^k
-        e = k < -126 ? -126 : k;
-    }
-    return static_cast<uint32_t>(e + 127);
+// One 64-byte record per binary internal node (format: crt_walk4.cuh): the
+// node's two children, then twice the internal child of largest area opened
+// into its own two.  Every step is rounded outward by directed float rounding:
+// the child's box grown by g = 4 * abs_eps, the origin the least corner, the
+// step the least power of two with 255 of them covering the node's extent.
+// Any node may be entered, so every rank gets a record (64 B read in order, at
+// most two more gathered from L2, 64 B written per node); opening by area
+// fills the slots better than taking the grandchildren (which leave a slot
+// empty beside every leaf) and visits fewer nodes.
+__device__ __forceinline__ float half_area(float4 mn, float4 mx) {
+    const float x = mx.x - mn.x, y = mx.y - mn.y, z = mx.z - mn.z;
+    return x * y + y * z + z * x;
 }
 
-__global__ void __launch_bounds__(256) cwide_kernel(const float4* __restrict__ wide, const uint8_t* __restrict__ depth_odd,
-                                                    uint32_t n_internal, uint4* __restrict__ cwide, uint32_t* err) {
-    const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= n_internal || depth_odd[i]) return;
-    float mn[4][3], mx[4][3];
+__device__ __forceinline__ void cwide_node(const float4* __restrict__ wide, uint32_t i, uint32_t n_internal,
+                                           float abs_eps, uint4* __restrict__ out, uint32_t* bad) {
+    float4 mn[4], mx[4];
     uint32_t ref[4];
-    int k = 0;
     const float4* w = wide + 4 * static_cast<size_t>(i);
-    const float4 w0 = w[0], w1 = w[1], w2 = w[2], w3 = w[3];
-    const float4 cmn[2] = {w0, w2}, cmx[2] = {w1, w3};
-    const uint32_t cref[2] = {__float_as_uint(w0.w), __float_as_uint(w1.w)};
-    auto put = [&](float4 a, float4 b, uint32_t r) {
-        mn[k][0] = a.x; mn[k][1] = a.y; mn[k][2] = a.z;
-        mx[k][0] = b.x; mx[k][1] = b.y; mx[k][2] = b.z;
-        ref[k++] = r;
-    };
+    const float4 w0 = __ldg(w), w1 = __ldg(w + 1), w2 = __ldg(w + 2), w3 = __ldg(w + 3);
+    mn[0] = w0; mx[0] = w1; ref[0] = __float_as_uint(w0.w);
+    mn[1] = w2; mx[1] = w3; ref[1] = __float_as_uint(w1.w);
+    const float inf = __int_as_float(0x7F800000);
 #pragma unroll
-    for (int c = 0; c < 2; ++c) {
-        if (cref[c] & kLeafRef) {
-            put(cmn[c], cmx[c], cref[c]);
-        } else {
-            const float4* g = wide + 4 * static_cast<size_t>(cref[c]);
-            const float4 g0 = g[0], g1 = g[1], g2 = g[2], g3 = g[3];
-            put(g0, g1, __float_as_uint(g0.w));
-            put(g2, g3, __float_as_uint(g1.w));
-        }
+    for (int c = 2; c < 4; ++c) {
+        mn[c] = make_float4(inf, inf, inf, 0.f);
+        mx[c] = make_float4(-inf, -inf, -inf, 0.f);
+        ref[c] = kNoChild;
     }
-    const int n = k;
-    float o[3];
-    uint32_t ex[3];
-    bool ok = true;
+#pragma unroll
+    for (int c = 2; c < 4; ++c) {  // slots 0 .. c-1 are taken
+        int best = -1;
+        float area = -1.f;
+#pragma unroll
+        for (int k = 0; k < c; ++k) {
+            const float a = half_area(mn[k], mx[k]);
+            if (!(ref[k] & kLeafRef) && a > area) { area = a; best = k; }
+        }
+        uint32_t open = kNoChild;
+#pragma unroll
+        for (int k = 0; k < c; ++k)
+            if (k == best) open = ref[k];
+        if (open >= n_internal) continue;  // no internal child (or a non-finite area)
+        const float4* g = wide + 4 * static_cast<size_t>(open);
+        const float4 g0 = __ldg(g), g1 = __ldg(g + 1), g2 = __ldg(g + 2), g3 = __ldg(g + 3);
+#pragma unroll
+        for (int k = 0; k < c; ++k)
+            if (k == best) { mn[k] = g0; mx[k] = g1; ref[k] = __float_as_uint(g0.w); }
+        mn[c] = g2; mx[c] = g3; ref[c] = __float_as_uint(g1.w);
+    }
+    bool ok = abs_eps >= 8.673617379884035e-19f && abs_eps <= 1073741824.f;  // a range of 2^-40 .. 2^50
+#pragma unroll
+    for (int c = 0; c < 4; ++c)  // the walk follows references unchecked
+        ok = ok && (ref[c] == kNoChild || ((ref[c] & kLeafRef) ? (ref[c] & ~kLeafRef) <= n_internal : ref[c] < n_internal));
+    const float grow = 4.f * abs_eps;
+    const float lo[3][4] = {{mn[0].x, mn[1].x, mn[2].x, mn[3].x}, {mn[0].y, mn[1].y, mn[2].y, mn[3].y},
+                            {mn[0].z, mn[1].z, mn[2].z, mn[3].z}};
+    const float hi[3][4] = {{mx[0].x, mx[1].x, mx[2].x, mx[3].x}, {mx[0].y, mx[1].y, mx[2].y, mx[3].y},
+                            {mx[0].z, mx[1].z, mx[2].z, mx[3].z}};
+    float org[3];
+    uint32_t ex = 0, q[6];
 #pragma unroll
     for (int a = 0; a < 3; ++a) {
-        float lo = mn[0][a], hi = mx[0][a];
-        for (int c = 1; c < n; ++c) {
-            lo = min_std(lo, mn[c][a]);
-            hi = max_std(hi, mx[c][a]);
-        }
-        ok = ok && isfinite(lo) && isfinite(hi) && lo <= hi;
-        o[a] = lo;
-        ex[a] = quant_step_exp(static_cast<double>(hi) - static_cast<double>(lo));
-        ok = ok && ex[a] <= 254u;
-    }
-    uint32_t q[6] = {0u, 0u, 0u, 0u, 0u, 0u};  // lo x, y, z, hi x, y, z; byte c = child c
-    if (ok) {
-        for (int c = 0; c < n; ++c)
+        // NaN coordinates must not be skipped by fminf: they fail the isfinite tests below
+        const float l = __fadd_rd(fminf(fminf(lo[a][0], lo[a][1]), fminf(lo[a][2], lo[a][3])), -grow);
+        const float h = __fadd_ru(fmaxf(fmaxf(hi[a][0], hi[a][1]), fmaxf(hi[a][2], hi[a][3])), grow);
+        ok = ok && isfinite(l) && isfinite(h);
+        // the least biased exponent whose power of two is >= extent / 255 (1/255 rounded up)
+        const float need = __fmul_ru(__fsub_ru(h, l), 0.00392156886f);
+        const uint32_t e = min(max((__float_as_uint(need) + 0x7FFFFFu) >> 23, 1u), 180u);
+        const float inv_step = __uint_as_float((254u - e) << 23);  // 2^(127 - e)
+        org[a] = l * 8.673617379884035e-19f;
+        ex |= (e + 73u) << (8 * a);
+        uint32_t ql = 0, qh = 0;
 #pragma unroll
-            for (int a = 0; a < 3; ++a) {
-                const double step = ldexp(1.0, static_cast<int>(ex[a]) - 127);
-                const float fstep = __uint_as_float(ex[a] << 23);
-                double dl = floor((static_cast<double>(mn[c][a]) - o[a]) / step);
-                double dh = ceil((static_cast<double>(mx[c][a]) - o[a]) / step);
-                int ql = dl < 0.0 ? 0 : (dl > 255.0 ? 255 : static_cast<int>(dl));
-                int qh = dh < 0.0 ? 0 : (dh > 255.0 ? 255 : static_cast<int>(dh));
-                // settle the counts against the decoder's own float arithmetic
-                while (ql > 0 && o[a] + static_cast<float>(ql) * fstep > mn[c][a]) --ql;
-                while (qh < 255 && o[a] + static_cast<float>(qh) * fstep < mx[c][a]) ++qh;
-                ok = ok && !(o[a] + static_cast<float>(ql) * fstep > mn[c][a]) &&
-                     !(o[a] + static_cast<float>(qh) * fstep < mx[c][a]);
-                q[a] |= static_cast<uint32_t>(ql) << (8 * c);
-                q[3 + a] |= static_cast<uint32_t>(qh) << (8 * c);
+        for (int c = 0; c < 4; ++c) {
+            uint32_t bl = 255u, bh = 0u;  // an empty slot: inverted planes
+            if (ref[c] != kNoChild) {
+                ok = ok && isfinite(lo[a][c]) && isfinite(hi[a][c]);
+                const float dl = __fsub_rd(__fadd_rd(lo[a][c], -grow), l), dh = __fsub_ru(__fadd_ru(hi[a][c], grow), l);
+                bl = static_cast<uint32_t>(fminf(fmaxf(floorf(dl * inv_step), 0.f), 255.f));
+                const float up = ceilf(dh * inv_step);
+                ok = ok && up >= 0.f && up <= 255.f;
+                bh = static_cast<uint32_t>(fminf(fmaxf(up, 0.f), 255.f));
             }
+            ql |= bl << (8 * c);
+            qh |= bh << (8 * c);
+        }
+        q[a] = ql;
+        q[3 + a] = qh;
     }
-    if (!ok) raise_corrupt(err, 16, i, 0u);
-    for (int c = n; c < 4; ++c) ref[c] = kNoChild;
-    uint4* out = cwide + 4 * static_cast<size_t>(i);
-    out[0] = make_uint4(__float_as_uint(o[0]), __float_as_uint(o[1]), __float_as_uint(o[2]),
-                        ex[0] | (ex[1] << 8) | (ex[2] << 16) | (static_cast<uint32_t>(n) << 24));
-    out[1] = make_uint4(q[0], q[1], q[2], q[3]);
-    out[2] = make_uint4(q[4], q[5], 0u, 0u);
-    out[3] = make_uint4(ref[0], ref[1], ref[2], ref[3]);
+    if (!ok) atomicOr(bad, 1u);
+    uint4* o = out + 4 * static_cast<size_t>(i);
+    o[0] = make_uint4(__float_as_uint(org[0]), __float_as_uint(org[1]), __float_as_uint(org[2]), ex);
+    o[1] = make_uint4(q[0], q[1], q[2], q[3]);
+    o[2] = make_uint4(q[4], q[5], 0u, 0u);
+    o[3] = make_uint4(ref[0], ref[1], ref[2], ref[3]);
 }
 
-void launch_cwide(const float4* wide, const uint8_t* depth_odd, uint32_t n_internal, uint4* cwide, uint32_t* err,
-                  cudaStream_t s) {
+__global__ void __launch_bounds__(256) cwide_kernel(const float4* __restrict__ wide, uint32_t n_internal, float abs_eps,
+                                                    uint4* __restrict__ cwide, uint32_t* bad) {
+    const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i < n_internal) cwide_node(wide, i, n_internal, abs_eps, cwide, bad);
+}
+
+__global__ void __launch_bounds__(256) cwide_batch_kernel(const float4* __restrict__ wide,
+                                                          const BatchScene* __restrict__ scenes, uint32_t n_scenes,
+                                                          uint32_t n_total, uint4* __restrict__ cwide, uint32_t* bad) {
+    const uint32_t j = blockIdx.x * blockDim.x + threadIdx.x;
+    if (j >= n_total) return;
+    uint32_t lo = 0, hi = n_scenes - 1;  // the last scene whose first triangle is <= j
+    while (lo < hi) {
+        const uint32_t mid = (lo + hi + 1) >> 1;
+        if (__ldg(&scenes[mid].tri_off) <= j) lo = mid; else hi = mid - 1;
+    }
+    const BatchScene sc = scenes[lo];
+    const uint32_t i = j - sc.tri_off;
+    if (i + 1 >= sc.n_tris) return;
+    const size_t base = 4 * static_cast<size_t>(sc.wide_off);
+    cwide_node(wide + base, i, sc.n_tris - 1, sc.abs_eps, cwide + base, bad);
+}
+
+void launch_cwide(const float4* wide, uint32_t n_internal, float abs_eps, uint4* cwide, uint32_t* bad, cudaStream_t s) {
+    cudaMemsetAsync(bad, 0, 4, s);
     if (n_internal == 0) return;
-    cwide_kernel<<<(n_internal + 255) / 256, 256, 0, s>>>(wide, depth_odd, n_internal, cwide, err);
+    cwide_kernel<<<(n_internal + 255) / 256, 256, 0, s>>>(wide, n_internal, abs_eps, cwide, bad);
+}
+
+void launch_cwide_batch(const float4* wide, const BatchScene* scenes, uint32_t n_scenes, uint32_t n_total, uint4* cwide,
+                        uint32_t* bad, cudaStream_t s) {
+    cudaMemsetAsync(bad, 0, 4, s);
+    cwide_batch_kernel<<<(n_total + 255) / 256, 256, 0, s>>>(wide, scenes, n_scenes, n_total, cwide, bad);
 }
 
 void launch_wide4(const float4* wide, const uint8_t* depth_odd, uint32_t n_internal, float4* wide4, cudaStream_t s) {

@@ -100,11 +100,10 @@ void launch_layout_emit(const float4* node_box, const uint4* node_kids, const ui
                         const uint32_t* dfs, crt_bvh_node* out, float4* wide, float4* wide_wt, uint8_t* depth_odd,
                         LeafOut leaves, const SceneState* st, uint32_t* err, cudaStream_t s);
 void launch_wide4(const float4* wide, const uint8_t* depth_odd, uint32_t n_internal, float4* wide4, cudaStream_t s);
-// 64-byte compressed 4-wide nodes (CRT_TRACE_COMPRESSED) from the binary
-// traversal nodes; raises kDevCorrupt where a box cannot be quantized
-// (non-finite coordinates).
-void launch_cwide(const float4* wide, const uint8_t* depth_odd, uint32_t n_internal, uint4* cwide, uint32_t* err,
-                  cudaStream_t s);
+// 64-byte compressed 4-wide nodes (crt_walk4.cuh) from the binary traversal
+// nodes, one per binary node; *bad (zeroed here) is set where a box cannot be
+// quantised (non-finite coordinates, a scene range outside 2^-40 .. 2^50).
+void launch_cwide(const float4* wide, uint32_t n_internal, float abs_eps, uint4* cwide, uint32_t* bad, cudaStream_t s);
 void launch_single_leaf(const float4* node_box, crt_bvh_node* out, LeafOut leaves, cudaStream_t s);
 // All PLOC iterations and the DFS layout in one cooperative launch; returns
 // cudaErrorNotSupported when a cooperative launch is unavailable.
@@ -144,6 +143,7 @@ struct TraceParams {
                              // traces: boxes already grown by abs_eps)
     const float4* wide4;     // 128-B 4-wide traversal nodes (even-depth internal nodes)
     const uint4* cwide = nullptr;  // 64-B compressed 4-wide traversal nodes (same indices)
+    const uint32_t* cw_bad = nullptr;  // nonzero: some box of cwide could not be quantised (walk the binary nodes)
     const float4* xtri;      // 3 float4 per leaf (tree order): transformed p0 | tri id, p1 | model id, p2
     const crt_ray* rays;
     crt_hit* hits;
@@ -162,10 +162,12 @@ struct TraceParams {
     const uint32_t* order = nullptr;
 };
 void launch_trace(const TraceParams& p, uint32_t flags, int block, cudaStream_t s);
-// Closest hit of many rays by persistent warps that refill finished lanes from
-// a ray counter (next_ray: one device word, reset here); binary nodes, no
-// seeding, rays in caller order or p.order.
-void launch_trace_pool(const TraceParams& p, uint32_t flags, uint32_t* next_ray, cudaStream_t s);
+// Many rays by persistent warps that refill finished lanes from a ray counter;
+// compressed nodes, no seeding, rays in caller order or p.order.  pool:
+// trace_pool_bytes(n_rays) of device memory (counters, reset here, and the list
+// of rays left to the binary walk).
+size_t trace_pool_bytes(uint32_t n_rays);
+void launch_trace_pool(const TraceParams& p, uint32_t flags, uint32_t* pool, cudaStream_t s);
 
 // Shading (getColor + imageStore) inputs; the BVH, leaf records and error
 // word come from the TraceParams it runs with.
@@ -211,10 +213,13 @@ struct BatchScene {
 static_assert(sizeof(BatchScene) == 48, "batch scene record");
 void launch_trace_batch(const TraceParams& p, const BatchScene* scenes, uint32_t n_scenes, uint32_t n_rays,
                         uint32_t flags, int block, bool deep, cudaStream_t s);
-// The persistent ray pool over a batch: closest hit, no seeding; p holds the
-// batch's node arrays and p.n_rays the batch's ray count.
+// The same nodes for every scene of a batch of n_total triangles.
+void launch_cwide_batch(const float4* wide, const struct BatchScene* scenes, uint32_t n_scenes, uint32_t n_total,
+                        uint4* cwide, uint32_t* bad, cudaStream_t s);
+// The persistent ray pool over a batch: no seeding; p holds the batch's node
+// arrays and p.n_rays the batch's ray count.
 void launch_trace_batch_pool(const TraceParams& p, const BatchScene* scenes, uint32_t n_scenes, uint32_t flags,
-                             bool deep, uint32_t* next_ray, cudaStream_t s);
+                             bool deep, uint32_t* pool, cudaStream_t s);
 // CRT_TRACE_SORT_RAYS: order[k] = k-th ray by coherence key (origin cell,
 // direction; with scenes, scene first).  scratch: ray_order_scratch_bytes(n).
 size_t ray_order_scratch_bytes(uint32_t n);

@@ -1,0 +1,535 @@
+// The 64-byte compressed 4-wide nodes and the persistent closest-hit / any-hit
+// walk over them (crt_trace.cu).  Compiled with -fmad=false.
+//
+// Record of binary internal node i (any node can be entered, so the array is
+// indexed by the binary rank): its subtree's top opened twice, the internal
+// child of largest area first, so up to four children.
+//   words 0-2   origin (minimum corner over the children) * 2^-60
+//   word  3     per axis the biased exponent of step * 2^73, one byte each
+//   words 4-9   8-bit steps of the children's planes: min x, y, z, max x, y, z;
+//               byte c of a word belongs to child c
+//   words 12-15 child references (leaf flag | place in tree order, or rank;
+//               kNoChild in an empty slot, whose planes are inverted)
+// The planes origin + q * step enclose, as real numbers, the child's box grown
+// by 4 * abs_eps (crt_build.cu rounds every step outward).
+//
+// Decoding.  A float whose bits are q << 16 is exactly q * 2^-133 (denormal up
+// to q = 127, the first normals above, same spacing), so one byte permute and
+// one fused multiply-add give a slab distance with a single rounding: with
+// R = 2^-40 / d, A = step * 2^73 * R and B = origin * 2^-60 * R - o * 2^-60 * R,
+// fma(q * 2^-133, A, B) is the distance times 2^-100.  All distances the walk
+// compares (entry distances, the pruning bound) carry that factor.
+//
+// Exactness.  B and the product round once each, as slab_wt's form does; with
+// origins within 8 times the scene's range the error stays below
+// 26 * 2^-24 of that range, and the shader's own slab form adds at most
+// 18 * 2^-24, both inside the 4 * abs_eps = 2^-18 the boxes are grown by.
+// So every box the binary walk enters is entered here, and
+//   * the watertight predicate needs no more (its hits do not depend on boxes);
+//   * the shader's predicate tests a leaf only if its exact box passes the
+//     shader's slab test (leaf_box_passes), which is the shader's tested set.
+// Rays outside that range (far origins, zero or extreme 1/d, negative tmin),
+// scenes whose boxes cannot be quantised and walks that outgrow their stack
+// take the binary walk (trace_one), one call per ray.
+#pragma once
+
+#include <cstdint>
+#include <cuda_runtime.h>
+
+#include "crt_build.cuh"
+#include "crt_common.cuh"
+#include "crt_traverse.cuh"
+
+namespace crt {
+
+struct Walk4Node {
+    float ox, oy, oz;
+    uint32_t ex;
+    uint32_t nx, ny, nz, xx, xy, xz;
+    uint32_t ref[4];
+};
+
+__device__ __forceinline__ Walk4Node load_walk4(const uint4* __restrict__ node) {
+    uint32_t w[16];
+    asm("ld.global.nc.v8.b32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];"
+        : "=r"(w[0]), "=r"(w[1]), "=r"(w[2]), "=r"(w[3]), "=r"(w[4]), "=r"(w[5]), "=r"(w[6]), "=r"(w[7])
+        : "l"(node));
+    asm("ld.global.nc.v8.b32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];"
+        : "=r"(w[8]), "=r"(w[9]), "=r"(w[10]), "=r"(w[11]), "=r"(w[12]), "=r"(w[13]), "=r"(w[14]), "=r"(w[15])
+        : "l"(node + 2));
+    Walk4Node n;
+    n.ox = __uint_as_float(w[0]);
+    n.oy = __uint_as_float(w[1]);
+    n.oz = __uint_as_float(w[2]);
+    n.ex = w[3];
+    n.nx = w[4]; n.ny = w[5]; n.nz = w[6];
+    n.xx = w[7]; n.xy = w[8]; n.xz = w[9];
+#pragma unroll
+    for (int c = 0; c < 4; ++c) n.ref[c] = w[12 + c];
+    return n;
+}
+
+constexpr float kWalk4TScale = 7.888609052210118e-31f;  // 2^-100: slab distances
+constexpr float kWalk4RScale = 9.094947017729282e-13f;  // 2^-40: 1/d
+constexpr float kWalk4OScale = 8.673617379884035e-19f;  // 2^-60: origins
+
+// A ray's constants: R = 2^-40 / d per axis and -(o * 2^-60) * R.
+struct Walk4Ray {
+    float rx, ry, rz;
+    float bx, by, bz;
+};
+
+// False: this ray takes the binary walk.  reach = 8 * range of the scene.
+__device__ __forceinline__ bool walk4_setup(Walk4Ray& w, float3 o, float3 d, float tmin, float abs_eps) {
+    const float range = abs_eps * 1048576.f;  // largest coordinate or extent (scene_abs_eps)
+    const float ix = 1.0f / d.x, iy = 1.0f / d.y, iz = 1.0f / d.z;
+    const float far = fmaxf(fabsf(o.x), fmaxf(fabsf(o.y), fabsf(o.z)));
+    const float big = fmaxf(fabsf(ix), fmaxf(fabsf(iy), fabsf(iz))) * range;
+    const float small = fminf(fabsf(ix), fminf(fabsf(iy), fabsf(iz))) * range;
+    w.rx = ix * kWalk4RScale;
+    w.ry = iy * kWalk4RScale;
+    w.rz = iz * kWalk4RScale;
+    w.bx = -((o.x * kWalk4OScale) * w.rx);
+    w.by = -((o.y * kWalk4OScale) * w.ry);
+    w.bz = -((o.z * kWalk4OScale) * w.rz);
+    // NaNs fail every comparison; the products are 2^-20 .. 2^60 in the distance unit
+    return tmin >= 0.f && far <= 8.f * range && big <= 1.152921504606846976e18f && small >= 9.5367431640625e-07f &&
+           isfinite(o.x) && isfinite(o.y) && isfinite(o.z) && !isnan(d.x) && !isnan(d.y) && !isnan(d.z);
+}
+
+template <int C>
+__device__ __forceinline__ float walk4_plane(uint32_t word, float a, float b) {
+    // byte C of word to bits 16-23, zeros elsewhere
+    const float q = __uint_as_float(__byte_perm(word, 0u, 0x4044u | (static_cast<uint32_t>(C) << 8)));
+    return __fmaf_rn(q, a, b);
+}
+
+// Entry distance (clamped to 0) of child C if the ray meets its box no farther
+// than bound, else +inf.
+template <int C>
+__device__ __forceinline__ float walk4_child(const uint32_t (&near)[3], const uint32_t (&far)[3], const float (&a)[3],
+                                             const float (&b)[3], float bound) {
+    const float t0 = fmaxf(fmaxf(walk4_plane<C>(near[0], a[0], b[0]), walk4_plane<C>(near[1], a[1], b[1])),
+                           fmaxf(walk4_plane<C>(near[2], a[2], b[2]), 0.f));
+    const float t1 = fminf(fminf(walk4_plane<C>(far[0], a[0], b[0]), walk4_plane<C>(far[1], a[1], b[1])),
+                           fminf(walk4_plane<C>(far[2], a[2], b[2]), bound));
+    return t0 <= t1 ? t0 : __int_as_float(0x7F800000);
+}
+
+__device__ __forceinline__ void walk4_children(const Walk4Node& n, const Walk4Ray& w, float bound, float (&t)[4]) {
+    const float a[3] = {__uint_as_float((n.ex & 0xFFu) << 23) * w.rx, __uint_as_float((n.ex << 15) & 0x7F800000u) * w.ry,
+                        __uint_as_float((n.ex << 7) & 0x7F800000u) * w.rz};
+    const float b[3] = {__fmaf_rn(n.ox, w.rx, w.bx), __fmaf_rn(n.oy, w.ry, w.by), __fmaf_rn(n.oz, w.rz, w.bz)};
+    const bool sx = w.rx < 0.f, sy = w.ry < 0.f, sz = w.rz < 0.f;
+    const uint32_t near[3] = {sx ? n.xx : n.nx, sy ? n.xy : n.ny, sz ? n.xz : n.nz};
+    const uint32_t far[3] = {sx ? n.nx : n.xx, sy ? n.ny : n.xy, sz ? n.nz : n.xz};
+    t[0] = walk4_child<0>(near, far, a, b, bound);
+    t[1] = walk4_child<1>(near, far, a, b, bound);
+    t[2] = walk4_child<2>(near, far, a, b, bound);
+    t[3] = walk4_child<3>(near, far, a, b, bound);
+}
+
+// Orders the four (distance, reference) pairs, nearest first (FARTHEST: the
+// farthest met child first); missed children (+inf) go last either way.
+template <bool FARTHEST>
+__device__ __forceinline__ void walk4_sort(float (&t)[4], uint32_t (&r)[4]) {
+    const float inf = __int_as_float(0x7F800000);
+    if (FARTHEST)
+#pragma unroll
+        for (int c = 0; c < 4; ++c) t[c] = t[c] == inf ? inf : -t[c];
+#define CRT_CSWAP(x, y)                                   \
+    {                                                     \
+        const bool s = t[y] < t[x];                       \
+        const float tx = t[x], ty = t[y];                 \
+        const uint32_t rx = r[x], ry = r[y];              \
+        t[x] = s ? ty : tx; t[y] = s ? tx : ty;           \
+        r[x] = s ? ry : rx; r[y] = s ? rx : ry;           \
+    }
+    CRT_CSWAP(0, 1) CRT_CSWAP(2, 3) CRT_CSWAP(0, 2) CRT_CSWAP(1, 3) CRT_CSWAP(1, 2)
+#undef CRT_CSWAP
+}
+
+// The shader's predicate tests a leaf only if its exact box (that of its
+// stored triangle) passes the shader's slab test.
+__device__ __forceinline__ bool leaf_box_passes(const RayCtx& r, float4 a, float4 b, float4 c, float bound) {
+    const float4 mn = make_float4(min_std(a.x, min_std(b.x, c.x)), min_std(a.y, min_std(b.y, c.y)),
+                                  min_std(a.z, min_std(b.z, c.z)), 0.f);
+    const float4 mx = make_float4(max_std(a.x, max_std(b.x, c.x)), max_std(a.y, max_std(b.y, c.y)),
+                                  max_std(a.z, max_std(b.z, c.z)), 0.f);
+    float te;
+    return slab<false>(r, mn, mx, 0.f, te) && te <= bound;
+}
+
+// The binary walk of one ray (see the head of this file).
+template <bool ANY, bool WT, int STACK>
+__device__ __noinline__ uint4 trace_binary(const TraceParams& p, uint32_t i, float4 r0, float4 r1) {
+    return trace_one<ANY, WT, STACK, false, 0>(p, i, r0, r1);
+}
+
+// Launch shape (GB300; 8.4 M bounce rays over 4.19 M triangles in caller order /
+// 64 uneven scenes built and traced): entries in shared memory 14 / 20 / 22:
+// 8.17 / 6.67 / 6.53 ms (28 drop a resident block: 10.8); blocked lanes that
+// start the leaf tests 3 / 4 / 6 / 12: 6.67 / 6.67 / 6.78 / 7.56; idle lanes
+// that refill 4 / 6 / 8 / 12: 6.68 / 6.63 / 6.67 / 7.43 (batch 6.79 / 6.64 /
+// 6.60 / 7.25); two or three pops per step instead of one: 7.05 / 7.49; 56
+// registers for 9 blocks per SM with 18 entries: 6.54 (batch 6.73).
+constexpr int kWalk4Shared = 22, kWalk4Local = 64, kWalk4Flush = 4, kWalk4Refill = 6, kWalk4Blocks = 8;
+constexpr int kWalk4Block = 128;
+
+// The scene whose ray range holds ray i.
+__device__ __forceinline__ uint32_t batch_scene_of(const uint32_t* ray_off, uint32_t n_scenes, uint32_t i) {
+    uint32_t lo = 0, hi = n_scenes - 1;
+    while (lo < hi) {
+        const uint32_t mid = (lo + hi + 1) >> 1;
+        if (ray_off[mid] <= i) lo = mid; else hi = mid - 1;
+    }
+    return lo;
+}
+
+__device__ __forceinline__ uint2 walk4_lds(uint32_t a) {
+    uint2 e;
+    asm volatile("ld.shared.v2.u32 {%0, %1}, [%2];" : "=r"(e.x), "=r"(e.y) : "r"(a));
+    return e;
+}
+__device__ __forceinline__ void walk4_sts(uint32_t a, uint2 e) {
+    asm volatile("st.shared.v2.u32 [%0], {%1, %2};" ::"r"(a), "r"(e.x), "r"(e.y) : "memory");
+}
+
+// Persistent warps over a ray pool, one ray per lane.  In a step each lane
+// without a node (cur < 0) pops one stack entry: an internal node
+// becomes cur, the first leaf is parked, a second leaf stays on the stack and
+// blocks the lane; then each lane with a node visits it.  The warp tests its
+// parked leaves together once kWalk4Flush lanes are blocked (or hold one
+// with nothing else left), or no lane has a node.  Lanes whose ray is done take new
+// rays from the counter once kWalk4Refill of them wait.
+//
+// What bounds it (ncu, 1 M rays): the ALU pipe (68 % busy: byte permutes,
+// minima, selects; issue slots 65 %), about 21 of 32 lanes visiting in a step.
+// The walk over the binary nodes with persistent warps it replaces was bound by
+// L1 wavefronts (65-70 % busy, one per lane and 16-byte load, four per visit)
+// at 12.7 active threads per instruction: 8.4 M bounce rays over 4.19 M
+// triangles 12.7 -> 6.5 ms in caller order (660 -> 1290 Mrays/s), 12.2 -> 7.1
+// in predicted order with its inference and sort; 1.5 M sorted rays over 0.3 M
+// triangles 1.60 -> 1.04 ms.  Any hit, one thread per ray before: 4.2 M rays
+// 6.70 -> 2.69 ms.  Deriving the nodes takes 75 us at 4.19 M triangles, less
+// than the 65,536 rays of the smallest launch gain (0.53 -> 0.43 ms with it,
+// 0.36 without).
+//
+// The stack's newest entries sit in shared memory (a column per thread, so any
+// mix of depths is free of bank conflicts), older ones move to local memory
+// eight at a time.  An entry is (reference, entry distance); its low two
+// distance bits count the siblings pushed just below it, which are farther, so
+// one too-far entry drops them all.
+//
+// Rays the compressed walk cannot take (walk4_setup, unquantised scenes, one-leaf
+// trees, walks deeper than the stack) go to the list left[0 .. pool[1]) for
+// walk4_left_kernel, launched right after; pool[0] counts the rays taken.
+template <bool ANY, bool WT, bool BATCH>
+__global__ void __launch_bounds__(kWalk4Block, kWalk4Blocks)
+    trace_walk4_kernel(const TraceParams p, uint32_t* __restrict__ pool, uint32_t* __restrict__ left,
+                       const BatchScene* __restrict__ scenes, uint32_t n_scenes) {
+    constexpr uint32_t SH = kWalk4Shared, LOC = kWalk4Local, kRow = kWalk4Block * 8, kSpill = 8;
+    static_assert(SH >= kSpill + 4 && LOC % kSpill == 0, "stack shape");
+    constexpr uint32_t kIdle = 0xFFFFFFFFu, kDone = 0xFFFFFFFEu, kNoLeaf = 0xFFFFFFFFu;
+    __shared__ uint2 s_st[SH + 1][kWalk4Block];  // row 0 is read (and ignored) below an empty stack
+    __shared__ uint32_t s_ray_off[BATCH ? kMaxBatchScenes + 1 : 1];
+    if (BATCH) {
+        for (uint32_t k = threadIdx.x; k <= n_scenes; k += kWalk4Block)
+            s_ray_off[k] = k < n_scenes ? scenes[k].ray_off : scenes[n_scenes - 1].ray_off + scenes[n_scenes - 1].n_rays;
+        __syncthreads();
+    }
+    const uint32_t lane = threadIdx.x & 31u;
+    const uint32_t s_base = static_cast<uint32_t>(__cvta_generic_to_shared(&s_st[1][threadIdx.x]));
+    const bool quantised = __ldg(p.cw_bad) == 0u;
+    uint2 st[LOC];
+    // the scene of the lane's ray
+    const uint4* cw = p.cwide;
+    const float4* xtri = p.xtri;
+    float abs_eps = p.abs_eps;
+    uint32_t n_leaves = (p.n_nodes + 1) / 2;
+    // the lane's ray
+    Walk4Ray w;
+    WRay wt{};
+    float3 o, d;
+    float tmin = 0.f, bt = 0.f, bu = 0.f, bv = 0.f, bound = 0.f;  // bt: tmax until a hit is found
+    float pend_t = 0.f;                                            // entry distance of the parked leaf
+    uint32_t btri = CRT_MISS, bleaf = 0, pend = kNoLeaf, i = kIdle;  // bleaf: the shader's tie order
+    int cur = -1;
+    uint32_t top = s_base, spilled = 0;  // next free shared entry; entries moved to local memory
+
+    auto set_bound = [&]() { bound = prune_bound(bt, abs_eps) * kWalk4TScale; };
+    auto stop = [&]() {  // nothing left of this walk
+        cur = -1;
+        top = s_base;
+        spilled = 0;
+        pend = kNoLeaf;
+    };
+    auto leave = [&]() {
+        left[atomicAdd(pool + 1, 1u)] = i;
+        i = kIdle;
+        stop();
+    };
+    auto test_leaf = [&](uint32_t leaf) {
+        if (leaf == kNoChild) return;  // an empty slot whose planes collapsed in rounding
+        const uint32_t L = leaf & ~kLeafRef;
+        const float4* t = xtri + 3 * static_cast<size_t>(L);
+        const float4 a = __ldg(t), b = __ldg(t + 1), c = __ldg(t + 2);
+        if (!WT) {
+            RayCtx r;
+            r.o = o;
+            r.d = d;
+            r.inv = make_float3(1.0f / d.x, 1.0f / d.y, 1.0f / d.z);
+            r.exact = false;  // walk4_setup admits only rays with finite, nonzero 1/d
+            if (!leaf_box_passes(r, a, b, c, prune_bound(bt, abs_eps))) return;
+        }
+        const float3 A = make_float3(a.x, a.y, a.z), B = make_float3(b.x, b.y, b.z), C = make_float3(c.x, c.y, c.z);
+        // accepted only up to the best hit (bt <= tmax)
+        const HitRes h = WT ? tri_watertight(o, tmin, bt, wt, A, B, C) : tri_reference(o, d, tmin, bt, A, B, C);
+        if (!h.did) return;
+        const uint32_t tri = __float_as_uint(a.w);
+        if (btri == CRT_MISS || h.t < bt || (h.t == bt && (WT ? tri < btri : L > bleaf))) {
+            bt = h.t; bu = h.u; bv = h.v; btri = tri;
+            if (!WT) bleaf = L;
+            set_bound();
+        }
+    };
+
+    bool pool_left = true;
+    while (true) {
+        const uint32_t need = __ballot_sync(0xFFFFFFFFu, i == kIdle);
+        if (need && pool_left) {
+            const uint32_t take = static_cast<uint32_t>(__popc(need));
+            const int leader = __ffs(need) - 1;
+            uint32_t base = 0;
+            if (lane == static_cast<uint32_t>(leader)) base = atomicAdd(pool, take);
+            base = __shfl_sync(0xFFFFFFFFu, base, leader);
+            pool_left = base < p.n_rays && p.n_rays - base > take;
+            const uint32_t k = base + static_cast<uint32_t>(__popc(need & ((1u << lane) - 1u)));
+            if (i == kIdle && k < p.n_rays && k >= base) {
+                i = p.order ? __ldg(p.order + k) : k;
+                if (i >= p.n_rays) {
+                    raise_corrupt(p.err, 7, k, i);
+                    i = kIdle;
+                } else {
+                    if (BATCH) {
+                        const BatchScene bs = scenes[batch_scene_of(s_ray_off, n_scenes, i)];
+                        cw = p.cwide + 4 * static_cast<size_t>(bs.wide_off);
+                        xtri = p.xtri + 3 * static_cast<size_t>(bs.tri_off);
+                        abs_eps = bs.abs_eps;
+                        n_leaves = bs.n_tris;
+                    }
+                    const float4 r0 = __ldg(reinterpret_cast<const float4*>(p.rays + i));
+                    const float4 r1 = __ldg(reinterpret_cast<const float4*>(p.rays + i) + 1);
+                    o = make_float3(r0.x, r0.y, r0.z);
+                    d = make_float3(r1.x, r1.y, r1.z);
+                    tmin = r0.w;
+                    bt = r1.w;
+                    bu = bv = 0.f;
+                    btri = CRT_MISS;
+                    cur = 0;  // the root: its children are tested, not its own box
+                    set_bound();
+                    if (WT) wt = wt_setup(d);
+                    if (!(tmin <= bt)) stop();
+                    else if (!walk4_setup(w, o, d, tmin, abs_eps) || !quantised || n_leaves < 2) leave();
+                }
+            }
+        }
+        if (i == kIdle && !pool_left) i = kDone;
+        if (__all_sync(0xFFFFFFFFu, i == kDone)) break;
+#pragma unroll 1
+        while (true) {
+            bool blocked = false, over = false;
+            if (cur < 0) {
+                if (spilled) {  // rare: older entries come back
+                    if (top == s_base) {
+                        const uint32_t n = min(spilled, kSpill);
+                        spilled -= n;
+                        for (uint32_t k = 0; k < n; ++k, top += kRow) walk4_sts(top, st[spilled + k]);
+                    }
+                }
+                const uint2 e = walk4_lds(top - kRow);
+                const bool some = top != s_base, full = pend != kNoLeaf;
+                const bool near = (ANY ? fabsf(__uint_as_float(e.y)) : __uint_as_float(e.y)) <= bound;
+                const bool leaf = static_cast<int>(e.x) < 0;
+                blocked = full && (!some || (near && leaf));
+                over = !some && !full;
+                if (some && near && !leaf) cur = static_cast<int>(e.x);
+                if (some && near && leaf && !full) {
+                    pend = e.x;
+                    pend_t = __uint_as_float(e.y);
+                }
+                uint32_t drop = near ? kRow : kRow + kRow * (e.y & 3u);
+                if (!some || blocked) drop = 0u;
+                if (spilled) {  // rare: some of the siblings were moved
+                    const uint32_t have = top - s_base;
+                    if (have < drop) {
+                        spilled -= (drop - have) / kRow;
+                        drop = have;
+                    }
+                }
+                top -= drop;
+            }
+            const uint32_t wm = __ballot_sync(0xFFFFFFFFu, cur >= 0);
+            const uint32_t bm = __ballot_sync(0xFFFFFFFFu, blocked);
+            if (__popc(bm) >= kWalk4Flush || !wm) {
+                if (pend != kNoLeaf) {
+                    if ((ANY ? fabsf(pend_t) : pend_t) <= bound) test_leaf(pend);
+                    pend = kNoLeaf;
+                    if (ANY && btri != CRT_MISS) {
+                        stop();
+                        over = true;
+                    }
+                }
+            }
+            const uint32_t om = __ballot_sync(0xFFFFFFFFu, over);
+            if (om == 0xFFFFFFFFu || (pool_left && __popc(om) >= kWalk4Refill)) break;
+            if (cur >= 0) {
+                Walk4Node n = load_walk4(cw + 4 * static_cast<size_t>(static_cast<uint32_t>(cur)));
+                if (top > s_base + (SH - 4) * kRow) {  // rare: the oldest entries move to local memory
+                    if (spilled + kSpill > LOC) {  // the walk outgrows the stack: start over on the binary nodes
+                        leave();
+                        continue;
+                    }
+                    for (uint32_t k = 0; k < kSpill; ++k) st[spilled + k] = walk4_lds(s_base + k * kRow);
+                    for (uint32_t q = s_base; q + kSpill * kRow < top; q += kRow)
+                        walk4_sts(q, walk4_lds(q + kSpill * kRow));
+                    top -= kSpill * kRow;
+                    spilled += kSpill;
+                }
+                float t[4];
+                walk4_children(n, w, bound, t);
+                walk4_sort<ANY>(t, n.ref);
+                const float inf = __int_as_float(0x7F800000);
+                uint32_t below = 0;
+                // each entry is stored where the next one goes unless it counts: four rows are free above top
+#pragma unroll
+                for (int c = 3; c >= 1; --c) {
+                    walk4_sts(top, make_uint2(n.ref[c], (__float_as_uint(t[c]) & ~3u) | below));
+                    if (t[c] < inf) {
+                        top += kRow;
+                        ++below;
+                    }
+                }
+                // the nearest child is entered; a leaf goes through the stack
+                walk4_sts(top, make_uint2(n.ref[0], (__float_as_uint(t[0]) & ~3u) | below));
+                const bool met = t[0] < inf;
+                cur = met ? static_cast<int>(n.ref[0]) : -1;
+                if (met && cur < 0) top += kRow;
+            }
+        }
+        // over: the walk has ended with no leaf parked
+        if (i < kDone && cur < 0 && top == s_base && !spilled && pend == kNoLeaf) {
+            reinterpret_cast<uint4*>(p.hits)[i] =
+                btri != CRT_MISS ? make_uint4(btri, __float_as_uint(bt), __float_as_uint(bu), __float_as_uint(bv))
+                                 : make_uint4(CRT_MISS, 0u, 0u, 0u);
+            i = kIdle;
+        }
+    }
+}
+
+// The binary walk of the rays a trace_walk4_kernel launch left over (few or none).
+template <bool ANY, bool WT, int STACK, bool BATCH>
+__global__ void __launch_bounds__(kWalk4Block)
+    walk4_left_kernel(const TraceParams p, const uint32_t* __restrict__ pool, const uint32_t* __restrict__ left,
+                      const BatchScene* __restrict__ scenes, uint32_t n_scenes) {
+    const uint32_t n = min(pool[1], p.n_rays);
+    for (uint32_t k = blockIdx.x * kWalk4Block + threadIdx.x; k < n; k += gridDim.x * kWalk4Block) {
+        const uint32_t i = left[k];
+        if (i >= p.n_rays) { raise_corrupt(p.err, 7, k, i); continue; }
+        TraceParams q = p;
+        if (BATCH) {
+            uint32_t lo = 0, hi = n_scenes - 1;
+            while (lo < hi) {
+                const uint32_t mid = (lo + hi + 1) >> 1;
+                if (__ldg(&scenes[mid].ray_off) <= i) lo = mid; else hi = mid - 1;
+            }
+            const BatchScene bs = scenes[lo];
+            q.nodes = p.nodes + bs.node_off;
+            q.wide = p.wide + 4 * static_cast<size_t>(bs.wide_off);
+            q.xtri = p.xtri + 3 * static_cast<size_t>(bs.tri_off);
+            q.abs_eps = bs.abs_eps;
+            q.n_nodes = 2 * bs.n_tris - 1;
+        }
+        trace_ray<ANY, WT, STACK, false, 0>(q, i);
+    }
+}
+
+// One thread's whole walk over the compressed nodes (leaves tested as they are
+// met), with the binary walk where walk4_setup or the stack asks for it.
+template <bool ANY, bool WT, int STACK>
+__device__ __forceinline__ uint4 trace_walk4_one(const TraceParams& p, const uint32_t i, const float4 r0,
+                                                 const float4 r1) {
+    const float3 o = make_float3(r0.x, r0.y, r0.z), d = make_float3(r1.x, r1.y, r1.z);
+    const float tmin = r0.w, tmax = r1.w;
+    if (!(tmin <= tmax)) return make_uint4(CRT_MISS, 0u, 0u, 0u);
+    const uint32_t n_leaves = (p.n_nodes + 1) / 2;
+    Walk4Ray w;
+    if (!walk4_setup(w, o, d, tmin, p.abs_eps) || n_leaves < 2 || __ldg(p.cw_bad) != 0u)
+        return trace_binary<ANY, WT, STACK>(p, i, r0, r1);
+    WRay wt{};
+    if (WT) wt = wt_setup(d);
+    float bt = tmax, bu = 0.f, bv = 0.f, bound = prune_bound(bt, p.abs_eps) * kWalk4TScale;
+    uint32_t bkey = 0xFFFFFFFFu, btri = CRT_MISS, cur = 0, fetched = 0, tested = 0;
+    bool corrupt = false;
+    constexpr int kCap = 64;
+    uint2 st[kCap];
+    int sp = 0;
+    auto test_leaf = [&](uint32_t leaf) {
+        const uint32_t L = leaf & ~kLeafRef;
+        if (L >= n_leaves) { corrupt = true; return; }
+        const float4* t = p.xtri + 3 * static_cast<size_t>(L);
+        const float4 a = __ldg(t), b = __ldg(t + 1), c = __ldg(t + 2);
+        if (!WT) {
+            RayCtx r;
+            r.o = o;
+            r.d = d;
+            r.inv = make_float3(1.0f / d.x, 1.0f / d.y, 1.0f / d.z);
+            r.exact = false;
+            if (!leaf_box_passes(r, a, b, c, prune_bound(bt, p.abs_eps))) return;
+        }
+        ++tested;
+        const float3 A = make_float3(a.x, a.y, a.z), B = make_float3(b.x, b.y, b.z), C = make_float3(c.x, c.y, c.z);
+        const HitRes h = WT ? tri_watertight(o, tmin, tmax, wt, A, B, C) : tri_reference(o, d, tmin, tmax, A, B, C);
+        if (!h.did) return;
+        const uint32_t tri = __float_as_uint(a.w);
+        const uint32_t key = WT ? tri : ~L;
+        if (btri == CRT_MISS || h.t < bt || (h.t == bt && key < bkey)) {
+            bt = h.t; bu = h.u; bv = h.v; bkey = key; btri = tri;
+            bound = prune_bound(bt, p.abs_eps) * kWalk4TScale;
+        }
+    };
+    const float inf = __int_as_float(0x7F800000);
+    while (true) {
+        if (cur & kLeafRef) {
+            if (cur != kNoChild) test_leaf(cur);
+            if (ANY && btri != CRT_MISS) break;
+        } else {
+            if (cur >= n_leaves - 1) { corrupt = true; break; }
+            if (sp + 3 > kCap) return trace_binary<ANY, WT, STACK>(p, i, r0, r1);
+            ++fetched;
+            Walk4Node n = load_walk4(p.cwide + 4 * static_cast<size_t>(cur));
+            float t[4];
+            walk4_children(n, w, bound, t);
+            walk4_sort<ANY>(t, n.ref);
+#pragma unroll
+            for (int c = 3; c >= 1; --c)
+                if (t[c] < inf) st[sp++] = make_uint2(n.ref[c], __float_as_uint(t[c]));
+            if (t[0] < inf) { cur = n.ref[0]; continue; }
+        }
+        bool more = false;
+        while (sp > 0) {
+            const uint2 e = st[--sp];
+            if (fabsf(__uint_as_float(e.y)) <= bound) { cur = e.x; more = true; break; }
+        }
+        if (!more) break;
+    }
+    if (corrupt) raise_corrupt(p.err, 5, i, 0u);
+    if (p.stats) {
+        atomicAdd(p.stats + 0, static_cast<unsigned long long>(fetched));
+        atomicAdd(p.stats + 1, static_cast<unsigned long long>(tested));
+    }
+    return btri != CRT_MISS ? make_uint4(btri, __float_as_uint(bt), __float_as_uint(bu), __float_as_uint(bv))
+                            : make_uint4(CRT_MISS, 0u, 0u, 0u);
+}
+
+}  // namespace crt
