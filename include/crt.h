@@ -128,11 +128,12 @@ typedef struct crt_camera {
 #define CRT_TRACE_SORT_RAYS   0x40u /* trace the rays ordered by origin cell and direction (same hits) */
 #define CRT_TRACE_COMPRESSED  0x80u /* walk 64-byte compressed 4-wide nodes: 8-bit child boxes rounded
                                        outward, exact leaf boxes re-checked (same hits); the reference
-                                       layout stays the export format */
-#define CRT_TRACE_PER_RAY_THREADS 0x100u /* closest-hit crt_trace of >= 65,536 rays normally runs on
-                                       persistent warps whose lanes take a new ray as soon as theirs
-                                       is done; this flag keeps one thread per ray for its whole walk
-                                       instead (same hits) */
+                                       layout stays the export format.  Traces of >= 65,536 rays and
+                                       frames take them without the flag */
+#define CRT_TRACE_PER_RAY_THREADS 0x100u /* crt_trace of >= 65,536 rays normally runs on persistent warps
+                                       over the compressed nodes whose lanes take a new ray as soon as
+                                       theirs is done; this flag keeps one thread per ray for its whole
+                                       walk of the binary nodes instead (same hits) */
 
 typedef struct crt_config {
     int device;                 /* CUDA device ordinal, default 0 */
@@ -315,9 +316,11 @@ crt_status crt_shadow_rays(crt_ctx* ctx, const crt_ray* primary, const crt_hit* 
 /* ---- trace: replaces getClosestHitBVH (raytracer.glsl:246-295) ---------- */
 crt_status crt_trace(crt_ctx* ctx, const crt_bvh* bvh, const crt_ray* rays, uint32_t n_rays,
                      uint32_t flags, crt_hit* hits);
-/* Counters of the last crt_trace issued with CRT_TRACE_STATS:
+/* Counters of the last crt_trace (or frame) issued with CRT_TRACE_STATS:
  * out[0] = traversal nodes fetched (64-byte binary, or 128-byte 4-wide with
- * CRT_TRACE_WIDE), out[1] = triangles tested. */
+ * CRT_TRACE_WIDE, or 64-byte compressed 4-wide with CRT_TRACE_COMPRESSED and
+ * in one-launch frames), out[1] = triangles tested.  crt_trace counts with one
+ * thread per ray, whatever the batch's size. */
 crt_status crt_last_trace_stats(crt_ctx* ctx, uint64_t out[2]);
 /* Device time of the last traversal issued through crt_trace,
  * crt_trace_seeded or the multi-launch frame paths, from CUDA events on the

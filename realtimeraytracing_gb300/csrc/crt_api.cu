@@ -135,6 +135,7 @@ struct crt_bvh {
     mutable bool wide4_ready = false;
     mutable bool cwide_ready = false;  // the compressed 4-wide nodes, derived likewise
     uint32_t* cw_bad() const { return reinterpret_cast<uint32_t*>(cwide.as<char>() + 64ull * n); }
+    mutable uint64_t frame_pixels = 0;  // pixels of the frames of the current tree
     // Refit topology of the last build (crt_refit, derived on its first call).
     DevBuf refit_link, refit_leaf, refit_dfs, refit_cnt;
     bool refit_ready = false;
@@ -196,7 +197,6 @@ struct crt_ctx {
     DevBuf mesh_vertices, mesh_indices, mesh_out;  // crt_triangles_from_indexed staging
     DevBuf probe_flag;                             // crt_selftest_wait
     DevBuf step_in, step_out;                      // crt_radix_digit_counts / _offsets
-    DevBuf pool;                                   // persistent traversal: its counters and left-over rays
     DevBuf opt_scratch;                            // crt_optimize
     uint64_t last_trace_stats[2] = {0, 0};
     // pinned host staging
@@ -327,7 +327,7 @@ crt_status crt_destroy(crt_ctx* x) {
                       &x->ray_order, &x->ray_order_scratch, &x->shade_models, &x->shade_materials,
                       &x->shade_rays, &x->shade_hits, &x->image, &x->refit_state, &x->xtri_sorted,
                       &x->mesh_vertices, &x->mesh_indices, &x->mesh_out, &x->probe_flag, &x->step_in,
-                      &x->step_out, &x->pool};
+                      &x->step_out};
     for (DevBuf* b : bufs) b->release();
     for (auto& e : x->ev)
         if (e) cudaEventDestroy(e);
@@ -515,8 +515,10 @@ crt_status build_impl(crt_ctx* x, crt_bvh* b, const crt_triangle* tris, uint32_t
     CRT_TRY(b->wide_wt.reserve(64ull * N));
     b->wide4_ready = false;
     b->cwide_ready = false;
+    b->frame_pixels = 0;
     b->refit_ready = false;
     b->node_boxes_stale = false;
+    CRT_TRY(b->cwide.reserve(64ull * N + 16));  // derived by the first trace that walks them, which then allocates nothing
     CRT_TRY(b->depth_odd.reserve(N));
     CRT_TRY(b->inv_perm.reserve(4ull * N));
     CRT_TRY(b->codes.reserve(4ull * N));
@@ -723,6 +725,19 @@ crt_status ensure_cwide(crt_ctx* x, const crt_bvh* b) {
     return CRT_OK;
 }
 
+// One-launch frames walk the compressed nodes once the frames of the current
+// tree have a quarter as many pixels as it has triangles: deriving the nodes
+// takes 0.035 ns per triangle (73 us at 2.0 M) and a pixel gains 0.05-0.2 ns.
+crt_status frame_walk4(crt_ctx* x, const crt_bvh* b, uint32_t pixels, crt::TraceParams* p) {
+    b->frame_pixels += pixels;
+    if (b->n < 2 || (!b->cwide_ready && 4 * b->frame_pixels < b->n)) return CRT_OK;
+    CRT_TRY(ensure_cwide(x, b));
+    CRT_TRY(x->node_box.reserve(crt::trace_pool_bytes(pixels)));  // build scratch, idle between builds
+    p->cwide = b->cwide.as<uint4>();
+    p->cw_bad = b->cw_bad();
+    return CRT_OK;
+}
+
 // Enqueues one traversal launch on device-resident rays/hits (no sync).
 constexpr uint32_t kPoolMinRays = 65536;  // below this a launch of one thread per ray fills the GPU as well
                                           // (measured sides at the kernel, crt_walk4.cuh)
@@ -810,9 +825,9 @@ crt_status trace_device(crt_ctx* x, const crt_bvh* b, const crt_ray* d_rays, uin
     const bool deep = (b->depth_bound + 2 > 64) || (3 * ((b->depth_bound + 2) / 2) + 3 > 96);
     const uint32_t launch_flags =
         (flags & (CRT_TRACE_ANY | CRT_TRI_WATERTIGHT | CRT_TRACE_WIDE | CRT_TRACE_COMPRESSED)) | (deep ? (1u << 16) : 0u);
-    if (pool) CRT_TRY(x->pool.reserve(crt::trace_pool_bytes(n_rays)));
+    if (pool) CRT_TRY(x->node_box.reserve(crt::trace_pool_bytes(n_rays)));  // build scratch, idle between builds
     CRT_CUDA(cudaEventRecord(x->tev[1], x->stream));
-    if (pool) crt::launch_trace_pool(p, launch_flags, x->pool.as<uint32_t>(), x->stream);
+    if (pool) crt::launch_trace_pool(p, launch_flags, x->node_box.as<uint32_t>(), x->stream);
     else crt::launch_trace(p, launch_flags, static_cast<int>(x->cfg.trace_block), x->stream);
     CRT_CUDA(cudaGetLastError());
     CRT_CUDA(cudaEventRecord(x->tev[2], x->stream));
@@ -899,6 +914,7 @@ crt_status crt_refit(crt_ctx* x, crt_bvh* b, const crt_triangle* tris, uint32_t 
                              cudaMemcpyDeviceToHost, s));
     b->wide4_ready = false;
     b->cwide_ready = false;
+    b->frame_pixels = 0;
     b->node_boxes_stale = N > 1;
     const crt_status st = x->check_device_error();
     if (st != CRT_OK) {
@@ -1040,7 +1056,7 @@ crt_status crt_bvh_from_nodes(crt_ctx* x, const crt_bvh_node* nodes, uint32_t n_
     crt_status st = CRT_OK;
     if ((st = b->nodes.reserve(sizeof(crt_bvh_node) * n_nodes)) != CRT_OK || (st = b->xtri.reserve(48ull * N)) != CRT_OK ||
         (st = b->wide.reserve(64ull * n_int_alloc)) != CRT_OK || (st = b->wide_wt.reserve(64ull * n_int_alloc)) != CRT_OK ||
-        (st = b->depth_odd.reserve(n_int_alloc)) != CRT_OK || (st = b->inv_perm.reserve(4ull * N)) != CRT_OK)
+        (st = b->cwide.reserve(64ull * N + 16)) != CRT_OK || (st = b->depth_odd.reserve(n_int_alloc)) != CRT_OK || (st = b->inv_perm.reserve(4ull * N)) != CRT_OK)
         return fail_free(st);
     // staging: idx (n_nodes) | int_pos (N-1) | leaf counts (N-1, uint2) | leaf_pos (N), each part
     // starting on a 256-byte boundary (the uint2 loads need 8-byte alignment)
@@ -1161,6 +1177,7 @@ crt_status crt_optimize(crt_ctx* x, crt_bvh* b, uint32_t passes) {
     CRT_CUDA(cudaGetLastError());
     b->wide4_ready = false;
     b->cwide_ready = false;
+    b->frame_pixels = 0;
     b->refit_ready = false;
     b->node_boxes_stale = false;
     b->depth_bound = H;
@@ -1472,6 +1489,7 @@ crt_status crt_trace_frame(crt_ctx* x, const crt_bvh* b, const crt_camera* cam, 
         p.abs_eps = b->abs_eps;
         p.err = x->err.as<uint32_t>();
         p.tile_width = tw;
+        CRT_TRY(frame_walk4(x, b, n, &p));
         if (flags & CRT_TRACE_STATS) {
             CRT_CUDA(cudaMemsetAsync(x->trace_stats.p, 0, 16, x->stream));
             p.stats = x->trace_stats.as<unsigned long long>();
@@ -1482,7 +1500,7 @@ crt_status crt_trace_frame(crt_ctx* x, const crt_bvh* b, const crt_camera* cam, 
         // hits are copied out on a second stream while the next band runs was
         // measured slower at every band count (2, 4, 8) on GB300.
         crt::launch_frame(p, d_cam, width, height, 0, height, light, d_hs, kflags, static_cast<int>(x->cfg.trace_block),
-                          nullptr, x->stream);
+                          nullptr, x->node_box.as<uint32_t>(), x->stream);
         CRT_CUDA(cudaGetLastError());
         if (!dev_p)
             CRT_CUDA(cudaMemcpyAsync(hits_primary, d_hp, sizeof(crt_hit) * static_cast<size_t>(n), cudaMemcpyDeviceToHost,
@@ -2530,6 +2548,7 @@ crt_status crt_render_frame(crt_ctx* x, const crt_bvh* b, const crt_camera* cam,
         crt::TraceParams p = bvh_params(x, b, flags);
         p.n_rays = n;
         p.tile_width = tw;
+        CRT_TRY(frame_walk4(x, b, n, &p));
         if (flags & CRT_TRACE_STATS) {
             CRT_CUDA(cudaMemsetAsync(x->trace_stats.p, 0, 16, x->stream));
             p.stats = x->trace_stats.as<unsigned long long>();
@@ -2537,7 +2556,7 @@ crt_status crt_render_frame(crt_ctx* x, const crt_bvh* b, const crt_camera* cam,
         const bool deep = b->depth_bound + 2 > 64;
         const uint32_t kflags = (flags & CRT_TRI_WATERTIGHT) | (deep ? (1u << 16) : 0u);
         crt::launch_frame(p, d_cam, width, height, 0, height, nullptr, nullptr, kflags,
-                          static_cast<int>(x->cfg.trace_block), &sp, x->stream);
+                          static_cast<int>(x->cfg.trace_block), &sp, x->node_box.as<uint32_t>(), x->stream);
         CRT_CUDA(cudaGetLastError());
     } else {
         CRT_TRY(x->frame_rays.reserve(sizeof(crt_ray) * static_cast<size_t>(n)));

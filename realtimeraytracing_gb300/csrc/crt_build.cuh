@@ -189,10 +189,11 @@ void launch_shade(const TraceParams& p, const ShadeParams& sp, cudaStream_t s);
 // Camera rays of image rows [y0, y0 + rows) traced to the closest hit into
 // p.hits (may be null with shading) and, with a light, their shadow rays to
 // any hit into hits_shadow, and with shade, their texels into shade->image,
-// in one launch (p.tile_width: width for 8x4 pixel tiles, or 0).
+// in one launch (p.tile_width: width for 8x4 pixel tiles, or 0).  With p.cwide
+// over the compressed nodes, with pool (trace_pool_bytes of the image's pixels).
 void launch_frame(const TraceParams& p, const crt_camera* cam, uint32_t width, uint32_t height, uint32_t y0,
                   uint32_t rows, const float* light, crt_hit* hits_shadow, uint32_t flags, int block,
-                  const ShadeParams* shade, cudaStream_t s);
+                  const ShadeParams* shade, uint32_t* pool, cudaStream_t s);
 
 // Batched scenes: per-scene offsets into the concatenated arrays.
 constexpr uint32_t kMaxBatchScenes = 256;

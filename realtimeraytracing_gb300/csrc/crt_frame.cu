@@ -14,6 +14,7 @@
 #include "crt_build.cuh"
 #include "crt_common.cuh"
 #include "crt_traverse.cuh"
+#include "crt_walk4.cuh"
 
 namespace crt {
 
@@ -130,74 +131,186 @@ void launch_shade(const TraceParams& p, const ShadeParams& sp, cudaStream_t s) {
 }
 
 // ------------------------------------------------------------- frames
-// One frame in one launch (crt_trace_frame, crt_render_frame): thread t
-// takes pixel ray_of_thread(t) of the image rows [y0, y0 + rows), generates
-// its camera ray, traces it to the closest hit and, with a light, traces
-// that hit's shadow ray to any hit at once, while the nodes around the hit
-// are still cached; with SHADE it also writes the pixel's texel.  The rays,
-// hits and texels are the ones the separate raygen, trace, shadow-ray and
-// shade calls produce.
-template <bool WT, int STACK, int BLOCK, bool SHADE>
-__global__ void __launch_bounds__(BLOCK) frame_kernel(TraceParams p, const crt_camera* __restrict__ cam, uint32_t width,
-                                                      uint32_t height, uint32_t y0, uint32_t rows, int shadows,
-                                                      float lx, float ly, float lz, crt_hit* __restrict__ hits_shadow,
-                                                      ShadeParams sp) {
-    const uint32_t t_id = blockIdx.x * BLOCK + threadIdx.x;
-    if (t_id >= width * rows) return;
-    const uint32_t i = y0 * width + ray_of_thread(t_id, p.tile_width);
-    const uint32_t y = i / width, x = i - y * width;
+// One frame in one launch (crt_trace_frame, crt_render_frame): a thread
+// generates pixel i's camera ray, traces it to the closest hit and, with a
+// light, traces that hit's shadow ray to any hit at once, while the nodes
+// around the hit are still cached; with SHADE it also writes the pixel's
+// texel.  The rays, hits and texels are the ones the separate raygen, trace,
+// shadow-ray and shade calls produce.
+struct FrameParams {
+    const crt_camera* cam;
+    uint32_t width, height, y0, rows;
+    int shadows;
+    float lx, ly, lz;
+    crt_hit* hits_shadow;
+};
+
+// Pixel i over the binary nodes.
+template <bool WT, int STACK, bool SHADE>
+__device__ __forceinline__ void frame_pixel(const TraceParams& p, const FrameParams& f, const ShadeParams& sp, uint32_t i) {
+    const uint32_t y = i / f.width, x = i - y * f.width;
     float4 r0, r1;
-    camera_ray(cam, x, y, width, height, r0, r1);
+    camera_ray(f.cam, x, y, f.width, f.height, r0, r1);
     const uint4 h = trace_one<false, WT, STACK, false, 0>(p, i, r0, r1);
     if (!SHADE || p.hits) reinterpret_cast<uint4*>(p.hits)[i] = h;
     if (SHADE) sp.image[i] = shade_texel(p, sp, h, r0, r1);
-    if (!shadows) return;
+    if (!f.shadows) return;
     uint4 hs = make_uint4(CRT_MISS, 0u, 0u, 0u);
     if (h.x != CRT_MISS) {
         float4 s0, s1;
-        shadow_ray(r0, r1, h, lx, ly, lz, s0, s1);
+        shadow_ray(r0, r1, h, f.lx, f.ly, f.lz, s0, s1);
         hs = trace_one<true, WT, STACK, false, 0>(p, i, s0, s1);
     }
-    reinterpret_cast<uint4*>(hits_shadow)[i] = hs;
+    reinterpret_cast<uint4*>(f.hits_shadow)[i] = hs;
+}
+
+// Thread t takes pixel ray_of_thread(t) of the image rows [y0, y0 + rows).
+template <bool WT, int STACK, int BLOCK, bool SHADE>
+__global__ void __launch_bounds__(BLOCK) frame_kernel(TraceParams p, FrameParams f, ShadeParams sp) {
+    const uint32_t t_id = blockIdx.x * BLOCK + threadIdx.x;
+    if (t_id >= f.width * f.rows) return;
+    frame_pixel<WT, STACK, SHADE>(p, f, sp, f.y0 * f.width + ray_of_thread(t_id, p.tile_width));
+}
+
+// The same over the compressed nodes: a warp takes a tile of 32 pixels (warp w
+// tile w, then tiles from the counter pool[0] while there are any), walks its
+// camera rays together, then their shadow rays, testing a leaf as soon as a
+// lane holds one (coherent lanes reach theirs together; waiting for two: 3 %
+// slower).  Pixels with a ray of the binary walk go to left[0 .. pool[1]) for
+// frame_left_kernel.
+//
+// Bound by the ALU pipe (65-71 % busy, 18-22 of 32 threads per instruction) and
+// by the rays of the longest walks at the end (an SM is busy 82-86 % of the
+// launch).  Against one thread per pixel over the binary nodes (41 %, 10-15
+// threads): 160x120 over 2,003 triangles 36 -> 25 us, 512x512 over 65,536 (the
+// shader's predicate) 244 -> 180 us, 1920x1080 with shadow rays over 1.31 M 831 ->
+// 720 us, 1280x720 over 2.0 M clustered 540 -> 372 us.  One thread per pixel over
+// these nodes, its stack in local memory, was slower than either (65,536: 414 us
+// a call against 282).
+template <bool WT, bool SHADE, bool COUNT>
+__global__ void __launch_bounds__(kWalk4Block, kWalk4Blocks)
+    frame_walk4_kernel(const TraceParams p, const FrameParams f, const ShadeParams sp, uint32_t* __restrict__ pool,
+                       uint32_t* __restrict__ left) {
+    __shared__ uint2 s_st[kWalk4Shared + 1][kWalk4Block];
+    const uint32_t lane = threadIdx.x & 31u;
+    const uint32_t s_base = static_cast<uint32_t>(__cvta_generic_to_shared(&s_st[1][threadIdx.x]));
+    const uint32_t n = f.width * f.rows, tiles = (n + 31u) / 32u, warps = gridDim.x * (kWalk4Block / 32);
+    const bool walkable = __ldg(p.cw_bad) == 0u && p.n_nodes > 2;
+    uint2 st[kWalk4Local];
+    Walk4Lane L{};
+    L.cw = p.cwide;
+    L.xtri = p.xtri;
+    L.abs_eps = p.abs_eps;
+    uint32_t tile = blockIdx.x * (kWalk4Block / 32) + (threadIdx.x >> 5);
+    while (tile < tiles) {
+        const uint32_t t = 32u * tile + lane;
+        const bool valid = t < n;
+        const uint32_t i = f.y0 * f.width + ray_of_thread(valid ? t : 0u, p.tile_width);
+        const uint32_t y = i / f.width, x = i - y * f.width;
+        float4 r0, r1;
+        camera_ray(f.cam, x, y, f.width, f.height, r0, r1);
+        bool redo = !L.template start<WT>(s_base, r0, r1, walkable);
+        if (!valid) L.stop(s_base);
+        walk4_run<false, WT, 1, COUNT>(L, s_base, st, 32);
+        redo = redo || L.redo;
+        const uint4 h = redo ? make_uint4(CRT_MISS, 0u, 0u, 0u) : L.hit();
+        // the ray again: what the walk keeps of it
+        r0 = make_float4(L.o.x, L.o.y, L.o.z, 0.f);
+        r1 = make_float4(L.d.x, L.d.y, L.d.z, __int_as_float(0x7F800000));
+        if (valid && !redo) {
+            if (!SHADE || p.hits) reinterpret_cast<uint4*>(p.hits)[i] = h;
+            if (SHADE) sp.image[i] = shade_texel(p, sp, h, r0, r1);
+        }
+        if (f.shadows) {
+            float4 s0, s1;
+            shadow_ray(r0, r1, h, f.lx, f.ly, f.lz, s0, s1);  // empty where the primary ray missed
+            redo = !L.template start<WT>(s_base, s0, s1, walkable) || redo;
+            if (!valid) L.stop(s_base);
+            walk4_run<true, WT, 1, COUNT>(L, s_base, st, 32);
+            redo = redo || L.redo;
+            if (valid && !redo) reinterpret_cast<uint4*>(f.hits_shadow)[i] = L.hit();
+        }
+        if (valid && redo) left[atomicAdd(pool + 1, 1u)] = i;
+        uint32_t next = tiles;
+        if (tiles > warps) {
+            if (lane == 0) next = warps + atomicAdd(pool, 1u);
+            next = __shfl_sync(0xFFFFFFFFu, next, 0);
+        }
+        tile = next;
+    }
+    if (COUNT && p.stats) {
+        atomicAdd(p.stats + 0, static_cast<unsigned long long>(L.fetched));
+        atomicAdd(p.stats + 1, static_cast<unsigned long long>(L.tested));
+    }
+}
+
+template <bool WT, int STACK, bool SHADE>
+__global__ void __launch_bounds__(kWalk4Block)
+    frame_left_kernel(TraceParams p, FrameParams f, ShadeParams sp, const uint32_t* __restrict__ pool,
+                      const uint32_t* __restrict__ left) {
+    const uint32_t n = min(pool[1], p.n_rays);
+    for (uint32_t k = blockIdx.x * kWalk4Block + threadIdx.x; k < n; k += gridDim.x * kWalk4Block) {
+        const uint32_t i = left[k];
+        if (i >= p.n_rays) raise_corrupt(p.err, 7, k, i);
+        else frame_pixel<WT, STACK, SHADE>(p, f, sp, i);
+    }
+}
+
+template <bool WT, bool SHADE>
+static void launch_frame_walk4(const TraceParams& p, const FrameParams& f, const ShadeParams& sp, bool deep,
+                               uint32_t* pool, cudaStream_t s) {
+    static int grid = 0;
+    if (grid == 0) {
+        int per_sm = 0;
+        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, frame_walk4_kernel<WT, SHADE, false>, kWalk4Block, 0);
+        grid = kNumSms * (per_sm > 0 ? per_sm : 1);
+    }
+    const uint32_t want = (f.width * f.rows + kWalk4Block - 1) / kWalk4Block;
+    const uint32_t blocks = want < static_cast<uint32_t>(grid) ? want : static_cast<uint32_t>(grid);
+    uint32_t* left = pool + 4;
+    cudaMemsetAsync(pool, 0, 8, s);
+    if (p.stats) frame_walk4_kernel<WT, SHADE, true><<<blocks, kWalk4Block, 0, s>>>(p, f, sp, pool, left);
+    else frame_walk4_kernel<WT, SHADE, false><<<blocks, kWalk4Block, 0, s>>>(p, f, sp, pool, left);
+    const uint32_t few = want < static_cast<uint32_t>(kNumSms) ? want : static_cast<uint32_t>(kNumSms);
+    if (deep) frame_left_kernel<WT, 1024, SHADE><<<few, kWalk4Block, 0, s>>>(p, f, sp, pool, left);
+    else frame_left_kernel<WT, 64, SHADE><<<few, kWalk4Block, 0, s>>>(p, f, sp, pool, left);
 }
 
 template <bool WT, int BLOCK, bool SHADE>
 static void launch_frame_s(const TraceParams& p, const crt_camera* cam, uint32_t width, uint32_t height, uint32_t y0,
                            uint32_t rows, const float* light, crt_hit* hits_shadow, bool deep, const ShadeParams& sp,
-                           cudaStream_t s) {
+                           uint32_t* pool, cudaStream_t s) {
     const uint32_t grid = (width * rows + BLOCK - 1) / BLOCK;
     if (grid == 0) return;
     const int sh = light != nullptr;
-    const float lx = sh ? light[0] : 0.f, ly = sh ? light[1] : 0.f, lz = sh ? light[2] : 0.f;
-    if (deep)
-        frame_kernel<WT, 1024, BLOCK, SHADE>
-            <<<grid, BLOCK, 0, s>>>(p, cam, width, height, y0, rows, sh, lx, ly, lz, hits_shadow, sp);
-    else
-        frame_kernel<WT, 64, BLOCK, SHADE>
-            <<<grid, BLOCK, 0, s>>>(p, cam, width, height, y0, rows, sh, lx, ly, lz, hits_shadow, sp);
+    const FrameParams f{cam, width, height, y0, rows, sh, sh ? light[0] : 0.f, sh ? light[1] : 0.f, sh ? light[2] : 0.f,
+                        hits_shadow};
+    if (p.cwide) launch_frame_walk4<WT, SHADE>(p, f, sp, deep, pool, s);
+    else if (deep) frame_kernel<WT, 1024, BLOCK, SHADE><<<grid, BLOCK, 0, s>>>(p, f, sp);
+    else frame_kernel<WT, 64, BLOCK, SHADE><<<grid, BLOCK, 0, s>>>(p, f, sp);
 }
 
 template <bool WT, int BLOCK>
 static void launch_frame_b(const TraceParams& p, const crt_camera* cam, uint32_t width, uint32_t height, uint32_t y0,
                            uint32_t rows, const float* light, crt_hit* hits_shadow, bool deep, const ShadeParams* shade,
-                           cudaStream_t s) {
-    if (shade) launch_frame_s<WT, BLOCK, true>(p, cam, width, height, y0, rows, light, hits_shadow, deep, *shade, s);
-    else launch_frame_s<WT, BLOCK, false>(p, cam, width, height, y0, rows, light, hits_shadow, deep, ShadeParams{}, s);
+                           uint32_t* pool, cudaStream_t s) {
+    if (shade) launch_frame_s<WT, BLOCK, true>(p, cam, width, height, y0, rows, light, hits_shadow, deep, *shade, pool, s);
+    else launch_frame_s<WT, BLOCK, false>(p, cam, width, height, y0, rows, light, hits_shadow, deep, ShadeParams{}, pool, s);
 }
 
 void launch_frame(const TraceParams& p, const crt_camera* cam, uint32_t width, uint32_t height, uint32_t y0,
                   uint32_t rows, const float* light, crt_hit* hits_shadow, uint32_t flags, int block,
-                  const ShadeParams* shade, cudaStream_t s) {
+                  const ShadeParams* shade, uint32_t* pool, cudaStream_t s) {
     const bool wt = flags & CRT_TRI_WATERTIGHT;
     const bool deep = (flags >> 16) != 0;
     if (wt) {
-        if (block == 256) launch_frame_b<true, 256>(p, cam, width, height, y0, rows, light, hits_shadow, deep, shade, s);
-        else if (block == 64) launch_frame_b<true, 64>(p, cam, width, height, y0, rows, light, hits_shadow, deep, shade, s);
-        else launch_frame_b<true, 128>(p, cam, width, height, y0, rows, light, hits_shadow, deep, shade, s);
+        if (block == 256) launch_frame_b<true, 256>(p, cam, width, height, y0, rows, light, hits_shadow, deep, shade, pool, s);
+        else if (block == 64) launch_frame_b<true, 64>(p, cam, width, height, y0, rows, light, hits_shadow, deep, shade, pool, s);
+        else launch_frame_b<true, 128>(p, cam, width, height, y0, rows, light, hits_shadow, deep, shade, pool, s);
     } else {
-        if (block == 256) launch_frame_b<false, 256>(p, cam, width, height, y0, rows, light, hits_shadow, deep, shade, s);
-        else if (block == 64) launch_frame_b<false, 64>(p, cam, width, height, y0, rows, light, hits_shadow, deep, shade, s);
-        else launch_frame_b<false, 128>(p, cam, width, height, y0, rows, light, hits_shadow, deep, shade, s);
+        if (block == 256) launch_frame_b<false, 256>(p, cam, width, height, y0, rows, light, hits_shadow, deep, shade, pool, s);
+        else if (block == 64) launch_frame_b<false, 64>(p, cam, width, height, y0, rows, light, hits_shadow, deep, shade, pool, s);
+        else launch_frame_b<false, 128>(p, cam, width, height, y0, rows, light, hits_shadow, deep, shade, pool, s);
     }
 }
 

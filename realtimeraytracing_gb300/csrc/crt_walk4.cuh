@@ -28,9 +28,14 @@
 //   * the watertight predicate needs no more (its hits do not depend on boxes);
 //   * the shader's predicate tests a leaf only if its exact box passes the
 //     shader's slab test (leaf_box_passes), which is the shader's tested set.
-// Rays outside that range (far origins, zero or extreme 1/d, negative tmin),
-// scenes whose boxes cannot be quantised and walks that outgrow their stack
-// take the binary walk (trace_one), one call per ray.
+// A ray parallel to an axis plane (1/d infinite) meets the shader's NaNs where a
+// box plane passes through its origin.  They reject a box of which every box
+// inside is rejected too, but for leaves flat in the ray's own plane, whose
+// triangles the shader's predicate rejects (a = 0): the tested leaves that can
+// hit are still those whose own box passes.
+// Rays outside that range (far origins, extreme scales, negative tmin), scenes
+// whose boxes cannot be quantised and walks that outgrow their stack take the
+// binary walk (trace_one), one call per ray.
 #pragma once
 
 #include <cstdint>
@@ -79,21 +84,23 @@ struct Walk4Ray {
     float bx, by, bz;
 };
 
-// False: this ray takes the binary walk.  reach = 8 * range of the scene.
+// False: this ray takes the binary walk.  Components below 2^-40 of the largest
+// count as that much: over the scene (t * |d| <= 10 ranges) it moves the ray by
+// 10 * 2^-40 of the range, far inside the boxes' growth.
 __device__ __forceinline__ bool walk4_setup(Walk4Ray& w, float3 o, float3 d, float tmin, float abs_eps) {
     const float range = abs_eps * 1048576.f;  // largest coordinate or extent (scene_abs_eps)
-    const float ix = 1.0f / d.x, iy = 1.0f / d.y, iz = 1.0f / d.z;
     const float far = fmaxf(fabsf(o.x), fmaxf(fabsf(o.y), fabsf(o.z)));
-    const float big = fmaxf(fabsf(ix), fmaxf(fabsf(iy), fabsf(iz))) * range;
-    const float small = fminf(fabsf(ix), fminf(fabsf(iy), fabsf(iz))) * range;
-    w.rx = ix * kWalk4RScale;
-    w.ry = iy * kWalk4RScale;
-    w.rz = iz * kWalk4RScale;
+    const float big = fmaxf(fabsf(d.x), fmaxf(fabsf(d.y), fabsf(d.z)));
+    const float least = big * 9.094947017729282e-13f;
+    w.rx = kWalk4RScale / copysignf(fmaxf(fabsf(d.x), least), d.x);
+    w.ry = kWalk4RScale / copysignf(fmaxf(fabsf(d.y), least), d.y);
+    w.rz = kWalk4RScale / copysignf(fmaxf(fabsf(d.z), least), d.z);
     w.bx = -((o.x * kWalk4OScale) * w.rx);
     w.by = -((o.y * kWalk4OScale) * w.ry);
     w.bz = -((o.z * kWalk4OScale) * w.rz);
-    // NaNs fail every comparison; the products are 2^-20 .. 2^60 in the distance unit
-    return tmin >= 0.f && far <= 8.f * range && big <= 1.152921504606846976e18f && small >= 9.5367431640625e-07f &&
+    // NaNs fail the comparisons or the tests after them; range / big, the distance
+    // unit, lies in 2^-20 .. 2^20, so every product above and below is normal
+    return tmin >= 0.f && far <= 8.f * range && big <= range * 1048576.f && range <= big * 1048576.f &&
            isfinite(o.x) && isfinite(o.y) && isfinite(o.z) && !isnan(d.x) && !isnan(d.y) && !isnan(d.z);
 }
 
@@ -166,15 +173,18 @@ __device__ __noinline__ uint4 trace_binary(const TraceParams& p, uint32_t i, flo
     return trace_one<ANY, WT, STACK, false, 0>(p, i, r0, r1);
 }
 
-// Launch shape (GB300; 8.4 M bounce rays over 4.19 M triangles in caller order /
-// 64 uneven scenes built and traced): entries in shared memory 14 / 20 / 22:
-// 8.17 / 6.67 / 6.53 ms (28 drop a resident block: 10.8); blocked lanes that
-// start the leaf tests 3 / 4 / 6 / 12: 6.67 / 6.67 / 6.78 / 7.56; idle lanes
-// that refill 4 / 6 / 8 / 12: 6.68 / 6.63 / 6.67 / 7.43 (batch 6.79 / 6.64 /
-// 6.60 / 7.25); two or three pops per step instead of one: 7.05 / 7.49; 56
-// registers for 9 blocks per SM with 18 entries: 6.54 (batch 6.73).
+// Stack entries in shared memory per thread, entries beyond them in local
+// memory, blocked lanes that start the warp's leaf tests, idle lanes that
+// refill, resident blocks per SM.  GB300, 8.4 M bounce rays over 4.19 M triangles
+// in caller order (64 uneven scenes built and traced): 14 / 20 / 22 entries 8.17 /
+// 6.67 / 6.53 ms (28 drop a resident block: 10.8); leaf tests at 3 / 4 / 6 / 12
+// lanes 6.67 / 6.67 / 6.78 / 7.56; refill at 4 / 6 / 8 / 12 idle lanes 6.68 / 6.63
+// / 6.67 / 7.43 (6.79 / 6.64 / 6.60 / 7.25); two or three pops per step instead
+// of one 7.05 / 7.49; 56 registers for 9 blocks per SM with 18 entries 6.54 (6.73).
 constexpr int kWalk4Shared = 22, kWalk4Local = 64, kWalk4Flush = 4, kWalk4Refill = 6, kWalk4Blocks = 8;
 constexpr int kWalk4Block = 128;
+constexpr uint32_t kWalk4Row = kWalk4Block * 8, kWalk4Spill = 8;
+static_assert(kWalk4Shared >= kWalk4Spill + 4 && kWalk4Local % kWalk4Spill == 0, "stack shape");
 
 // The scene whose ray range holds ray i.
 __device__ __forceinline__ uint32_t batch_scene_of(const uint32_t* ray_off, uint32_t n_scenes, uint32_t i) {
@@ -195,13 +205,186 @@ __device__ __forceinline__ void walk4_sts(uint32_t a, uint2 e) {
     asm volatile("st.shared.v2.u32 [%0], {%1, %2};" ::"r"(a), "r"(e.x), "r"(e.y) : "memory");
 }
 
-// Persistent warps over a ray pool, one ray per lane.  In a step each lane
-// without a node (cur < 0) pops one stack entry: an internal node
-// becomes cur, the first leaf is parked, a second leaf stays on the stack and
-// blocks the lane; then each lane with a node visits it.  The warp tests its
-// parked leaves together once kWalk4Flush lanes are blocked (or hold one
-// with nothing else left), or no lane has a node.  Lanes whose ray is done take new
-// rays from the counter once kWalk4Refill of them wait.
+// One lane's walk.  cur: the internal node to visit next, or -1 (pop one); pend:
+// a parked leaf.  The stack's newest entries sit in shared memory (a column per
+// thread, so any mix of depths is free of bank conflicts), older ones move to
+// local memory eight at a time.  An entry is (reference, entry distance); its low
+// two distance bits count the siblings pushed just below it, which are farther,
+// so one too-far entry drops them all.
+struct Walk4Lane {
+    static constexpr uint32_t kNoLeaf = 0xFFFFFFFFu;
+    const uint4* cw;      // the scene: nodes, leaf triangles, slack
+    const float4* xtri;
+    float abs_eps;
+    Walk4Ray w;           // the ray
+    WRay wt;
+    float3 o, d;
+    float tmin;
+    float bt, bu, bv, bound;  // best hit (bt: tmax until there is one), pruning bound
+    uint32_t btri, bleaf;     // bleaf: the shader's tie order
+    int cur;
+    uint32_t pend, top, spilled;
+    float pend_t;
+    bool redo;                // the walk outgrew its stack: to be done on the binary nodes
+    uint32_t fetched, tested; // nodes and triangles (walk4_run with COUNT)
+
+    __device__ __forceinline__ void stop(uint32_t s_base) {
+        cur = -1;
+        top = s_base;
+        spilled = 0;
+        pend = kNoLeaf;
+    }
+    __device__ __forceinline__ void set_bound() { bound = prune_bound(bt, abs_eps) * kWalk4TScale; }
+    // Starts ray (r0, r1) at the root (whose children are tested, not its own
+    // box); false for a ray of the binary walk, which is then stopped.
+    template <bool WT>
+    __device__ __forceinline__ bool start(uint32_t s_base, float4 r0, float4 r1, bool walkable) {
+        o = make_float3(r0.x, r0.y, r0.z);
+        d = make_float3(r1.x, r1.y, r1.z);
+        tmin = r0.w;
+        bt = r1.w;
+        bu = bv = 0.f;
+        btri = CRT_MISS;
+        redo = false;
+        stop(s_base);
+        set_bound();
+        if (WT) wt = wt_setup(d);
+        if (!(tmin <= bt)) return true;  // an empty ray
+        if (!walk4_setup(w, o, d, tmin, abs_eps) || !walkable) return false;
+        cur = 0;
+        return true;
+    }
+    template <bool WT>
+    __device__ __forceinline__ void test_leaf(uint32_t leaf) {
+        if (leaf == kNoChild) return;  // an empty slot whose planes collapsed in rounding
+        const uint32_t L = leaf & ~kLeafRef;
+        const float4* t = xtri + 3 * static_cast<size_t>(L);
+        const float4 a = __ldg(t), b = __ldg(t + 1), c = __ldg(t + 2);
+        if (!WT) {
+            RayCtx r;
+            r.o = o;
+            r.d = d;
+            r.inv = make_float3(1.0f / d.x, 1.0f / d.y, 1.0f / d.z);
+            r.exact = !(isfinite(r.inv.x) && isfinite(r.inv.y) && isfinite(r.inv.z));
+            if (!leaf_box_passes(r, a, b, c, prune_bound(bt, abs_eps))) return;
+        }
+        const float3 A = make_float3(a.x, a.y, a.z), B = make_float3(b.x, b.y, b.z), C = make_float3(c.x, c.y, c.z);
+        // accepted only up to the best hit (bt <= tmax)
+        const HitRes h = WT ? tri_watertight(o, tmin, bt, wt, A, B, C) : tri_reference(o, d, tmin, bt, A, B, C);
+        if (!h.did) return;
+        const uint32_t tri = __float_as_uint(a.w);
+        if (btri == CRT_MISS || h.t < bt || (h.t == bt && (WT ? tri < btri : L > bleaf))) {
+            bt = h.t; bu = h.u; bv = h.v; btri = tri;
+            if (!WT) bleaf = L;
+            set_bound();
+        }
+    }
+    __device__ __forceinline__ uint4 hit() const {
+        return btri != CRT_MISS ? make_uint4(btri, __float_as_uint(bt), __float_as_uint(bu), __float_as_uint(bv))
+                                : make_uint4(CRT_MISS, 0u, 0u, 0u);
+    }
+};
+
+// Steps the warp's walks until at least `limit` lanes are over (lanes without a
+// ray are) and returns their mask.  In a step each lane without a node pops one
+// stack entry: an internal node becomes cur, the first leaf is parked, a second
+// leaf stays on the stack and blocks the lane; then each lane with a node visits
+// it.  The warp tests its parked leaves together once FLUSH lanes are blocked (or
+// hold one with nothing else left), or no lane has a node.
+// s_base: the lane's first shared entry (the row below it is readable).
+template <bool ANY, bool WT, int FLUSH, bool COUNT = false>
+__device__ __forceinline__ uint32_t walk4_run(Walk4Lane& L, uint32_t s_base, uint2* __restrict__ st, int limit) {
+    constexpr uint32_t kRow = kWalk4Row, kNoLeaf = Walk4Lane::kNoLeaf;
+#pragma unroll 1
+    while (true) {
+        bool blocked = false, over = false;
+        if (L.cur < 0) {
+            if (L.spilled) {  // rare: older entries come back
+                if (L.top == s_base) {
+                    const uint32_t n = min(L.spilled, kWalk4Spill);
+                    L.spilled -= n;
+                    for (uint32_t k = 0; k < n; ++k, L.top += kRow) walk4_sts(L.top, st[L.spilled + k]);
+                }
+            }
+            const uint2 e = walk4_lds(L.top - kRow);
+            const bool some = L.top != s_base, full = L.pend != kNoLeaf;
+            const bool near = (ANY ? fabsf(__uint_as_float(e.y)) : __uint_as_float(e.y)) <= L.bound;
+            const bool leaf = static_cast<int>(e.x) < 0;
+            blocked = full && (!some || (near && leaf));
+            over = !some && !full;
+            if (some && near && !leaf) L.cur = static_cast<int>(e.x);
+            if (some && near && leaf && !full) {
+                L.pend = e.x;
+                L.pend_t = __uint_as_float(e.y);
+            }
+            uint32_t drop = near ? kRow : kRow + kRow * (e.y & 3u);
+            if (!some || blocked) drop = 0u;
+            if (L.spilled) {  // rare: some of the siblings were moved
+                const uint32_t have = L.top - s_base;
+                if (have < drop) {
+                    L.spilled -= (drop - have) / kRow;
+                    drop = have;
+                }
+            }
+            L.top -= drop;
+        }
+        const uint32_t wm = __ballot_sync(0xFFFFFFFFu, L.cur >= 0);
+        const uint32_t bm = __ballot_sync(0xFFFFFFFFu, blocked);
+        if (__popc(bm) >= FLUSH || !wm) {
+            if (L.pend != kNoLeaf) {
+                if ((ANY ? fabsf(L.pend_t) : L.pend_t) <= L.bound) {
+                    L.template test_leaf<WT>(L.pend);
+                    if (COUNT) ++L.tested;
+                }
+                L.pend = kNoLeaf;
+                if (ANY && L.btri != CRT_MISS) {
+                    L.stop(s_base);
+                    over = true;
+                }
+            }
+        }
+        const uint32_t om = __ballot_sync(0xFFFFFFFFu, over);
+        if (__popc(om) >= limit) return om;
+        if (L.cur >= 0) {
+            Walk4Node n = load_walk4(L.cw + 4 * static_cast<size_t>(static_cast<uint32_t>(L.cur)));
+            if (COUNT) ++L.fetched;
+            if (L.top > s_base + (kWalk4Shared - 4) * kRow) {  // rare: the oldest entries move to local memory
+                if (L.spilled + kWalk4Spill > kWalk4Local) {
+                    L.redo = true;
+                    L.stop(s_base);
+                    continue;
+                }
+                for (uint32_t k = 0; k < kWalk4Spill; ++k) st[L.spilled + k] = walk4_lds(s_base + k * kRow);
+                for (uint32_t q = s_base; q + kWalk4Spill * kRow < L.top; q += kRow)
+                    walk4_sts(q, walk4_lds(q + kWalk4Spill * kRow));
+                L.top -= kWalk4Spill * kRow;
+                L.spilled += kWalk4Spill;
+            }
+            float t[4];
+            walk4_children(n, L.w, L.bound, t);
+            walk4_sort<ANY>(t, n.ref);
+            const float inf = __int_as_float(0x7F800000);
+            uint32_t below = 0;
+            // each entry is stored where the next one goes unless it counts: four rows are free above top
+#pragma unroll
+            for (int c = 3; c >= 1; --c) {
+                walk4_sts(L.top, make_uint2(n.ref[c], (__float_as_uint(t[c]) & ~3u) | below));
+                if (t[c] < inf) {
+                    L.top += kRow;
+                    ++below;
+                }
+            }
+            // the nearest child is entered; a leaf goes through the stack
+            walk4_sts(L.top, make_uint2(n.ref[0], (__float_as_uint(t[0]) & ~3u) | below));
+            const bool met = t[0] < inf;
+            L.cur = met ? static_cast<int>(n.ref[0]) : -1;
+            if (met && L.cur < 0) L.top += kRow;
+        }
+    }
+}
+
+// Persistent warps over a ray pool, one ray per lane; lanes whose ray is done take
+// new rays from the counter once kWalk4Refill of them wait.
 //
 // What bounds it (ncu, 1 M rays): the ALU pipe (68 % busy: byte permutes,
 // minima, selects; issue slots 65 %), about 21 of 32 lanes visiting in a step.
@@ -215,12 +398,6 @@ __device__ __forceinline__ void walk4_sts(uint32_t a, uint2 e) {
 // than the 65,536 rays of the smallest launch gain (0.53 -> 0.43 ms with it,
 // 0.36 without).
 //
-// The stack's newest entries sit in shared memory (a column per thread, so any
-// mix of depths is free of bank conflicts), older ones move to local memory
-// eight at a time.  An entry is (reference, entry distance); its low two
-// distance bits count the siblings pushed just below it, which are farther, so
-// one too-far entry drops them all.
-//
 // Rays the compressed walk cannot take (walk4_setup, unquantised scenes, one-leaf
 // trees, walks deeper than the stack) go to the list left[0 .. pool[1]) for
 // walk4_left_kernel, launched right after; pool[0] counts the rays taken.
@@ -228,10 +405,8 @@ template <bool ANY, bool WT, bool BATCH>
 __global__ void __launch_bounds__(kWalk4Block, kWalk4Blocks)
     trace_walk4_kernel(const TraceParams p, uint32_t* __restrict__ pool, uint32_t* __restrict__ left,
                        const BatchScene* __restrict__ scenes, uint32_t n_scenes) {
-    constexpr uint32_t SH = kWalk4Shared, LOC = kWalk4Local, kRow = kWalk4Block * 8, kSpill = 8;
-    static_assert(SH >= kSpill + 4 && LOC % kSpill == 0, "stack shape");
-    constexpr uint32_t kIdle = 0xFFFFFFFFu, kDone = 0xFFFFFFFEu, kNoLeaf = 0xFFFFFFFFu;
-    __shared__ uint2 s_st[SH + 1][kWalk4Block];  // row 0 is read (and ignored) below an empty stack
+    constexpr uint32_t kIdle = 0xFFFFFFFFu, kDone = 0xFFFFFFFEu;
+    __shared__ uint2 s_st[kWalk4Shared + 1][kWalk4Block];  // row 0 is read (and ignored) below an empty stack
     __shared__ uint32_t s_ray_off[BATCH ? kMaxBatchScenes + 1 : 1];
     if (BATCH) {
         for (uint32_t k = threadIdx.x; k <= n_scenes; k += kWalk4Block)
@@ -241,59 +416,14 @@ __global__ void __launch_bounds__(kWalk4Block, kWalk4Blocks)
     const uint32_t lane = threadIdx.x & 31u;
     const uint32_t s_base = static_cast<uint32_t>(__cvta_generic_to_shared(&s_st[1][threadIdx.x]));
     const bool quantised = __ldg(p.cw_bad) == 0u;
-    uint2 st[LOC];
-    // the scene of the lane's ray
-    const uint4* cw = p.cwide;
-    const float4* xtri = p.xtri;
-    float abs_eps = p.abs_eps;
-    uint32_t n_leaves = (p.n_nodes + 1) / 2;
-    // the lane's ray
-    Walk4Ray w;
-    WRay wt{};
-    float3 o, d;
-    float tmin = 0.f, bt = 0.f, bu = 0.f, bv = 0.f, bound = 0.f;  // bt: tmax until a hit is found
-    float pend_t = 0.f;                                            // entry distance of the parked leaf
-    uint32_t btri = CRT_MISS, bleaf = 0, pend = kNoLeaf, i = kIdle;  // bleaf: the shader's tie order
-    int cur = -1;
-    uint32_t top = s_base, spilled = 0;  // next free shared entry; entries moved to local memory
-
-    auto set_bound = [&]() { bound = prune_bound(bt, abs_eps) * kWalk4TScale; };
-    auto stop = [&]() {  // nothing left of this walk
-        cur = -1;
-        top = s_base;
-        spilled = 0;
-        pend = kNoLeaf;
-    };
-    auto leave = [&]() {
-        left[atomicAdd(pool + 1, 1u)] = i;
-        i = kIdle;
-        stop();
-    };
-    auto test_leaf = [&](uint32_t leaf) {
-        if (leaf == kNoChild) return;  // an empty slot whose planes collapsed in rounding
-        const uint32_t L = leaf & ~kLeafRef;
-        const float4* t = xtri + 3 * static_cast<size_t>(L);
-        const float4 a = __ldg(t), b = __ldg(t + 1), c = __ldg(t + 2);
-        if (!WT) {
-            RayCtx r;
-            r.o = o;
-            r.d = d;
-            r.inv = make_float3(1.0f / d.x, 1.0f / d.y, 1.0f / d.z);
-            r.exact = false;  // walk4_setup admits only rays with finite, nonzero 1/d
-            if (!leaf_box_passes(r, a, b, c, prune_bound(bt, abs_eps))) return;
-        }
-        const float3 A = make_float3(a.x, a.y, a.z), B = make_float3(b.x, b.y, b.z), C = make_float3(c.x, c.y, c.z);
-        // accepted only up to the best hit (bt <= tmax)
-        const HitRes h = WT ? tri_watertight(o, tmin, bt, wt, A, B, C) : tri_reference(o, d, tmin, bt, A, B, C);
-        if (!h.did) return;
-        const uint32_t tri = __float_as_uint(a.w);
-        if (btri == CRT_MISS || h.t < bt || (h.t == bt && (WT ? tri < btri : L > bleaf))) {
-            bt = h.t; bu = h.u; bv = h.v; btri = tri;
-            if (!WT) bleaf = L;
-            set_bound();
-        }
-    };
-
+    uint2 st[kWalk4Local];
+    Walk4Lane L{};
+    L.cw = p.cwide;
+    L.xtri = p.xtri;
+    L.abs_eps = p.abs_eps;
+    L.stop(s_base);
+    bool walkable = quantised && p.n_nodes > 2;
+    uint32_t i = kIdle;
     bool pool_left = true;
     while (true) {
         const uint32_t need = __ballot_sync(0xFFFFFFFFu, i == kIdle);
@@ -313,115 +443,23 @@ __global__ void __launch_bounds__(kWalk4Block, kWalk4Blocks)
                 } else {
                     if (BATCH) {
                         const BatchScene bs = scenes[batch_scene_of(s_ray_off, n_scenes, i)];
-                        cw = p.cwide + 4 * static_cast<size_t>(bs.wide_off);
-                        xtri = p.xtri + 3 * static_cast<size_t>(bs.tri_off);
-                        abs_eps = bs.abs_eps;
-                        n_leaves = bs.n_tris;
+                        L.cw = p.cwide + 4 * static_cast<size_t>(bs.wide_off);
+                        L.xtri = p.xtri + 3 * static_cast<size_t>(bs.tri_off);
+                        L.abs_eps = bs.abs_eps;
+                        walkable = quantised && bs.n_tris > 1;
                     }
                     const float4 r0 = __ldg(reinterpret_cast<const float4*>(p.rays + i));
                     const float4 r1 = __ldg(reinterpret_cast<const float4*>(p.rays + i) + 1);
-                    o = make_float3(r0.x, r0.y, r0.z);
-                    d = make_float3(r1.x, r1.y, r1.z);
-                    tmin = r0.w;
-                    bt = r1.w;
-                    bu = bv = 0.f;
-                    btri = CRT_MISS;
-                    cur = 0;  // the root: its children are tested, not its own box
-                    set_bound();
-                    if (WT) wt = wt_setup(d);
-                    if (!(tmin <= bt)) stop();
-                    else if (!walk4_setup(w, o, d, tmin, abs_eps) || !quantised || n_leaves < 2) leave();
+                    L.redo = !L.template start<WT>(s_base, r0, r1, walkable);
                 }
             }
         }
         if (i == kIdle && !pool_left) i = kDone;
         if (__all_sync(0xFFFFFFFFu, i == kDone)) break;
-#pragma unroll 1
-        while (true) {
-            bool blocked = false, over = false;
-            if (cur < 0) {
-                if (spilled) {  // rare: older entries come back
-                    if (top == s_base) {
-                        const uint32_t n = min(spilled, kSpill);
-                        spilled -= n;
-                        for (uint32_t k = 0; k < n; ++k, top += kRow) walk4_sts(top, st[spilled + k]);
-                    }
-                }
-                const uint2 e = walk4_lds(top - kRow);
-                const bool some = top != s_base, full = pend != kNoLeaf;
-                const bool near = (ANY ? fabsf(__uint_as_float(e.y)) : __uint_as_float(e.y)) <= bound;
-                const bool leaf = static_cast<int>(e.x) < 0;
-                blocked = full && (!some || (near && leaf));
-                over = !some && !full;
-                if (some && near && !leaf) cur = static_cast<int>(e.x);
-                if (some && near && leaf && !full) {
-                    pend = e.x;
-                    pend_t = __uint_as_float(e.y);
-                }
-                uint32_t drop = near ? kRow : kRow + kRow * (e.y & 3u);
-                if (!some || blocked) drop = 0u;
-                if (spilled) {  // rare: some of the siblings were moved
-                    const uint32_t have = top - s_base;
-                    if (have < drop) {
-                        spilled -= (drop - have) / kRow;
-                        drop = have;
-                    }
-                }
-                top -= drop;
-            }
-            const uint32_t wm = __ballot_sync(0xFFFFFFFFu, cur >= 0);
-            const uint32_t bm = __ballot_sync(0xFFFFFFFFu, blocked);
-            if (__popc(bm) >= kWalk4Flush || !wm) {
-                if (pend != kNoLeaf) {
-                    if ((ANY ? fabsf(pend_t) : pend_t) <= bound) test_leaf(pend);
-                    pend = kNoLeaf;
-                    if (ANY && btri != CRT_MISS) {
-                        stop();
-                        over = true;
-                    }
-                }
-            }
-            const uint32_t om = __ballot_sync(0xFFFFFFFFu, over);
-            if (om == 0xFFFFFFFFu || (pool_left && __popc(om) >= kWalk4Refill)) break;
-            if (cur >= 0) {
-                Walk4Node n = load_walk4(cw + 4 * static_cast<size_t>(static_cast<uint32_t>(cur)));
-                if (top > s_base + (SH - 4) * kRow) {  // rare: the oldest entries move to local memory
-                    if (spilled + kSpill > LOC) {  // the walk outgrows the stack: start over on the binary nodes
-                        leave();
-                        continue;
-                    }
-                    for (uint32_t k = 0; k < kSpill; ++k) st[spilled + k] = walk4_lds(s_base + k * kRow);
-                    for (uint32_t q = s_base; q + kSpill * kRow < top; q += kRow)
-                        walk4_sts(q, walk4_lds(q + kSpill * kRow));
-                    top -= kSpill * kRow;
-                    spilled += kSpill;
-                }
-                float t[4];
-                walk4_children(n, w, bound, t);
-                walk4_sort<ANY>(t, n.ref);
-                const float inf = __int_as_float(0x7F800000);
-                uint32_t below = 0;
-                // each entry is stored where the next one goes unless it counts: four rows are free above top
-#pragma unroll
-                for (int c = 3; c >= 1; --c) {
-                    walk4_sts(top, make_uint2(n.ref[c], (__float_as_uint(t[c]) & ~3u) | below));
-                    if (t[c] < inf) {
-                        top += kRow;
-                        ++below;
-                    }
-                }
-                // the nearest child is entered; a leaf goes through the stack
-                walk4_sts(top, make_uint2(n.ref[0], (__float_as_uint(t[0]) & ~3u) | below));
-                const bool met = t[0] < inf;
-                cur = met ? static_cast<int>(n.ref[0]) : -1;
-                if (met && cur < 0) top += kRow;
-            }
-        }
-        // over: the walk has ended with no leaf parked
-        if (i < kDone && cur < 0 && top == s_base && !spilled && pend == kNoLeaf) {
-            reinterpret_cast<uint4*>(p.hits)[i] =
-                btri != CRT_MISS ? make_uint4(btri, __float_as_uint(bt), __float_as_uint(bu), __float_as_uint(bv))
-                                 : make_uint4(CRT_MISS, 0u, 0u, 0u);
+        const uint32_t om = walk4_run<ANY, WT, kWalk4Flush>(L, s_base, st, pool_left ? kWalk4Refill : 32);
+        if ((om >> lane & 1u) && i < kDone) {
+            if (L.redo) left[atomicAdd(pool + 1, 1u)] = i;
+            else reinterpret_cast<uint4*>(p.hits)[i] = L.hit();
             i = kIdle;
         }
     }
@@ -484,7 +522,7 @@ __device__ __forceinline__ uint4 trace_walk4_one(const TraceParams& p, const uin
             r.o = o;
             r.d = d;
             r.inv = make_float3(1.0f / d.x, 1.0f / d.y, 1.0f / d.z);
-            r.exact = false;
+            r.exact = !(isfinite(r.inv.x) && isfinite(r.inv.y) && isfinite(r.inv.z));
             if (!leaf_box_passes(r, a, b, c, prune_bound(bt, p.abs_eps))) return;
         }
         ++tested;
