@@ -1828,7 +1828,6 @@ struct crt_batch {
     DevBuf node_box, node_kids, pf, clus_a, clus_b, it, ploc_lb, hist, sort_lb;
     DevBuf nodes, wide, wide_wt, depth_odd, xtri, xtri_sorted, inv_perm;
     DevBuf ray_order, ray_order_scratch;  // CRT_TRACE_SORT_RAYS
-    DevBuf pool;                          // the persistent trace's counters and left-over rays
     DevBuf cwide;                         // compressed 4-wide nodes (and their bad flag) of the scenes' current trees
     bool cwide_ready = false;
     bool g_cwide = false;                 // the captured graph derives them
@@ -1927,7 +1926,7 @@ crt_status batch_trace_enqueue(crt_ctx* x, crt_batch* bt, const crt_ray* rays, u
         p.cwide = bt->cwide.as<uint4>();
         p.cw_bad = bt->cw_bad();
         crt::launch_trace_batch_pool(p, bt->scenes.as<crt::BatchScene>(), bt->n_scenes,
-                                     flags & (CRT_TRACE_ANY | CRT_TRI_WATERTIGHT), deep, bt->pool.as<uint32_t>(), s);
+                                     flags & (CRT_TRACE_ANY | CRT_TRI_WATERTIGHT), deep, bt->node_box.as<uint32_t>(), s);
     } else
         crt::launch_trace_batch(p, bt->scenes.as<crt::BatchScene>(), bt->n_scenes, bt->n_rays,
                                 flags & (CRT_TRACE_ANY | CRT_TRI_WATERTIGHT), static_cast<int>(bt->cfg.trace_block), deep,
@@ -2005,13 +2004,8 @@ crt_status batch_enqueue(crt_ctx* x, crt_batch* bt, const crt_triangle* tris, co
     return CRT_OK;
 }
 
-// Buffers of a batch's trace (compressed nodes, the scratch of CRT_TRACE_SORT_RAYS),
-// reserved outside graph capture.
-crt_status batch_trace_buffers(crt_batch* bt, uint32_t flags) {
-    if (batch_pool(bt, flags)) {
-        CRT_TRY(bt->cwide.reserve(64ull * bt->n_tris + 16));
-        CRT_TRY(bt->pool.reserve(crt::trace_pool_bytes(bt->ray_cap)));
-    }
+// Scratch of CRT_TRACE_SORT_RAYS for a batch, reserved outside graph capture.
+crt_status batch_order_buffers(crt_batch* bt, uint32_t flags) {
     // sized for the batch's ray capacity, so a later crt_batch_set_ray_counts
     // never moves a buffer that a captured graph points at
     if (!(flags & CRT_TRACE_SORT_RAYS) || bt->ray_cap <= 1) return CRT_OK;
@@ -2100,7 +2094,9 @@ crt_status crt_batch_create(crt_ctx* x, const uint32_t* tri_counts, const uint32
                       &bt->inv_perm})
         R(*b, 4ull * N);
     R(bt->node_kids, 16ull * N);
-    R(bt->node_box, 32ull * (2ull * N));
+    // node_box also holds the trace's ray pool: it is build scratch, idle between builds
+    R(bt->node_box, std::max<size_t>(32ull * (2ull * N), crt::trace_pool_bytes(bt->ray_cap)));
+    R(bt->cwide, 64ull * N + 16);
     R(bt->pf, 8ull * N);
     R(bt->clus_a, 32ull * N);
     R(bt->clus_b, 32ull * N);
@@ -2145,7 +2141,7 @@ crt_status crt_batch_free(crt_batch* bt) {
                       &bt->codes_a, &bt->codes_b, &bt->vals_a, &bt->vals_b, &bt->codes, &bt->perm_global,
                       &bt->perm_local, &bt->node_box, &bt->node_kids, &bt->pf, &bt->clus_a, &bt->clus_b, &bt->it,
                       &bt->ploc_lb, &bt->hist, &bt->sort_lb, &bt->nodes, &bt->wide, &bt->wide_wt, &bt->depth_odd, &bt->xtri, &bt->ray_order, &bt->ray_order_scratch,
-                      &bt->inv_perm, &bt->xtri_sorted, &bt->pool, &bt->cwide};
+                      &bt->inv_perm, &bt->xtri_sorted, &bt->cwide};
     for (DevBuf* b : bufs) b->release();
     delete bt;
     return CRT_OK;
@@ -2235,7 +2231,7 @@ crt_status crt_batch_trace(crt_ctx* x, crt_batch* bt, const crt_ray* rays, uint3
     CRT_TRY(check_aligned16(rays, "crt_batch_trace: rays"));
     CRT_TRY(check_aligned16(hits, "crt_batch_trace: hits"));
     CRT_CUDA(cudaSetDevice(x->device));
-    CRT_TRY(batch_trace_buffers(bt, flags));
+    CRT_TRY(batch_order_buffers(bt, flags));
     CRT_CUDA(cudaMemsetAsync(bt->err.p, 0, 16, x->stream));
     const bool deep = bt->cfg.stack_depth > 64 || bt->max_iters + 2 > 64;
     CRT_TRY(batch_trace_enqueue(x, bt, rays, flags, hits, deep));
@@ -2248,7 +2244,7 @@ crt_status crt_batch_run(crt_ctx* x, crt_batch* bt, const crt_triangle* tris, co
     CRT_TRY(batch_trace_flags(bt, flags, "crt_batch_run"));
     CRT_TRY(check_batch_buffers(tris, rays, hits, "crt_batch_run"));
     CRT_CUDA(cudaSetDevice(x->device));
-    CRT_TRY(batch_trace_buffers(bt, flags));  // before any graph capture: no allocation inside it
+    CRT_TRY(batch_order_buffers(bt, flags));  // before any graph capture: no allocation inside it
     if (graph_used) *graph_used = 0;
     if (bt->max_iters + 2 > 64) bt->cfg.stack_depth = 1024;
     if (use_graph) {
@@ -2360,7 +2356,7 @@ crt_status crt_batch_autotune(crt_ctx* x, crt_batch* bt, const crt_triangle* tri
     if (!x || !bt || !tris || !rays || !hits) return fail(CRT_ERR_INVALID_ARG, "crt_batch_autotune: null argument");
     CRT_TRY(check_batch_buffers(tris, rays, hits, "crt_batch_autotune"));
     CRT_CUDA(cudaSetDevice(x->device));
-    CRT_TRY(batch_trace_buffers(bt, flags));
+    CRT_TRY(batch_order_buffers(bt, flags));
     cudaEvent_t e0, e1, e2;
     CRT_CUDA(cudaEventCreate(&e0));
     CRT_CUDA(cudaEventCreate(&e1));
