@@ -161,15 +161,36 @@ __device__ __forceinline__ float load_h(const unsigned char* tile, int Kd, int r
     return __half2float(*reinterpret_cast<const __half*>(tile + kmajor_offset(row, k, Kd)));
 }
 
-// Issue D = A * B^T over Kd columns (Kd / 16 MMAs) from one thread.
+// Sum of row `row` of a K-major tile of 128 fp16 columns, in column order.
+__device__ __forceinline__ float row_sum128(const unsigned char* tile, int row) {
+    float acc = 0.f;
+#pragma unroll 4
+    for (int c = 0; c < 128; c += 8) {
+        const uint4 q = *reinterpret_cast<const uint4*>(tile + kmajor_offset(row, c, 128));
+        const __half* h = reinterpret_cast<const __half*>(&q);
+#pragma unroll
+        for (int j = 0; j < 8; ++j) acc += __half2float(h[j]);
+    }
+    return acc;
+}
+
+// Four floats added to global memory in one reduction.
+__device__ __forceinline__ void red_add4(float* dst, const float* v) {
+    asm volatile("red.relaxed.gpu.global.add.v4.f32 [%0], {%1, %2, %3, %4};" ::"l"(dst), "f"(v[0]), "f"(v[1]), "f"(v[2]),
+                 "f"(v[3])
+                 : "memory");
+}
+
+// Issue D = A * B^T over Kd columns (Kd / 16 MMAs) from one thread; with add,
+// D += A * B^T.
 __device__ __forceinline__ void gemm(uint32_t d_tmem, const unsigned char* A, const unsigned char* B, int Kd, int M,
-                                     int N) {
+                                     int N, bool add = false) {
     const uint32_t sbo = static_cast<uint32_t>(Kd / 8) * 128u;
     const uint32_t a0 = tc::smem_u32(A), b0 = tc::smem_u32(B);
     const uint32_t id = tc::idesc_f16_f32(M, N);
     for (int kk = 0; kk < Kd / 16; ++kk)
         tc::mma_f16(d_tmem, tc::smem_desc(a0 + kk * 256, tc::kLbo, sbo), tc::smem_desc(b0 + kk * 256, tc::kLbo, sbo),
-                    id, kk > 0);
+                    id, add || kk > 0);
 }
 
 constexpr uint32_t kMmaWaitLimit = 1u << 26;  // try_wait rounds before a tile gives up
@@ -402,15 +423,20 @@ __global__ void __launch_bounds__(128) infer_kernel(PredictorDev P, const crt_bv
 }
 
 // ------------------------------------------------------------ training
-// One 128-sample tile per CTA: forward, softmax cross-entropy gradient
-// (p - onehot, unscaled; the optimiser divides by the sample count), backward
-// GEMMs, FP32 atomics into the gradient buffers.  Shared memory:
+// Persistent, one CTA per SM over 128-sample tiles: forward, softmax
+// cross-entropy gradient (p - onehot, unscaled; the optimiser divides by the
+// sample count), backward GEMMs.  The weight gradients accumulate in TMEM and
+// the bias gradients and the loss in registers over the CTA's tiles and are
+// added to global memory once; the embedding gradients (a row per sample) by
+// four-float reductions.  With one tile per CTA and an atomic per weight and
+// tile, 262,145 samples took 617 us, 13.5 waves bound by the atomics on the
+// 14,592 shared weights; now TRAIN_US.  Shared memory:
 //   weights  W1 W1T W2 W2T W3 W3T                       56 KB
 //   acts     X XT H1 H1T H2 H2T                         80 KB
 //   grads    G3 G3T, then G2 G2T(padded to 128 rows),
 //            then G1 G1T(padded)                       64 KB
-// TMEM (256 cols): D1 0-63, D2 64-127, logits 128-255; then dW3 0-63,
-// dH2 64-127; dW2 128-191, dH1 192-255; dW1 0-31, dX 32-63.
+// TMEM (512 cols): D1 0-63, D2 64-127, logits 128-255; then dH2 64-127,
+// dH1 192-255, dX 32-63; dW3 256-319, dW2 320-383 and dW1 384-415 throughout.
 constexpr int kTrainSmem = 56 * 1024 + 80 * 1024 + 64 * 1024 + 256 * 4 + 64;
 
 __global__ void __launch_bounds__(128) train_kernel(PredictorDev P, const crt_bvh_node* nodes, const crt_ray* rays,
@@ -447,205 +473,208 @@ __global__ void __launch_bounds__(128) train_kernel(PredictorDev P, const crt_bv
     load_kmajor(sW3T, P.w16 + hW3T, 64, 128);
     for (int i = threadIdx.x; i < 256; i += 128)
         sB[i] = i < 64 ? P.master[oB1 + i] : (i < 128 ? P.master[oB2 + i - 64] : P.master[oB3 + i - 128]);
-    if (threadIdx.x < 32) { tc::tmem_alloc(sT, 256); tc::tmem_relinquish(); }
+    if (threadIdx.x < 32) { tc::tmem_alloc(sT, 512); tc::tmem_relinquish(); }
     if (threadIdx.x == 0) tc::mbar_init(sM, 1);
     const int tid = threadIdx.x;
-    const uint32_t s = blockIdx.x * 128 + tid;
-    const uint64_t ri = static_cast<uint64_t>(s) * stride + offset;
-    const bool valid = s < n_samples && ri < n_rays;
-    uint32_t cell = 0, bin = 0;
-    int target = -1;
-    uint4 e[4] = {};
-    if (valid) {
-        const float4 r0 = __ldg(reinterpret_cast<const float4*>(rays + ri));
-        const float4 r1 = __ldg(reinterpret_cast<const float4*>(rays + ri) + 1);
-        uint32_t scene, cell_raw;
-        ray_features(P, nodes, scene_frame(nodes), static_cast<uint32_t>(ri), r0, r1, cell, bin, scene, cell_raw);
-        const uint4* eo = reinterpret_cast<const uint4*>(P.w16 + hEo + static_cast<size_t>(cell) * kEmb);
-        const uint4* ed = reinterpret_cast<const uint4*>(P.w16 + hEd + static_cast<size_t>(bin) * kEmb);
-        e[0] = __ldg(eo); e[1] = __ldg(eo + 1); e[2] = __ldg(ed); e[3] = __ldg(ed + 1);
-        if (targets) {
-            target = targets[ri];
-        } else {
-            target = hit_class(P, scene, __ldg(reinterpret_cast<const uint32_t*>(hits + ri)));
-        }
-        if (target < 0 || target >= kClasses) target = kMissClass;
-    }
-#pragma unroll
-    for (int c = 0; c < 4; ++c) {
-        *reinterpret_cast<uint4*>(sX + kmajor_offset(tid, 8 * c, 32)) = e[c];
-        const __half* hv = reinterpret_cast<const __half*>(&e[c]);
-#pragma unroll
-        for (int j = 0; j < 8; ++j)
-            *reinterpret_cast<__half*>(sXT + kmajor_offset(8 * c + j, tid, 128)) = hv[j];
-    }
     Sync sy{sM, 0, err};
     sy.before_mma();
     const uint32_t tb = *sT;
+    // the CTA's sums over its tiles: weight gradients in these TMEM columns
+    // (lane = output unit), bias gradients and loss in registers
+    const uint32_t cW3 = tb + 256, cW2 = tb + 320, cW1 = tb + 384;
+    float db3 = 0.f, db2 = 0.f, db1 = 0.f, loss = 0.f;
+    bool first = true, ok = true;
+    for (uint32_t tile = blockIdx.x; tile * 128u < n_samples; tile += gridDim.x) {
+        ok = false;  // until the tile's last MMA wait has succeeded
+        const uint32_t s = tile * 128u + tid;
+        const uint64_t ri = static_cast<uint64_t>(s) * stride + offset;
+        const bool valid = s < n_samples && ri < n_rays;
+        uint32_t cell = 0, bin = 0;
+        int target = -1;
+        uint4 e[4] = {};
+        if (valid) {
+            const float4 r0 = __ldg(reinterpret_cast<const float4*>(rays + ri));
+            const float4 r1 = __ldg(reinterpret_cast<const float4*>(rays + ri) + 1);
+            uint32_t scene, cell_raw;
+            ray_features(P, nodes, scene_frame(nodes), static_cast<uint32_t>(ri), r0, r1, cell, bin, scene, cell_raw);
+            const uint4* eo = reinterpret_cast<const uint4*>(P.w16 + hEo + static_cast<size_t>(cell) * kEmb);
+            const uint4* ed = reinterpret_cast<const uint4*>(P.w16 + hEd + static_cast<size_t>(bin) * kEmb);
+            e[0] = __ldg(eo); e[1] = __ldg(eo + 1); e[2] = __ldg(ed); e[3] = __ldg(ed + 1);
+            if (targets) {
+                target = targets[ri];
+            } else {
+                target = hit_class(P, scene, __ldg(reinterpret_cast<const uint32_t*>(hits + ri)));
+            }
+            if (target < 0 || target >= kClasses) target = kMissClass;
+        }
+#pragma unroll
+        for (int c = 0; c < 4; ++c) {
+            *reinterpret_cast<uint4*>(sX + kmajor_offset(tid, 8 * c, 32)) = e[c];
+            const __half* hv = reinterpret_cast<const __half*>(&e[c]);
+#pragma unroll
+            for (int j = 0; j < 8; ++j)
+                *reinterpret_cast<__half*>(sXT + kmajor_offset(8 * c + j, tid, 128)) = hv[j];
+        }
+        sy.before_mma();
 
-    // One pass through the tile; a timed-out MMA wait leaves it (break) to
-    // the TMEM release below.
-    do {
-        // ---- forward
-        if (tid == 0) gemm(tb + 0, sX, sW1, 32, 128, 64);
-        if (!sy.commit_and_wait()) break;
-        for (int c = 0; c < 64; c += 16) {
-            float v[16];
-            tc::tmem_ld16(lane_addr(tb, c), v);
-#pragma unroll
-            for (int j = 0; j < 16; ++j) {
-                v[j] = __half2float(__float2half_rn(fmaxf(v[j] + sB[c + j], 0.f)));
-                store_h(sH1T, 128, c + j, tid, v[j]);
-            }
-            store_row8(sH1, 64, tid, c, v);
-            store_row8(sH1, 64, tid, c + 8, v + 8);
-        }
-        sy.before_mma();
-        if (tid == 0) gemm(tb + 64, sH1, sW2, 64, 128, 64);
-        if (!sy.commit_and_wait()) break;
-        for (int c = 0; c < 64; c += 16) {
-            float v[16];
-            tc::tmem_ld16(lane_addr(tb, 64 + c), v);
-#pragma unroll
-            for (int j = 0; j < 16; ++j) {
-                v[j] = __half2float(__float2half_rn(fmaxf(v[j] + sB[64 + c + j], 0.f)));
-                store_h(sH2T, 128, c + j, tid, v[j]);
-            }
-            store_row8(sH2, 64, tid, c, v);
-            store_row8(sH2, 64, tid, c + 8, v + 8);
-        }
-        sy.before_mma();
-        if (tid == 0) gemm(tb + 128, sH2, sW3, 64, 128, 128);
-        if (!sy.commit_and_wait()) break;
-
-        // ---- softmax cross-entropy: G3 = p - onehot(target)
-        float mx = -INFINITY;
-        for (int c = 0; c < 128; c += 16) {
-            float v[16];
-            tc::tmem_ld16(lane_addr(tb, 128 + c), v);
-#pragma unroll
-            for (int j = 0; j < 16; ++j) mx = fmaxf(mx, v[j] + sB[128 + c + j]);
-        }
-        float sum = 0.f;
-        for (int c = 0; c < 128; c += 16) {
-            float v[16];
-            tc::tmem_ld16(lane_addr(tb, 128 + c), v);
-#pragma unroll
-            for (int j = 0; j < 16; ++j) sum += __expf(v[j] + sB[128 + c + j] - mx);
-        }
-        const float inv = 1.f / sum;
-        for (int c = 0; c < 128; c += 16) {
-            float v[16];
-            tc::tmem_ld16(lane_addr(tb, 128 + c), v);
-#pragma unroll
-            for (int j = 0; j < 16; ++j) {
-                const float l = v[j] + sB[128 + c + j];
-                const float p = __expf(l - mx) * inv;
-                float g = p - ((c + j) == target ? 1.f : 0.f);
-                if (!valid) g = 0.f;
-                if (valid && (c + j) == target) atomicAdd(loss_sum, -(l - mx - __logf(sum)));
-                v[j] = __half2float(__float2half_rn(g));
-                store_h(sG3T, 128, c + j, tid, v[j]);
-            }
-            store_row8(sG3, 128, tid, c, v);
-            store_row8(sG3, 128, tid, c + 8, v + 8);
-        }
-        // ---- dW3 = G3^T H2 and dH2 = G3 W3
-        sy.before_mma();
-        if (tid == 0) {
-            gemm(tb + 0, sG3T, sH2T, 128, 128, 64);
-            gemm(tb + 64, sG3, sW3T, 128, 128, 64);
-        }
-        if (!sy.commit_and_wait()) break;
-        {
-            float acc = 0.f;  // db3[tid] = sum over samples of G3[:, tid]
-            for (int b = 0; b < 128; ++b) acc += load_h(sG3T, 128, tid, b);
-            atomicAdd(grad + oB3 + tid, acc);
-        }
-        for (int c = 0; c < 64; c += 16) {
-            float v[16];
-            tc::tmem_ld16(lane_addr(tb, c), v);
-#pragma unroll
-            for (int j = 0; j < 16; ++j) atomicAdd(grad + oW3 + tid * 64 + c + j, v[j]);
-        }
-        float dh[64];
-        for (int c = 0; c < 64; c += 16) tc::tmem_ld16(lane_addr(tb, 64 + c), dh + c);
-        tc::fence_before_sync();
-        __syncthreads();  // G3 / G3T fully consumed
-        zero_bytes(sGT + 64 * 128 * 2, 64 * 128 * 2);  // padding rows 64..127 of G2T
-#pragma unroll
-        for (int j = 0; j < 64; ++j) {
-            dh[j] = (load_h(sH2, 64, tid, j) > 0.f) ? __half2float(__float2half_rn(dh[j])) : 0.f;
-            store_h(sGT, 128, j, tid, dh[j]);
-        }
-        for (int c = 0; c < 64; c += 8) store_row8(sG, 64, tid, c, dh + c);
-        // ---- dW2 = G2^T H1 and dH1 = G2 W2
-        sy.before_mma();
-        if (tid == 0) {
-            gemm(tb + 128, sGT, sH1T, 128, 128, 64);
-            gemm(tb + 192, sG, sW2T, 64, 128, 64);
-        }
-        if (!sy.commit_and_wait()) break;
-        if (tid < 64) {
-            float acc = 0.f;
-            for (int b = 0; b < 128; ++b) acc += load_h(sGT, 128, tid, b);
-            atomicAdd(grad + oB2 + tid, acc);
-        }
-        for (int c = 0; c < 64; c += 16) {
-            float v[16];
-            tc::tmem_ld16(lane_addr(tb, 128 + c), v);
-            if (tid < 64) {
-#pragma unroll
-                for (int j = 0; j < 16; ++j) atomicAdd(grad + oW2 + tid * 64 + c + j, v[j]);
-            }
-        }
-        for (int c = 0; c < 64; c += 16) tc::tmem_ld16(lane_addr(tb, 192 + c), dh + c);
-        tc::fence_before_sync();
-        __syncthreads();
-        zero_bytes(sGT + 64 * 128 * 2, 64 * 128 * 2);
-#pragma unroll
-        for (int j = 0; j < 64; ++j) {
-            dh[j] = (load_h(sH1, 64, tid, j) > 0.f) ? __half2float(__float2half_rn(dh[j])) : 0.f;
-            store_h(sGT, 128, j, tid, dh[j]);
-        }
-        for (int c = 0; c < 64; c += 8) store_row8(sG, 64, tid, c, dh + c);
-        // ---- dW1 = G1^T X and dX = G1 W1
-        sy.before_mma();
-        if (tid == 0) {
-            gemm(tb + 0, sGT, sXT, 128, 128, 32);
-            gemm(tb + 32, sG, sW1T, 64, 128, 32);
-        }
-        if (!sy.commit_and_wait()) break;
-        if (tid < 64) {
-            float acc = 0.f;
-            for (int b = 0; b < 128; ++b) acc += load_h(sGT, 128, tid, b);
-            atomicAdd(grad + oB1 + tid, acc);
-        }
-        for (int c = 0; c < 32; c += 16) {
-            float v[16];
-            tc::tmem_ld16(lane_addr(tb, c), v);
-            if (tid < 64) {
-#pragma unroll
-                for (int j = 0; j < 16; ++j) atomicAdd(grad + oW1 + tid * 32 + c + j, v[j]);
-            }
-        }
-        for (int c = 0; c < 32; c += 16) {
-            float v[16];
-            tc::tmem_ld16(lane_addr(tb, 32 + c), v);
-            if (valid) {
+        // One pass through the tile; a timed-out MMA wait leaves it (break), and then
+        // the tile loop, to the TMEM release below.
+        do {
+            // ---- forward
+            if (tid == 0) gemm(tb + 0, sX, sW1, 32, 128, 64);
+            if (!sy.commit_and_wait()) break;
+            for (int c = 0; c < 64; c += 16) {
+                float v[16];
+                tc::tmem_ld16(lane_addr(tb, c), v);
 #pragma unroll
                 for (int j = 0; j < 16; ++j) {
-                    const int ee = c + j;
-                    float* dst = ee < kEmb ? grad + oEo + static_cast<size_t>(cell) * kEmb + ee
-                                           : grad + oEd + static_cast<size_t>(bin) * kEmb + (ee - kEmb);
-                    atomicAdd(dst, v[j]);
+                    v[j] = __half2float(__float2half_rn(fmaxf(v[j] + sB[c + j], 0.f)));
+                    store_h(sH1T, 128, c + j, tid, v[j]);
+                }
+                store_row8(sH1, 64, tid, c, v);
+                store_row8(sH1, 64, tid, c + 8, v + 8);
+            }
+            sy.before_mma();
+            if (tid == 0) gemm(tb + 64, sH1, sW2, 64, 128, 64);
+            if (!sy.commit_and_wait()) break;
+            for (int c = 0; c < 64; c += 16) {
+                float v[16];
+                tc::tmem_ld16(lane_addr(tb, 64 + c), v);
+#pragma unroll
+                for (int j = 0; j < 16; ++j) {
+                    v[j] = __half2float(__float2half_rn(fmaxf(v[j] + sB[64 + c + j], 0.f)));
+                    store_h(sH2T, 128, c + j, tid, v[j]);
+                }
+                store_row8(sH2, 64, tid, c, v);
+                store_row8(sH2, 64, tid, c + 8, v + 8);
+            }
+            sy.before_mma();
+            if (tid == 0) gemm(tb + 128, sH2, sW3, 64, 128, 128);
+            if (!sy.commit_and_wait()) break;
+
+            // ---- softmax cross-entropy: G3 = p - onehot(target)
+            float mx = -INFINITY;
+            for (int c = 0; c < 128; c += 16) {
+                float v[16];
+                tc::tmem_ld16(lane_addr(tb, 128 + c), v);
+#pragma unroll
+                for (int j = 0; j < 16; ++j) mx = fmaxf(mx, v[j] + sB[128 + c + j]);
+            }
+            float sum = 0.f;
+            for (int c = 0; c < 128; c += 16) {
+                float v[16];
+                tc::tmem_ld16(lane_addr(tb, 128 + c), v);
+#pragma unroll
+                for (int j = 0; j < 16; ++j) sum += __expf(v[j] + sB[128 + c + j] - mx);
+            }
+            const float inv = 1.f / sum;
+            for (int c = 0; c < 128; c += 16) {
+                float v[16];
+                tc::tmem_ld16(lane_addr(tb, 128 + c), v);
+#pragma unroll
+                for (int j = 0; j < 16; ++j) {
+                    const float l = v[j] + sB[128 + c + j];
+                    const float p = __expf(l - mx) * inv;
+                    float g = p - ((c + j) == target ? 1.f : 0.f);
+                    if (!valid) g = 0.f;
+                    if (valid && (c + j) == target) loss -= l - mx - __logf(sum);
+                    v[j] = __half2float(__float2half_rn(g));
+                    store_h(sG3T, 128, c + j, tid, v[j]);
+                }
+                store_row8(sG3, 128, tid, c, v);
+                store_row8(sG3, 128, tid, c + 8, v + 8);
+            }
+            // ---- dW3 = G3^T H2 and dH2 = G3 W3
+            sy.before_mma();
+            if (tid == 0) {
+                gemm(cW3, sG3T, sH2T, 128, 128, 64, !first);
+                gemm(tb + 64, sG3, sW3T, 128, 128, 64);
+            }
+            if (!sy.commit_and_wait()) break;
+            db3 += row_sum128(sG3T, tid);  // sum over samples of G3[:, tid]
+            float dh[64];
+            for (int c = 0; c < 64; c += 16) tc::tmem_ld16(lane_addr(tb, 64 + c), dh + c);
+            tc::fence_before_sync();
+            __syncthreads();  // G3 / G3T fully consumed
+            zero_bytes(sGT + 64 * 128 * 2, 64 * 128 * 2);  // padding rows 64..127 of G2T
+#pragma unroll
+            for (int j = 0; j < 64; ++j) {
+                dh[j] = (load_h(sH2, 64, tid, j) > 0.f) ? __half2float(__float2half_rn(dh[j])) : 0.f;
+                store_h(sGT, 128, j, tid, dh[j]);
+            }
+            for (int c = 0; c < 64; c += 8) store_row8(sG, 64, tid, c, dh + c);
+            // ---- dW2 = G2^T H1 and dH1 = G2 W2
+            sy.before_mma();
+            if (tid == 0) {
+                gemm(cW2, sGT, sH1T, 128, 128, 64, !first);
+                gemm(tb + 192, sG, sW2T, 64, 128, 64);
+            }
+            if (!sy.commit_and_wait()) break;
+            if (tid < 64) db2 += row_sum128(sGT, tid);
+            for (int c = 0; c < 64; c += 16) tc::tmem_ld16(lane_addr(tb, 192 + c), dh + c);
+            tc::fence_before_sync();
+            __syncthreads();
+            zero_bytes(sGT + 64 * 128 * 2, 64 * 128 * 2);
+#pragma unroll
+            for (int j = 0; j < 64; ++j) {
+                dh[j] = (load_h(sH1, 64, tid, j) > 0.f) ? __half2float(__float2half_rn(dh[j])) : 0.f;
+                store_h(sGT, 128, j, tid, dh[j]);
+            }
+            for (int c = 0; c < 64; c += 8) store_row8(sG, 64, tid, c, dh + c);
+            // ---- dW1 = G1^T X and dX = G1 W1
+            sy.before_mma();
+            if (tid == 0) {
+                gemm(cW1, sGT, sXT, 128, 128, 32, !first);
+                gemm(tb + 32, sG, sW1T, 64, 128, 32);
+            }
+            if (!sy.commit_and_wait()) break;
+            if (tid < 64) db1 += row_sum128(sGT, tid);
+            for (int c = 0; c < 32; c += 16) {
+                float v[16];
+                tc::tmem_ld16(lane_addr(tb, 32 + c), v);
+                if (valid) {
+                    float* dst = c == 0 ? grad + oEo + static_cast<size_t>(cell) * kEmb : grad + oEd + static_cast<size_t>(bin) * kEmb;
+#pragma unroll
+                    for (int j = 0; j < 16; j += 4) red_add4(dst + j, v + j);
                 }
             }
+            ok = true;
+        } while (false);
+        if (!ok) break;
+        first = false;
+        // the next tile's operands overwrite what this tile's threads still read
+        tc::fence_before_sync();
+        __syncthreads();
+    }
+    if (ok && !first) {
+        for (int c = 0; c < 64; c += 16) {
+            float v[16];
+            tc::tmem_ld16(lane_addr(cW3, c), v);
+#pragma unroll
+            for (int j = 0; j < 16; j += 4) red_add4(grad + oW3 + tid * 64 + c + j, v + j);
+            tc::tmem_ld16(lane_addr(cW2, c), v);
+            if (tid < 64) {
+#pragma unroll
+                for (int j = 0; j < 16; j += 4) red_add4(grad + oW2 + tid * 64 + c + j, v + j);
+            }
+            if (c >= 32) continue;
+            tc::tmem_ld16(lane_addr(cW1, c), v);
+            if (tid < 64) {
+#pragma unroll
+                for (int j = 0; j < 16; j += 4) red_add4(grad + oW1 + tid * 32 + c + j, v + j);
+            }
         }
-    } while (false);
+        atomicAdd(grad + oB3 + tid, db3);
+        if (tid < 64) {
+            atomicAdd(grad + oB2 + tid, db2);
+            atomicAdd(grad + oB1 + tid, db1);
+        }
+        for (int m = 16; m > 0; m >>= 1) loss += __shfl_xor_sync(0xFFFFFFFFu, loss, m);
+        if ((tid & 31) == 0) atomicAdd(loss_sum, loss);
+    }
     tc::fence_before_sync();
     __syncthreads();
-    if (threadIdx.x < 32) tc::tmem_dealloc(tb, 256);
+    if (threadIdx.x < 32) tc::tmem_dealloc(tb, 512);
 }
 
 // ---------------------------------------------- failure-detection probe
@@ -1115,8 +1144,9 @@ cudaError_t pred_train_step(const PredictorDev& P, const crt_bvh_node* nodes, co
         if (e != cudaSuccess) return e;
         attr = true;
     }
-    const uint32_t grid = (n_samples + 127) / 128;
-    if (grid == 0) return cudaSuccess;
+    const uint32_t tiles = (n_samples + 127) / 128;
+    if (tiles == 0) return cudaSuccess;
+    const uint32_t grid = tiles < static_cast<uint32_t>(kNumSms) ? tiles : static_cast<uint32_t>(kNumSms);
     pred::train_kernel<<<grid, 128, pred::kTrainSmem, s>>>(P, nodes, rays, n_rays, hits, targets, n_samples, stride,
                                                           offset, P.grad, loss_sum, err);
     return cudaGetLastError();
