@@ -161,12 +161,12 @@ __device__ __forceinline__ float load_h(const unsigned char* tile, int Kd, int r
     return __half2float(*reinterpret_cast<const __half*>(tile + kmajor_offset(row, k, Kd)));
 }
 
-// Sum of row `row` of a K-major tile of 128 fp16 columns, in column order.
-__device__ __forceinline__ float row_sum128(const unsigned char* tile, int row) {
+// Sum of columns [c0, c0 + 32) of row `row` of a K-major tile of 128 fp16 columns.
+__device__ __forceinline__ float row_sum32(const unsigned char* tile, int row, int c0) {
     float acc = 0.f;
-#pragma unroll 4
-    for (int c = 0; c < 128; c += 8) {
-        const uint4 q = *reinterpret_cast<const uint4*>(tile + kmajor_offset(row, c, 128));
+#pragma unroll
+    for (int c = 0; c < 32; c += 8) {
+        const uint4 q = *reinterpret_cast<const uint4*>(tile + kmajor_offset(row, c0 + c, 128));
         const __half* h = reinterpret_cast<const __half*>(&q);
 #pragma unroll
         for (int j = 0; j < 8; ++j) acc += __half2float(h[j]);
@@ -430,19 +430,22 @@ __global__ void __launch_bounds__(128) infer_kernel(PredictorDev P, const crt_bv
 // added to global memory once; the embedding gradients (a row per sample) by
 // four-float reductions.  With one tile per CTA and an atomic per weight and
 // tile, 262,145 samples took 617 us, 13.5 waves bound by the atomics on the
-// 14,592 shared weights; now TRAIN_US.  Shared memory:
+// 14,592 shared weights; now 177 us (363 with
+// 128 threads per CTA).  Shared memory:
 //   weights  W1 W1T W2 W2T W3 W3T                       56 KB
 //   acts     X XT H1 H1T H2 H2T                         80 KB
 //   grads    G3 G3T, then G2 G2T(padded to 128 rows),
 //            then G1 G1T(padded)                       64 KB
 // TMEM (512 cols): D1 0-63, D2 64-127, logits 128-255; then dH2 64-127,
 // dH1 192-255, dX 32-63; dW3 256-319, dW2 320-383 and dW1 384-415 throughout.
-constexpr int kTrainSmem = 56 * 1024 + 80 * 1024 + 64 * 1024 + 256 * 4 + 64;
+constexpr int kTrainThreads = 512;  // four groups of 128: a thread per row and quarter of the columns
+constexpr int kTrainSmem = 56 * 1024 + 80 * 1024 + 64 * 1024 + 256 * 4 + 1024 * 4 + 64;
 
-__global__ void __launch_bounds__(128) train_kernel(PredictorDev P, const crt_bvh_node* nodes, const crt_ray* rays,
-                                                    uint32_t n_rays, const crt_hit* hits, const uint16_t* targets,
-                                                    uint32_t n_samples, uint32_t stride, uint32_t offset,
-                                                    float* grad, float* loss_sum, uint32_t* err) {
+__global__ void __launch_bounds__(kTrainThreads) train_kernel(PredictorDev P, const crt_bvh_node* nodes, const crt_ray* rays,
+                                                              uint32_t n_rays, const crt_hit* hits,
+                                                              const uint16_t* targets, uint32_t n_samples,
+                                                              uint32_t stride, uint32_t offset, float* grad,
+                                                              float* loss_sum, uint32_t* err) {
     extern __shared__ __align__(1024) unsigned char smem[];
     unsigned char* sW1 = smem;
     unsigned char* sW1T = sW1 + 4096;
@@ -458,7 +461,8 @@ __global__ void __launch_bounds__(128) train_kernel(PredictorDev P, const crt_bv
     unsigned char* sH2T = sH2 + 16384;
     unsigned char* sGA = sH2T + 16384;
     float* sB = reinterpret_cast<float*>(sGA + 65536);
-    uint32_t* sT = reinterpret_cast<uint32_t*>(sB + 256);
+    float* sRed = sB + 256;  // [4][128]: the groups' row maxima, then row sums
+    uint32_t* sT = reinterpret_cast<uint32_t*>(sRed + 1024);
     uint64_t* sM = reinterpret_cast<uint64_t*>(sT + 2);
     unsigned char* sG3 = sGA;
     unsigned char* sG3T = sGA + 32768;
@@ -471,169 +475,175 @@ __global__ void __launch_bounds__(128) train_kernel(PredictorDev P, const crt_bv
     load_kmajor(sW2T, P.w16 + hW2T, 64, 64);
     load_kmajor(sW3, P.w16 + hW3, 128, 64);
     load_kmajor(sW3T, P.w16 + hW3T, 64, 128);
-    for (int i = threadIdx.x; i < 256; i += 128)
+    if (threadIdx.x < 256) {
+        const int i = threadIdx.x;
         sB[i] = i < 64 ? P.master[oB1 + i] : (i < 128 ? P.master[oB2 + i - 64] : P.master[oB3 + i - 128]);
+    }
     if (threadIdx.x < 32) { tc::tmem_alloc(sT, 512); tc::tmem_relinquish(); }
     if (threadIdx.x == 0) tc::mbar_init(sM, 1);
-    const int tid = threadIdx.x;
+    // row: the sample (or output unit) this thread works on, one TMEM lane; q: the
+    // group of columns it takes
+    const int row = threadIdx.x & 127, q = threadIdx.x >> 7;
     Sync sy{sM, 0, err};
     sy.before_mma();
     const uint32_t tb = *sT;
+    // a warp reads the lane quadrant of its place in its group
+    auto lane = [&](uint32_t col) { return tb + ((32u * (static_cast<uint32_t>(row) >> 5)) << 16) + col; };
     // the CTA's sums over its tiles: weight gradients in these TMEM columns
     // (lane = output unit), bias gradients and loss in registers
-    const uint32_t cW3 = tb + 256, cW2 = tb + 320, cW1 = tb + 384;
+    constexpr uint32_t cW3 = 256, cW2 = 320, cW1 = 384;
     float db3 = 0.f, db2 = 0.f, db1 = 0.f, loss = 0.f;
     bool first = true, ok = true;
     for (uint32_t tile = blockIdx.x; tile * 128u < n_samples; tile += gridDim.x) {
         ok = false;  // until the tile's last MMA wait has succeeded
-        const uint32_t s = tile * 128u + tid;
+        const uint32_t s = tile * 128u + row;
         const uint64_t ri = static_cast<uint64_t>(s) * stride + offset;
         const bool valid = s < n_samples && ri < n_rays;
         uint32_t cell = 0, bin = 0;
         int target = -1;
-        uint4 e[4] = {};
+        uint4 e = make_uint4(0u, 0u, 0u, 0u);  // features 8q .. 8q+7
         if (valid) {
             const float4 r0 = __ldg(reinterpret_cast<const float4*>(rays + ri));
             const float4 r1 = __ldg(reinterpret_cast<const float4*>(rays + ri) + 1);
             uint32_t scene, cell_raw;
             ray_features(P, nodes, scene_frame(nodes), static_cast<uint32_t>(ri), r0, r1, cell, bin, scene, cell_raw);
-            const uint4* eo = reinterpret_cast<const uint4*>(P.w16 + hEo + static_cast<size_t>(cell) * kEmb);
-            const uint4* ed = reinterpret_cast<const uint4*>(P.w16 + hEd + static_cast<size_t>(bin) * kEmb);
-            e[0] = __ldg(eo); e[1] = __ldg(eo + 1); e[2] = __ldg(ed); e[3] = __ldg(ed + 1);
-            if (targets) {
-                target = targets[ri];
-            } else {
-                target = hit_class(P, scene, __ldg(reinterpret_cast<const uint32_t*>(hits + ri)));
-            }
+            e = __ldg(reinterpret_cast<const uint4*>(P.w16 + (q < 2 ? hEo + static_cast<size_t>(cell) * kEmb
+                                                                     : hEd + static_cast<size_t>(bin) * kEmb)) + (q & 1));
+            if (targets) target = targets[ri];
+            else target = hit_class(P, scene, __ldg(reinterpret_cast<const uint32_t*>(hits + ri)));
             if (target < 0 || target >= kClasses) target = kMissClass;
         }
+        *reinterpret_cast<uint4*>(sX + kmajor_offset(row, 8 * q, 32)) = e;
+        {
+            const __half* hv = reinterpret_cast<const __half*>(&e);
 #pragma unroll
-        for (int c = 0; c < 4; ++c) {
-            *reinterpret_cast<uint4*>(sX + kmajor_offset(tid, 8 * c, 32)) = e[c];
-            const __half* hv = reinterpret_cast<const __half*>(&e[c]);
-#pragma unroll
-            for (int j = 0; j < 8; ++j)
-                *reinterpret_cast<__half*>(sXT + kmajor_offset(8 * c + j, tid, 128)) = hv[j];
+            for (int j = 0; j < 8; ++j) *reinterpret_cast<__half*>(sXT + kmajor_offset(8 * q + j, row, 128)) = hv[j];
         }
         sy.before_mma();
 
-        // One pass through the tile; a timed-out MMA wait leaves it (break), and then
-        // the tile loop, to the TMEM release below.
+        // One pass through the tile; a timed-out MMA wait leaves it (break), and
+        // then the tile loop, to the TMEM release below.
         do {
-            // ---- forward
-            if (tid == 0) gemm(tb + 0, sX, sW1, 32, 128, 64);
+            // ---- forward: columns 16q .. 16q+15 of each hidden layer
+            const int c0 = 16 * q;
+            float v[16];
+            if (threadIdx.x == 0) gemm(tb + 0, sX, sW1, 32, 128, 64);
             if (!sy.commit_and_wait()) break;
-            for (int c = 0; c < 64; c += 16) {
-                float v[16];
-                tc::tmem_ld16(lane_addr(tb, c), v);
+            tc::tmem_ld16(lane(c0), v);
 #pragma unroll
-                for (int j = 0; j < 16; ++j) {
-                    v[j] = __half2float(__float2half_rn(fmaxf(v[j] + sB[c + j], 0.f)));
-                    store_h(sH1T, 128, c + j, tid, v[j]);
-                }
-                store_row8(sH1, 64, tid, c, v);
-                store_row8(sH1, 64, tid, c + 8, v + 8);
+            for (int j = 0; j < 16; ++j) {
+                v[j] = __half2float(__float2half_rn(fmaxf(v[j] + sB[c0 + j], 0.f)));
+                store_h(sH1T, 128, c0 + j, row, v[j]);
             }
+            store_row8(sH1, 64, row, c0, v);
+            store_row8(sH1, 64, row, c0 + 8, v + 8);
+            uint32_t on1 = 0, on2 = 0;  // bit j: hidden unit c0 + j is active (its activation as stored is > 0)
+#pragma unroll
+            for (int j = 0; j < 16; ++j) on1 |= (v[j] > 0.f ? 1u : 0u) << j;
             sy.before_mma();
-            if (tid == 0) gemm(tb + 64, sH1, sW2, 64, 128, 64);
+            if (threadIdx.x == 0) gemm(tb + 64, sH1, sW2, 64, 128, 64);
             if (!sy.commit_and_wait()) break;
-            for (int c = 0; c < 64; c += 16) {
-                float v[16];
-                tc::tmem_ld16(lane_addr(tb, 64 + c), v);
+            tc::tmem_ld16(lane(64 + c0), v);
 #pragma unroll
-                for (int j = 0; j < 16; ++j) {
-                    v[j] = __half2float(__float2half_rn(fmaxf(v[j] + sB[64 + c + j], 0.f)));
-                    store_h(sH2T, 128, c + j, tid, v[j]);
-                }
-                store_row8(sH2, 64, tid, c, v);
-                store_row8(sH2, 64, tid, c + 8, v + 8);
+            for (int j = 0; j < 16; ++j) {
+                v[j] = __half2float(__float2half_rn(fmaxf(v[j] + sB[64 + c0 + j], 0.f)));
+                store_h(sH2T, 128, c0 + j, row, v[j]);
             }
+            store_row8(sH2, 64, row, c0, v);
+            store_row8(sH2, 64, row, c0 + 8, v + 8);
+#pragma unroll
+            for (int j = 0; j < 16; ++j) on2 |= (v[j] > 0.f ? 1u : 0u) << j;
             sy.before_mma();
-            if (tid == 0) gemm(tb + 128, sH2, sW3, 64, 128, 128);
+            if (threadIdx.x == 0) gemm(tb + 128, sH2, sW3, 64, 128, 128);
             if (!sy.commit_and_wait()) break;
 
-            // ---- softmax cross-entropy: G3 = p - onehot(target)
-            float mx = -INFINITY;
-            for (int c = 0; c < 128; c += 16) {
-                float v[16];
-                tc::tmem_ld16(lane_addr(tb, 128 + c), v);
+            // ---- softmax cross-entropy: G3 = p - onehot(target), columns 32q .. 32q+31
+            {
+                const int l0 = 32 * q;
+                float l[32];
+                tc::tmem_ld16(lane(128 + l0), l);
+                tc::tmem_ld16(lane(128 + l0 + 16), l + 16);
+                float mx = -INFINITY;
 #pragma unroll
-                for (int j = 0; j < 16; ++j) mx = fmaxf(mx, v[j] + sB[128 + c + j]);
-            }
-            float sum = 0.f;
-            for (int c = 0; c < 128; c += 16) {
-                float v[16];
-                tc::tmem_ld16(lane_addr(tb, 128 + c), v);
-#pragma unroll
-                for (int j = 0; j < 16; ++j) sum += __expf(v[j] + sB[128 + c + j] - mx);
-            }
-            const float inv = 1.f / sum;
-            for (int c = 0; c < 128; c += 16) {
-                float v[16];
-                tc::tmem_ld16(lane_addr(tb, 128 + c), v);
-#pragma unroll
-                for (int j = 0; j < 16; ++j) {
-                    const float l = v[j] + sB[128 + c + j];
-                    const float p = __expf(l - mx) * inv;
-                    float g = p - ((c + j) == target ? 1.f : 0.f);
-                    if (!valid) g = 0.f;
-                    if (valid && (c + j) == target) loss -= l - mx - __logf(sum);
-                    v[j] = __half2float(__float2half_rn(g));
-                    store_h(sG3T, 128, c + j, tid, v[j]);
+                for (int j = 0; j < 32; ++j) {
+                    l[j] += sB[128 + l0 + j];
+                    mx = fmaxf(mx, l[j]);
                 }
-                store_row8(sG3, 128, tid, c, v);
-                store_row8(sG3, 128, tid, c + 8, v + 8);
+                sRed[q * 128 + row] = mx;
+                __syncthreads();
+                mx = fmaxf(fmaxf(sRed[row], sRed[128 + row]), fmaxf(sRed[256 + row], sRed[384 + row]));
+                float sum = 0.f;
+#pragma unroll
+                for (int j = 0; j < 32; ++j) {
+                    if (valid && l0 + j == target) loss -= l[j] - mx;
+                    l[j] = __expf(l[j] - mx);
+                    sum += l[j];
+                }
+                sRed[512 + q * 128 + row] = sum;
+                __syncthreads();
+                sum = (sRed[512 + row] + sRed[640 + row]) + (sRed[768 + row] + sRed[896 + row]);
+                if (valid && q == 0) loss += __logf(sum);
+                const float inv = 1.f / sum;
+#pragma unroll
+                for (int j = 0; j < 32; ++j) {
+                    float g = l[j] * inv - (l0 + j == target ? 1.f : 0.f);
+                    if (!valid) g = 0.f;
+                    l[j] = __half2float(__float2half_rn(g));
+                    store_h(sG3T, 128, l0 + j, row, l[j]);
+                }
+#pragma unroll
+                for (int j = 0; j < 32; j += 8) store_row8(sG3, 128, row, l0 + j, l + j);
             }
-            // ---- dW3 = G3^T H2 and dH2 = G3 W3
+            // ---- dW3 += G3^T H2 and dH2 = G3 W3
             sy.before_mma();
-            if (tid == 0) {
-                gemm(cW3, sG3T, sH2T, 128, 128, 64, !first);
+            if (threadIdx.x == 0) {
+                gemm(tb + cW3, sG3T, sH2T, 128, 128, 64, !first);
                 gemm(tb + 64, sG3, sW3T, 128, 128, 64);
             }
             if (!sy.commit_and_wait()) break;
-            db3 += row_sum128(sG3T, tid);  // sum over samples of G3[:, tid]
-            float dh[64];
-            for (int c = 0; c < 64; c += 16) tc::tmem_ld16(lane_addr(tb, 64 + c), dh + c);
+            db3 += row_sum32(sG3T, row, 32 * q);  // G3[:, row] over samples 32q .. 32q+31
+            tc::tmem_ld16(lane(64 + c0), v);
             tc::fence_before_sync();
             __syncthreads();  // G3 / G3T fully consumed
             zero_bytes(sGT + 64 * 128 * 2, 64 * 128 * 2);  // padding rows 64..127 of G2T
 #pragma unroll
-            for (int j = 0; j < 64; ++j) {
-                dh[j] = (load_h(sH2, 64, tid, j) > 0.f) ? __half2float(__float2half_rn(dh[j])) : 0.f;
-                store_h(sGT, 128, j, tid, dh[j]);
+            for (int j = 0; j < 16; ++j) {
+                v[j] = (on2 >> j & 1u) ? __half2float(__float2half_rn(v[j])) : 0.f;
+                store_h(sGT, 128, c0 + j, row, v[j]);
             }
-            for (int c = 0; c < 64; c += 8) store_row8(sG, 64, tid, c, dh + c);
-            // ---- dW2 = G2^T H1 and dH1 = G2 W2
+            store_row8(sG, 64, row, c0, v);
+            store_row8(sG, 64, row, c0 + 8, v + 8);
+            // ---- dW2 += G2^T H1 and dH1 = G2 W2
             sy.before_mma();
-            if (tid == 0) {
-                gemm(cW2, sGT, sH1T, 128, 128, 64, !first);
+            if (threadIdx.x == 0) {
+                gemm(tb + cW2, sGT, sH1T, 128, 128, 64, !first);
                 gemm(tb + 192, sG, sW2T, 64, 128, 64);
             }
             if (!sy.commit_and_wait()) break;
-            if (tid < 64) db2 += row_sum128(sGT, tid);
-            for (int c = 0; c < 64; c += 16) tc::tmem_ld16(lane_addr(tb, 192 + c), dh + c);
+            if (row < 64) db2 += row_sum32(sGT, row, 32 * q);
+            tc::tmem_ld16(lane(192 + c0), v);
             tc::fence_before_sync();
             __syncthreads();
-            zero_bytes(sGT + 64 * 128 * 2, 64 * 128 * 2);
 #pragma unroll
-            for (int j = 0; j < 64; ++j) {
-                dh[j] = (load_h(sH1, 64, tid, j) > 0.f) ? __half2float(__float2half_rn(dh[j])) : 0.f;
-                store_h(sGT, 128, j, tid, dh[j]);
+            for (int j = 0; j < 16; ++j) {
+                v[j] = (on1 >> j & 1u) ? __half2float(__float2half_rn(v[j])) : 0.f;
+                store_h(sGT, 128, c0 + j, row, v[j]);
             }
-            for (int c = 0; c < 64; c += 8) store_row8(sG, 64, tid, c, dh + c);
-            // ---- dW1 = G1^T X and dX = G1 W1
+            store_row8(sG, 64, row, c0, v);
+            store_row8(sG, 64, row, c0 + 8, v + 8);
+            // ---- dW1 += G1^T X and dX = G1 W1
             sy.before_mma();
-            if (tid == 0) {
-                gemm(cW1, sGT, sXT, 128, 128, 32, !first);
+            if (threadIdx.x == 0) {
+                gemm(tb + cW1, sGT, sXT, 128, 128, 32, !first);
                 gemm(tb + 32, sG, sW1T, 64, 128, 32);
             }
             if (!sy.commit_and_wait()) break;
-            if (tid < 64) db1 += row_sum128(sGT, tid);
-            for (int c = 0; c < 32; c += 16) {
-                float v[16];
-                tc::tmem_ld16(lane_addr(tb, 32 + c), v);
+            if (row < 64) db1 += row_sum32(sGT, row, 32 * q);
+            if (q < 2) {
+                tc::tmem_ld16(lane(32 + 16 * q), v);
                 if (valid) {
-                    float* dst = c == 0 ? grad + oEo + static_cast<size_t>(cell) * kEmb : grad + oEd + static_cast<size_t>(bin) * kEmb;
+                    float* dst = q == 0 ? grad + oEo + static_cast<size_t>(cell) * kEmb
+                                        : grad + oEd + static_cast<size_t>(bin) * kEmb;
 #pragma unroll
                     for (int j = 0; j < 16; j += 4) red_add4(dst + j, v + j);
                 }
@@ -647,30 +657,29 @@ __global__ void __launch_bounds__(128) train_kernel(PredictorDev P, const crt_bv
         __syncthreads();
     }
     if (ok && !first) {
-        for (int c = 0; c < 64; c += 16) {
-            float v[16];
-            tc::tmem_ld16(lane_addr(cW3, c), v);
+        float v[16];
+        tc::tmem_ld16(lane(cW3 + 16 * q), v);
 #pragma unroll
-            for (int j = 0; j < 16; j += 4) red_add4(grad + oW3 + tid * 64 + c + j, v + j);
-            tc::tmem_ld16(lane_addr(cW2, c), v);
-            if (tid < 64) {
+        for (int j = 0; j < 16; j += 4) red_add4(grad + oW3 + row * 64 + 16 * q + j, v + j);
+        tc::tmem_ld16(lane(cW2 + 16 * q), v);
+        if (row < 64) {
 #pragma unroll
-                for (int j = 0; j < 16; j += 4) red_add4(grad + oW2 + tid * 64 + c + j, v + j);
-            }
-            if (c >= 32) continue;
-            tc::tmem_ld16(lane_addr(cW1, c), v);
-            if (tid < 64) {
+            for (int j = 0; j < 16; j += 4) red_add4(grad + oW2 + row * 64 + 16 * q + j, v + j);
+        }
+        if (q < 2) {
+            tc::tmem_ld16(lane(cW1 + 16 * q), v);
+            if (row < 64) {
 #pragma unroll
-                for (int j = 0; j < 16; j += 4) red_add4(grad + oW1 + tid * 32 + c + j, v + j);
+                for (int j = 0; j < 16; j += 4) red_add4(grad + oW1 + row * 32 + 16 * q + j, v + j);
             }
         }
-        atomicAdd(grad + oB3 + tid, db3);
-        if (tid < 64) {
-            atomicAdd(grad + oB2 + tid, db2);
-            atomicAdd(grad + oB1 + tid, db1);
+        atomicAdd(grad + oB3 + row, db3);
+        if (row < 64) {
+            atomicAdd(grad + oB2 + row, db2);
+            atomicAdd(grad + oB1 + row, db1);
         }
         for (int m = 16; m > 0; m >>= 1) loss += __shfl_xor_sync(0xFFFFFFFFu, loss, m);
-        if ((tid & 31) == 0) atomicAdd(loss_sum, loss);
+        if ((threadIdx.x & 31) == 0) atomicAdd(loss_sum, loss);
     }
     tc::fence_before_sync();
     __syncthreads();
@@ -1147,7 +1156,7 @@ cudaError_t pred_train_step(const PredictorDev& P, const crt_bvh_node* nodes, co
     const uint32_t tiles = (n_samples + 127) / 128;
     if (tiles == 0) return cudaSuccess;
     const uint32_t grid = tiles < static_cast<uint32_t>(kNumSms) ? tiles : static_cast<uint32_t>(kNumSms);
-    pred::train_kernel<<<grid, 128, pred::kTrainSmem, s>>>(P, nodes, rays, n_rays, hits, targets, n_samples, stride,
+    pred::train_kernel<<<grid, pred::kTrainThreads, pred::kTrainSmem, s>>>(P, nodes, rays, n_rays, hits, targets, n_samples, stride,
                                                           offset, P.grad, loss_sum, err);
     return cudaGetLastError();
 }
