@@ -501,6 +501,7 @@ class Context:
         _check(lib().crt_create(C.byref(h), C.byref(cfg)))
         self.handle = h
         self.device = device
+        self._stream = self.stream
         self._ext = None
 
     def _after_torch(self):
@@ -509,14 +510,13 @@ class Context:
         the library reads them (an event wait on the GPU, no host sync).  The
         library's calls return with their outputs complete."""
         t = sys.modules.get("torch")
-        if t is None or not t.cuda.is_available() or not t.cuda.is_initialized():
+        if t is None or not t.cuda.is_initialized():
             return
-        dev = t.device("cuda", self.device)
-        cur = t.cuda.current_stream(dev)
-        if cur.cuda_stream == self.stream:
+        cur = t.cuda.current_stream(self.device)
+        if cur.cuda_stream == self._stream or cur.query():  # the library's own, or nothing queued
             return
         if self._ext is None:
-            self._ext = t.cuda.ExternalStream(self.stream, device=dev)
+            self._ext = t.cuda.ExternalStream(self._stream, device=t.device("cuda", self.device))
         self._ext.wait_stream(cur)
 
     def close(self):

@@ -8,6 +8,7 @@
 #include <cstdio>
 #include <cstring>
 #include <cuda_runtime.h>
+#include <functional>
 #include <vector>
 
 #include "crt.h"
@@ -199,6 +200,16 @@ struct crt_ctx {
     DevBuf step_in, step_out;                      // crt_radix_digit_counts / _offsets
     DevBuf opt_scratch;                            // crt_optimize
     uint64_t last_trace_stats[2] = {0, 0};
+    // Page-locked words the GPU writes directly: [0..3] error word of the calls
+    // that only raise errors (traces, frames, shading, refit, predictor), so that
+    // they neither clear nor copy one; [4] rays the last persistent trace left over.
+    uint32_t* hw = nullptr;
+    uint32_t* hw_dev = nullptr;
+    DevBuf walk_ctr;  // persistent walks' counters (zero between launches)
+    // The launch of the rays that the last persistent walk left over, until its
+    // number is known (finish_walk).
+    std::function<void(uint32_t)> left_over;
+    bool err_dirty = true;  // the device error word may hold something
     // pinned host staging
     void* pinned = nullptr;
     size_t pinned_cap = 0;
@@ -224,10 +235,33 @@ struct crt_ctx {
         pinned_cap = bytes;
         return CRT_OK;
     }
+    // Host-visible error word: nothing of this context runs between its calls, so
+    // the host clears it.  It also follows a failed call's kernels here.
+    crt_status begin_host_error() {
+        if (hw[0] == 0u) return CRT_OK;
+        CRT_CUDA(cudaStreamSynchronize(stream));
+        for (int k = 0; k < 4; ++k) hw[k] = 0u;
+        return CRT_OK;
+    }
+    crt_status check_host_error() {
+        CRT_CUDA(cudaStreamSynchronize(stream));
+        const uint32_t ew[4] = {hw[0], hw[1], hw[2], hw[3]};
+        for (int k = 0; k < 4; ++k) hw[k] = 0u;
+        return describe_error(ew);
+    }
+    crt_status begin_device_error() {
+        if (err_dirty) CRT_CUDA(cudaMemsetAsync(err.p, 0, 16, stream));
+        err_dirty = true;
+        return CRT_OK;
+    }
     crt_status check_device_error() {
-        uint32_t ew[4] = {0, 0, 0, 0};
+        uint32_t* ew = static_cast<uint32_t*>(pinned) + pinned_cap / 4 - 4;
         CRT_CUDA(cudaMemcpyAsync(ew, err.p, 16, cudaMemcpyDeviceToHost, stream));
         CRT_CUDA(cudaStreamSynchronize(stream));
+        err_dirty = ew[0] != 0u;
+        return describe_error(ew);
+    }
+    static crt_status describe_error(const uint32_t* ew) {
         const uint32_t e = ew[0];
         if (e & crt::kDevTimeout) return fail(CRT_ERR_DEVICE_TIMEOUT, "a bounded device wait gave up (err=0x%x)", e);
         if (e & crt::kDevBadModel) return fail(CRT_ERR_BAD_INPUT, "a triangle references model id >= 64");
@@ -302,6 +336,12 @@ crt_status crt_create(crt_ctx** out, const crt_config* cfg) {
     if (s == CRT_OK) s = x->cam.reserve(sizeof(crt_camera));
     if (s == CRT_OK) s = x->trace_stats.reserve(16);
     if (s == CRT_OK) s = x->pinned_reserve(1 << 16);
+    if (s == CRT_OK) s = x->walk_ctr.reserve(16);
+    if (s == CRT_OK && (cudaMemset(x->walk_ctr.p, 0, 16) != cudaSuccess ||
+                        cudaHostAlloc(reinterpret_cast<void**>(&x->hw), 64, cudaHostAllocMapped) != cudaSuccess ||
+                        cudaHostGetDevicePointer(reinterpret_cast<void**>(&x->hw_dev), x->hw, 0) != cudaSuccess))
+        s = fail(CRT_ERR_CUDA, "host-visible words");
+    if (s == CRT_OK) std::memset(x->hw, 0, 64);
     if (s == CRT_OK) {
         crt::SceneState init{};
         for (int a = 0; a < 3; ++a) { init.key_max[a] = 0ull; init.key_min[a] = ~0ull; }
@@ -327,8 +367,9 @@ crt_status crt_destroy(crt_ctx* x) {
                       &x->ray_order, &x->ray_order_scratch, &x->shade_models, &x->shade_materials,
                       &x->shade_rays, &x->shade_hits, &x->image, &x->refit_state, &x->xtri_sorted,
                       &x->mesh_vertices, &x->mesh_indices, &x->mesh_out, &x->probe_flag, &x->step_in,
-                      &x->step_out};
+                      &x->step_out, &x->walk_ctr};
     for (DevBuf* b : bufs) b->release();
+    if (x->hw) cudaFreeHost(x->hw);
     for (auto& e : x->ev)
         if (e) cudaEventDestroy(e);
     for (auto& e : x->tev)
@@ -349,7 +390,7 @@ crt_status crt_selftest_wait(crt_ctx* x, int set_flag, uint32_t spin_limit) {
     if (!x) return fail(CRT_ERR_INVALID_ARG, "null context");
     CRT_CUDA(cudaSetDevice(x->device));
     CRT_TRY(x->probe_flag.reserve(4));
-    CRT_CUDA(cudaMemsetAsync(x->err.p, 0, 16, x->stream));
+    CRT_TRY(x->begin_device_error());
     CRT_CUDA(cudaMemsetAsync(x->probe_flag.p, set_flag ? 0xFF : 0, 4, x->stream));
     crt::launch_wait_probe(x->probe_flag.as<unsigned int>(), spin_limit ? spin_limit : x->cfg.spin_limit,
                            x->err.as<uint32_t>(), x->stream);
@@ -361,7 +402,7 @@ crt_status crt_selftest_tc_wait(crt_ctx* x, int complete, uint32_t spin_limit) {
     if (!x) return fail(CRT_ERR_INVALID_ARG, "null context");
     CRT_CUDA(cudaSetDevice(x->device));
     CRT_TRY(x->probe_flag.reserve(128 * sizeof(float)));
-    CRT_CUDA(cudaMemsetAsync(x->err.p, 0, 16, x->stream));
+    CRT_TRY(x->begin_device_error());
     CRT_CUDA(cudaMemsetAsync(x->probe_flag.p, 0, 128 * sizeof(float), x->stream));
     CRT_CUDA(crt::tc_wait_probe(complete, spin_limit, x->err.as<uint32_t>(), x->probe_flag.as<float>(), x->stream));
     const crt_status st = x->check_device_error();
@@ -446,18 +487,14 @@ namespace {
 crt_status stage_model_matrices(crt_ctx* x, const crt_mesh_model* models, uint32_t n_models) {
     float* hm = static_cast<float*>(x->pinned);
     CRT_CUDA(cudaStreamSynchronize(x->stream));  // the pinned staging area may still feed an earlier copy
-    const bool dev = n_models > 0 && is_device_ptr(models);
+    crt_mesh_model from_device[64];
+    if (n_models > 0 && is_device_ptr(models)) {
+        CRT_CUDA(cudaMemcpy(from_device, models, sizeof(crt_mesh_model) * n_models, cudaMemcpyDeviceToHost));
+        models = from_device;
+    }
     for (uint32_t m = 0; m < 64; ++m) {
         for (int k = 0; k < 16; ++k) hm[16 * m + k] = (k % 5 == 0) ? 1.f : 0.f;
-        if (m < n_models) {
-            crt_mesh_model mm;
-            if (dev) {
-                CRT_CUDA(cudaMemcpy(&mm, models + m, sizeof(mm), cudaMemcpyDeviceToHost));
-            } else {
-                std::memcpy(&mm, models + m, sizeof(mm));
-            }
-            std::memcpy(hm + 16 * m, mm.m, 64);
-        }
+        if (m < n_models) std::memcpy(hm + 16 * m, reinterpret_cast<const char*>(models + m), 64);
     }
     const volatile float third = 1.f / 3.f;
     for (int k = 0; k < 64 * 16; ++k) hm[64 * 16 + k] = third * hm[k];
@@ -528,7 +565,7 @@ crt_status build_impl(crt_ctx* x, crt_bvh* b, const crt_triangle* tris, uint32_t
     const float* d_models = x->models.as<float>();
     const float* d_models3 = d_models + 64 * 16;
 
-    CRT_CUDA(cudaMemsetAsync(x->err.p, 0, 16, s));
+    CRT_TRY(x->begin_device_error());
     CRT_CUDA(cudaMemsetAsync(x->hist.p, 0, 4 * hist_words, s));
     CRT_CUDA(cudaMemsetAsync(x->sort_lb.p, 0, 4 * sort_lb_words, s));
     CRT_CUDA(cudaMemsetAsync(x->ploc_lb.p, 0, 8ull * (2ull * ploc_tiles) + 64, s));
@@ -570,6 +607,9 @@ crt_status build_impl(crt_ctx* x, crt_bvh* b, const crt_triangle* tris, uint32_t
     uint32_t iters = 0;
     bool laid_out = false;
     float layout_in_kernel_ms = 0.f;  // the persistent launch's layout phase, from its timer stamps
+    // read back in page-locked memory, past the model matrices that may still be on their way
+    uint32_t* h_tail = static_cast<uint32_t*>(x->pinned) + 2 * 64 * 16;
+    crt::SceneState* h_state = reinterpret_cast<crt::SceneState*>(h_tail + 16);
     if (N > 1 && !x->force_multi_launch) {
         // one cooperative launch: every PLOC iteration, then the DFS layout
         unsigned long long* lb = x->ploc_lb.as<unsigned long long>();
@@ -582,14 +622,8 @@ crt_status build_impl(crt_ctx* x, crt_bvh* b, const crt_triangle* tris, uint32_t
             err, x->cfg.spin_limit, s);
         if (e == cudaSuccess) {
             CRT_CUDA(cudaEventRecord(x->ev[3], s));
-            uint32_t* hp = static_cast<uint32_t*>(x->pinned);
-            CRT_CUDA(cudaMemcpyAsync(hp, tail + 4, 32, cudaMemcpyDeviceToHost, s));
-            CRT_CUDA(cudaStreamSynchronize(s));
-            iters = hp[0];
-            unsigned long long stamp[3];
-            std::memcpy(stamp, hp + 2, sizeof(stamp));
-            if (stamp[2] > stamp[1]) layout_in_kernel_ms = static_cast<float>(static_cast<double>(stamp[2] - stamp[1]) * 1e-6);
-            laid_out = true;
+            CRT_CUDA(cudaMemcpyAsync(h_tail, tail + 4, 32, cudaMemcpyDeviceToHost, s));
+            laid_out = true;  // its iteration count and stamps are read at the end
         } else if (e != cudaErrorNotSupported && e != cudaErrorCooperativeLaunchTooLarge) {
             return fail(CRT_ERR_CUDA, "PLOC launch failed: %s", cudaGetErrorString(e));
         } else {
@@ -660,10 +694,15 @@ crt_status build_impl(crt_ctx* x, crt_bvh* b, const crt_triangle* tris, uint32_t
     }
     CRT_CUDA(cudaGetLastError());
     CRT_CUDA(cudaEventRecord(x->ev[4], s));
-    CRT_TRY(x->check_device_error());
-
-    crt::SceneState hs;
-    CRT_CUDA(cudaMemcpy(&hs, st, sizeof(hs), cudaMemcpyDeviceToHost));
+    CRT_CUDA(cudaMemcpyAsync(h_state, st, sizeof(crt::SceneState), cudaMemcpyDeviceToHost, s));
+    CRT_TRY(x->check_device_error());  // the build's one wait
+    const crt::SceneState hs = *h_state;
+    if (laid_out) {
+        iters = h_tail[0];
+        unsigned long long stamp[3];
+        std::memcpy(stamp, h_tail + 2, sizeof(stamp));
+        if (stamp[2] > stamp[1]) layout_in_kernel_ms = static_cast<float>(static_cast<double>(stamp[2] - stamp[1]) * 1e-6);
+    }
     float ms[4];
     for (int k = 0; k < 4; ++k) CRT_CUDA(cudaEventElapsedTime(&ms[k], x->ev[k], x->ev[k + 1]));
     x->stats.n_tris = N;
@@ -725,6 +764,31 @@ crt_status ensure_cwide(crt_ctx* x, const crt_bvh* b) {
     return CRT_OK;
 }
 
+// Scratch of a persistent walk of n rays: the list of left-over rays lies in
+// build scratch, idle between builds.
+crt_status walk_scratch(crt_ctx* x, uint32_t n, bool wait, crt::WalkScratch* w) {
+    CRT_TRY(x->node_box.reserve(4ull * n));
+    w->ctr = x->walk_ctr.as<uint32_t>();
+    w->left = x->node_box.as<uint32_t>();
+    w->host_left = wait ? x->hw_dev + 4 : nullptr;
+    return CRT_OK;
+}
+
+// Waits for a persistent walk issued with host_left and launches the rays it
+// left over.
+crt_status finish_walk(crt_ctx* x) {
+    if (!x->left_over) return CRT_OK;
+    auto launch = std::move(x->left_over);
+    x->left_over = nullptr;
+    CRT_CUDA(cudaStreamSynchronize(x->stream));
+    const uint32_t n = reinterpret_cast<volatile uint32_t*>(x->hw)[4];
+    if (n != 0) {
+        launch(n);
+        CRT_CUDA(cudaGetLastError());
+    }
+    return CRT_OK;
+}
+
 // One-launch frames walk the compressed nodes once the frames of the current
 // tree have a quarter as many pixels as it has triangles: deriving the nodes
 // takes 0.035 ns per triangle (73 us at 2.0 M) and a pixel gains 0.05-0.2 ns.
@@ -732,10 +796,25 @@ crt_status frame_walk4(crt_ctx* x, const crt_bvh* b, uint32_t pixels, crt::Trace
     b->frame_pixels += pixels;
     if (b->n < 2 || (!b->cwide_ready && 4 * b->frame_pixels < b->n)) return CRT_OK;
     CRT_TRY(ensure_cwide(x, b));
-    CRT_TRY(x->node_box.reserve(crt::trace_pool_bytes(pixels)));  // build scratch, idle between builds
     p->cwide = b->cwide.as<uint4>();
     p->cw_bad = b->cw_bad();
     return CRT_OK;
+}
+
+// A one-launch frame, and the pixels it leaves to the binary walk.
+crt_status frame_launch(crt_ctx* x, const crt::TraceParams& p, const crt_camera* cam, uint32_t width, uint32_t height,
+                        const float* light, crt_hit* hits_shadow, uint32_t flags, const crt::ShadeParams* sp) {
+    crt::WalkScratch ws;
+    if (p.cwide) CRT_TRY(walk_scratch(x, p.n_rays, true, &ws));
+    auto launch = [&](uint32_t left) {
+        crt::launch_frame(p, cam, width, height, 0, height, light, hits_shadow, flags,
+                          static_cast<int>(x->cfg.trace_block), sp, ws, left, x->stream);
+    };
+    launch(0);
+    CRT_CUDA(cudaGetLastError());
+    if (!p.cwide) return CRT_OK;
+    x->left_over = launch;
+    return finish_walk(x);
 }
 
 // Enqueues one traversal launch on device-resident rays/hits (no sync).
@@ -746,9 +825,10 @@ constexpr uint32_t kChunkedCopyMinRays = 1u << 20;  // crt_trace: smaller host b
 // classes_ready: the predictor's classes of these rays are already in its
 // class buffer, and with CRT_TRACE_PREDICTOR_ORDER their order keys in its
 // order scratch (crt_trace's chunked copy ran the inference per chunk).
+// wait: the caller calls finish_walk before it uses the hits.
 crt_status trace_device(crt_ctx* x, const crt_bvh* b, const crt_ray* d_rays, uint32_t n_rays, uint32_t flags,
                         crt_hit* d_hits, const uint16_t* seed_classes = nullptr, uint32_t tile_width = 0,
-                        bool classes_ready = false) {
+                        bool classes_ready = false, bool wait = false) {
     if (n_rays == 0) return CRT_OK;
     if (flags & CRT_TRACE_WIDE) CRT_TRY(ensure_wide4(x, b));
     // Large batches over one scene: persistent warps over the compressed nodes;
@@ -772,7 +852,7 @@ crt_status trace_device(crt_ctx* x, const crt_bvh* b, const crt_ray* d_rays, uin
     p.n_rays = n_rays;
     p.n_nodes = 2 * b->n - 1;
     p.abs_eps = b->abs_eps;
-    p.err = x->err.as<uint32_t>();
+    p.err = x->hw_dev;
     p.stats = nullptr;
     p.tile_width = tile_width;
     if (flags & CRT_TRACE_STATS) {
@@ -797,7 +877,7 @@ crt_status trace_device(crt_ctx* x, const crt_bvh* b, const crt_ray* d_rays, uin
             uint32_t *okeys = nullptr, *ohist = nullptr;
             if (fuse) crt::pred_order_begin(pr->order_scratch.p, n_rays, &okeys, &ohist, x->stream);
             CRT_CUDA(crt::pred_infer(pr->dev(), b->nodes.as<crt_bvh_node>(), d_rays, n_rays, pr->classes.as<uint16_t>(),
-                                     pr->cfg.miss_threshold, !(flags & CRT_TRACE_USE_PREDICTOR), x->err.as<uint32_t>(),
+                                     pr->cfg.miss_threshold, !(flags & CRT_TRACE_USE_PREDICTOR), x->hw_dev,
                                      x->stream, okeys, ohist));
         }
         if (flags & CRT_TRACE_USE_PREDICTOR) {
@@ -807,7 +887,7 @@ crt_status trace_device(crt_ctx* x, const crt_bvh* b, const crt_ray* d_rays, uin
         }
         if (flags & CRT_TRACE_PREDICTOR_ORDER) {  // includes the coherence order of CRT_TRACE_SORT_RAYS
             crt::pred_order(pr->dev(), b->nodes.as<crt_bvh_node>(), d_rays, pr->classes.as<uint16_t>(), n_rays,
-                            pr->order.as<uint32_t>(), pr->order_scratch.p, x->err.as<uint32_t>(), x->cfg.spin_limit,
+                            pr->order.as<uint32_t>(), pr->order_scratch.p, x->hw_dev, x->cfg.spin_limit,
                             x->stream, fuse);
             CRT_CUDA(cudaGetLastError());
             p.order = pr->order.as<uint32_t>();
@@ -817,7 +897,7 @@ crt_status trace_device(crt_ctx* x, const crt_bvh* b, const crt_ray* d_rays, uin
         CRT_TRY(x->ray_order.reserve(4ull * n_rays));
         CRT_TRY(x->ray_order_scratch.reserve(crt::ray_order_scratch_bytes(n_rays)));
         crt::launch_ray_order(d_rays, n_rays, b->nodes.as<crt_bvh_node>(), nullptr, 0, x->ray_order.as<uint32_t>(),
-                              x->ray_order_scratch.p, x->err.as<uint32_t>(), x->cfg.spin_limit, x->stream);
+                              x->ray_order_scratch.p, x->hw_dev, x->cfg.spin_limit, x->stream);
         CRT_CUDA(cudaGetLastError());
         p.order = x->ray_order.as<uint32_t>();
     }
@@ -825,13 +905,19 @@ crt_status trace_device(crt_ctx* x, const crt_bvh* b, const crt_ray* d_rays, uin
     const bool deep = (b->depth_bound + 2 > 64) || (3 * ((b->depth_bound + 2) / 2) + 3 > 96);
     const uint32_t launch_flags =
         (flags & (CRT_TRACE_ANY | CRT_TRI_WATERTIGHT | CRT_TRACE_WIDE | CRT_TRACE_COMPRESSED)) | (deep ? (1u << 16) : 0u);
-    if (pool) CRT_TRY(x->node_box.reserve(crt::trace_pool_bytes(n_rays)));  // build scratch, idle between builds
+    crt::WalkScratch ws;
+    if (pool) CRT_TRY(walk_scratch(x, n_rays, wait, &ws));
     CRT_CUDA(cudaEventRecord(x->tev[1], x->stream));
-    if (pool) crt::launch_trace_pool(p, launch_flags, x->node_box.as<uint32_t>(), x->stream);
+    if (pool) crt::launch_trace_pool(p, launch_flags, ws, x->stream);
     else crt::launch_trace(p, launch_flags, static_cast<int>(x->cfg.trace_block), x->stream);
     CRT_CUDA(cudaGetLastError());
     CRT_CUDA(cudaEventRecord(x->tev[2], x->stream));
     x->tev_valid = true;
+    if (ws.host_left)
+        x->left_over = [=](uint32_t n) {
+            crt::launch_trace_left(p, launch_flags, ws, n, x->stream);
+            cudaEventRecord(x->tev[2], x->stream);
+        };
     return CRT_OK;
 }
 
@@ -862,6 +948,7 @@ crt_status crt_rebuild(crt_ctx* x, crt_bvh* b, const crt_triangle* tris, uint32_
 // Brings the node array's boxes up to date after a refit (on x's stream).
 static crt_status ensure_node_boxes(crt_ctx* x, const crt_bvh* b) {
     if (!b->node_boxes_stale) return CRT_OK;
+    x->err_dirty = true;
     crt::launch_refit_nodes(b->wide.as<float4>(), b->refit_dfs.as<uint32_t>(), b->n,
                             const_cast<crt_bvh_node*>(b->nodes.as<crt_bvh_node>()), x->err.as<uint32_t>(), x->stream);
     CRT_CUDA(cudaGetLastError());
@@ -889,7 +976,7 @@ crt_status crt_refit(crt_ctx* x, crt_bvh* b, const crt_triangle* tris, uint32_t 
     }
     CRT_TRY(stage_model_matrices(x, models, n_models));
     CRT_TRY(x->refit_state.reserve(sizeof(crt::RefitState)));
-    CRT_CUDA(cudaMemsetAsync(x->err.p, 0, 16, s));
+    CRT_TRY(x->begin_host_error());
     if (!b->refit_ready) {
         const size_t n_int = std::max<size_t>(N - 1, 1);
         CRT_TRY(b->refit_leaf.reserve(16ull * N));
@@ -899,7 +986,7 @@ crt_status crt_refit(crt_ctx* x, crt_bvh* b, const crt_triangle* tris, uint32_t 
         // the counters' buffer holds the per-block counts of the topology pass first
         crt::launch_refit_topology(b->nodes.as<crt_bvh_node>(), b->wide.as<float4>(), N, b->refit_leaf.as<uint4>(),
                                    b->refit_link.as<uint4>(), b->refit_dfs.as<uint32_t>(), b->refit_cnt.as<uint32_t>(),
-                                   x->err.as<uint32_t>(), s);
+                                   x->hw_dev, s);
         CRT_CUDA(cudaGetLastError());
         b->refit_ready = true;
     }
@@ -907,7 +994,7 @@ crt_status crt_refit(crt_ctx* x, crt_bvh* b, const crt_triangle* tris, uint32_t 
     crt::launch_refit(d_tris, N, x->models.as<float>(), b->refit_leaf.as<uint4>(), b->refit_link.as<uint4>(),
                       b->refit_cnt.as<uint32_t>(), b->nodes.as<crt_bvh_node>(), b->xtri.as<float4>(),
                       b->wide.as<float4>(), b->wide_wt.as<float4>(), x->refit_state.as<crt::RefitState>(),
-                      x->err.as<uint32_t>(), s);
+                      x->hw_dev, s);
     CRT_CUDA(cudaGetLastError());
     float* h_eps = static_cast<float*>(x->pinned);
     CRT_CUDA(cudaMemcpyAsync(h_eps, &x->refit_state.as<crt::RefitState>()->abs_eps, sizeof(float),
@@ -916,7 +1003,7 @@ crt_status crt_refit(crt_ctx* x, crt_bvh* b, const crt_triangle* tris, uint32_t 
     b->cwide_ready = false;
     b->frame_pixels = 0;
     b->node_boxes_stale = N > 1;
-    const crt_status st = x->check_device_error();
+    const crt_status st = x->check_host_error();
     if (st != CRT_OK) {
         b->refit_ready = false;  // derive the topology again next time
         return st;
@@ -1086,7 +1173,7 @@ crt_status crt_bvh_from_nodes(crt_ctx* x, const crt_bvh_node* nodes, uint32_t n_
     // the traversal slack of the root box, as a refit derives it
     const float smin[3] = {h[0].mn[0], h[0].mn[1], h[0].mn[2]}, smax[3] = {h[0].mx[0], h[0].mx[1], h[0].mx[2]};
     const float grow = crt::scene_abs_eps(smin, smax);
-    if (cudaMemsetAsync(x->err.p, 0, 16, s) != cudaSuccess) return fail_free(fail(CRT_ERR_CUDA, "crt_bvh_from_nodes: memset"));
+    if ((st = x->begin_device_error()) != CRT_OK) return fail_free(st);
     crt::launch_import(b->nodes.as<crt_bvh_node>(), N, reinterpret_cast<const uint32_t*>(base),
                        reinterpret_cast<const uint32_t*>(base + o_int), reinterpret_cast<const uint2*>(base + o_lc),
                        reinterpret_cast<const uint32_t*>(base + o_leaf), d_tris, x->models.as<float>(), grow,
@@ -1136,7 +1223,7 @@ crt_status crt_optimize(crt_ctx* x, crt_bvh* b, uint32_t passes) {
     v.karea = reinterpret_cast<float2*>(base + o_karea);
     v.cnt = reinterpret_cast<uint32_t*>(base + o_cnt);
     v.N = N;
-    CRT_CUDA(cudaMemsetAsync(x->err.p, 0, 16, s));
+    CRT_TRY(x->begin_device_error());
     crt::launch_opt_init(b->wide.as<float4>(), b->xtri.as<float4>(), v, err, s);
     for (uint32_t k = 0; k < passes; ++k) crt::launch_opt_pass(v, true, err, s);
     if (passes == 0) crt::launch_opt_pass(v, false, err, s);
@@ -1304,7 +1391,7 @@ crt_status crt_trace(crt_ctx* x, const crt_bvh* b, const crt_ray* rays, uint32_t
     if (is_device_ptr(hits)) CRT_TRY(check_aligned16(hits, "crt_trace: hits"));
     const crt_ray* d_rays = rays;
     bool classes_ready = false;
-    CRT_CUDA(cudaMemsetAsync(x->err.p, 0, 16, x->stream));
+    CRT_TRY(x->begin_host_error());
     if (!is_device_ptr(rays)) {
         // Page-locked host rays are read in place by the trace kernel when it
         // reads each ray once, in order; reordered or predicted traces read
@@ -1329,7 +1416,7 @@ crt_status crt_trace(crt_ctx* x, const crt_bvh* b, const crt_ray* rays, uint32_t
             uint32_t *okeys = nullptr, *ohist = nullptr;
             crt::pred_order_begin(pr->order_scratch.p, n_rays, &okeys, &ohist, x->stream);
             CRT_CUDA(crt::pred_infer(pr->dev(), b->nodes.as<crt_bvh_node>(), static_cast<const crt_ray*>(mi), n_rays,
-                                     pr->classes.as<uint16_t>(), pr->cfg.miss_threshold, true, x->err.as<uint32_t>(),
+                                     pr->classes.as<uint16_t>(), pr->cfg.miss_threshold, true, x->hw_dev,
                                      x->stream, okeys, ohist, x->rays_in.as<crt_ray>()));
             d_rays = x->rays_in.as<crt_ray>();
             classes_ready = true;
@@ -1359,7 +1446,7 @@ crt_status crt_trace(crt_ctx* x, const crt_bvh* b, const crt_ray* rays, uint32_t
                 CRT_CUDA(cudaStreamWaitEvent(x->stream, x->copy_ev[c], 0));
                 CRT_CUDA(crt::pred_infer(pr->dev(), b->nodes.as<crt_bvh_node>(), dst + off, cnt,
                                          pr->classes.as<uint16_t>() + off, pr->cfg.miss_threshold, true,
-                                         x->err.as<uint32_t>(), x->stream, okeys + off, ohist));
+                                         x->hw_dev, x->stream, okeys + off, ohist));
             }
             d_rays = dst;
             classes_ready = true;
@@ -1381,9 +1468,10 @@ crt_status crt_trace(crt_ctx* x, const crt_bvh* b, const crt_ray* rays, uint32_t
         CRT_TRY(x->hits_out.reserve(sizeof(crt_hit) * n_rays));
         d_hits = x->hits_out.as<crt_hit>();
     }
-    CRT_TRY(trace_device(x, b, d_rays, n_rays, flags, d_hits, nullptr, 0, classes_ready));
+    CRT_TRY(trace_device(x, b, d_rays, n_rays, flags, d_hits, nullptr, 0, classes_ready, true));
+    CRT_TRY(finish_walk(x));
     if (!dev_out) CRT_CUDA(cudaMemcpyAsync(hits, d_hits, sizeof(crt_hit) * n_rays, cudaMemcpyDeviceToHost, x->stream));
-    CRT_TRY(x->check_device_error());
+    CRT_TRY(x->check_host_error());
     if (flags & CRT_TRACE_STATS)
         CRT_CUDA(cudaMemcpy(x->last_trace_stats, x->trace_stats.p, 16, cudaMemcpyDeviceToHost));
     return CRT_OK;
@@ -1402,9 +1490,9 @@ crt_status crt_trace_seeded(crt_ctx* x, const crt_bvh* b, const crt_ray* rays, u
     CRT_TRY(check_aligned16(hits, "crt_trace_seeded: hits"));
     if (reinterpret_cast<uintptr_t>(classes) & 1u)
         return fail(CRT_ERR_INVALID_ARG, "crt_trace_seeded: classes must be 2-byte aligned");
-    CRT_CUDA(cudaMemsetAsync(x->err.p, 0, 16, x->stream));
+    CRT_TRY(x->begin_host_error());
     CRT_TRY(trace_device(x, b, rays, n_rays, flags & ~CRT_TRACE_USE_PREDICTOR, hits, classes));
-    CRT_TRY(x->check_device_error());
+    CRT_TRY(x->check_host_error());
     if (flags & CRT_TRACE_STATS)
         CRT_CUDA(cudaMemcpy(x->last_trace_stats, x->trace_stats.p, 16, cudaMemcpyDeviceToHost));
     return CRT_OK;
@@ -1458,7 +1546,7 @@ crt_status crt_trace_frame(crt_ctx* x, const crt_bvh* b, const crt_camera* cam, 
     } else {
         CRT_TRY(check_aligned16(cam, "camera"));
     }
-    CRT_CUDA(cudaMemsetAsync(x->err.p, 0, 16, x->stream));
+    CRT_TRY(x->begin_host_error());
     const uint32_t tw = (width % 8 == 0 && height % 4 == 0) ? width : 0u;  // 8x4 pixel tiles per warp
     if (fused) {
         // one launch: camera ray, closest hit, shadow ray, any hit per pixel.
@@ -1487,7 +1575,7 @@ crt_status crt_trace_frame(crt_ctx* x, const crt_bvh* b, const crt_camera* cam, 
         p.n_rays = n;
         p.n_nodes = 2 * b->n - 1;
         p.abs_eps = b->abs_eps;
-        p.err = x->err.as<uint32_t>();
+        p.err = x->hw_dev;
         p.tile_width = tw;
         CRT_TRY(frame_walk4(x, b, n, &p));
         if (flags & CRT_TRACE_STATS) {
@@ -1499,9 +1587,7 @@ crt_status crt_trace_frame(crt_ctx* x, const crt_bvh* b, const crt_camera* cam, 
         // One launch for the whole image.  Splitting it into row bands whose
         // hits are copied out on a second stream while the next band runs was
         // measured slower at every band count (2, 4, 8) on GB300.
-        crt::launch_frame(p, d_cam, width, height, 0, height, light, d_hs, kflags, static_cast<int>(x->cfg.trace_block),
-                          nullptr, x->node_box.as<uint32_t>(), x->stream);
-        CRT_CUDA(cudaGetLastError());
+        CRT_TRY(frame_launch(x, p, d_cam, width, height, light, d_hs, kflags, nullptr));
         if (!dev_p)
             CRT_CUDA(cudaMemcpyAsync(hits_primary, d_hp, sizeof(crt_hit) * static_cast<size_t>(n), cudaMemcpyDeviceToHost,
                                      x->stream));
@@ -1512,7 +1598,7 @@ crt_status crt_trace_frame(crt_ctx* x, const crt_bvh* b, const crt_camera* cam, 
             CRT_CUDA(cudaStreamSynchronize(x->stream));
             CRT_CUDA(cudaMemcpy(x->last_trace_stats, x->trace_stats.p, 16, cudaMemcpyDeviceToHost));
         }
-        return x->check_device_error();
+        return x->check_host_error();
     }
     CRT_TRY(x->frame_rays.reserve(sizeof(crt_ray) * static_cast<size_t>(n)));
     crt_ray* rays = x->frame_rays.as<crt_ray>();
@@ -1532,7 +1618,7 @@ crt_status crt_trace_frame(crt_ctx* x, const crt_bvh* b, const crt_camera* cam, 
         CRT_TRY(trace_device(x, b, sh, n, (flags & ~CRT_TRACE_STATS) | CRT_TRACE_ANY, d_hs, nullptr, tw));
         if (!dev_s) CRT_CUDA(cudaMemcpyAsync(hits_shadow, d_hs, sizeof(crt_hit) * static_cast<size_t>(n), cudaMemcpyDeviceToHost, x->stream));
     }
-    return x->check_device_error();
+    return x->check_host_error();
 }
 
 }  // extern "C"
@@ -1669,21 +1755,21 @@ crt_status crt_predictor_train(crt_ctx* x, crt_predictor* pr, const crt_ray* ray
     CRT_TRY(stage_in(x, pr->hits_in, hits, sizeof(crt_hit) * static_cast<size_t>(n_rays), &d_hits));
     const uint32_t stride = pr->cfg.train_stride;
     const uint32_t total = offset < n_rays ? (n_rays - offset + stride - 1) / stride : 0;
-    CRT_CUDA(cudaMemsetAsync(x->err.p, 0, 16, x->stream));
+    CRT_TRY(x->begin_host_error());
     CRT_CUDA(cudaMemsetAsync(pr->scratch.p, 0, 16, x->stream));
     for (uint32_t done = 0; done < total; done += pr->cfg.batch) {
         const uint32_t nb = std::min(pr->cfg.batch, total - done);
         CRT_CUDA(crt::pred_train_step(pr->dev(), pr->nodes(),
                                       static_cast<const crt_ray*>(d_rays), n_rays, static_cast<const crt_hit*>(d_hits),
                                       nullptr, nb, stride, offset + done * stride, pr->scratch.as<float>(),
-                                      x->err.as<uint32_t>(), x->stream));
+                                      x->hw_dev, x->stream));
         ++pr->step;
         crt::pred_adam(pr->dev(), 1.f / static_cast<float>(nb), pr->cfg.lr, pr->step, x->stream);
         CRT_CUDA(cudaGetLastError());
     }
     float ls = 0.f;
     CRT_CUDA(cudaMemcpyAsync(&ls, pr->scratch.p, 4, cudaMemcpyDeviceToHost, x->stream));
-    CRT_TRY(x->check_device_error());
+    CRT_TRY(x->check_host_error());
     if (loss) *loss = total ? ls / static_cast<float>(total) : 0.f;
     return CRT_OK;
 }
@@ -1702,11 +1788,11 @@ crt_status crt_predictor_infer(crt_ctx* x, crt_predictor* pr, const crt_ray* ray
         CRT_TRY(pr->classes.reserve(2ull * n));
         d_out = pr->classes.as<uint16_t>();
     }
-    CRT_CUDA(cudaMemsetAsync(x->err.p, 0, 16, x->stream));
+    CRT_TRY(x->begin_host_error());
     CRT_CUDA(crt::pred_infer(pr->dev(), pr->nodes(), static_cast<const crt_ray*>(d_rays), n,
-                             d_out, pr->cfg.miss_threshold, false, x->err.as<uint32_t>(), x->stream));
+                             d_out, pr->cfg.miss_threshold, false, x->hw_dev, x->stream));
     if (!dev_out) CRT_CUDA(cudaMemcpyAsync(classes, d_out, 2ull * n, cudaMemcpyDeviceToHost, x->stream));
-    return x->check_device_error();
+    return x->check_host_error();
 }
 
 crt_status crt_predictor_classes_of_hits(crt_ctx* x, crt_predictor* pr, const crt_hit* hits, uint32_t n,
@@ -1742,16 +1828,16 @@ crt_status crt_predictor_gradients(crt_ctx* x, crt_predictor* pr, const crt_ray*
     const crt::PredictorDev d = pr->dev();
     CRT_CUDA(cudaMemsetAsync(d.grad, 0, sizeof(float) * crt::pred::kParams, x->stream));
     CRT_CUDA(cudaMemsetAsync(pr->scratch.p, 0, 16, x->stream));
-    CRT_CUDA(cudaMemsetAsync(x->err.p, 0, 16, x->stream));
+    CRT_TRY(x->begin_host_error());
     CRT_CUDA(crt::pred_train_step(d, pr->nodes(), static_cast<const crt_ray*>(d_rays), n, nullptr,
                                   static_cast<const uint16_t*>(d_t), n, 1, 0, pr->scratch.as<float>(),
-                                  x->err.as<uint32_t>(), x->stream));
+                                  x->hw_dev, x->stream));
     CRT_CUDA(cudaMemcpyAsync(grad, d.grad, sizeof(float) * crt::pred::kParams,
                              is_device_ptr(grad) ? cudaMemcpyDeviceToDevice : cudaMemcpyDeviceToHost, x->stream));
     float ls = 0.f;
     CRT_CUDA(cudaMemcpyAsync(&ls, pr->scratch.p, 4, cudaMemcpyDeviceToHost, x->stream));
     CRT_CUDA(cudaMemsetAsync(d.grad, 0, sizeof(float) * crt::pred::kParams, x->stream));
-    CRT_TRY(x->check_device_error());
+    CRT_TRY(x->check_host_error());
     if (loss) *loss = ls;
     return CRT_OK;
 }
@@ -1832,6 +1918,7 @@ struct crt_batch {
     bool cwide_ready = false;
     bool g_cwide = false;                 // the captured graph derives them
     uint32_t* cw_bad() const { return reinterpret_cast<uint32_t*>(cwide.as<char>() + 64ull * n_tris); }
+    DevBuf walk_ctr;                      // the persistent trace's counters (zero between launches)
     bool models_set = false;
     cudaGraphExec_t graph = nullptr;
     const void* g_tris = nullptr;
@@ -1926,7 +2013,8 @@ crt_status batch_trace_enqueue(crt_ctx* x, crt_batch* bt, const crt_ray* rays, u
         p.cwide = bt->cwide.as<uint4>();
         p.cw_bad = bt->cw_bad();
         crt::launch_trace_batch_pool(p, bt->scenes.as<crt::BatchScene>(), bt->n_scenes,
-                                     flags & (CRT_TRACE_ANY | CRT_TRI_WATERTIGHT), deep, bt->node_box.as<uint32_t>(), s);
+                                     flags & (CRT_TRACE_ANY | CRT_TRI_WATERTIGHT), deep,
+                                     crt::WalkScratch{bt->walk_ctr.as<uint32_t>(), bt->node_box.as<uint32_t>(), nullptr}, s);
     } else
         crt::launch_trace_batch(p, bt->scenes.as<crt::BatchScene>(), bt->n_scenes, bt->n_rays,
                                 flags & (CRT_TRACE_ANY | CRT_TRI_WATERTIGHT), static_cast<int>(bt->cfg.trace_block), deep,
@@ -2015,11 +2103,13 @@ crt_status batch_order_buffers(crt_batch* bt, uint32_t flags) {
 }
 
 crt_status batch_check(crt_ctx* x, crt_batch* bt) {
-    uint32_t ew[4] = {0, 0, 0, 0};
+    static_assert(sizeof(crt::BatchScene) * crt::kMaxBatchScenes + 16 <= 1 << 16, "page-locked staging");
+    uint32_t* ew = static_cast<uint32_t*>(x->pinned);
     CRT_CUDA(cudaMemcpyAsync(ew, bt->err.p, 16, cudaMemcpyDeviceToHost, x->stream));
-    CRT_CUDA(cudaMemcpyAsync(bt->hs.data(), bt->scenes.p, sizeof(crt::BatchScene) * bt->n_scenes, cudaMemcpyDeviceToHost,
+    CRT_CUDA(cudaMemcpyAsync(ew + 4, bt->scenes.p, sizeof(crt::BatchScene) * bt->n_scenes, cudaMemcpyDeviceToHost,
                              x->stream));
     CRT_CUDA(cudaStreamSynchronize(x->stream));
+    std::memcpy(bt->hs.data(), ew + 4, sizeof(crt::BatchScene) * bt->n_scenes);
     bt->max_iters = 0;
     for (const auto& sc : bt->hs) bt->max_iters = std::max(bt->max_iters, sc.iters);
     if (ew[0] & crt::kDevTimeout) return fail(CRT_ERR_DEVICE_TIMEOUT, "batch: a bounded device wait gave up");
@@ -2094,8 +2184,9 @@ crt_status crt_batch_create(crt_ctx* x, const uint32_t* tri_counts, const uint32
                       &bt->inv_perm})
         R(*b, 4ull * N);
     R(bt->node_kids, 16ull * N);
-    // node_box also holds the trace's ray pool: it is build scratch, idle between builds
-    R(bt->node_box, std::max<size_t>(32ull * (2ull * N), crt::trace_pool_bytes(bt->ray_cap)));
+    // node_box also holds the trace's left-over rays: it is build scratch, idle between builds
+    R(bt->node_box, std::max<size_t>(32ull * (2ull * N), 4ull * bt->ray_cap));
+    R(bt->walk_ctr, 16);
     R(bt->cwide, 64ull * N + 16);
     R(bt->pf, 8ull * N);
     R(bt->clus_a, 32ull * N);
@@ -2116,7 +2207,8 @@ crt_status crt_batch_create(crt_ctx* x, const uint32_t* tri_counts, const uint32
     seg[n_scenes] = N;
     bt->tri_off = seg;
     st = CRT_OK;
-    if (cudaMemcpy(bt->scenes.p, hs.data(), sizeof(crt::BatchScene) * n_scenes, cudaMemcpyHostToDevice) != cudaSuccess ||
+    if (cudaMemset(bt->walk_ctr.p, 0, 16) != cudaSuccess ||
+        cudaMemcpy(bt->scenes.p, hs.data(), sizeof(crt::BatchScene) * n_scenes, cudaMemcpyHostToDevice) != cudaSuccess ||
         cudaMemcpy(bt->seg_off.p, seg.data(), 4ull * seg.size(), cudaMemcpyHostToDevice) != cudaSuccess ||
         cudaMemcpy(bt->seg_hist.p, segh.data(), 4ull * 256, cudaMemcpyHostToDevice) != cudaSuccess ||
         cudaMemcpy(bt->chunks.p, chunks.data(), 4ull * chunks.size(), cudaMemcpyHostToDevice) != cudaSuccess) {
@@ -2141,7 +2233,7 @@ crt_status crt_batch_free(crt_batch* bt) {
                       &bt->codes_a, &bt->codes_b, &bt->vals_a, &bt->vals_b, &bt->codes, &bt->perm_global,
                       &bt->perm_local, &bt->node_box, &bt->node_kids, &bt->pf, &bt->clus_a, &bt->clus_b, &bt->it,
                       &bt->ploc_lb, &bt->hist, &bt->sort_lb, &bt->nodes, &bt->wide, &bt->wide_wt, &bt->depth_odd, &bt->xtri, &bt->ray_order, &bt->ray_order_scratch,
-                      &bt->inv_perm, &bt->xtri_sorted, &bt->cwide};
+                      &bt->inv_perm, &bt->xtri_sorted, &bt->cwide, &bt->walk_ctr};
     for (DevBuf* b : bufs) b->release();
     delete bt;
     return CRT_OK;
@@ -2480,7 +2572,7 @@ crt::TraceParams bvh_params(crt_ctx* x, const crt_bvh* b, uint32_t flags) {
     p.wide = (flags & CRT_TRI_WATERTIGHT) ? b->wide_wt.as<float4>() : b->wide.as<float4>();
     p.n_nodes = 2 * b->n - 1;
     p.abs_eps = b->abs_eps;
-    p.err = x->err.as<uint32_t>();
+    p.err = x->hw_dev;
     return p;
 }
 
@@ -2510,11 +2602,11 @@ crt_status crt_shade(crt_ctx* x, const crt_bvh* b, const crt_ray* rays, const cr
     p.rays = static_cast<const crt_ray*>(d_rays);
     p.hits = static_cast<crt_hit*>(const_cast<void*>(d_hits));
     p.n_rays = n;
-    CRT_CUDA(cudaMemsetAsync(x->err.p, 0, 16, x->stream));
+    CRT_TRY(x->begin_host_error());
     crt::launch_shade(p, sp, x->stream);
     CRT_CUDA(cudaGetLastError());
     if (copy_out) CRT_CUDA(cudaMemcpyAsync(rgba, sp.image, 16 * static_cast<size_t>(n), cudaMemcpyDeviceToHost, x->stream));
-    return x->check_device_error();
+    return x->check_host_error();
 }
 
 crt_status crt_render_frame(crt_ctx* x, const crt_bvh* b, const crt_camera* cam, uint32_t width, uint32_t height,
@@ -2537,7 +2629,7 @@ crt_status crt_render_frame(crt_ctx* x, const crt_bvh* b, const crt_camera* cam,
     } else {
         CRT_TRY(check_aligned16(cam, "camera"));
     }
-    CRT_CUDA(cudaMemsetAsync(x->err.p, 0, 16, x->stream));
+    CRT_TRY(x->begin_host_error());
     const uint32_t tw = (width % 8 == 0 && height % 4 == 0) ? width : 0u;  // 8x4 pixel tiles per warp
     if (!(flags & (CRT_TRACE_USE_PREDICTOR | CRT_TRACE_WIDE | CRT_TRACE_COMPRESSED))) {
         // one launch: camera ray, closest hit and texel per pixel
@@ -2551,9 +2643,7 @@ crt_status crt_render_frame(crt_ctx* x, const crt_bvh* b, const crt_camera* cam,
         }
         const bool deep = b->depth_bound + 2 > 64;
         const uint32_t kflags = (flags & CRT_TRI_WATERTIGHT) | (deep ? (1u << 16) : 0u);
-        crt::launch_frame(p, d_cam, width, height, 0, height, nullptr, nullptr, kflags,
-                          static_cast<int>(x->cfg.trace_block), &sp, x->node_box.as<uint32_t>(), x->stream);
-        CRT_CUDA(cudaGetLastError());
+        CRT_TRY(frame_launch(x, p, d_cam, width, height, nullptr, nullptr, kflags, &sp));
     } else {
         CRT_TRY(x->frame_rays.reserve(sizeof(crt_ray) * static_cast<size_t>(n)));
         CRT_TRY(x->frame_hits.reserve(sizeof(crt_hit) * static_cast<size_t>(n)));
@@ -2569,7 +2659,7 @@ crt_status crt_render_frame(crt_ctx* x, const crt_bvh* b, const crt_camera* cam,
         CRT_CUDA(cudaGetLastError());
     }
     if (copy_out) CRT_CUDA(cudaMemcpyAsync(rgba, sp.image, 16 * static_cast<size_t>(n), cudaMemcpyDeviceToHost, x->stream));
-    CRT_TRY(x->check_device_error());
+    CRT_TRY(x->check_host_error());
     if (flags & CRT_TRACE_STATS) CRT_CUDA(cudaMemcpy(x->last_trace_stats, x->trace_stats.p, 16, cudaMemcpyDeviceToHost));
     return CRT_OK;
 }
@@ -2612,7 +2702,7 @@ crt_status crt_triangles_from_indexed(crt_ctx* x, const float* vertices, uint32_
     } else if (!aligned(out, 16)) {
         return fail(CRT_ERR_INVALID_ARG, "crt_triangles_from_indexed: out must be 16-byte aligned");
     }
-    CRT_CUDA(cudaMemsetAsync(x->err.p, 0, 16, x->stream));
+    CRT_TRY(x->begin_device_error());
     crt::launch_indexed(static_cast<const float*>(d_v), n_vertices, static_cast<const uint32_t*>(d_i), n_triangles,
                         model_id, d_out, x->err.as<uint32_t>(), x->stream);
     CRT_CUDA(cudaGetLastError());

@@ -162,12 +162,20 @@ struct TraceParams {
     const uint32_t* order = nullptr;
 };
 void launch_trace(const TraceParams& p, uint32_t flags, int block, cudaStream_t s);
+// Scratch of a persistent walk over the compressed nodes: 16 bytes of counters,
+// zero before its first use and again after each launch, room for the index of
+// every ray, and optionally a page-locked word for the number of rays left to the
+// binary walk.  With it the caller waits for the launch and then launches the
+// left-over rays itself; without, they are launched right away.
+struct WalkScratch {
+    uint32_t* ctr = nullptr;
+    uint32_t* left = nullptr;
+    uint32_t* host_left = nullptr;
+};
 // Many rays by persistent warps that refill finished lanes from a ray counter;
-// compressed nodes, no seeding, rays in caller order or p.order.  pool:
-// trace_pool_bytes(n_rays) of device memory (counters, reset here, and the list
-// of rays left to the binary walk).
-size_t trace_pool_bytes(uint32_t n_rays);
-void launch_trace_pool(const TraceParams& p, uint32_t flags, uint32_t* pool, cudaStream_t s);
+// compressed nodes, no seeding, rays in caller order or p.order.
+void launch_trace_pool(const TraceParams& p, uint32_t flags, const WalkScratch& w, cudaStream_t s);
+void launch_trace_left(const TraceParams& p, uint32_t flags, const WalkScratch& w, uint32_t n, cudaStream_t s);
 
 // Shading (getColor + imageStore) inputs; the BVH, leaf records and error
 // word come from the TraceParams it runs with.
@@ -190,10 +198,11 @@ void launch_shade(const TraceParams& p, const ShadeParams& sp, cudaStream_t s);
 // p.hits (may be null with shading) and, with a light, their shadow rays to
 // any hit into hits_shadow, and with shade, their texels into shade->image,
 // in one launch (p.tile_width: width for 8x4 pixel tiles, or 0).  With p.cwide
-// over the compressed nodes, with pool (trace_pool_bytes of the image's pixels).
+// over the compressed nodes (w with host_left); left != 0: the pixels such a
+// launch left over.
 void launch_frame(const TraceParams& p, const crt_camera* cam, uint32_t width, uint32_t height, uint32_t y0,
                   uint32_t rows, const float* light, crt_hit* hits_shadow, uint32_t flags, int block,
-                  const ShadeParams* shade, uint32_t* pool, cudaStream_t s);
+                  const ShadeParams* shade, const WalkScratch& w, uint32_t left, cudaStream_t s);
 
 // Batched scenes: per-scene offsets into the concatenated arrays.
 constexpr uint32_t kMaxBatchScenes = 256;
@@ -220,7 +229,7 @@ void launch_cwide_batch(const float4* wide, const struct BatchScene* scenes, uin
 // The persistent ray pool over a batch: no seeding; p holds the batch's node
 // arrays and p.n_rays the batch's ray count.
 void launch_trace_batch_pool(const TraceParams& p, const BatchScene* scenes, uint32_t n_scenes, uint32_t flags,
-                             bool deep, uint32_t* pool, cudaStream_t s);
+                             bool deep, const WalkScratch& w, cudaStream_t s);
 // CRT_TRACE_SORT_RAYS: order[k] = k-th ray by coherence key (origin cell,
 // direction; with scenes, scene first).  scratch: ray_order_scratch_bytes(n).
 size_t ray_order_scratch_bytes(uint32_t n);

@@ -173,10 +173,10 @@ __global__ void __launch_bounds__(BLOCK) frame_kernel(TraceParams p, FrameParams
 }
 
 // The same over the compressed nodes: a warp takes a tile of 32 pixels (warp w
-// tile w, then tiles from the counter pool[0] while there are any), walks its
+// tile w, then tiles from the counter while there are any), walks its
 // camera rays together, then their shadow rays, testing a leaf as soon as a
 // lane holds one (coherent lanes reach theirs together; waiting for two: 3 %
-// slower).  Pixels with a ray of the binary walk go to left[0 .. pool[1]) for
+// slower).  Pixels with a ray of the binary walk go to the list `left` for
 // frame_left_kernel.
 //
 // Bound by the ALU pipe (65-71 % busy, 18-22 of 32 threads per instruction) and
@@ -189,8 +189,8 @@ __global__ void __launch_bounds__(BLOCK) frame_kernel(TraceParams p, FrameParams
 // a call against 282).
 template <bool WT, bool SHADE, bool COUNT>
 __global__ void __launch_bounds__(kWalk4Block, kWalk4Blocks)
-    frame_walk4_kernel(const TraceParams p, const FrameParams f, const ShadeParams sp, uint32_t* __restrict__ pool,
-                       uint32_t* __restrict__ left) {
+    frame_walk4_kernel(const TraceParams p, const FrameParams f, const ShadeParams sp, Walk4Counters* ctr,
+                       uint32_t* __restrict__ left, uint32_t* host_left) {
     __shared__ uint2 s_st[kWalk4Shared + 1][kWalk4Block];
     const uint32_t lane = threadIdx.x & 31u;
     const uint32_t s_base = static_cast<uint32_t>(__cvta_generic_to_shared(&s_st[1][threadIdx.x]));
@@ -230,10 +230,10 @@ __global__ void __launch_bounds__(kWalk4Block, kWalk4Blocks)
             redo = redo || L.redo;
             if (valid && !redo) reinterpret_cast<uint4*>(f.hits_shadow)[i] = L.hit();
         }
-        if (valid && redo) left[atomicAdd(pool + 1, 1u)] = i;
+        if (valid && redo) left[atomicAdd(&ctr->left, 1u)] = i;
         uint32_t next = tiles;
         if (tiles > warps) {
-            if (lane == 0) next = warps + atomicAdd(pool, 1u);
+            if (lane == 0) next = warps + atomicAdd(&ctr->taken, 1u);
             next = __shfl_sync(0xFFFFFFFFu, next, 0);
         }
         tile = next;
@@ -242,13 +242,13 @@ __global__ void __launch_bounds__(kWalk4Block, kWalk4Blocks)
         atomicAdd(p.stats + 0, static_cast<unsigned long long>(L.fetched));
         atomicAdd(p.stats + 1, static_cast<unsigned long long>(L.tested));
     }
+    walk4_finish(ctr, host_left);
 }
 
 template <bool WT, int STACK, bool SHADE>
 __global__ void __launch_bounds__(kWalk4Block)
-    frame_left_kernel(TraceParams p, FrameParams f, ShadeParams sp, const uint32_t* __restrict__ pool,
-                      const uint32_t* __restrict__ left) {
-    const uint32_t n = min(pool[1], p.n_rays);
+    frame_left_kernel(TraceParams p, FrameParams f, ShadeParams sp, uint32_t n, const uint32_t* __restrict__ left) {
+    n = min(n, p.n_rays);
     for (uint32_t k = blockIdx.x * kWalk4Block + threadIdx.x; k < n; k += gridDim.x * kWalk4Block) {
         const uint32_t i = left[k];
         if (i >= p.n_rays) raise_corrupt(p.err, 7, k, i);
@@ -256,36 +256,39 @@ __global__ void __launch_bounds__(kWalk4Block)
     }
 }
 
+// The frame, or with left != 0 the pixels that its launch left over.
 template <bool WT, bool SHADE>
 static void launch_frame_walk4(const TraceParams& p, const FrameParams& f, const ShadeParams& sp, bool deep,
-                               uint32_t* pool, cudaStream_t s) {
+                               const WalkScratch& w, uint32_t left, cudaStream_t s) {
     static int grid = 0;
     if (grid == 0) {
         int per_sm = 0;
         cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, frame_walk4_kernel<WT, SHADE, false>, kWalk4Block, 0);
         grid = kNumSms * (per_sm > 0 ? per_sm : 1);
     }
+    if (left != 0) {
+        const uint32_t few = (left + kWalk4Block - 1) / kWalk4Block;
+        if (deep) frame_left_kernel<WT, 1024, SHADE><<<few, kWalk4Block, 0, s>>>(p, f, sp, left, w.left);
+        else frame_left_kernel<WT, 64, SHADE><<<few, kWalk4Block, 0, s>>>(p, f, sp, left, w.left);
+        return;
+    }
+    Walk4Counters* ctr = reinterpret_cast<Walk4Counters*>(w.ctr);
     const uint32_t want = (f.width * f.rows + kWalk4Block - 1) / kWalk4Block;
     const uint32_t blocks = want < static_cast<uint32_t>(grid) ? want : static_cast<uint32_t>(grid);
-    uint32_t* left = pool + 4;
-    cudaMemsetAsync(pool, 0, 8, s);
-    if (p.stats) frame_walk4_kernel<WT, SHADE, true><<<blocks, kWalk4Block, 0, s>>>(p, f, sp, pool, left);
-    else frame_walk4_kernel<WT, SHADE, false><<<blocks, kWalk4Block, 0, s>>>(p, f, sp, pool, left);
-    const uint32_t few = want < static_cast<uint32_t>(kNumSms) ? want : static_cast<uint32_t>(kNumSms);
-    if (deep) frame_left_kernel<WT, 1024, SHADE><<<few, kWalk4Block, 0, s>>>(p, f, sp, pool, left);
-    else frame_left_kernel<WT, 64, SHADE><<<few, kWalk4Block, 0, s>>>(p, f, sp, pool, left);
+    if (p.stats) frame_walk4_kernel<WT, SHADE, true><<<blocks, kWalk4Block, 0, s>>>(p, f, sp, ctr, w.left, w.host_left);
+    else frame_walk4_kernel<WT, SHADE, false><<<blocks, kWalk4Block, 0, s>>>(p, f, sp, ctr, w.left, w.host_left);
 }
 
 template <bool WT, int BLOCK, bool SHADE>
 static void launch_frame_s(const TraceParams& p, const crt_camera* cam, uint32_t width, uint32_t height, uint32_t y0,
                            uint32_t rows, const float* light, crt_hit* hits_shadow, bool deep, const ShadeParams& sp,
-                           uint32_t* pool, cudaStream_t s) {
+                           const WalkScratch& w, uint32_t left, cudaStream_t s) {
     const uint32_t grid = (width * rows + BLOCK - 1) / BLOCK;
     if (grid == 0) return;
     const int sh = light != nullptr;
     const FrameParams f{cam, width, height, y0, rows, sh, sh ? light[0] : 0.f, sh ? light[1] : 0.f, sh ? light[2] : 0.f,
                         hits_shadow};
-    if (p.cwide) launch_frame_walk4<WT, SHADE>(p, f, sp, deep, pool, s);
+    if (p.cwide) launch_frame_walk4<WT, SHADE>(p, f, sp, deep, w, left, s);
     else if (deep) frame_kernel<WT, 1024, BLOCK, SHADE><<<grid, BLOCK, 0, s>>>(p, f, sp);
     else frame_kernel<WT, 64, BLOCK, SHADE><<<grid, BLOCK, 0, s>>>(p, f, sp);
 }
@@ -293,24 +296,24 @@ static void launch_frame_s(const TraceParams& p, const crt_camera* cam, uint32_t
 template <bool WT, int BLOCK>
 static void launch_frame_b(const TraceParams& p, const crt_camera* cam, uint32_t width, uint32_t height, uint32_t y0,
                            uint32_t rows, const float* light, crt_hit* hits_shadow, bool deep, const ShadeParams* shade,
-                           uint32_t* pool, cudaStream_t s) {
-    if (shade) launch_frame_s<WT, BLOCK, true>(p, cam, width, height, y0, rows, light, hits_shadow, deep, *shade, pool, s);
-    else launch_frame_s<WT, BLOCK, false>(p, cam, width, height, y0, rows, light, hits_shadow, deep, ShadeParams{}, pool, s);
+                           const WalkScratch& w, uint32_t left, cudaStream_t s) {
+    if (shade) launch_frame_s<WT, BLOCK, true>(p, cam, width, height, y0, rows, light, hits_shadow, deep, *shade, w, left, s);
+    else launch_frame_s<WT, BLOCK, false>(p, cam, width, height, y0, rows, light, hits_shadow, deep, ShadeParams{}, w, left, s);
 }
 
 void launch_frame(const TraceParams& p, const crt_camera* cam, uint32_t width, uint32_t height, uint32_t y0,
                   uint32_t rows, const float* light, crt_hit* hits_shadow, uint32_t flags, int block,
-                  const ShadeParams* shade, uint32_t* pool, cudaStream_t s) {
+                  const ShadeParams* shade, const WalkScratch& w, uint32_t left, cudaStream_t s) {
     const bool wt = flags & CRT_TRI_WATERTIGHT;
     const bool deep = (flags >> 16) != 0;
     if (wt) {
-        if (block == 256) launch_frame_b<true, 256>(p, cam, width, height, y0, rows, light, hits_shadow, deep, shade, pool, s);
-        else if (block == 64) launch_frame_b<true, 64>(p, cam, width, height, y0, rows, light, hits_shadow, deep, shade, pool, s);
-        else launch_frame_b<true, 128>(p, cam, width, height, y0, rows, light, hits_shadow, deep, shade, pool, s);
+        if (block == 256) launch_frame_b<true, 256>(p, cam, width, height, y0, rows, light, hits_shadow, deep, shade, w, left, s);
+        else if (block == 64) launch_frame_b<true, 64>(p, cam, width, height, y0, rows, light, hits_shadow, deep, shade, w, left, s);
+        else launch_frame_b<true, 128>(p, cam, width, height, y0, rows, light, hits_shadow, deep, shade, w, left, s);
     } else {
-        if (block == 256) launch_frame_b<false, 256>(p, cam, width, height, y0, rows, light, hits_shadow, deep, shade, pool, s);
-        else if (block == 64) launch_frame_b<false, 64>(p, cam, width, height, y0, rows, light, hits_shadow, deep, shade, pool, s);
-        else launch_frame_b<false, 128>(p, cam, width, height, y0, rows, light, hits_shadow, deep, shade, pool, s);
+        if (block == 256) launch_frame_b<false, 256>(p, cam, width, height, y0, rows, light, hits_shadow, deep, shade, w, left, s);
+        else if (block == 64) launch_frame_b<false, 64>(p, cam, width, height, y0, rows, light, hits_shadow, deep, shade, w, left, s);
+        else launch_frame_b<false, 128>(p, cam, width, height, y0, rows, light, hits_shadow, deep, shade, w, left, s);
     }
 }
 

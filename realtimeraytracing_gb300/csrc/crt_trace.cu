@@ -200,43 +200,48 @@ static void launch_trace_t(const TraceParams& p, int block, bool deep, bool seed
 }
 
 template <bool ANY, bool WT, bool BATCH>
-static void launch_walk4_t(const TraceParams& p, bool deep, uint32_t* pool, const BatchScene* scenes, uint32_t n_scenes,
-                           cudaStream_t s) {
+static void launch_walk4_t(const TraceParams& p, bool deep, const WalkScratch& w, uint32_t left, const BatchScene* scenes,
+                           uint32_t n_scenes, cudaStream_t s) {
     static int grid = 0;
     if (grid == 0) {
         int per_sm = 0;
         cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, trace_walk4_kernel<ANY, WT, BATCH>, kWalk4Block, 0);
         grid = kNumSms * (per_sm > 0 ? per_sm : 1);
     }
-    uint32_t* left = pool + 4;
-    cudaMemsetAsync(pool, 0, 8, s);
+    Walk4Counters* ctr = reinterpret_cast<Walk4Counters*>(w.ctr);
     const uint32_t want = (p.n_rays + kWalk4Block - 1) / kWalk4Block;
-    const uint32_t blocks = std::min(want, static_cast<uint32_t>(grid));
-    trace_walk4_kernel<ANY, WT, BATCH><<<blocks, kWalk4Block, 0, s>>>(p, pool, left, scenes, n_scenes);
-    const uint32_t few = std::min(want, static_cast<uint32_t>(kNumSms * 4));
-    if (deep) walk4_left_kernel<ANY, WT, 1024, BATCH><<<few, kWalk4Block, 0, s>>>(p, pool, left, scenes, n_scenes);
-    else walk4_left_kernel<ANY, WT, 64, BATCH><<<few, kWalk4Block, 0, s>>>(p, pool, left, scenes, n_scenes);
+    if (left == 0) {
+        trace_walk4_kernel<ANY, WT, BATCH><<<std::min(want, static_cast<uint32_t>(grid)), kWalk4Block, 0, s>>>(
+            p, ctr, w.left, w.host_left, scenes, n_scenes);
+        if (w.host_left) return;
+    }
+    const uint32_t* count = left == 0 ? &ctr->last_left : nullptr;
+    const uint32_t few = std::min(left == 0 ? want : (left + kWalk4Block - 1) / kWalk4Block, static_cast<uint32_t>(kNumSms * 16));
+    if (deep) walk4_left_kernel<ANY, WT, 1024, BATCH><<<few, kWalk4Block, 0, s>>>(p, count, left, w.left, scenes, n_scenes);
+    else walk4_left_kernel<ANY, WT, 64, BATCH><<<few, kWalk4Block, 0, s>>>(p, count, left, w.left, scenes, n_scenes);
 }
 
 template <bool BATCH>
-static void launch_walk4(const TraceParams& p, uint32_t flags, bool deep, uint32_t* pool, const BatchScene* scenes,
-                         uint32_t n_scenes, cudaStream_t s) {
+static void launch_walk4(const TraceParams& p, uint32_t flags, bool deep, const WalkScratch& w, uint32_t left,
+                         const BatchScene* scenes, uint32_t n_scenes, cudaStream_t s) {
     const bool any = flags & CRT_TRACE_ANY, wt = flags & CRT_TRI_WATERTIGHT;
-    if (any && wt) launch_walk4_t<true, true, BATCH>(p, deep, pool, scenes, n_scenes, s);
-    else if (any) launch_walk4_t<true, false, BATCH>(p, deep, pool, scenes, n_scenes, s);
-    else if (wt) launch_walk4_t<false, true, BATCH>(p, deep, pool, scenes, n_scenes, s);
-    else launch_walk4_t<false, false, BATCH>(p, deep, pool, scenes, n_scenes, s);
+    if (any && wt) launch_walk4_t<true, true, BATCH>(p, deep, w, left, scenes, n_scenes, s);
+    else if (any) launch_walk4_t<true, false, BATCH>(p, deep, w, left, scenes, n_scenes, s);
+    else if (wt) launch_walk4_t<false, true, BATCH>(p, deep, w, left, scenes, n_scenes, s);
+    else launch_walk4_t<false, false, BATCH>(p, deep, w, left, scenes, n_scenes, s);
 }
 
-size_t trace_pool_bytes(uint32_t n_rays) { return 16 + 4ull * n_rays; }
+void launch_trace_pool(const TraceParams& p, uint32_t flags, const WalkScratch& w, cudaStream_t s) {
+    if (p.n_rays != 0) launch_walk4<false>(p, flags, (flags >> 16) != 0, w, 0, nullptr, 0, s);
+}
 
-void launch_trace_pool(const TraceParams& p, uint32_t flags, uint32_t* pool, cudaStream_t s) {
-    if (p.n_rays != 0) launch_walk4<false>(p, flags, (flags >> 16) != 0, pool, nullptr, 0, s);
+void launch_trace_left(const TraceParams& p, uint32_t flags, const WalkScratch& w, uint32_t n, cudaStream_t s) {
+    if (n != 0) launch_walk4<false>(p, flags, (flags >> 16) != 0, w, n, nullptr, 0, s);
 }
 
 void launch_trace_batch_pool(const TraceParams& p, const BatchScene* scenes, uint32_t n_scenes, uint32_t flags,
-                             bool deep, uint32_t* pool, cudaStream_t s) {
-    if (p.n_rays != 0 && n_scenes != 0) launch_walk4<true>(p, flags, deep, pool, scenes, n_scenes, s);
+                             bool deep, const WalkScratch& w, cudaStream_t s) {
+    if (p.n_rays != 0 && n_scenes != 0) launch_walk4<true>(p, flags, deep, w, 0, scenes, n_scenes, s);
 }
 
 void launch_trace(const TraceParams& p, uint32_t flags, int block, cudaStream_t s) {

@@ -383,6 +383,26 @@ __device__ __forceinline__ uint32_t walk4_run(Walk4Lane& L, uint32_t s_base, uin
     }
 }
 
+// A persistent walk's counters in device memory.  The launch's last block zeroes
+// them for the next one (no clear in between) and hands the number of rays left
+// over to the device (last_left) and, where given, to page-locked host memory,
+// so that a caller that waits for the launch anyway starts walk4_left_kernel only
+// when there are any.
+struct Walk4Counters {
+    uint32_t taken, left, blocks, last_left;
+};
+__device__ __forceinline__ void walk4_finish(Walk4Counters* ctr, uint32_t* host_left) {
+    __syncthreads();
+    if (threadIdx.x != 0) return;
+    __threadfence();
+    if (atomicInc(&ctr->blocks, gridDim.x - 1) != gridDim.x - 1) return;
+    __threadfence();
+    const uint32_t n = atomicExch(&ctr->left, 0u);
+    ctr->taken = 0u;
+    ctr->last_left = n;
+    if (host_left) *reinterpret_cast<volatile uint32_t*>(host_left) = n;
+}
+
 // Persistent warps over a ray pool, one ray per lane; lanes whose ray is done take
 // new rays from the counter once kWalk4Refill of them wait.
 //
@@ -399,11 +419,11 @@ __device__ __forceinline__ uint32_t walk4_run(Walk4Lane& L, uint32_t s_base, uin
 // 0.36 without).
 //
 // Rays the compressed walk cannot take (walk4_setup, unquantised scenes, one-leaf
-// trees, walks deeper than the stack) go to the list left[0 .. pool[1]) for
-// walk4_left_kernel, launched right after; pool[0] counts the rays taken.
+// trees, walks deeper than the stack) go to the list `left` for walk4_left_kernel.
+// ctr (Walk4Counters, zero between launches): the rays taken and left.
 template <bool ANY, bool WT, bool BATCH>
 __global__ void __launch_bounds__(kWalk4Block, kWalk4Blocks)
-    trace_walk4_kernel(const TraceParams p, uint32_t* __restrict__ pool, uint32_t* __restrict__ left,
+    trace_walk4_kernel(const TraceParams p, Walk4Counters* ctr, uint32_t* __restrict__ left, uint32_t* host_left,
                        const BatchScene* __restrict__ scenes, uint32_t n_scenes) {
     constexpr uint32_t kIdle = 0xFFFFFFFFu, kDone = 0xFFFFFFFEu;
     __shared__ uint2 s_st[kWalk4Shared + 1][kWalk4Block];  // row 0 is read (and ignored) below an empty stack
@@ -431,7 +451,7 @@ __global__ void __launch_bounds__(kWalk4Block, kWalk4Blocks)
             const uint32_t take = static_cast<uint32_t>(__popc(need));
             const int leader = __ffs(need) - 1;
             uint32_t base = 0;
-            if (lane == static_cast<uint32_t>(leader)) base = atomicAdd(pool, take);
+            if (lane == static_cast<uint32_t>(leader)) base = atomicAdd(&ctr->taken, take);
             base = __shfl_sync(0xFFFFFFFFu, base, leader);
             pool_left = base < p.n_rays && p.n_rays - base > take;
             const uint32_t k = base + static_cast<uint32_t>(__popc(need & ((1u << lane) - 1u)));
@@ -458,19 +478,21 @@ __global__ void __launch_bounds__(kWalk4Block, kWalk4Blocks)
         if (__all_sync(0xFFFFFFFFu, i == kDone)) break;
         const uint32_t om = walk4_run<ANY, WT, kWalk4Flush>(L, s_base, st, pool_left ? kWalk4Refill : 32);
         if ((om >> lane & 1u) && i < kDone) {
-            if (L.redo) left[atomicAdd(pool + 1, 1u)] = i;
+            if (L.redo) left[atomicAdd(&ctr->left, 1u)] = i;
             else reinterpret_cast<uint4*>(p.hits)[i] = L.hit();
             i = kIdle;
         }
     }
+    walk4_finish(ctr, host_left);
 }
 
-// The binary walk of the rays a trace_walk4_kernel launch left over (few or none).
+// The binary walk of the rays a trace_walk4_kernel launch left over (few or none):
+// n of them, or as many as *count says.
 template <bool ANY, bool WT, int STACK, bool BATCH>
 __global__ void __launch_bounds__(kWalk4Block)
-    walk4_left_kernel(const TraceParams p, const uint32_t* __restrict__ pool, const uint32_t* __restrict__ left,
-                      const BatchScene* __restrict__ scenes, uint32_t n_scenes) {
-    const uint32_t n = min(pool[1], p.n_rays);
+    walk4_left_kernel(const TraceParams p, const uint32_t* __restrict__ count, uint32_t n,
+                      const uint32_t* __restrict__ left, const BatchScene* __restrict__ scenes, uint32_t n_scenes) {
+    n = min(count ? *count : n, p.n_rays);
     for (uint32_t k = blockIdx.x * kWalk4Block + threadIdx.x; k < n; k += gridDim.x * kWalk4Block) {
         const uint32_t i = left[k];
         if (i >= p.n_rays) { raise_corrupt(p.err, 7, k, i); continue; }
