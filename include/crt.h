@@ -156,7 +156,7 @@ typedef struct crt_build_stats {
     float ms_morton;     /* scene box + Morton codes */
     float ms_sort;       /* radix sort of (code, index) */
     float ms_ploc;       /* PLOC iterations */
-    float ms_layout;     /* DFS node layout (inside the one-launch path: from its own timer stamps) */
+    float ms_layout;     /* DFS node layout */
     float ms_total;
     float scene_box[6];  /* min xyz, max xyz over the scanned buffer */
 } crt_build_stats;

@@ -543,7 +543,7 @@ crt_status build_impl(crt_ctx* x, crt_bvh* b, const crt_triangle* tris, uint32_t
     CRT_TRY(x->clus_a.reserve(32ull * N));
     CRT_TRY(x->clus_b.reserve(32ull * N));
     CRT_TRY(x->iters.reserve(8ull * (N + 2)));
-    // + tail: tickets[2], barrier[2], iteration count, finished blocks, 3 timer stamps
+    // + tail: tickets[2], barrier[2], iteration count
     CRT_TRY(x->ploc_lb.reserve(8ull * (2ull * ploc_tiles) + 64));
     CRT_TRY(b->nodes.reserve(sizeof(crt_bvh_node) * (2ull * N - 1)));
     CRT_TRY(b->xtri.reserve(48ull * N));
@@ -600,30 +600,27 @@ crt_status build_impl(crt_ctx* x, crt_bvh* b, const crt_triangle* tris, uint32_t
     // ---- K3: leaf clusters + PLOC iterations
     uint2* d_it = x->iters.as<uint2>();
     crt::launch_leaf_init(d_tris, N, d_models, b->perm.as<uint32_t>(), x->node_box.as<float4>(), x->clus_a.as<float4>(),
-                          x->xtri_sorted.as<float4>(), d_it, err, s);
+                          x->xtri_sorted.as<float4>(), d_it, x->pos.as<uint2>(), err, s);
     const crt::LeafOut leaves{x->xtri_sorted.as<float4>(), b->xtri.as<float4>(), b->inv_perm.as<uint32_t>()};
     CRT_CUDA(cudaGetLastError());
     x->it_host.assign(1, make_uint2(N, N));
     uint32_t iters = 0;
     bool laid_out = false;
-    float layout_in_kernel_ms = 0.f;  // the persistent launch's layout phase, from its timer stamps
     // read back in page-locked memory, past the model matrices that may still be on their way
     uint32_t* h_tail = static_cast<uint32_t*>(x->pinned) + 2 * 64 * 16;
     crt::SceneState* h_state = reinterpret_cast<crt::SceneState*>(h_tail + 16);
     if (N > 1 && !x->force_multi_launch) {
-        // one cooperative launch: every PLOC iteration, then the DFS layout
         unsigned long long* lb = x->ploc_lb.as<unsigned long long>();
         uint32_t* tail = reinterpret_cast<uint32_t*>(lb + 2ull * ploc_tiles);
-        const cudaError_t e = crt::launch_ploc_persistent(
+        const cudaError_t e = crt::launch_ploc_layout(
             x->clus_a.as<float4>(), x->clus_b.as<float4>(), x->node_box.as<float4>(), x->node_kids.as<uint4>(), d_it, N,
             static_cast<int>(x->cfg.ploc_radius), lb, tail, ploc_tiles, x->pos.as<uint2>(), b->nodes.as<crt_bvh_node>(),
             b->wide.as<float4>(), b->wide_wt.as<float4>(), b->depth_odd.as<uint8_t>(), leaves, st,
             reinterpret_cast<unsigned long long*>(tail + 2), tail + 4,
-            err, x->cfg.spin_limit, s);
+            err, x->cfg.spin_limit, x->ev[3], s);
         if (e == cudaSuccess) {
-            CRT_CUDA(cudaEventRecord(x->ev[3], s));
-            CRT_CUDA(cudaMemcpyAsync(h_tail, tail + 4, 32, cudaMemcpyDeviceToHost, s));
-            laid_out = true;  // its iteration count and stamps are read at the end
+            CRT_CUDA(cudaMemcpyAsync(h_tail, tail + 4, 4, cudaMemcpyDeviceToHost, s));
+            laid_out = true;  // its iteration count is read at the end
         } else if (e != cudaErrorNotSupported && e != cudaErrorCooperativeLaunchTooLarge) {
             return fail(CRT_ERR_CUDA, "PLOC launch failed: %s", cudaGetErrorString(e));
         } else {
@@ -697,20 +694,15 @@ crt_status build_impl(crt_ctx* x, crt_bvh* b, const crt_triangle* tris, uint32_t
     CRT_CUDA(cudaMemcpyAsync(h_state, st, sizeof(crt::SceneState), cudaMemcpyDeviceToHost, s));
     CRT_TRY(x->check_device_error());  // the build's one wait
     const crt::SceneState hs = *h_state;
-    if (laid_out) {
-        iters = h_tail[0];
-        unsigned long long stamp[3];
-        std::memcpy(stamp, h_tail + 2, sizeof(stamp));
-        if (stamp[2] > stamp[1]) layout_in_kernel_ms = static_cast<float>(static_cast<double>(stamp[2] - stamp[1]) * 1e-6);
-    }
+    if (laid_out) iters = h_tail[0];
     float ms[4];
     for (int k = 0; k < 4; ++k) CRT_CUDA(cudaEventElapsedTime(&ms[k], x->ev[k], x->ev[k + 1]));
     x->stats.n_tris = N;
     x->stats.ploc_iterations = iters;
     x->stats.ms_morton = ms[0];
     x->stats.ms_sort = ms[1];
-    x->stats.ms_ploc = ms[2] - layout_in_kernel_ms;
-    x->stats.ms_layout = ms[3] + layout_in_kernel_ms;
+    x->stats.ms_ploc = ms[2];
+    x->stats.ms_layout = ms[3];
     x->stats.ms_total = ms[0] + ms[1] + ms[2] + ms[3];
     for (int a = 0; a < 3; ++a) {
         x->stats.scene_box[a] = hs.scene_min[a];

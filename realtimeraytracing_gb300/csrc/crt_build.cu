@@ -4,6 +4,7 @@
 // Reference: srcCommon/scene/geometry/bvh.cpp (CPU, OpenMP) and the DFS
 // flattening in srcOpenGL/scene/scene.cpp:189-208.  Every float result is
 // bit-identical to the reference's (this file is compiled with -fmad=false).
+#include <cooperative_groups.h>
 #include <cstdint>
 #include <cuda_runtime.h>
 
@@ -409,6 +410,8 @@ __global__ void __launch_bounds__(BLOCK, 3) onesweep_kernel(const uint32_t* __re
     }
 }
 
+constexpr uint32_t kLayoutUnset = 0xFFFFFFFFu;  // a place not yet published (dataflow layout)
+
 // ==================================================== leaf clusters
 // plocPreprocessing (bvh.cpp:26-46): sorted position i holds the leaf of
 // triangle perm[i] with AABB::buildFromTriangle's box (bvh.cpp:383-399).
@@ -418,10 +421,12 @@ __global__ void __launch_bounds__(256) leaf_init_kernel(const crt_triangle* __re
                                                         const float* __restrict__ models,
                                                         const uint32_t* __restrict__ perm,
                                                         float4* __restrict__ node_box, float4* __restrict__ clusters,
-                                                        float4* __restrict__ xtri, uint2* it, uint32_t* err) {
+                                                        float4* __restrict__ xtri, uint2* it, uint2* __restrict__ pf,
+                                                        uint32_t* err) {
     const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i == 0) it[0] = make_uint2(n, n);
     if (i >= n) return;
+    pf[i] = make_uint2(kLayoutUnset, 0u);  // the layout's places arrive from each node's parent
     const uint32_t ti = perm[i];
     if (ti >= n) { raise_corrupt(err, 1, i, ti); return; }
     const TriRec t = load_tri(tris, ti);
@@ -1004,8 +1009,6 @@ __global__ void __launch_bounds__(BLOCK) ploc_iteration_kernel(const float4* __r
 // transformed triangle into that order.  The traversal's tie rule (equal t:
 // the leaf later in DFS order, which the shader visits first) and every
 // subtree's leaves forming one contiguous range rest on this order.
-constexpr uint32_t kLayoutUnset = 0xFFFFFFFFu;  // a position not yet published (dataflow layout)
-
 __device__ __forceinline__ uint2 layout_place(uint32_t X, const uint2* __restrict__ pf, uint32_t N) {
     // (DFS position, first leaf below | depth parity << 31) of X; the root sits at (0, 0)
     return (X == 2 * N - 2) ? make_uint2(0u, 0u) : __ldcg(pf + (X - N));
@@ -1180,32 +1183,296 @@ __device__ __forceinline__ bool grid_barrier(unsigned long long* bar, unsigned l
     return (ld_acquire_u32(err) & kDevTimeout) == 0u;
 }
 
+// =============================== K3 on a cluster: the last PLOC iterations
+// Once the live clusters fit in the shared memory of one thread-block cluster
+// (n <= ploc_cluster_max), it runs the remaining iterations there: block c holds
+// the positions [c seg, (c + 1) seg) and a halo of 2R on each side in the window
+// layout of a tile that starts at its first position.  An iteration is the
+// reference's, as in ploc_tile: nearest neighbours, mutual pairs merged at the
+// lower position, exclusive scan of survivors and merges (over the block, then
+// over the blocks' totals, which every block stores to every other), compaction
+// (each survivor stored straight into the window, and the halos, of the blocks
+// that hold its new position).  Two cluster barriers separate the steps, so no
+// iteration waits for the grid, a look-back or global memory; only new nodes and
+// the iteration records are written out.  When one segment holds every cluster the
+// other blocks leave and block 0 finishes alone.
+//
+// What it replaces (one grid barrier per iteration down to 992 clusters, then one
+// block): 9-20 us per iteration of latency, here 1.5-5 us; a 20,011-triangle
+// build PADDED_OLD -> PADDED_NEW us of PLOC.  Beyond 32,256 clusters (radius 16) the
+// whole GPU's search is faster than sixteen SMs'.
+constexpr int kClusterBlocks = 16, kClusterThreads = 512, kClusterTile = 4 * kClusterThreads;
+constexpr int kClusterMinSeg = 96;  // >= 2 * kPlocMaxRadius: a halo reaches only the adjacent segment
+static_assert(kClusterMinSeg >= 2 * kPlocMaxRadius, "halo");
+struct ClusterSmem {
+    PlocSmem<kClusterTile, kClusterThreads, kPlocMaxRadius> w;
+    uint32_t totals[2][kClusterBlocks];
+    uint32_t lcj[kClusterTile / kClusterThreads][kClusterThreads];  // a merge's right child's leaves
+};
+
+// Nearest neighbours of the positions [s - R, e + R) into nn (position s - R first).
+// Up to 128 positions: four threads each take a quarter of a position's 2R
+// candidates; the strict minimum, lowest j on ties, of ascending candidates is
+// the lexicographic minimum of (area, j).
+template <int RC, typename Smem>
+__device__ __forceinline__ void cluster_nearest(Smem& S, int s, int e, int n, int R_rt) {
+    const int R = RC > 0 ? RC : R_rt;
+    const int cnt = e - s + 2 * R;
+    if (cnt > kClusterThreads) {
+        ploc_nearest<RC>(S, s, e, n, R);
+        return;
+    }
+    if (cnt > kClusterThreads / 4) {
+        const int t = threadIdx.x, q = s - R + t;
+        if (t < cnt && q >= 0 && q < n) S.nn[t] = ploc_nearest_at<RC>(S, q, t + R, R);
+        return;
+    }
+    const int t = threadIdx.x >> 2, part = threadIdx.x & 3, q = s - R + t, w = t + R;
+    float best = __int_as_float(0x7F800000);
+    int bj = q;
+    if (t < cnt) {
+        const float amnx = S.mnx[w], amny = S.mny[w], amnz = S.mnz[w], amxx = S.mxx[w], amxy = S.mxy[w], amxz = S.mxz[w];
+        // offsets -R .. -1, 1 .. R in four runs
+        const int per = (2 * R + 3) / 4;
+        auto visit = [&](int k) {
+            const int d = k < R ? k - R : k - R + 1;
+            const int wj = w + d;
+            const float dx = fmaxf(amxx, S.mxx[wj]) - fminf(amnx, S.mnx[wj]);
+            const float dy = fmaxf(amxy, S.mxy[wj]) - fminf(amny, S.mny[wj]);
+            const float dz = fmaxf(amxz, S.mxz[wj]) - fminf(amnz, S.mnz[wj]);
+            const float v = 2.0f * (dx * dy + dy * dz + dz * dx);
+            if (v < best) { best = v; bj = q + d; }
+        };
+        if (RC > 0) {
+#pragma unroll
+            for (int u = 0; u < (RC + 1) / 2; ++u) visit(part * per + u);
+        } else {
+            for (int k = part * per; k < min(2 * R, (part + 1) * per); ++k) visit(k);
+        }
+    }
+#pragma unroll
+    for (int m = 1; m < 4; m <<= 1) {
+        const float ov = __shfl_xor_sync(0xFFFFFFFFu, best, m);
+        const int oj = __shfl_xor_sync(0xFFFFFFFFu, bj, m);
+        if (ov < best || (ov == best && oj < bj)) { best = ov; bj = oj; }
+    }
+    if (t < cnt && part == 0 && q >= 0 && q < n) S.nn[t] = static_cast<uint32_t>(bj);
+}
+
+template <int RC>
+__device__ __forceinline__ void ploc_cluster_r(ClusterSmem& C, int iter, const float4* __restrict__ cin,
+                                               float4* __restrict__ node_box, uint4* __restrict__ node_kids, uint2* it,
+                                               uint32_t N, int R_rt, uint32_t* iters_out, uint32_t* err) {
+    namespace cg = cooperative_groups;
+    auto cluster = cg::this_cluster();
+    auto& S = C.w;
+    constexpr int PMAX = kClusterTile / kClusterThreads;
+    const int R = RC > 0 ? RC : R_rt;
+    const int rank = static_cast<int>(cluster.block_rank()), blocks = static_cast<int>(cluster.num_blocks());
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const float inf = __int_as_float(0x7F800000);
+    auto segment = [&](int n) { return max((n + blocks - 1) / blocks, kClusterMinSeg); };
+    uint2 cur = __ldcg(it + iter);
+    int n = static_cast<int>(cur.x);
+    uint32_t idb = cur.y;
+    int seg = segment(n);
+    if (seg + 2 * R > kClusterTile) {  // the caller checked n <= ploc_cluster_max; only corruption gets here
+        if (rank == 0 && threadIdx.x == 0) raise_corrupt(err, 12, static_cast<uint32_t>(iter), static_cast<uint32_t>(n));
+        return;
+    }
+    int s = min(n, rank * seg), e = min(n, s + seg);
+    for (int w = threadIdx.x; w < seg + 4 * R; w += kClusterThreads) {
+        const int p = s + w - 2 * R;
+        if (p >= 0 && p < n) {
+            const float4 a = __ldcg(cin + 2 * static_cast<size_t>(p));
+            const float4 b = __ldcg(cin + 2 * static_cast<size_t>(p) + 1);
+            S.mnx[w] = a.x; S.mny[w] = a.y; S.mnz[w] = a.z; S.id[w] = __float_as_uint(a.w);
+            S.mxx[w] = b.x; S.mxy[w] = b.y; S.mxz[w] = b.z; S.lc[w] = __float_as_uint(b.w);
+        } else {
+            S.mnx[w] = -inf; S.mny[w] = -inf; S.mnz[w] = -inf;
+            S.mxx[w] = inf; S.mxy[w] = inf; S.mxz[w] = inf;
+        }
+    }
+    bool solo = false;  // one segment holds everything: this block alone
+    if (n <= seg) {
+        solo = true;
+        cluster.sync();  // nothing is stored to a block after this
+        if (rank != 0) return;
+    } else {
+        cluster.sync();  // every block has started: its memory may be stored to
+    }
+    for (int par = 0; n > 1; par ^= 1) {
+        if (static_cast<uint32_t>(iter) + 1 >= N) {  // uniform over the cluster
+            if (rank == 0 && threadIdx.x == 0) raise_error(err, kDevIterLimit);
+            break;
+        }
+        if (s < e) cluster_nearest<RC>(S, s, e, n, R);
+        __syncthreads();
+        const int k = (e - s + kClusterThreads - 1) / kClusterThreads;
+        const int p0 = s + k * static_cast<int>(threadIdx.x);
+        uint32_t flags = 0, nv = 0, nm = 0;
+#pragma unroll
+        for (int q = 0; q < PMAX; ++q) {
+            const int p = p0 + q;
+            if (q >= k || p >= e) continue;
+            const int j = static_cast<int>(S.nn[p - s + R]);
+            const bool mutual = (j != p) && (static_cast<int>(S.nn[j - s + R]) == p);
+            if (!(mutual && p > j)) { flags |= 1u << q; ++nv; }
+            if (mutual && p < j) { flags |= 1u << (16 + q); ++nm; }
+        }
+        // exclusive scan of (survivors, merges) in position order, 16|16 bits
+        const uint32_t packed = (nv << 16) | nm;
+        uint32_t incl = packed;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const uint32_t y = __shfl_up_sync(0xFFFFFFFFu, incl, o);
+            if (lane >= o) incl += y;
+        }
+        if (lane == 31) S.wsum[warp] = incl;
+        __syncthreads();
+        if (warp == 0) {
+            const uint32_t ws = lane < kClusterThreads / 32 ? static_cast<uint32_t>(S.wsum[lane]) : 0u;
+            uint32_t wi = ws;
+#pragma unroll
+            for (int o = 1; o < 32; o <<= 1) {
+                const uint32_t y = __shfl_up_sync(0xFFFFFFFFu, wi, o);
+                if (lane >= o) wi += y;
+            }
+            if (lane < kClusterThreads / 32) S.wsum[lane] = wi - ws;
+            const uint32_t total = __shfl_sync(0xFFFFFFFFu, wi, 31);
+            if (solo) {
+                if (lane == 0) C.totals[par][0] = total;
+            } else if (lane < blocks) {
+                cluster.map_shared_rank(&C.totals[par][0], lane)[rank] = total;
+            }
+        }
+        // the survivors' records, from this iteration's window
+        float4 omn[PMAX], omx[PMAX];
+        uint32_t part[PMAX];  // the merged partner's window index
+#pragma unroll
+        for (int q = 0; q < PMAX; ++q) {
+            if (!(flags & (1u << q))) continue;
+            const int wp = p0 + q - s + 2 * R;
+            omn[q] = make_float4(S.mnx[wp], S.mny[wp], S.mnz[wp], __uint_as_float(S.id[wp]));
+            omx[q] = make_float4(S.mxx[wp], S.mxy[wp], S.mxz[wp], __uint_as_float(S.lc[wp]));
+            part[q] = 0u;
+            if (flags & (1u << (16 + q))) {
+                const int wj = static_cast<int>(S.nn[p0 + q - s + R]) - s + 2 * R;
+                float4 m0, m1;  // AABB::merge (bvh.cpp:401-413), first argument = lower position
+                m0.x = min_std(omn[q].x, S.mnx[wj]); m0.y = min_std(omn[q].y, S.mny[wj]); m0.z = min_std(omn[q].z, S.mnz[wj]);
+                m1.x = max_std(omx[q].x, S.mxx[wj]); m1.y = max_std(omx[q].y, S.mxy[wj]); m1.z = max_std(omx[q].z, S.mxz[wj]);
+                m0.w = omn[q].w;  // left child id
+                m1.w = omx[q].w;  // left child's leaves
+                omn[q] = m0;
+                omx[q] = m1;
+                part[q] = S.id[wj];
+                C.lcj[q][threadIdx.x] = S.lc[wj];
+            }
+        }
+        if (solo) __syncthreads(); else cluster.sync();  // totals are in; every read of the windows is done
+        // (survivors and merges summed separately: the packed halves may overflow over the blocks)
+        uint32_t n_next = 0, merges = 0, bv = 0, bm = 0;
+        for (int r = 0; r < (solo ? 1 : blocks); ++r) {
+            const uint32_t v = C.totals[par][r];
+            n_next += v >> 16;
+            merges += v & 0xFFFFu;
+            if (r < rank) { bv += v >> 16; bm += v & 0xFFFFu; }
+        }
+        const uint32_t excl = static_cast<uint32_t>(S.wsum[warp]) + (incl - packed);
+        uint32_t out_v = bv + (excl >> 16);
+        uint32_t out_m = idb + bm + (excl & 0xFFFFu);
+        const int seg2 = solo ? seg : segment(static_cast<int>(n_next));
+        int owner = solo ? 0 : static_cast<int>(out_v) / seg2;
+        auto put = [&](int b, int w, const float4& mn, const float4& mx) {
+            auto& D = solo ? S : cluster.map_shared_rank(&C, b)->w;
+            D.mnx[w] = mn.x; D.mny[w] = mn.y; D.mnz[w] = mn.z; D.id[w] = __float_as_uint(mn.w);
+            D.mxx[w] = mx.x; D.mxy[w] = mx.y; D.mxz[w] = mx.z; D.lc[w] = __float_as_uint(mx.w);
+        };
+#pragma unroll
+        for (int q = 0; q < PMAX; ++q) {
+            if (!(flags & (1u << q))) continue;
+            float4 mn = omn[q], mx = omx[q];
+            if (flags & (1u << (16 + q))) {
+                const uint32_t id = out_m++;
+                if (id >= 2 * N - 1 || id < N) {
+                    raise_corrupt(err, 13 + (iter << 8), p0 + q, id);
+                } else {
+                    const uint32_t lcl = __float_as_uint(mx.w), lcr = C.lcj[q][threadIdx.x];
+                    node_box[2 * static_cast<size_t>(id)] = mn;
+                    node_box[2 * static_cast<size_t>(id) + 1] = make_float4(mx.x, mx.y, mx.z, __uint_as_float(part[q]));
+                    node_kids[id - N] = make_uint4(__float_as_uint(mn.w), part[q], lcl, lcr);
+                    mn.w = __uint_as_float(id);
+                    mx.w = __uint_as_float(lcl + lcr);
+                }
+            }
+            if (out_v >= n_next) { raise_corrupt(err, 14 + (iter << 8), p0 + q, out_v); continue; }
+            while (!solo && static_cast<int>(out_v) >= (owner + 1) * seg2) ++owner;
+            const int at = static_cast<int>(out_v) - owner * seg2;  // place in its segment
+            put(owner, at + 2 * R, mn, mx);
+            if (!solo) {
+                if (at < 2 * R && owner > 0) put(owner - 1, at + seg2 + 2 * R, mn, mx);
+                if (at >= seg2 - 2 * R && owner + 1 < blocks && (owner + 1) * seg2 < static_cast<int>(n_next))
+                    put(owner + 1, at - seg2 + 2 * R, mn, mx);
+            }
+            ++out_v;
+        }
+        s = min(static_cast<int>(n_next), rank * seg2);
+        e = min(static_cast<int>(n_next), s + seg2);
+        if (s < e)  // window entries past the last cluster
+            for (int w = static_cast<int>(n_next) - s + 2 * R + static_cast<int>(threadIdx.x); w < seg2 + 4 * R; w += kClusterThreads) {
+                S.mnx[w] = -inf; S.mny[w] = -inf; S.mnz[w] = -inf;
+                S.mxx[w] = inf; S.mxy[w] = inf; S.mxz[w] = inf;
+            }
+        n = static_cast<int>(n_next);
+        idb += merges;
+        seg = seg2;
+        ++iter;
+        if (rank == 0 && threadIdx.x == 0) it[iter] = make_uint2(n_next, idb);
+        if (solo) {
+            __syncthreads();
+        } else {
+            cluster.sync();
+            if (n <= seg) {
+                solo = true;
+                if (rank != 0) return;
+            }
+        }
+    }
+    if (rank == 0 && threadIdx.x == 0) iters_out[0] = static_cast<uint32_t>(iter);
+}
+
+template <int MAXR>
+__global__ void __launch_bounds__(kClusterThreads) ploc_cluster_kernel(const float4* ca, const float4* cb,
+                                                                       float4* __restrict__ node_box,
+                                                                       uint4* __restrict__ node_kids, uint2* it, uint32_t N,
+                                                                       int R, uint32_t* iters_out, uint32_t* err) {
+    extern __shared__ __align__(16) unsigned char cluster_smem[];
+    ClusterSmem& C = *reinterpret_cast<ClusterSmem*>(cluster_smem);
+    const int iter = static_cast<int>(__ldcg(iters_out));
+    const float4* cin = (iter & 1) ? cb : ca;
+    switch (R) {
+        case 8: ploc_cluster_r<8>(C, iter, cin, node_box, node_kids, it, N, R, iters_out, err); break;
+        case 16: ploc_cluster_r<16>(C, iter, cin, node_box, node_kids, it, N, R, iters_out, err); break;
+        case 32: ploc_cluster_r<32>(C, iter, cin, node_box, node_kids, it, N, R, iters_out, err); break;
+        default: ploc_cluster_r<0>(C, iter, cin, node_box, node_kids, it, N, R, iters_out, err); break;
+    }
+}
+
 template <int TILE, int BLOCK, int MAXR>
 __global__ void __launch_bounds__(BLOCK, kPlocBlocksPerSm) ploc_persistent_kernel(float4* ca, float4* cb, float4* __restrict__ node_box,
                                                                 uint4* __restrict__ node_kids, uint2* it, uint32_t N,
-                                                                int R, unsigned long long* lookback, uint32_t* tickets,
-                                                                uint32_t n_tiles_cap, uint2* pf, crt_bvh_node* out,
-                                                                float4* wide, float4* wide_wt, uint8_t* depth_odd,
-                                                                LeafOut lv, const SceneState* st, unsigned long long* bar,
-                                                                uint32_t* iters_out, uint32_t* err, uint32_t spin_limit) {
+                                                                int R, uint32_t stop_n, unsigned long long* lookback,
+                                                                uint32_t* tickets, uint32_t n_tiles_cap,
+                                                                unsigned long long* bar, uint32_t* iters_out,
+                                                                uint32_t* err, uint32_t spin_limit) {
     __shared__ PlocSmem<TILE, BLOCK, MAXR> S;
     __shared__ uint32_t s_tile;
     unsigned long long bar_target = 0;  // grid barriers passed x gridDim (thread 0)
-    // iters_out[0]: iterations; [1]: blocks finished; then 64-bit globaltimer
-    // stamps: start, end of the PLOC loop, end of the layout.
-    unsigned long long* stamp = reinterpret_cast<unsigned long long*>(iters_out + 2);
-    if (blockIdx.x == 0 && threadIdx.x == 0) stamp[0] = global_ns();
-    // The layout's records start unset: a node's position arrives from its
-    // parent (pf is not touched by the PLOC iterations, whose grid barriers
-    // order this reset before the layout).
-    for (uint32_t j = blockIdx.x * BLOCK + threadIdx.x; j + 1 < N; j += gridDim.x * BLOCK)
-        pf[j] = make_uint2(kLayoutUnset, 0u);
     int iter = 0;
-    bool tail = false;
     for (;; ++iter) {
         const uint2 cur = __ldcg(it + iter);
         if (cur.x <= 1u) break;
-        if (cur.x <= ploc_own(R)) { tail = true; break; }  // every block reads the same record
+        if (cur.x <= stop_n) break;  // every block reads the same record; the cluster kernel takes over
         const float4* cin = (iter & 1) ? cb : ca;
         float4* cout = (iter & 1) ? ca : cb;
         unsigned long long* lb_cur = lookback + static_cast<size_t>(iter & 1) * n_tiles_cap;
@@ -1262,30 +1529,20 @@ __global__ void __launch_bounds__(BLOCK, kPlocBlocksPerSm) ploc_persistent_kerne
         if (!grid_barrier(bar, bar_target, err, spin_limit)) return;
         if (static_cast<uint32_t>(iter) + 1 >= N) { raise_error(err, kDevIterLimit); return; }
     }
-    if (tail) {
-        // The remaining iterations fit in one tile each (the last few hundred
-        // clusters, which merge a few pairs per iteration): block 0 runs them
-        // alone on shared memory, while the others wait once.
-        if (blockIdx.x == 0) {
-            iter = ploc_tail<TILE, BLOCK, MAXR>(S, iter, (iter & 1) ? cb : ca, node_box, node_kids, it, N, R, err);
-            if (threadIdx.x == 0) iters_out[0] = static_cast<uint32_t>(iter);
-        }
-        if (!grid_barrier(bar, bar_target, err, spin_limit)) return;
-        iter = static_cast<int>(__ldcg(iters_out));
-    }
-    if (blockIdx.x == 0 && threadIdx.x == 0) {
-        iters_out[0] = static_cast<uint32_t>(iter);
-        stamp[1] = global_ns();
-    }
+    if (blockIdx.x == 0 && threadIdx.x == 0) iters_out[0] = static_cast<uint32_t>(iter);
+}
+
+// The layout's position pass in one cooperative launch.
+template <int BLOCK>
+__global__ void __launch_bounds__(BLOCK) layout_places_kernel(uint32_t* __restrict__ dfs, const uint4* __restrict__ node_kids,
+                                                              uint32_t N, uint2* pf, uint32_t* err, uint32_t spin_limit) {
     // DFS layout, position pass as dataflow: internal node ids grow with the
     // PLOC iteration that made them, so a parent's id is larger than its
     // children's and decreasing ids are a top-down order.  Every thread takes
     // the ids 2N-2, 2N-3, ... in grid-stride order and, before laying node X
     // out, waits (bounded) until X's parent has published X's position.  The
     // unfinished node with the largest id never waits (its parent is done), so
-    // the co-resident grid always progresses; one grid barrier before the
-    // emit pass replaces one barrier per PLOC level.
-    uint32_t* dfs = reinterpret_cast<uint32_t*>(ca);
+    // the co-resident grid always progresses, with no barrier per PLOC level.
     bool gave_up = false;
     for (uint32_t t = blockIdx.x * BLOCK + threadIdx.x; t + 1 < N && !gave_up; t += gridDim.x * BLOCK) {
         const uint32_t X = 2 * N - 2 - t;
@@ -1316,12 +1573,6 @@ __global__ void __launch_bounds__(BLOCK, kPlocBlocksPerSm) ploc_persistent_kerne
         if (top) layout_publish_grandchildren(me, kids, kc, pf, N);
         layout_down_at<true>(X, me, kids, pf, N, dfs, err);
     }
-    if (!grid_barrier(bar, bar_target, err, spin_limit)) return;
-    const float grow = st->abs_eps;
-    for (uint32_t p = blockIdx.x * BLOCK + threadIdx.x; p < 2 * N - 1; p += gridDim.x * BLOCK)
-        layout_emit(p, node_box, node_kids, pf, N, dfs, out, wide, wide_wt, depth_odd, lv, grow, err);
-    __syncthreads();
-    if (threadIdx.x == 0 && atomicAdd(iters_out + 1, 1u) + 1u == gridDim.x) stamp[2] = global_ns();
 }
 
 __global__ void single_leaf_kernel(const float4* __restrict__ node_box, crt_bvh_node* __restrict__ out, LeafOut lv) {
@@ -1619,8 +1870,8 @@ bool launch_digit_offsets(const uint32_t* counts, uint32_t places, int bits, uin
 }
 
 void launch_leaf_init(const crt_triangle* tris, uint32_t n, const float* models, const uint32_t* perm, float4* node_box,
-                      float4* clusters, float4* xtri_sorted, uint2* it, uint32_t* err, cudaStream_t s) {
-    leaf_init_kernel<<<(n + 255) / 256, 256, 0, s>>>(tris, n, models, perm, node_box, clusters, xtri_sorted, it, err);
+                      float4* clusters, float4* xtri_sorted, uint2* it, uint2* pf, uint32_t* err, cudaStream_t s) {
+    leaf_init_kernel<<<(n + 255) / 256, 256, 0, s>>>(tris, n, models, perm, node_box, clusters, xtri_sorted, it, pf, err);
 }
 
 void launch_ploc_iteration(const float4* cin, float4* cout, float4* node_box, uint4* node_kids, uint2* it,
@@ -1665,17 +1916,78 @@ int ploc_persistent_grid() {
     return grid;
 }
 
-cudaError_t launch_ploc_persistent(float4* ca, float4* cb, float4* node_box, uint4* node_kids, uint2* it, uint32_t N,
-                                   int radius, unsigned long long* lookback, uint32_t* tickets, uint32_t n_tiles_cap,
-                                   uint2* pf, crt_bvh_node* out, float4* wide, float4* wide_wt, uint8_t* depth_odd,
-                                   LeafOut lv, const SceneState* st, unsigned long long* bar, uint32_t* iters_out,
-                                   uint32_t* err, uint32_t spin_limit, cudaStream_t s) {
-    const int grid = ploc_persistent_grid();
-    if (grid <= 0) return cudaErrorNotSupported;
-    void* args[] = {&ca, &cb, &node_box, &node_kids, &it, &N, &radius, &lookback, &tickets, &n_tiles_cap, &pf, &out,
-                    &wide, &wide_wt, &depth_odd, &lv, &st, &bar, &iters_out, &err, &spin_limit};
-    return cudaLaunchCooperativeKernel(reinterpret_cast<const void*>(ploc_persistent_kernel<kPlocSpan, 256, kPlocMaxRadius>),
-                                       dim3(grid), dim3(256), args, 0, s);
+// Blocks of the cluster kernel's cluster on this device (0: it cannot run).
+static int ploc_cluster_blocks() {
+    static int blocks = -1;
+    if (blocks < 0) {
+        blocks = 0;
+        const void* f = reinterpret_cast<const void*>(ploc_cluster_kernel<kPlocMaxRadius>);
+        cudaFuncSetAttribute(f, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
+        cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(sizeof(ClusterSmem)));
+        for (int b = kClusterBlocks; b >= 8 && blocks == 0; b /= 2) {
+            cudaLaunchConfig_t c{};
+            cudaLaunchAttribute a{};
+            a.id = cudaLaunchAttributeClusterDimension;
+            a.val.clusterDim.x = b;
+            a.val.clusterDim.y = a.val.clusterDim.z = 1;
+            c.gridDim = dim3(b);
+            c.blockDim = dim3(kClusterThreads);
+            c.dynamicSmemBytes = sizeof(ClusterSmem);
+            c.attrs = &a;
+            c.numAttrs = 1;
+            int active = 0;
+            if (cudaOccupancyMaxActiveClusters(&active, f, &c) == cudaSuccess && active > 0) blocks = b;
+        }
+        cudaGetLastError();
+    }
+    return blocks;
+}
+
+cudaError_t launch_ploc_layout(float4* ca, float4* cb, float4* node_box, uint4* node_kids, uint2* it, uint32_t N,
+                               int radius, unsigned long long* lookback, uint32_t* tickets, uint32_t n_tiles_cap,
+                               uint2* pf, crt_bvh_node* out, float4* wide, float4* wide_wt, uint8_t* depth_odd,
+                               LeafOut lv, const SceneState* st, unsigned long long* bar, uint32_t* iters_out,
+                               uint32_t* err, uint32_t spin_limit, cudaEvent_t ploc_done, cudaStream_t s) {
+    const int grid = ploc_persistent_grid(), blocks = ploc_cluster_blocks();
+    if (grid <= 0 || blocks <= 0) return cudaErrorNotSupported;
+    uint32_t stop_n = static_cast<uint32_t>(blocks * (kClusterTile - 2 * radius));
+    cudaError_t e = cudaSuccess;
+    if (N > stop_n) {
+        void* args[] = {&ca, &cb, &node_box, &node_kids, &it, &N, &radius, &stop_n, &lookback, &tickets, &n_tiles_cap,
+                        &bar, &iters_out, &err, &spin_limit};
+        e = cudaLaunchCooperativeKernel(reinterpret_cast<const void*>(ploc_persistent_kernel<kPlocSpan, 256, kPlocMaxRadius>),
+                                        dim3(grid), dim3(256), args, 0, s);
+        if (e != cudaSuccess) return e;
+    }
+    cudaLaunchConfig_t c{};
+    cudaLaunchAttribute a{};
+    a.id = cudaLaunchAttributeClusterDimension;
+    a.val.clusterDim.x = blocks;
+    a.val.clusterDim.y = a.val.clusterDim.z = 1;
+    c.gridDim = dim3(blocks);
+    c.blockDim = dim3(kClusterThreads);
+    c.dynamicSmemBytes = sizeof(ClusterSmem);
+    c.stream = s;
+    c.attrs = &a;
+    c.numAttrs = 1;
+    e = cudaLaunchKernelEx(&c, ploc_cluster_kernel<kPlocMaxRadius>, static_cast<const float4*>(ca),
+                           static_cast<const float4*>(cb), node_box, node_kids, it, N, radius, iters_out, err);
+    if (e != cudaSuccess) return e;
+    cudaEventRecord(ploc_done, s);
+    static int place_grid = 0;
+    if (place_grid == 0) {
+        int per_sm = 0;
+        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, layout_places_kernel<256>, 256, 0);
+        place_grid = kNumSms * (per_sm > 0 ? per_sm : 1);
+    }
+    const uint32_t want = (N + 254) / 256;  // N - 1 internal nodes
+    uint32_t* dfs = reinterpret_cast<uint32_t*>(ca);
+    void* args[] = {&dfs, &node_kids, &N, &pf, &err, &spin_limit};
+    e = cudaLaunchCooperativeKernel(reinterpret_cast<const void*>(layout_places_kernel<256>),
+                                    dim3(want < static_cast<uint32_t>(place_grid) ? want : place_grid), dim3(256), args, 0, s);
+    if (e != cudaSuccess) return e;
+    launch_layout_emit(node_box, node_kids, pf, N, dfs, out, wide, wide_wt, depth_odd, lv, st, err, s);
+    return cudaGetLastError();
 }
 
 // A wait on a flag, bounded like every look-back and grid-barrier wait: on

@@ -78,7 +78,7 @@ void launch_onesweep_segments(const uint32_t* keys_in, const uint32_t* vals_in, 
 // xtri_sorted: the leaves' transformed triangles in sorted (Morton) order;
 // the layout moves them into tree order.
 void launch_leaf_init(const crt_triangle* tris, uint32_t n, const float* models, const uint32_t* perm, float4* node_box,
-                      float4* clusters, float4* xtri_sorted, uint2* it, uint32_t* err, cudaStream_t s);
+                      float4* clusters, float4* xtri_sorted, uint2* it, uint2* pf, uint32_t* err, cudaStream_t s);
 void launch_ploc_iteration(const float4* cin, float4* cout, float4* node_box, uint4* node_kids, uint2* it,
                            int iter, uint32_t N, int radius, uint32_t n_upper,
                            unsigned long long* lookback, uint32_t* tickets, uint32_t n_tiles_cap, uint32_t* err,
@@ -105,13 +105,15 @@ void launch_wide4(const float4* wide, const uint8_t* depth_odd, uint32_t n_inter
 // quantised (non-finite coordinates, a scene range outside 2^-40 .. 2^50).
 void launch_cwide(const float4* wide, uint32_t n_internal, float abs_eps, uint4* cwide, uint32_t* bad, cudaStream_t s);
 void launch_single_leaf(const float4* node_box, crt_bvh_node* out, LeafOut leaves, cudaStream_t s);
-// All PLOC iterations and the DFS layout in one cooperative launch; returns
-// cudaErrorNotSupported when a cooperative launch is unavailable.
-cudaError_t launch_ploc_persistent(float4* ca, float4* cb, float4* node_box, uint4* node_kids, uint2* it, uint32_t N,
-                                   int radius, unsigned long long* lookback, uint32_t* tickets, uint32_t n_tiles_cap,
-                                   uint2* pf, crt_bvh_node* out, float4* wide, float4* wide_wt, uint8_t* depth_odd,
-                                   LeafOut leaves, const SceneState* st, unsigned long long* bar, uint32_t* iters_out,
-                                   uint32_t* err, uint32_t spin_limit, cudaStream_t s);
+// All PLOC iterations (a cooperative launch while the clusters are many, then one
+// thread-block cluster) and the DFS layout; ploc_done is recorded between the two.
+// iters_out[0] (zero before) receives the iteration count.
+// cudaErrorNotSupported when a cooperative or cluster launch is unavailable.
+cudaError_t launch_ploc_layout(float4* ca, float4* cb, float4* node_box, uint4* node_kids, uint2* it, uint32_t N,
+                               int radius, unsigned long long* lookback, uint32_t* tickets, uint32_t n_tiles_cap,
+                               uint2* pf, crt_bvh_node* out, float4* wide, float4* wide_wt, uint8_t* depth_odd,
+                               LeafOut leaves, const SceneState* st, unsigned long long* bar, uint32_t* iters_out,
+                               uint32_t* err, uint32_t spin_limit, cudaEvent_t ploc_done, cudaStream_t s);
 
 // Refit (crt_refit.cu).  The slack of the refit tree's root box goes to
 // abs_eps for the host.
