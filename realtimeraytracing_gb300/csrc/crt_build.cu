@@ -1185,7 +1185,7 @@ __device__ __forceinline__ bool grid_barrier(unsigned long long* bar, unsigned l
 
 // =============================== K3 on a cluster: the last PLOC iterations
 // Once the live clusters fit in the shared memory of one thread-block cluster
-// (n <= ploc_cluster_max), it runs the remaining iterations there: block c holds
+// (n <= 16 (2048 - 2R)), it runs the remaining iterations there: block c holds
 // the positions [c seg, (c + 1) seg) and a halo of 2R on each side in the window
 // layout of a tile that starts at its first position.  An iteration is the
 // reference's, as in ploc_tile: nearest neighbours, mutual pairs merged at the
@@ -1197,86 +1197,85 @@ __device__ __forceinline__ bool grid_barrier(unsigned long long* bar, unsigned l
 // the iteration records are written out.  When one segment holds every cluster the
 // other blocks leave and block 0 finishes alone.
 //
-// What it replaces (one grid barrier per iteration down to 992 clusters, then one
-// block): 9-20 us per iteration of latency, here 1.5-5 us; a 20,011-triangle
-// build PADDED_OLD -> PADDED_NEW us of PLOC.  Beyond 32,256 clusters (radius 16) the
-// whole GPU's search is faster than sixteen SMs'.
+// Bound by the latency of an iteration's chain: a search of 0.7-1.2 k cycles (2 R
+// candidates over four, two or one threads a position), two scans, and two cluster
+// barriers of ~1.3 k each; warps without positions only take the barriers.  What
+// it replaces (one grid barrier an iteration down to 992 clusters, then one block)
+// took 9-20 us an iteration, this 2.3-4.  PLOC of N clusters, us: 1,000 78, 4,000
+// 98, 16,000 127, 32,000 168, 65,536 227 (before, 20,011: 258, now 135).  With
+// 1,024 threads of two positions: 86, 113, 145, 186, 244 (more warps to wait for
+// at each barrier); with 8 blocks of 512 32,000 217 and 65,536 260.  Beyond 32,256
+// clusters (radius 16) the whole GPU's search is faster than sixteen SMs'.
 constexpr int kClusterBlocks = 16, kClusterThreads = 512, kClusterTile = 4 * kClusterThreads;
-constexpr int kClusterMinSeg = 96;  // >= 2 * kPlocMaxRadius: a halo reaches only the adjacent segment
+constexpr int kClusterMinSeg = 64;  // >= 2 * kPlocMaxRadius: a halo reaches only the adjacent segment
 static_assert(kClusterMinSeg >= 2 * kPlocMaxRadius, "halo");
-struct ClusterSmem {
-    PlocSmem<kClusterTile, kClusterThreads, kPlocMaxRadius> w;
-    uint32_t totals[2][kClusterBlocks];
-    uint32_t lcj[kClusterTile / kClusterThreads][kClusterThreads];  // a merge's right child's leaves
+struct ClusterSmem : PlocSmem<kClusterTile, kClusterThreads, kPlocMaxRadius> {
+    __align__(16) uint32_t totals[2][kClusterBlocks];  // every block's survivors << 16 | merges
+    uint32_t gsum[kClusterTile / 32];                  // the same per 32 positions
 };
 
-// Nearest neighbours of the positions [s - R, e + R) into nn (position s - R first).
-// Up to 128 positions: four threads each take a quarter of a position's 2R
-// candidates; the strict minimum, lowest j on ties, of ascending candidates is
-// the lexicographic minimum of (area, j).
-template <int RC, typename Smem>
-__device__ __forceinline__ void cluster_nearest(Smem& S, int s, int e, int n, int R_rt) {
+// Nearest neighbours of the positions [s - R, e + R) into nn (position s - R
+// first).  PARTS threads share a position's 2R candidates, in ascending runs; the
+// strict minimum, lowest j on ties, is the lexicographic minimum of (area, j).
+template <int RC, int PARTS>
+__device__ __forceinline__ void cluster_nearest(ClusterSmem& S, int s, int e, int n, int R_rt) {
     const int R = RC > 0 ? RC : R_rt;
-    const int cnt = e - s + 2 * R;
-    if (cnt > kClusterThreads) {
-        ploc_nearest<RC>(S, s, e, n, R);
-        return;
-    }
-    if (cnt > kClusterThreads / 4) {
-        const int t = threadIdx.x, q = s - R + t;
-        if (t < cnt && q >= 0 && q < n) S.nn[t] = ploc_nearest_at<RC>(S, q, t + R, R);
-        return;
-    }
-    const int t = threadIdx.x >> 2, part = threadIdx.x & 3, q = s - R + t, w = t + R;
-    float best = __int_as_float(0x7F800000);
-    int bj = q;
-    if (t < cnt) {
-        const float amnx = S.mnx[w], amny = S.mny[w], amnz = S.mnz[w], amxx = S.mxx[w], amxy = S.mxy[w], amxz = S.mxz[w];
-        // offsets -R .. -1, 1 .. R in four runs
-        const int per = (2 * R + 3) / 4;
-        auto visit = [&](int k) {
-            const int d = k < R ? k - R : k - R + 1;
-            const int wj = w + d;
-            const float dx = fmaxf(amxx, S.mxx[wj]) - fminf(amnx, S.mnx[wj]);
-            const float dy = fmaxf(amxy, S.mxy[wj]) - fminf(amny, S.mny[wj]);
-            const float dz = fmaxf(amxz, S.mxz[wj]) - fminf(amnz, S.mnz[wj]);
-            const float v = 2.0f * (dx * dy + dy * dz + dz * dx);
-            if (v < best) { best = v; bj = q + d; }
-        };
-        if (RC > 0) {
+    const int cnt = e - s + 2 * R, part = static_cast<int>(threadIdx.x) % PARTS;
+    // whole warps enter together (they exchange below)
+    for (int t0 = static_cast<int>(threadIdx.x & ~31u) / PARTS; t0 < cnt; t0 += kClusterThreads / PARTS) {
+        const int t = t0 + static_cast<int>(threadIdx.x & 31u) / PARTS, q = s - R + t, w = t + R;
+        float best = __int_as_float(0x7F800000);
+        int bj = q;
+        if (t < cnt) {
+            const float amnx = S.mnx[w], amny = S.mny[w], amnz = S.mnz[w], amxx = S.mxx[w], amxy = S.mxy[w], amxz = S.mxz[w];
+            auto visit = [&](int k) {  // candidate k of the offsets -R .. -1, 1 .. R
+                const int d = k < R ? k - R : k - R + 1;
+                const int wj = w + d;
+                const float dx = fmaxf(amxx, S.mxx[wj]) - fminf(amnx, S.mnx[wj]);
+                const float dy = fmaxf(amxy, S.mxy[wj]) - fminf(amny, S.mny[wj]);
+                const float dz = fmaxf(amxz, S.mxz[wj]) - fminf(amnz, S.mnz[wj]);
+                const float v = 2.0f * (dx * dy + dy * dz + dz * dx);
+                if (v < best) { best = v; bj = q + d; }
+            };
+            if (RC > 0) {
+                static_assert((2 * RC) % PARTS == 0, "equal runs");
 #pragma unroll
-            for (int u = 0; u < (RC + 1) / 2; ++u) visit(part * per + u);
-        } else {
-            for (int k = part * per; k < min(2 * R, (part + 1) * per); ++k) visit(k);
+                for (int u = 0; u < 2 * RC / PARTS; ++u) visit(part * (2 * RC / PARTS) + u);
+            } else {
+                const int per = (2 * R + PARTS - 1) / PARTS;
+                for (int k = part * per; k < min(2 * R, (part + 1) * per); ++k) visit(k);
+            }
         }
-    }
 #pragma unroll
-    for (int m = 1; m < 4; m <<= 1) {
-        const float ov = __shfl_xor_sync(0xFFFFFFFFu, best, m);
-        const int oj = __shfl_xor_sync(0xFFFFFFFFu, bj, m);
-        if (ov < best || (ov == best && oj < bj)) { best = ov; bj = oj; }
+        for (int m = 1; m < PARTS; m <<= 1) {
+            const float ov = __shfl_xor_sync(0xFFFFFFFFu, best, m);
+            const int oj = __shfl_xor_sync(0xFFFFFFFFu, bj, m);
+            if (ov < best || (ov == best && oj < bj)) { best = ov; bj = oj; }
+        }
+        if (t < cnt && part == 0 && q >= 0 && q < n) S.nn[t] = static_cast<uint32_t>(bj);
     }
-    if (t < cnt && part == 0 && q >= 0 && q < n) S.nn[t] = static_cast<uint32_t>(bj);
 }
 
 template <int RC>
-__device__ __forceinline__ void ploc_cluster_r(ClusterSmem& C, int iter, const float4* __restrict__ cin,
+__device__ __forceinline__ void ploc_cluster_r(ClusterSmem& S, int iter, const float4* __restrict__ cin,
                                                float4* __restrict__ node_box, uint4* __restrict__ node_kids, uint2* it,
                                                uint32_t N, int R_rt, uint32_t* iters_out, uint32_t* err) {
     namespace cg = cooperative_groups;
     auto cluster = cg::this_cluster();
-    auto& S = C.w;
-    constexpr int PMAX = kClusterTile / kClusterThreads;
+    constexpr int PMAX = kClusterTile / kClusterThreads, WARPS = kClusterThreads / 32;
+    static_assert(kClusterTile / 32 == 64, "the block scan takes 64 groups of positions in two rounds of lanes");
     const int R = RC > 0 ? RC : R_rt;
     const int rank = static_cast<int>(cluster.block_rank()), blocks = static_cast<int>(cluster.num_blocks());
+    const int log_blocks = 31 - __clz(blocks);
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const uint32_t lt_mask = (1u << lane) - 1u;
     const float inf = __int_as_float(0x7F800000);
-    auto segment = [&](int n) { return max((n + blocks - 1) / blocks, kClusterMinSeg); };
-    uint2 cur = __ldcg(it + iter);
+    auto segment = [&](int n) { return max((n + blocks - 1) >> log_blocks, kClusterMinSeg); };
+    const uint2 cur = __ldcg(it + iter);
     int n = static_cast<int>(cur.x);
     uint32_t idb = cur.y;
     int seg = segment(n);
-    if (seg + 2 * R > kClusterTile) {  // the caller checked n <= ploc_cluster_max; only corruption gets here
+    if (seg + 2 * R > kClusterTile) {  // the caller checked n <= blocks * (tile - 2R); only corruption gets here
         if (rank == 0 && threadIdx.x == 0) raise_corrupt(err, 12, static_cast<uint32_t>(iter), static_cast<uint32_t>(n));
         return;
     }
@@ -1293,128 +1292,147 @@ __device__ __forceinline__ void ploc_cluster_r(ClusterSmem& C, int iter, const f
             S.mxx[w] = inf; S.mxy[w] = inf; S.mxz[w] = inf;
         }
     }
-    bool solo = false;  // one segment holds everything: this block alone
-    if (n <= seg) {
-        solo = true;
-        cluster.sync();  // nothing is stored to a block after this
-        if (rank != 0) return;
-    } else {
-        cluster.sync();  // every block has started: its memory may be stored to
-    }
+    if (threadIdx.x < 2 * kClusterBlocks) (&S.totals[0][0])[threadIdx.x] = 0u;
+    // one segment holds everything: this block alone
+    bool solo = n <= seg;
+    cluster.sync();  // every block has started (its memory may be stored to), or is not needed
+    if (solo && rank != 0) return;
     for (int par = 0; n > 1; par ^= 1) {
         if (static_cast<uint32_t>(iter) + 1 >= N) {  // uniform over the cluster
             if (rank == 0 && threadIdx.x == 0) raise_error(err, kDevIterLimit);
             break;
         }
-        if (s < e) cluster_nearest<RC>(S, s, e, n, R);
+        if (s < e) {
+            const int cnt = e - s + 2 * R;
+            if (cnt <= kClusterThreads / 4) cluster_nearest<RC, 4>(S, s, e, n, R);
+            else if (cnt <= kClusterThreads / 2) cluster_nearest<RC, 2>(S, s, e, n, R);
+            else if (cnt <= 2 * kClusterThreads) cluster_nearest<RC, 1>(S, s, e, n, R);
+            else ploc_nearest<RC>(S, s, e, n, R);
+        }
         __syncthreads();
-        const int k = (e - s + kClusterThreads - 1) / kClusterThreads;
-        const int p0 = s + k * static_cast<int>(threadIdx.x);
-        uint32_t flags = 0, nv = 0, nm = 0;
+        // Thread t decides positions s + t, s + 512 + t, ...: what survives, what
+        // merges, and the prefix counts of both, by groups of 32 positions.
+        // Warps without positions only take part in the barriers: an iteration is
+        // bound by the instructions its blocks issue.
+        const int own = e - s, groups = (own + 31) >> 5;
+        uint32_t keep[PMAX], head[PMAX];  // the warp's lanes that survive / that merge
+        int nb[PMAX];                     // neighbour's window index
 #pragma unroll
         for (int q = 0; q < PMAX; ++q) {
-            const int p = p0 + q;
-            if (q >= k || p >= e) continue;
-            const int j = static_cast<int>(S.nn[p - s + R]);
-            const bool mutual = (j != p) && (static_cast<int>(S.nn[j - s + R]) == p);
-            if (!(mutual && p > j)) { flags |= 1u << q; ++nv; }
-            if (mutual && p < j) { flags |= 1u << (16 + q); ++nm; }
+            keep[q] = head[q] = 0u;
+            nb[q] = 0;
+            if (q * WARPS + warp >= groups) continue;
+            const int p = s + q * kClusterThreads + static_cast<int>(threadIdx.x);
+            bool kp = false, hd = false;
+            if (p < e) {
+                const int j = static_cast<int>(S.nn[p - s + R]);
+                const bool mutual = (j != p) && (static_cast<int>(S.nn[j - s + R]) == p);
+                kp = !(mutual && p > j);
+                hd = mutual && p < j;
+                nb[q] = j - s + 2 * R;
+            }
+            keep[q] = __ballot_sync(0xFFFFFFFFu, kp);
+            head[q] = __ballot_sync(0xFFFFFFFFu, hd);
+            if (lane == 0) S.gsum[q * WARPS + warp] = (static_cast<uint32_t>(__popc(keep[q])) << 16) | __popc(head[q]);
         }
-        // exclusive scan of (survivors, merges) in position order, 16|16 bits
-        const uint32_t packed = (nv << 16) | nm;
-        uint32_t incl = packed;
-#pragma unroll
-        for (int o = 1; o < 32; o <<= 1) {
-            const uint32_t y = __shfl_up_sync(0xFFFFFFFFu, incl, o);
-            if (lane >= o) incl += y;
-        }
-        if (lane == 31) S.wsum[warp] = incl;
         __syncthreads();
-        if (warp == 0) {
-            const uint32_t ws = lane < kClusterThreads / 32 ? static_cast<uint32_t>(S.wsum[lane]) : 0u;
-            uint32_t wi = ws;
+        // each such warp scans the groups' totals (survivors << 16 | merges)
+        uint32_t excl[PMAX] = {};
+        if (warp < groups || warp == 0) {
+            uint32_t total = 0;
 #pragma unroll
-            for (int o = 1; o < 32; o <<= 1) {
-                const uint32_t y = __shfl_up_sync(0xFFFFFFFFu, wi, o);
-                if (lane >= o) wi += y;
+            for (int r = 0; r < 2; ++r) {
+                if (r > 0 && groups <= 32) break;
+                const uint32_t v = 32 * r + lane < groups ? S.gsum[32 * r + lane] : 0u;
+                uint32_t incl = v;
+#pragma unroll
+                for (int o = 1; o < 32; o <<= 1) {
+                    const uint32_t y = __shfl_up_sync(0xFFFFFFFFu, incl, o);
+                    if (lane >= o) incl += y;
+                }
+#pragma unroll
+                for (int q = 0; q < PMAX; ++q) {
+                    const int g = q * WARPS + warp;  // this warp's groups are every WARPS-th
+                    const uint32_t x = __shfl_sync(0xFFFFFFFFu, incl - v, g & 31);
+                    if (g >> 5 == r) excl[q] = total + x;
+                }
+                total += __shfl_sync(0xFFFFFFFFu, incl, 31);
             }
-            if (lane < kClusterThreads / 32) S.wsum[lane] = wi - ws;
-            const uint32_t total = __shfl_sync(0xFFFFFFFFu, wi, 31);
-            if (solo) {
-                if (lane == 0) C.totals[par][0] = total;
-            } else if (lane < blocks) {
-                cluster.map_shared_rank(&C.totals[par][0], lane)[rank] = total;
-            }
+            if (warp == 0 && lane < (solo ? 1 : blocks)) cluster.map_shared_rank(&S.totals[par][0], lane)[rank] = total;
         }
         // the survivors' records, from this iteration's window
         float4 omn[PMAX], omx[PMAX];
-        uint32_t part[PMAX];  // the merged partner's window index
+        uint32_t right[PMAX], right_lc[PMAX];  // a merge's right child and its leaves
 #pragma unroll
         for (int q = 0; q < PMAX; ++q) {
-            if (!(flags & (1u << q))) continue;
-            const int wp = p0 + q - s + 2 * R;
+            if (!(keep[q] >> lane & 1u)) continue;
+            const int wp = q * kClusterThreads + static_cast<int>(threadIdx.x) + 2 * R;
             omn[q] = make_float4(S.mnx[wp], S.mny[wp], S.mnz[wp], __uint_as_float(S.id[wp]));
             omx[q] = make_float4(S.mxx[wp], S.mxy[wp], S.mxz[wp], __uint_as_float(S.lc[wp]));
-            part[q] = 0u;
-            if (flags & (1u << (16 + q))) {
-                const int wj = static_cast<int>(S.nn[p0 + q - s + R]) - s + 2 * R;
-                float4 m0, m1;  // AABB::merge (bvh.cpp:401-413), first argument = lower position
-                m0.x = min_std(omn[q].x, S.mnx[wj]); m0.y = min_std(omn[q].y, S.mny[wj]); m0.z = min_std(omn[q].z, S.mnz[wj]);
-                m1.x = max_std(omx[q].x, S.mxx[wj]); m1.y = max_std(omx[q].y, S.mxy[wj]); m1.z = max_std(omx[q].z, S.mxz[wj]);
-                m0.w = omn[q].w;  // left child id
-                m1.w = omx[q].w;  // left child's leaves
-                omn[q] = m0;
-                omx[q] = m1;
-                part[q] = S.id[wj];
-                C.lcj[q][threadIdx.x] = S.lc[wj];
+            if (head[q] >> lane & 1u) {  // AABB::merge (bvh.cpp:401-413), first argument = lower position
+                const int wj = nb[q];
+                omn[q].x = min_std(omn[q].x, S.mnx[wj]); omn[q].y = min_std(omn[q].y, S.mny[wj]); omn[q].z = min_std(omn[q].z, S.mnz[wj]);
+                omx[q].x = max_std(omx[q].x, S.mxx[wj]); omx[q].y = max_std(omx[q].y, S.mxy[wj]); omx[q].z = max_std(omx[q].z, S.mxz[wj]);
+                right[q] = S.id[wj];
+                right_lc[q] = S.lc[wj];
             }
         }
-        if (solo) __syncthreads(); else cluster.sync();  // totals are in; every read of the windows is done
-        // (survivors and merges summed separately: the packed halves may overflow over the blocks)
-        uint32_t n_next = 0, merges = 0, bv = 0, bm = 0;
-        for (int r = 0; r < (solo ? 1 : blocks); ++r) {
-            const uint32_t v = C.totals[par][r];
-            n_next += v >> 16;
-            merges += v & 0xFFFFu;
-            if (r < rank) { bv += v >> 16; bm += v & 0xFFFFu; }
+        uint32_t n_next = 0u, merges = 0u, bv = 0u, bm = 0u;
+        if (solo) {
+            __syncthreads();  // every read of the window is done, the total is in
+            n_next = S.totals[par][0] >> 16;
+            merges = S.totals[par][0] & 0xFFFFu;
+        } else {
+            cluster.sync();
+#pragma unroll
+            for (int r = 0; r < kClusterBlocks; r += 4) {
+                const uint4 t = *reinterpret_cast<const uint4*>(&S.totals[par][r]);  // 0 past the cluster's blocks
+                const uint32_t v[4] = {t.x, t.y, t.z, t.w};
+#pragma unroll
+                for (int u = 0; u < 4; ++u) {
+                    if (r + u == rank) { bv = n_next; bm = merges; }
+                    n_next += v[u] >> 16;
+                    merges += v[u] & 0xFFFFu;
+                }
+            }
         }
-        const uint32_t excl = static_cast<uint32_t>(S.wsum[warp]) + (incl - packed);
-        uint32_t out_v = bv + (excl >> 16);
-        uint32_t out_m = idb + bm + (excl & 0xFFFFu);
         const int seg2 = solo ? seg : segment(static_cast<int>(n_next));
-        int owner = solo ? 0 : static_cast<int>(out_v) / seg2;
+        const float per_seg = 1.0f / static_cast<float>(seg2);
         auto put = [&](int b, int w, const float4& mn, const float4& mx) {
-            auto& D = solo ? S : cluster.map_shared_rank(&C, b)->w;
+            ClusterSmem& D = solo ? S : *cluster.map_shared_rank(&S, b);
             D.mnx[w] = mn.x; D.mny[w] = mn.y; D.mnz[w] = mn.z; D.id[w] = __float_as_uint(mn.w);
             D.mxx[w] = mx.x; D.mxy[w] = mx.y; D.mxz[w] = mx.z; D.lc[w] = __float_as_uint(mx.w);
         };
 #pragma unroll
         for (int q = 0; q < PMAX; ++q) {
-            if (!(flags & (1u << q))) continue;
+            if (!(keep[q] >> lane & 1u)) continue;
+            const uint32_t out_v = bv + (excl[q] >> 16) + __popc(keep[q] & lt_mask);
             float4 mn = omn[q], mx = omx[q];
-            if (flags & (1u << (16 + q))) {
-                const uint32_t id = out_m++;
+            if (head[q] >> lane & 1u) {
+                const uint32_t id = idb + bm + (excl[q] & 0xFFFFu) + __popc(head[q] & lt_mask);
                 if (id >= 2 * N - 1 || id < N) {
-                    raise_corrupt(err, 13 + (iter << 8), p0 + q, id);
+                    raise_corrupt(err, 13 + (iter << 8), out_v, id);
                 } else {
-                    const uint32_t lcl = __float_as_uint(mx.w), lcr = C.lcj[q][threadIdx.x];
-                    node_box[2 * static_cast<size_t>(id)] = mn;
-                    node_box[2 * static_cast<size_t>(id) + 1] = make_float4(mx.x, mx.y, mx.z, __uint_as_float(part[q]));
-                    node_kids[id - N] = make_uint4(__float_as_uint(mn.w), part[q], lcl, lcr);
+                    const uint32_t left_lc = __float_as_uint(mx.w);
+                    node_box[2 * static_cast<size_t>(id)] = mn;  // .w: left child, then right child
+                    node_box[2 * static_cast<size_t>(id) + 1] = make_float4(mx.x, mx.y, mx.z, __uint_as_float(right[q]));
+                    node_kids[id - N] = make_uint4(__float_as_uint(mn.w), right[q], left_lc, right_lc[q]);
                     mn.w = __uint_as_float(id);
-                    mx.w = __uint_as_float(lcl + lcr);
+                    mx.w = __uint_as_float(left_lc + right_lc[q]);
                 }
             }
-            if (out_v >= n_next) { raise_corrupt(err, 14 + (iter << 8), p0 + q, out_v); continue; }
-            while (!solo && static_cast<int>(out_v) >= (owner + 1) * seg2) ++owner;
-            const int at = static_cast<int>(out_v) - owner * seg2;  // place in its segment
-            put(owner, at + 2 * R, mn, mx);
-            if (!solo) {
-                if (at < 2 * R && owner > 0) put(owner - 1, at + seg2 + 2 * R, mn, mx);
-                if (at >= seg2 - 2 * R && owner + 1 < blocks && (owner + 1) * seg2 < static_cast<int>(n_next))
-                    put(owner + 1, at - seg2 + 2 * R, mn, mx);
+            if (out_v >= n_next) { raise_corrupt(err, 14 + (iter << 8), out_v, n_next); continue; }
+            if (solo) {
+                put(0, static_cast<int>(out_v) + 2 * R, mn, mx);
+                continue;
             }
-            ++out_v;
+            int owner = __float2int_rz(static_cast<float>(out_v) * per_seg);  // the quotient, or next to it
+            int at = static_cast<int>(out_v) - owner * seg2;                  // place in its segment
+            if (at < 0) { --owner; at += seg2; }
+            if (at >= seg2) { ++owner; at -= seg2; }
+            put(owner, at + 2 * R, mn, mx);
+            if (at < 2 * R && owner > 0) put(owner - 1, at + seg2 + 2 * R, mn, mx);
+            if (at >= seg2 - 2 * R && (owner + 1) * seg2 < static_cast<int>(n_next)) put(owner + 1, at - seg2 + 2 * R, mn, mx);
         }
         s = min(static_cast<int>(n_next), rank * seg2);
         e = min(static_cast<int>(n_next), s + seg2);
@@ -1432,10 +1450,8 @@ __device__ __forceinline__ void ploc_cluster_r(ClusterSmem& C, int iter, const f
             __syncthreads();
         } else {
             cluster.sync();
-            if (n <= seg) {
-                solo = true;
-                if (rank != 0) return;
-            }
+            solo = n <= seg;
+            if (solo && rank != 0) return;
         }
     }
     if (rank == 0 && threadIdx.x == 0) iters_out[0] = static_cast<uint32_t>(iter);

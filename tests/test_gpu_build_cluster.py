@@ -1,0 +1,46 @@
+"""The PLOC iterations that one thread-block cluster runs in shared memory, at
+the sizes where its split can go wrong: one segment exactly full and one past it
+(64 positions), sixteen minimal segments (1,024), the largest number of clusters
+that fits (16 segments of 2,048 positions less two halos of R) and one past it,
+where the whole GPU runs the first iterations.  The tree is the oracle's, bit for
+bit, and the per-iteration launches' (srcCommon/scene/geometry/bvh.cpp)."""
+import numpy as np
+import pytest
+
+from oracle import oracle as O
+from realtimeraytracing_gb300 import crt
+from realtimeraytracing_gb300 import scenes as S
+
+pytestmark = pytest.mark.gpu
+
+
+def _fits(radius):
+    return 16 * (2048 - 2 * radius)
+
+
+def _check(tris, radius):
+    n = tris.shape[0]
+    ref = O.build_bvh(tris, n, S.identity_models(1), radius=radius)
+    want = ref["nodes"].view(np.uint32)
+    for multi in (False, True):
+        c = crt.Context(ploc_radius=radius, multi_launch_build=multi)
+        got = c.build(tris, models=S.identity_models(1)).nodes().view(np.uint32)
+        assert c.last_build_stats()["ploc_iterations"] == ref["iterations"]
+        c.close()
+        np.testing.assert_array_equal(got, want)
+
+
+@pytest.mark.parametrize("radius", [16, 8, 32, 5])
+@pytest.mark.parametrize("at", [64, 1024, "largest"])
+@pytest.mark.parametrize("off", [-1, 0, 1])
+def test_segment_edges(radius, at, off):
+    n = (_fits(radius) if at == "largest" else at) + off
+    _check(S.uniform_soup(n, seed=n + radius), radius)
+
+
+@pytest.mark.parametrize("radius", [16, 32, 7])
+def test_equal_boxes(radius):
+    """Groups of equal triangles: ties of the surface area go to the lowest
+    position, also where the candidates are split over threads."""
+    one = S.uniform_soup(40, seed=5)
+    _check(np.repeat(one, 37, axis=0), radius)
