@@ -2064,18 +2064,18 @@ crt_status batch_enqueue(crt_ctx* x, crt_batch* bt, const crt_triangle* tris, co
     crt::launch_batch_leaf_init(tris, bt->n_tris, bt->scenes.as<crt::BatchScene>(), bt->n_scenes, bt->models.as<float>(),
                                 bt->perm_global.as<uint32_t>(), bt->perm_local.as<uint32_t>(), bt->node_box.as<float4>(),
                                 bt->clus_a.as<float4>(), bt->xtri_sorted.as<float4>(), bt->xtri.as<float4>(),
-                                bt->inv_perm.as<uint32_t>(), bt->it.as<uint2>(), bt->nodes.as<crt_bvh_node>(), err, s);
+                                bt->inv_perm.as<uint32_t>(), bt->it.as<uint2>(), bt->nodes.as<crt_bvh_node>(),
+                                bt->pf.as<uint2>(), err, s);
     {
         unsigned long long* lb = bt->ploc_lb.as<unsigned long long>();
         uint32_t* tail = reinterpret_cast<uint32_t*>(lb + 2ull * bt->lb_cap);
         const cudaError_t e = crt::launch_batch_ploc(
-            bt->scenes.as<crt::BatchScene>(), bt->n_scenes, bt->clus_a.as<float4>(), bt->clus_b.as<float4>(),
-            bt->node_box.as<float4>(), bt->node_kids.as<uint4>(), bt->it.as<uint2>(), static_cast<int>(bt->cfg.ploc_radius),
+            bt->scenes.as<crt::BatchScene>(), bt->n_scenes, bt->n_tris, bt->max_n, bt->clus_a.as<float4>(),
+            bt->clus_b.as<float4>(), bt->node_box.as<float4>(), bt->node_kids.as<uint4>(), bt->it.as<uint2>(), static_cast<int>(bt->cfg.ploc_radius),
             lb, bt->lb_cap, tail, bt->pf.as<uint2>(), bt->nodes.as<crt_bvh_node>(), bt->wide.as<float4>(),
             bt->wide_wt.as<float4>(), bt->depth_odd.as<uint8_t>(),
             crt::LeafOut{bt->xtri_sorted.as<float4>(), bt->xtri.as<float4>(), bt->inv_perm.as<uint32_t>()},
-            reinterpret_cast<unsigned long long*>(tail + 2),
-            bt->max_n + 1, err, x->cfg.spin_limit, s);
+            reinterpret_cast<unsigned long long*>(tail + 2), err, x->cfg.spin_limit, s);
         if (e != cudaSuccess) return fail(CRT_ERR_UNSUPPORTED, "batched PLOC launch failed: %s", cudaGetErrorString(e));
     }
     CRT_CUDA(cudaGetLastError());

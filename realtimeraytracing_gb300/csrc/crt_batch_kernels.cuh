@@ -2,8 +2,9 @@
 // layout and grid-barrier device code).
 //
 // Many scenes in one pipeline (config 2): every stage is one launch over all
-// scenes, the PLOC iterations of all scenes run in lockstep inside one
-// persistent cooperative kernel, and the whole build + trace can be captured
+// scenes: the PLOC iterations run in lockstep inside one persistent cooperative
+// kernel while a scene is larger than its thread-block cluster holds, then one
+// cluster a scene, then the layout, and the whole build + trace can be captured
 // into a CUDA graph and replayed.  Each scene's BVH is bit-identical to the
 // one crt_build makes for that scene alone (same codes, same sort order,
 // same PLOC decisions), because every kernel only sees its scene's data
@@ -199,7 +200,8 @@ __global__ void __launch_bounds__(256) batch_leaf_init_kernel(const crt_triangle
                                                               float4* __restrict__ clusters,
                                                               float4* __restrict__ xtri_sorted, float4* __restrict__ xtri,
                                                               uint32_t* __restrict__ leaf_of_tri, uint2* __restrict__ it,
-                                                              crt_bvh_node* __restrict__ nodes, uint32_t* err) {
+                                                              crt_bvh_node* __restrict__ nodes, uint2* __restrict__ pf,
+                                                              uint32_t* err) {
     __shared__ uint32_t s_off[kMaxBatchScenes];
     for (uint32_t k = threadIdx.x; k < n_scenes; k += 256) s_off[k] = scenes[k].tri_off;
     __syncthreads();
@@ -216,6 +218,7 @@ __global__ void __launch_bounds__(256) batch_leaf_init_kernel(const crt_triangle
         scenes[s].iters = sc.n_tris > 1 ? 0u : 1u;   // one-triangle scenes need no iteration
     }
     perm_local[i] = tl;
+    pf[i] = make_uint2(kLayoutUnset, 0u);  // the layout's places arrive from each node's parent
     const TriRec t = load_tri(tris, tg);
     const float* M = models + 16 * (t.model & (kMaxModels - 1));
     const float4 p0 = mat_vec(M, t.p0), p1 = mat_vec(M, t.p1), p2 = mat_vec(M, t.p2);
@@ -246,75 +249,65 @@ __global__ void __launch_bounds__(256) batch_leaf_init_kernel(const crt_triangle
     }
 }
 
-// PLOC for all scenes in lockstep, then every scene's DFS layout.  Each
-// iteration: every block derives the running scenes' tile counts (a scene
-// converged once its iteration count is set), takes tiles from one ticket
-// counter, maps a ticket to (scene, tile) and runs the single-scene tile
-// code on that scene's slices.  A grid barrier separates iterations.
+// The sum of v over the threads before this one, and over all (BLOCK threads).
+template <int BLOCK>
+__device__ __forceinline__ uint32_t block_exclusive(uint32_t v, uint32_t* s_warp, uint32_t& total) {
+    uint32_t incl = v;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+        const uint32_t y = __shfl_up_sync(0xFFFFFFFFu, incl, o);
+        if ((threadIdx.x & 31u) >= o) incl += y;
+    }
+    if ((threadIdx.x & 31u) == 31u) s_warp[threadIdx.x >> 5] = incl;
+    __syncthreads();
+    uint32_t before = 0u;
+    total = 0u;
+#pragma unroll
+    for (uint32_t w = 0; w < BLOCK / 32; ++w) {
+        if (w < threadIdx.x >> 5) before += s_warp[w];
+        total += s_warp[w];
+    }
+    return before + incl - v;
+}
+
+// The PLOC iterations of the scenes of more than stop_n live clusters, in
+// lockstep.  Each iteration: every block derives the running scenes' tile counts,
+// takes tiles from one ticket counter, maps a ticket to (scene, tile) and runs the
+// single-scene tile code on that scene's slices.  A grid barrier separates
+// iterations.  A scene leaves with its iteration count in scenes[].iters once it
+// has stop_n clusters or fewer; batch_cluster_kernel finishes it.  Thread k of
+// every block keeps scene k, and the tile counts are scanned by the whole block:
+// a loop over the scenes in one thread cost 64 dependent steps an iteration.
+// Whole batch builds before and with the three launches below, us: 64 scenes of
+// 1,000-250,000 triangles 2,730 -> 1,663, 16 of 5,000-20,000 886 -> 403, 200 of
+// 100-5,000 1,795 -> 456, 2 of 1-1.5 M 2,493 -> 1,961.
 template <int TILE, int BLOCK, int MAXR>
 __global__ void __launch_bounds__(BLOCK, kPlocBlocksPerSm) batch_ploc_kernel(BatchScene* scenes, uint32_t n_scenes, float4* ca, float4* cb,
                                                            float4* node_box, uint4* node_kids, uint2* it, int R,
-                                                           unsigned long long* lookback, uint32_t lb_cap, uint32_t* tickets,
-                                                           uint2* pf, crt_bvh_node* nodes, float4* wide, float4* wide_wt,
-                                                           uint8_t* depth_odd, LeafOut lv, unsigned long long* bar,
-                                                           uint32_t max_iters, uint32_t* err, uint32_t spin_limit) {
+                                                           uint32_t stop_n, unsigned long long* lookback, uint32_t lb_cap,
+                                                           uint32_t* tickets, unsigned long long* bar, uint32_t max_iters,
+                                                           uint32_t* err, uint32_t spin_limit) {
+    static_assert(BLOCK >= static_cast<int>(kMaxBatchScenes), "a thread per scene");
     __shared__ PlocSmem<TILE, BLOCK, MAXR> S;
     unsigned long long bar_target = 0;  // grid barriers passed x gridDim (thread 0)
-    __shared__ uint32_t s_tile_pre[kMaxBatchScenes + 1];
-    __shared__ uint32_t s_n[kMaxBatchScenes];
+    __shared__ uint32_t s_tile_pre[BLOCK];
+    __shared__ uint32_t s_n[BLOCK];
+    __shared__ uint32_t s_warp[BLOCK / 32];
     __shared__ uint32_t s_tile;
-    __shared__ uint32_t s_running;
-    int iter = 0;
-    for (;; ++iter) {
-        __syncthreads();
-        if (threadIdx.x == 0) s_running = 0;
-        __syncthreads();
-        for (uint32_t k = threadIdx.x; k < n_scenes; k += BLOCK) {
-            const uint32_t done = __ldcg(&scenes[k].iters);
-            uint32_t n = 1;
-            if (done == 0u) {
-                n = __ldcg(it + scenes[k].it_off + iter).x;
-                if (n > 1) atomicAdd(&s_running, 1u);
-            }
-            s_n[k] = n;
+    const uint32_t k = threadIdx.x;
+    uint32_t n = k < n_scenes ? scenes[k].n_tris : 0u;  // scene k's live clusters; no longer read once <= stop_n
+    const uint32_t it_off = k < n_scenes ? scenes[k].it_off : 0u;
+    for (int iter = 0;; ++iter) {
+        if (iter > 0 && n > stop_n) {
+            n = __ldcg(it + it_off + iter).x;
+            if (n <= stop_n && blockIdx.x == 0) scenes[k].iters = static_cast<uint32_t>(iter);
         }
-        __syncthreads();
-        if (s_running == 0) break;
+        const uint32_t tiles = n > stop_n ? (n + ploc_own(R) - 1) / ploc_own(R) : 0u;
+        s_n[k] = n;
+        uint32_t total;
+        s_tile_pre[k] = block_exclusive<BLOCK>(tiles, s_warp, total);
+        if (total == 0u) break;  // uniform: every thread has the same total
         if (static_cast<uint32_t>(iter) >= max_iters) { raise_error(err, kDevIterLimit); return; }
-        // Once every running scene fits in one tile, each block finishes whole
-        // scenes alone (their remaining iterations, one tile each, with block
-        // barriers only) and one grid barrier ends the PLOC phase.
-        if (threadIdx.x == 0) {
-            uint32_t big = 0;
-            for (uint32_t k = 0; k < n_scenes; ++k) big += s_n[k] > ploc_own(R) ? 1u : 0u;
-            s_tile = big;
-        }
-        __syncthreads();
-        if (s_tile == 0u) {
-            for (uint32_t sc = blockIdx.x; sc < n_scenes; sc += gridDim.x) {
-                if (s_n[sc] <= 1u) continue;  // finished before this iteration
-                const BatchScene B = scenes[sc];
-                // the scene's remaining iterations on shared memory (ploc_tail);
-                // its iteration count cannot exceed the scene's N - 1
-                const float4* cin = ((iter & 1) ? cb : ca) + 2 * static_cast<size_t>(B.tri_off);
-                const int k = ploc_tail<TILE, BLOCK, MAXR>(S, iter, cin, node_box + 2 * static_cast<size_t>(B.node_off),
-                                                          node_kids + B.tri_off, it + B.it_off, B.n_tris, R, err);
-                if (threadIdx.x == 0) scenes[sc].iters = static_cast<uint32_t>(k);
-                __syncthreads();
-            }
-            if (!grid_barrier(bar, bar_target, err, spin_limit)) return;
-            break;
-        }
-        if (threadIdx.x == 0) {
-            uint32_t run = 0;
-            for (uint32_t k = 0; k < n_scenes; ++k) {
-                s_tile_pre[k] = run;
-                run += s_n[k] > 1 ? (s_n[k] + ploc_own(R) - 1) / ploc_own(R) : 0u;
-            }
-            s_tile_pre[n_scenes] = run;
-        }
-        __syncthreads();
-        const uint32_t total = s_tile_pre[n_scenes];
         for (;;) {
             __syncthreads();
             if (threadIdx.x == 0) s_tile = atomicAdd(&tickets[iter & 1], 1u);
@@ -336,75 +329,88 @@ __global__ void __launch_bounds__(BLOCK, kPlocBlocksPerSm) batch_ploc_kernel(Bat
             unsigned long long* lb_next = lookback + static_cast<size_t>((iter + 1) & 1) * lb_cap + B.lb_off;
             ploc_tile<TILE, BLOCK, MAXR>(S, tile, cur, iter, cin, cout, node_box + 2 * static_cast<size_t>(B.node_off),
                                          node_kids + B.tri_off, it + B.it_off, B.n_tris, R, lb_cur, lb_next, err, spin_limit);
-            if ((tile + 1) * ploc_own(R) >= cur.x && threadIdx.x == 0) {  // the scene's last tile wrote its next record
-                if (it[B.it_off + iter + 1].x <= 1u) scenes[sc].iters = static_cast<uint32_t>(iter + 1);
-            }
         }
         if (!grid_barrier(bar, bar_target, err, spin_limit)) return;
     }
-    // DFS layout: step r handles level (iters - 1 - r) of every scene that has
-    // it, recording node ids by DFS position in dfs (the first cluster buffer,
-    // free now); then every position is emitted in order.
-    uint32_t* dfs = reinterpret_cast<uint32_t*>(ca);
-    uint32_t max_it = 0;
-    for (uint32_t k = 0; k < n_scenes; ++k) max_it = max(max_it, __ldcg(&scenes[k].iters));
-    for (uint32_t r = 0; r < max_it; ++r) {
-        __syncthreads();
-        if (threadIdx.x == 0) {
-            uint32_t run = 0;
-            for (uint32_t k = 0; k < n_scenes; ++k) {
-                s_tile_pre[k] = run;
-                const uint32_t K = __ldcg(&scenes[k].iters);
-                if (scenes[k].n_tris > 1 && K > r) {
-                    const uint32_t lv = K - 1 - r;
-                    const uint32_t o = scenes[k].it_off;
-                    run += __ldcg(it + o + lv + 1).y - __ldcg(it + o + lv).y;
-                }
-            }
-            s_tile_pre[n_scenes] = run;
-        }
-        __syncthreads();
-        const uint32_t total = s_tile_pre[n_scenes];
-        for (uint32_t q = blockIdx.x * BLOCK + threadIdx.x; q < total; q += gridDim.x * BLOCK) {
-            uint32_t lo = 0, hi = n_scenes - 1;
-            while (lo < hi) {
-                const uint32_t mid = (lo + hi + 1) >> 1;
-                if (s_tile_pre[mid] <= q) lo = mid; else hi = mid - 1;
-            }
-            const BatchScene B = scenes[lo];
-            const uint32_t lv = B.iters - 1 - r;
-            const uint32_t X = __ldcg(it + B.it_off + lv).y + (q - s_tile_pre[lo]);
-            layout_down(X, node_kids + B.tri_off, pf + B.tri_off, B.n_tris,
-                        dfs + B.node_off, err);
-        }
-        if (!grid_barrier(bar, bar_target, err, spin_limit)) return;
+}
+
+// Every scene's remaining PLOC iterations, one cluster a scene (ploc_cluster_r);
+// scenes[].iters: iterations done before, then all of them.
+__global__ void __launch_bounds__(kClusterThreads) batch_cluster_kernel(BatchScene* scenes, const float4* ca, const float4* cb,
+                                                                        float4* node_box, uint4* node_kids, uint2* it, int R,
+                                                                        uint32_t* err) {
+    extern __shared__ __align__(16) unsigned char cluster_smem[];
+    ClusterSmem& C = *reinterpret_cast<ClusterSmem*>(cluster_smem);
+    BatchScene& B = scenes[blockIdx.x / cooperative_groups::this_cluster().num_blocks()];
+    const uint32_t N = B.n_tris;
+    if (N < 2) return;  // no node to make
+    const int iter = static_cast<int>(__ldcg(&B.iters));
+    const float4* cin = ((iter & 1) ? cb : ca) + 2 * static_cast<size_t>(B.tri_off);
+    float4* box = node_box + 2 * static_cast<size_t>(B.node_off);
+    uint4* kids = node_kids + B.tri_off;
+    uint2* rec = it + B.it_off;
+    switch (R) {
+        case 8: ploc_cluster_r<8>(C, iter, cin, box, kids, rec, N, R, &B.iters, err); break;
+        case 16: ploc_cluster_r<16>(C, iter, cin, box, kids, rec, N, R, &B.iters, err); break;
+        case 32: ploc_cluster_r<32>(C, iter, cin, box, kids, rec, N, R, &B.iters, err); break;
+        default: ploc_cluster_r<0>(C, iter, cin, box, kids, rec, N, R, &B.iters, err); break;
     }
-    // every DFS position of every scene with more than one triangle, in order
+}
+
+// The layout's position pass (layout_places_kernel) over all scenes.  A scene
+// has blocks of its own, one per `share` of its internal nodes, so the scenes'
+// chains of places run side by side (blocks that also held the end of the scene
+// before made one chain of them all: 64 scenes of 2.6 M triangles 1,350 us, now
+// 94).  A grid barrier a PLOC level, with a loop over the scenes in one thread, was
+// what both replace.
+template <int BLOCK>
+__global__ void __launch_bounds__(BLOCK) batch_places_kernel(const BatchScene* __restrict__ scenes, uint32_t n_scenes,
+                                                             uint32_t share, uint32_t* __restrict__ dfs,
+                                                             const uint4* __restrict__ node_kids, uint2* pf, uint32_t* err,
+                                                             uint32_t spin_limit) {
+    static_assert(BLOCK >= static_cast<int>(kMaxBatchScenes), "a thread per scene");
+    __shared__ uint32_t s_warp[BLOCK / 32];
+    __shared__ uint32_t s_mine[3];  // this block's scene, its place among the scene's blocks, their number
+    const uint32_t k = threadIdx.x;
+    const uint32_t blocks = k < n_scenes ? (scenes[k].n_tris - 1 + share - 1) / share : 0u;
+    uint32_t total;
+    const uint32_t first = block_exclusive<BLOCK>(blocks, s_warp, total);
+    if (blockIdx.x >= total) return;  // uniform
+    if (blockIdx.x - first < blocks) {
+        s_mine[0] = k;
+        s_mine[1] = blockIdx.x - first;
+        s_mine[2] = blocks;
+    }
     __syncthreads();
-    if (threadIdx.x == 0) {
-        uint32_t run = 0;
-        for (uint32_t k = 0; k < n_scenes; ++k) {
-            s_tile_pre[k] = run;
-            if (scenes[k].n_tris > 1) run += 2 * scenes[k].n_tris - 1;
-        }
-        s_tile_pre[n_scenes] = run;
+    const BatchScene B = scenes[s_mine[0]];
+    const uint32_t N = B.n_tris, stride = s_mine[2] * BLOCK;
+    for (uint32_t t = s_mine[1] * BLOCK + threadIdx.x; t + 1 < N; t += stride)
+        if (!layout_place_node(2 * N - 2 - t, t < stride, dfs + B.node_off, node_kids + B.tri_off, N, pf + B.tri_off, err,
+                               spin_limit))
+            return;
+}
+
+// Every DFS position of every scene with more than one triangle, in order.
+__global__ void __launch_bounds__(256) batch_emit_kernel(const BatchScene* __restrict__ scenes, uint32_t n_scenes,
+                                                         uint32_t n_slots, const float4* __restrict__ node_box,
+                                                         const uint4* __restrict__ node_kids, const uint2* __restrict__ pf,
+                                                         const uint32_t* __restrict__ dfs, crt_bvh_node* __restrict__ nodes,
+                                                         float4* __restrict__ wide, float4* __restrict__ wide_wt,
+                                                         uint8_t* __restrict__ depth_odd, LeafOut lv, uint32_t* err) {
+    const uint32_t q = blockIdx.x * 256 + threadIdx.x;
+    if (q >= n_slots) return;
+    uint32_t lo = 0, hi = n_scenes - 1;  // node_off: slots before the scene
+    while (lo < hi) {
+        const uint32_t mid = (lo + hi + 1) >> 1;
+        if (__ldg(&scenes[mid].node_off) <= q) lo = mid; else hi = mid - 1;
     }
-    __syncthreads();
-    const uint32_t total_slots = s_tile_pre[n_scenes];
-    for (uint32_t q = blockIdx.x * BLOCK + threadIdx.x; q < total_slots; q += gridDim.x * BLOCK) {
-        uint32_t lo = 0, hi = n_scenes - 1;
-        while (lo < hi) {
-            const uint32_t mid = (lo + hi + 1) >> 1;
-            if (s_tile_pre[mid] <= q) lo = mid; else hi = mid - 1;
-        }
-        const BatchScene B = scenes[lo];
-        const LeafOut slv{lv.xtri_sorted + 3 * static_cast<size_t>(B.tri_off), lv.xtri + 3 * static_cast<size_t>(B.tri_off),
-                          lv.leaf_of_tri + B.tri_off};
-        layout_emit(q - s_tile_pre[lo], node_box + 2 * static_cast<size_t>(B.node_off), node_kids + B.tri_off,
-                    pf + B.tri_off, B.n_tris, dfs + B.node_off, nodes + B.node_off,
-                    wide + 4 * static_cast<size_t>(B.wide_off), wide_wt + 4 * static_cast<size_t>(B.wide_off),
-                    depth_odd + B.wide_off, slv, B.abs_eps, err);
-    }
+    const BatchScene B = scenes[lo];
+    if (B.n_tris < 2) return;  // written with the leaves
+    const LeafOut slv{lv.xtri_sorted + 3 * static_cast<size_t>(B.tri_off), lv.xtri + 3 * static_cast<size_t>(B.tri_off),
+                      lv.leaf_of_tri + B.tri_off};
+    layout_emit(q - B.node_off, node_box + 2 * static_cast<size_t>(B.node_off), node_kids + B.tri_off, pf + B.tri_off,
+                B.n_tris, dfs + B.node_off, nodes + B.node_off, wide + 4 * static_cast<size_t>(B.wide_off),
+                wide_wt + 4 * static_cast<size_t>(B.wide_off), depth_odd + B.wide_off, slv, B.abs_eps, err);
 }
 
 // ------------------------------------------------------------------ launchers
@@ -444,25 +450,68 @@ void launch_batch_morton(const crt_triangle* tris, const void* chunks, uint32_t 
 void launch_batch_leaf_init(const crt_triangle* tris, uint32_t n_total, BatchScene* scenes, uint32_t n_scenes,
                             const float* models, const uint32_t* perm_global, uint32_t* perm_local, float4* node_box,
                             float4* clusters, float4* xtri_sorted, float4* xtri, uint32_t* leaf_of_tri, uint2* it,
-                            crt_bvh_node* nodes,
-                            uint32_t* err, cudaStream_t s) {
+                            crt_bvh_node* nodes, uint2* pf, uint32_t* err, cudaStream_t s) {
     batch_leaf_init_kernel<<<(n_total + 255) / 256, 256, 0, s>>>(tris, n_total, scenes, n_scenes, models, perm_global,
                                                                  perm_local, node_box, clusters, xtri_sorted, xtri,
-                                                                 leaf_of_tri, it, nodes,
-                                                                 err);
+                                                                 leaf_of_tri, it, nodes, pf, err);
 }
 
-cudaError_t launch_batch_ploc(BatchScene* scenes, uint32_t n_scenes, float4* ca, float4* cb, float4* node_box,
-                              uint4* node_kids, uint2* it, int radius, unsigned long long* lookback, uint32_t lb_cap,
-                              uint32_t* tickets, uint2* pf, crt_bvh_node* nodes, float4* wide, float4* wide_wt,
-                              uint8_t* depth_odd, LeafOut lv, unsigned long long* bar, uint32_t max_iters, uint32_t* err,
-                              uint32_t spin_limit, cudaStream_t s) {
-    const int grid = batch_ploc_grid();
-    if (grid <= 0) return cudaErrorNotSupported;
-    void* args[] = {&scenes, &n_scenes, &ca, &cb, &node_box, &node_kids, &it, &radius, &lookback, &lb_cap, &tickets,
-                    &pf, &nodes, &wide, &wide_wt, &depth_odd, &lv, &bar, &max_iters, &err, &spin_limit};
-    return cudaLaunchCooperativeKernel(reinterpret_cast<const void*>(batch_ploc_kernel<kPlocSpan, 256, kPlocMaxRadius>),
-                                       dim3(grid), dim3(256), args, 0, s);
+// Blocks of a scene's cluster: the most for which every scene's cluster is
+// resident at once (up to 16; 152 SMs hold 76 clusters of two, 8 of sixteen), so
+// that the scenes' chains of iterations run side by side.
+static int batch_cluster_blocks(uint32_t n_scenes) {
+    static int active[5] = {-1, -1, -1, -1, -1};  // clusters of 1 << i blocks the device holds
+    for (int i = 4; i >= 0; --i) {
+        if (active[i] < 0) active[i] = ClusterLaunch::active(reinterpret_cast<const void*>(batch_cluster_kernel), 1 << i);
+        if (active[i] > 0 && (static_cast<uint32_t>(active[i]) >= n_scenes || i == 0)) return 1 << i;
+    }
+    return 0;
+}
+
+cudaError_t launch_batch_ploc(BatchScene* scenes, uint32_t n_scenes, uint32_t n_total, uint32_t max_n, float4* ca,
+                              float4* cb, float4* node_box, uint4* node_kids, uint2* it, int radius,
+                              unsigned long long* lookback, uint32_t lb_cap, uint32_t* tickets, uint2* pf,
+                              crt_bvh_node* nodes, float4* wide, float4* wide_wt, uint8_t* depth_odd, LeafOut lv,
+                              unsigned long long* bar, uint32_t* err, uint32_t spin_limit, cudaStream_t s) {
+    const int grid = batch_ploc_grid(), blocks = batch_cluster_blocks(n_scenes);
+    if (grid <= 0 || blocks <= 0) return cudaErrorNotSupported;
+    cudaError_t e = cudaSuccess;
+    uint32_t stop_n = static_cast<uint32_t>(blocks * (kClusterTile - 2 * radius)), max_iters = max_n + 1;
+    if (max_n > stop_n) {
+        void* args[] = {&scenes, &n_scenes, &ca, &cb, &node_box, &node_kids, &it, &radius, &stop_n, &lookback, &lb_cap,
+                        &tickets, &bar, &max_iters, &err, &spin_limit};
+        e = cudaLaunchCooperativeKernel(reinterpret_cast<const void*>(batch_ploc_kernel<kPlocSpan, 256, kPlocMaxRadius>),
+                                        dim3(grid), dim3(256), args, 0, s);
+        if (e != cudaSuccess) return e;
+    }
+    const uint32_t inner = n_total - n_scenes;  // internal nodes
+    if (inner == 0) return cudaSuccess;
+    ClusterLaunch l(blocks, n_scenes, s);
+    e = cudaLaunchKernelEx(&l.c, batch_cluster_kernel, scenes, static_cast<const float4*>(ca), static_cast<const float4*>(cb),
+                           node_box, node_kids, it, radius, err);
+    if (e != cudaSuccess) return e;
+    static int place_grid = 0;
+    if (place_grid == 0) {
+        int per_sm = 0;
+        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, batch_places_kernel<256>, 256, 0);
+        place_grid = kNumSms * (per_sm > 0 ? per_sm : 1);
+    }
+    // whole blocks a scene: at most inner / share + n_scenes of them, all resident
+    if (place_grid <= static_cast<int>(n_scenes)) return cudaErrorNotSupported;
+    const uint32_t spread = static_cast<uint32_t>(place_grid) - n_scenes;
+    uint32_t share = (inner + spread - 1) / spread;
+    share = share > 256 ? share : 256;
+    uint32_t* dfs = reinterpret_cast<uint32_t*>(ca);  // node ids by DFS position: the clusters are done with
+    const BatchScene* cs = scenes;
+    const uint4* ck = node_kids;
+    void* args[] = {&cs, &n_scenes, &share, &dfs, &ck, &pf, &err, &spin_limit};
+    e = cudaLaunchCooperativeKernel(reinterpret_cast<const void*>(batch_places_kernel<256>),
+                                    dim3(inner / share + n_scenes), dim3(256), args, 0, s);
+    if (e != cudaSuccess) return e;
+    const uint32_t slots = n_total + inner;
+    batch_emit_kernel<<<(slots + 255) / 256, 256, 0, s>>>(cs, n_scenes, slots, node_box, node_kids, pf, dfs, nodes, wide,
+                                                          wide_wt, depth_odd, lv, err);
+    return cudaGetLastError();
 }
 
 size_t batch_box_state_bytes() { return sizeof(BatchBoxState); }

@@ -789,175 +789,6 @@ __device__ __forceinline__ void ploc_tile(PlocSmem<TILE, BLOCK, MAXR>& S, uint32
     }
 }
 
-// The same for a whole-array window (position q at window index q + 2R).
-template <int RC, int TILE, int BLOCK, int MAXR>
-__device__ __forceinline__ uint32_t ploc_nearest_one(const PlocSmem<TILE, BLOCK, MAXR>& S, int p, int R_rt) {
-    return ploc_nearest_at<RC>(S, p, p + 2 * (RC > 0 ? RC : R_rt), R_rt);
-}
-
-// The last PLOC iterations, once every live cluster fits in one tile (n <=
-// ploc_own(R)): one block runs them with the clusters held in shared memory,
-// in the window layout of a single tile starting at position 0 (position q at
-// index q + 2R, infinite boxes outside [0, n)), so an iteration costs no
-// global round trip; only the new nodes and the iteration records are written
-// out.  Each iteration is the same reference iteration as ploc_tile's: the
-// same nearest-neighbour search (ploc_nearest over the whole array while n >
-// BLOCK, one position per thread below), mutual pairs merged at the lower
-// position (AABB::merge), new ids in position order, survivors compacted in
-// order.  Thread t decides positions [k t, k t + k), k = ceil(n / BLOCK) <=
-// TILE / BLOCK; the compaction is in place, after a barrier that ends every
-// read of the iteration's clusters.  Returns the iteration count.
-template <int RC, int TILE, int BLOCK, int MAXR>
-__device__ __noinline__ int ploc_tail_r(PlocSmem<TILE, BLOCK, MAXR>& S, int iter, int n, uint32_t idb,
-                                           float4* __restrict__ node_box, uint4* __restrict__ node_kids, uint2* it,
-                                           uint32_t N, int R_rt, uint32_t* err) {
-    constexpr int PMAX = TILE / BLOCK;
-    const int R = RC > 0 ? RC : R_rt;
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const float inf = __int_as_float(0x7F800000);
-    while (n > 1) {
-        if (static_cast<uint32_t>(iter) + 1 >= N) {
-            if (threadIdx.x == 0) raise_error(err, kDevIterLimit);
-            break;
-        }
-        if (n > BLOCK) {
-            ploc_nearest<RC>(S, 0, n, n, R);  // S.nn[p + R] for p < n
-        } else if (static_cast<int>(threadIdx.x) < n) {
-            S.nn[threadIdx.x + R] = ploc_nearest_one<RC>(S, static_cast<int>(threadIdx.x), R);
-        }
-        __syncthreads();
-        const int k = (n + BLOCK - 1) / BLOCK;
-        const int p0 = k * static_cast<int>(threadIdx.x);
-        uint32_t flags = 0, nv = 0, nm = 0;
-#pragma unroll
-        for (int q = 0; q < PMAX; ++q) {
-            const int p = p0 + q;
-            if (q >= k || p >= n) continue;
-            const int j = static_cast<int>(S.nn[p + R]);
-            const bool mutual = (j != p) && (static_cast<int>(S.nn[j + R]) == p);
-            if (!(mutual && p > j)) { flags |= 1u << q; ++nv; }
-            if (mutual && p < j) { flags |= 1u << (16 + q); ++nm; }
-        }
-        // exclusive scan of (survivors, merges) in position order, 16|16 bits
-        const uint32_t packed = (nv << 16) | nm;
-        uint32_t incl = packed;
-#pragma unroll
-        for (int o = 1; o < 32; o <<= 1) {
-            const uint32_t y = __shfl_up_sync(0xFFFFFFFFu, incl, o);
-            if (lane >= o) incl += y;
-        }
-        if (lane == 31) S.wsum[warp] = incl;
-        __syncthreads();
-        if (warp == 0) {
-            const uint32_t ws = lane < BLOCK / 32 ? static_cast<uint32_t>(S.wsum[lane]) : 0u;
-            uint32_t wi = ws;
-#pragma unroll
-            for (int o = 1; o < 32; o <<= 1) {
-                const uint32_t y = __shfl_up_sync(0xFFFFFFFFu, wi, o);
-                if (lane >= o) wi += y;
-            }
-            if (lane < BLOCK / 32) S.wsum[lane] = wi - ws;
-            if (lane == 31) S.prefix = wi;  // block totals
-        }
-        __syncthreads();
-        const uint32_t excl = static_cast<uint32_t>(S.wsum[warp]) + (incl - packed);
-        const uint32_t total = static_cast<uint32_t>(S.prefix);
-        uint32_t out_v = excl >> 16;
-        uint32_t out_m = idb + (excl & 0xFFFFu);
-        float4 omn[PMAX], omx[PMAX];
-#pragma unroll
-        for (int q = 0; q < PMAX; ++q) {
-            if (!(flags & (1u << q))) continue;
-            const int p = p0 + q, wp = p + 2 * R;
-            float4 mn = make_float4(S.mnx[wp], S.mny[wp], S.mnz[wp], __uint_as_float(S.id[wp]));
-            float4 mx = make_float4(S.mxx[wp], S.mxy[wp], S.mxz[wp], __uint_as_float(S.lc[wp]));
-            if (flags & (1u << (16 + q))) {
-                const int wj = static_cast<int>(S.nn[p + R]) + 2 * R;
-                const uint32_t id = out_m++;
-                if (id >= 2 * N - 1 || id < N) {
-                    raise_corrupt(err, 13 + (iter << 8), p, id);
-                    flags &= ~(1u << q);
-                    continue;
-                }
-                float4 m0, m1;  // AABB::merge (bvh.cpp:401-413), first argument = lower position
-                m0.x = min_std(mn.x, S.mnx[wj]); m0.y = min_std(mn.y, S.mny[wj]); m0.z = min_std(mn.z, S.mnz[wj]);
-                m1.x = max_std(mx.x, S.mxx[wj]); m1.y = max_std(mx.y, S.mxy[wj]); m1.z = max_std(mx.z, S.mxz[wj]);
-                m0.w = mn.w;                      // left child id
-                m1.w = __uint_as_float(S.id[wj]); // right child id
-                node_box[2 * static_cast<size_t>(id)] = m0;
-                node_box[2 * static_cast<size_t>(id) + 1] = m1;
-                node_kids[id - N] = make_uint4(S.id[wp], S.id[wj], S.lc[wp], S.lc[wj]);
-                mn = make_float4(m0.x, m0.y, m0.z, __uint_as_float(id));
-                mx = make_float4(m1.x, m1.y, m1.z, __uint_as_float(S.lc[wp] + S.lc[wj]));
-            }
-            omn[q] = mn;
-            omx[q] = mx;
-        }
-        __syncthreads();  // every read of this iteration's clusters is done: compact in place
-        const int n_next = static_cast<int>(total >> 16);
-        const uint32_t merges = total & 0xFFFFu;
-#pragma unroll
-        for (int q = 0; q < PMAX; ++q) {
-            if (!(flags & (1u << q))) continue;
-            if (out_v >= static_cast<uint32_t>(n_next)) {
-                raise_corrupt(err, 14 + (iter << 8), p0 + q, out_v);
-                continue;
-            }
-            const int w = static_cast<int>(out_v) + 2 * R;
-            S.mnx[w] = omn[q].x; S.mny[w] = omn[q].y; S.mnz[w] = omn[q].z; S.id[w] = __float_as_uint(omn[q].w);
-            S.mxx[w] = omx[q].x; S.mxy[w] = omx[q].y; S.mxz[w] = omx[q].z; S.lc[w] = __float_as_uint(omx[q].w);
-            ++out_v;
-        }
-        for (int q = n_next + static_cast<int>(threadIdx.x); q < n; q += BLOCK) {  // vacated positions
-            const int w = q + 2 * R;
-            S.mnx[w] = -inf; S.mny[w] = -inf; S.mnz[w] = -inf;
-            S.mxx[w] = inf; S.mxy[w] = inf; S.mxz[w] = inf;
-        }
-        if (threadIdx.x == 0) it[iter + 1] = make_uint2(static_cast<uint32_t>(n_next), idb + merges);
-        n = n_next;
-        idb += merges;
-        ++iter;
-        __syncthreads();
-    }
-    return iter;
-}
-
-// Stages the tail's clusters (input of iteration iter) and runs ploc_tail_r
-// with the compile-time radius when there is one.
-template <int TILE, int BLOCK, int MAXR>
-__device__ __forceinline__ int ploc_tail(PlocSmem<TILE, BLOCK, MAXR>& S, int iter, const float4* __restrict__ cin,
-                                         float4* __restrict__ node_box, uint4* __restrict__ node_kids, uint2* it,
-                                         uint32_t N, int R, uint32_t* err) {
-    constexpr int kWin = PlocSmem<TILE, BLOCK, MAXR>::kWin;
-    __syncthreads();
-    const uint2 cur = __ldcg(it + iter);
-    const int n = static_cast<int>(cur.x);
-    if (n + 4 * R > kWin || n > TILE) {  // the caller checked n <= ploc_own(R); only corruption gets here
-        if (threadIdx.x == 0) raise_corrupt(err, 12, static_cast<uint32_t>(iter), static_cast<uint32_t>(n));
-        return iter;
-    }
-    const float inf = __int_as_float(0x7F800000);
-    for (int w = threadIdx.x; w < kWin; w += BLOCK) {
-        const int p = w - 2 * R;
-        if (p >= 0 && p < n) {
-            const float4 a = __ldcg(cin + 2 * static_cast<size_t>(p));
-            const float4 b = __ldcg(cin + 2 * static_cast<size_t>(p) + 1);
-            S.mnx[w] = a.x; S.mny[w] = a.y; S.mnz[w] = a.z; S.id[w] = __float_as_uint(a.w);
-            S.mxx[w] = b.x; S.mxy[w] = b.y; S.mxz[w] = b.z; S.lc[w] = __float_as_uint(b.w);
-        } else {
-            S.mnx[w] = -inf; S.mny[w] = -inf; S.mnz[w] = -inf;
-            S.mxx[w] = inf; S.mxy[w] = inf; S.mxz[w] = inf;
-        }
-    }
-    __syncthreads();
-    switch (R) {
-        case 8: return ploc_tail_r<8>(S, iter, n, cur.y, node_box, node_kids, it, N, R, err);
-        case 16: return ploc_tail_r<16>(S, iter, n, cur.y, node_box, node_kids, it, N, R, err);
-        case 32: return ploc_tail_r<32>(S, iter, n, cur.y, node_box, node_kids, it, N, R, err);
-        default: return ploc_tail_r<0>(S, iter, n, cur.y, node_box, node_kids, it, N, R, err);
-    }
-}
-
 template <int TILE, int BLOCK, int MAXR>
 __global__ void __launch_bounds__(BLOCK) ploc_iteration_kernel(const float4* __restrict__ cin, float4* __restrict__ cout,
                                                                float4* __restrict__ node_box, uint4* __restrict__ node_kids,
@@ -1548,6 +1379,38 @@ __global__ void __launch_bounds__(BLOCK, kPlocBlocksPerSm) ploc_persistent_kerne
     if (blockIdx.x == 0 && threadIdx.x == 0) iters_out[0] = static_cast<uint32_t>(iter);
 }
 
+// One internal node of the layout's dataflow pass: waits (bounded) for the
+// place of node X, lays X out and publishes its children's places; top: also
+// its grandchildren's.  False: the wait ran out.
+__device__ __forceinline__ bool layout_place_node(uint32_t X, bool top, uint32_t* __restrict__ dfs,
+                                                  const uint4* __restrict__ node_kids, uint32_t N, uint2* pf,
+                                                  uint32_t* err, uint32_t spin_limit) {
+    // X's record (and, at the top of the tree, where the chain of places is the
+    // latency that counts, its internal children's), in flight while X's place
+    // is awaited
+    const uint4 kids = __ldcg(node_kids + (X - N));
+    uint4 kc[2] = {make_uint4(0u, 0u, 0u, 0u), make_uint4(0u, 0u, 0u, 0u)};
+    if (top && kids.x >= N && kids.x - N < N - 1) kc[0] = __ldcg(node_kids + (kids.x - N));
+    if (top && kids.y >= N && kids.y - N < N - 1) kc[1] = __ldcg(node_kids + (kids.y - N));
+    uint2 me = make_uint2(0u, 0u);  // the root's place
+    if (X != 2 * N - 2) {
+        const unsigned long long* w = reinterpret_cast<const unsigned long long*>(pf + (X - N));
+        unsigned long long v = ld_relaxed_u64(w);
+        SpinBound spin(spin_limit);
+        while (static_cast<uint32_t>(v) == kLayoutUnset) {
+            if (!spin.step()) {
+                raise_error(err, kDevTimeout);
+                return false;
+            }
+            v = ld_relaxed_u64(w);
+        }
+        me = make_uint2(static_cast<uint32_t>(v), static_cast<uint32_t>(v >> 32));
+    }
+    if (top) layout_publish_grandchildren(me, kids, kc, pf, N);
+    layout_down_at<true>(X, me, kids, pf, N, dfs, err);
+    return true;
+}
+
 // The layout's position pass in one cooperative launch.
 template <int BLOCK>
 __global__ void __launch_bounds__(BLOCK) layout_places_kernel(uint32_t* __restrict__ dfs, const uint4* __restrict__ node_kids,
@@ -1559,36 +1422,8 @@ __global__ void __launch_bounds__(BLOCK) layout_places_kernel(uint32_t* __restri
     // out, waits (bounded) until X's parent has published X's position.  The
     // unfinished node with the largest id never waits (its parent is done), so
     // the co-resident grid always progresses, with no barrier per PLOC level.
-    bool gave_up = false;
-    for (uint32_t t = blockIdx.x * BLOCK + threadIdx.x; t + 1 < N && !gave_up; t += gridDim.x * BLOCK) {
-        const uint32_t X = 2 * N - 2 - t;
-        // X's record (and, for the grid's first round of nodes, the top of the
-        // tree, where the chain of places is the latency that counts, its
-        // internal children's), in flight while X's place is awaited
-        const bool top = t < gridDim.x * BLOCK;
-        const uint4 kids = __ldcg(node_kids + (X - N));
-        uint4 kc[2] = {make_uint4(0u, 0u, 0u, 0u), make_uint4(0u, 0u, 0u, 0u)};
-        if (top && kids.x >= N && kids.x - N < N - 1) kc[0] = __ldcg(node_kids + (kids.x - N));
-        if (top && kids.y >= N && kids.y - N < N - 1) kc[1] = __ldcg(node_kids + (kids.y - N));
-        uint2 me = make_uint2(0u, 0u);  // the root's place
-        if (X != 2 * N - 2) {
-            const unsigned long long* w = reinterpret_cast<const unsigned long long*>(pf + (X - N));
-            unsigned long long v = ld_relaxed_u64(w);
-            SpinBound spin(spin_limit);
-            while (static_cast<uint32_t>(v) == kLayoutUnset) {
-                if (!spin.step()) {
-                    raise_error(err, kDevTimeout);
-                    gave_up = true;
-                    break;
-                }
-                v = ld_relaxed_u64(w);
-            }
-            if (gave_up) break;
-            me = make_uint2(static_cast<uint32_t>(v), static_cast<uint32_t>(v >> 32));
-        }
-        if (top) layout_publish_grandchildren(me, kids, kc, pf, N);
-        layout_down_at<true>(X, me, kids, pf, N, dfs, err);
-    }
+    for (uint32_t t = blockIdx.x * BLOCK + threadIdx.x; t + 1 < N; t += gridDim.x * BLOCK)
+        if (!layout_place_node(2 * N - 2 - t, t < gridDim.x * BLOCK, dfs, node_kids, N, pf, err, spin_limit)) return;
 }
 
 __global__ void single_leaf_kernel(const float4* __restrict__ node_box, crt_bvh_node* __restrict__ out, LeafOut lv) {
@@ -1932,29 +1767,42 @@ int ploc_persistent_grid() {
     return grid;
 }
 
+// Launch of a PLOC cluster kernel: `clusters` clusters of `blocks` blocks.
+struct ClusterLaunch {
+    cudaLaunchConfig_t c{};
+    cudaLaunchAttribute a{};
+    ClusterLaunch(int blocks, uint32_t clusters, cudaStream_t s) {
+        a.id = cudaLaunchAttributeClusterDimension;
+        a.val.clusterDim.x = blocks;
+        a.val.clusterDim.y = a.val.clusterDim.z = 1;
+        c.gridDim = dim3(blocks * clusters);
+        c.blockDim = dim3(kClusterThreads);
+        c.dynamicSmemBytes = sizeof(ClusterSmem);
+        c.stream = s;
+        c.attrs = &a;
+        c.numAttrs = 1;
+    }
+    // Allows the kernel f clusters of kClusterBlocks; the clusters of `blocks`
+    // blocks that the device holds at once (0: it cannot run).
+    static int active(const void* f, int blocks) {
+        cudaFuncSetAttribute(f, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
+        cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(sizeof(ClusterSmem)));
+        ClusterLaunch l(blocks, 1, nullptr);
+        int n = 0;
+        if (cudaOccupancyMaxActiveClusters(&n, f, &l.c) != cudaSuccess) n = 0;
+        cudaGetLastError();
+        return n;
+    }
+};
+
 // Blocks of the cluster kernel's cluster on this device (0: it cannot run).
 static int ploc_cluster_blocks() {
     static int blocks = -1;
     if (blocks < 0) {
-        blocks = 0;
-        const void* f = reinterpret_cast<const void*>(ploc_cluster_kernel<kPlocMaxRadius>);
-        cudaFuncSetAttribute(f, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
-        cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(sizeof(ClusterSmem)));
-        for (int b = kClusterBlocks; b >= 8 && blocks == 0; b /= 2) {
-            cudaLaunchConfig_t c{};
-            cudaLaunchAttribute a{};
-            a.id = cudaLaunchAttributeClusterDimension;
-            a.val.clusterDim.x = b;
-            a.val.clusterDim.y = a.val.clusterDim.z = 1;
-            c.gridDim = dim3(b);
-            c.blockDim = dim3(kClusterThreads);
-            c.dynamicSmemBytes = sizeof(ClusterSmem);
-            c.attrs = &a;
-            c.numAttrs = 1;
-            int active = 0;
-            if (cudaOccupancyMaxActiveClusters(&active, f, &c) == cudaSuccess && active > 0) blocks = b;
-        }
-        cudaGetLastError();
+        int found = 0;
+        for (int b = kClusterBlocks; b >= 8 && found == 0; b /= 2)
+            if (ClusterLaunch::active(reinterpret_cast<const void*>(ploc_cluster_kernel<kPlocMaxRadius>), b) > 0) found = b;
+        blocks = found;
     }
     return blocks;
 }
@@ -1975,18 +1823,8 @@ cudaError_t launch_ploc_layout(float4* ca, float4* cb, float4* node_box, uint4* 
                                         dim3(grid), dim3(256), args, 0, s);
         if (e != cudaSuccess) return e;
     }
-    cudaLaunchConfig_t c{};
-    cudaLaunchAttribute a{};
-    a.id = cudaLaunchAttributeClusterDimension;
-    a.val.clusterDim.x = blocks;
-    a.val.clusterDim.y = a.val.clusterDim.z = 1;
-    c.gridDim = dim3(blocks);
-    c.blockDim = dim3(kClusterThreads);
-    c.dynamicSmemBytes = sizeof(ClusterSmem);
-    c.stream = s;
-    c.attrs = &a;
-    c.numAttrs = 1;
-    e = cudaLaunchKernelEx(&c, ploc_cluster_kernel<kPlocMaxRadius>, static_cast<const float4*>(ca),
+    ClusterLaunch l(blocks, 1, s);
+    e = cudaLaunchKernelEx(&l.c, ploc_cluster_kernel<kPlocMaxRadius>, static_cast<const float4*>(ca),
                            static_cast<const float4*>(cb), node_box, node_kids, it, N, radius, iters_out, err);
     if (e != cudaSuccess) return e;
     cudaEventRecord(ploc_done, s);

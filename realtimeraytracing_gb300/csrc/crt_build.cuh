@@ -249,12 +249,12 @@ void launch_batch_morton(const crt_triangle* tris, const void* chunks, uint32_t 
 void launch_batch_leaf_init(const crt_triangle* tris, uint32_t n_total, BatchScene* scenes, uint32_t n_scenes,
                             const float* models, const uint32_t* perm_global, uint32_t* perm_local, float4* node_box,
                             float4* clusters, float4* xtri_sorted, float4* xtri, uint32_t* leaf_of_tri, uint2* it,
-                            crt_bvh_node* nodes, uint32_t* err, cudaStream_t s);
-cudaError_t launch_batch_ploc(BatchScene* scenes, uint32_t n_scenes, float4* ca, float4* cb, float4* node_box,
-                              uint4* node_kids, uint2* it, int radius, unsigned long long* lookback, uint32_t lb_cap,
-                              uint32_t* tickets, uint2* pf, crt_bvh_node* nodes, float4* wide, float4* wide_wt,
-                              uint8_t* depth_odd, LeafOut leaves, unsigned long long* bar, uint32_t max_iters, uint32_t* err,
-                              uint32_t spin_limit, cudaStream_t s);
+                            crt_bvh_node* nodes, uint2* pf, uint32_t* err, cudaStream_t s);
+cudaError_t launch_batch_ploc(BatchScene* scenes, uint32_t n_scenes, uint32_t n_total, uint32_t max_n, float4* ca,
+                              float4* cb, float4* node_box, uint4* node_kids, uint2* it, int radius,
+                              unsigned long long* lookback, uint32_t lb_cap, uint32_t* tickets, uint2* pf,
+                              crt_bvh_node* nodes, float4* wide, float4* wide_wt, uint8_t* depth_odd, LeafOut leaves,
+                              unsigned long long* bar, uint32_t* err, uint32_t spin_limit, cudaStream_t s);
 // Treelet restructuring (crt_optimize.cu).  Ids: leaves 0..N-1 in tree
 // leaf order, internal nodes N + DFS rank (root N).
 struct OptView {

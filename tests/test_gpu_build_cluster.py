@@ -44,3 +44,25 @@ def test_equal_boxes(radius):
     position, also where the candidates are split over threads."""
     one = S.uniform_soup(40, seed=5)
     _check(np.repeat(one, 37, axis=0), radius)
+
+
+@pytest.mark.parametrize("n_scenes", [1, 6, 15, 30, 70, 200])
+def test_batches_of_scenes(n_scenes):
+    """A batch splits the SMs over its scenes' clusters (16 blocks a scene down to
+    one), and its layout the grid over their nodes: every scene is the oracle's tree,
+    for scenes around what each cluster size holds among tiny ones."""
+    torch = pytest.importorskip("torch")
+    edges = [b * 2016 + o for b in (1, 2, 4, 8, 16) for o in (0, 1, -1)] + [1, 2, 64, 65, 257]
+    sizes = [edges[(7 * k) % len(edges)] if k < len(edges) else 1 + (37 * k) % 90 for k in range(n_scenes)]
+    scenes = [S.uniform_soup(n, seed=3 * k + n) for k, n in enumerate(sizes)]
+    ctx = crt.Context()
+    batch = crt.Batch(ctx, sizes, [1] * n_scenes, models=S.identity_models(1))
+    tris = torch.from_numpy(np.concatenate(scenes)).cuda()
+    for _ in range(2):  # a second build starts from the first one's scratch
+        batch.build(tris)
+    for k, t in enumerate(scenes):
+        ref = O.build_bvh(t, sizes[k], S.identity_models(1))
+        np.testing.assert_array_equal(batch.nodes(k).view(np.uint32), ref["nodes"].view(np.uint32), err_msg=f"scene {k}")
+        assert batch.scene_info(k)["iterations"] == ref["iterations"]
+    batch.free()
+    ctx.close()
