@@ -1546,7 +1546,7 @@ __device__ __forceinline__ void cwide_node(const float4* __restrict__ wide, uint
     const float hi[3][4] = {{mx[0].x, mx[1].x, mx[2].x, mx[3].x}, {mx[0].y, mx[1].y, mx[2].y, mx[3].y},
                             {mx[0].z, mx[1].z, mx[2].z, mx[3].z}};
     float org[3];
-    uint32_t ex = 0, q[6];
+    uint32_t step[3], q[6];
 #pragma unroll
     for (int a = 0; a < 3; ++a) {
         // NaN coordinates must not be skipped by fminf: they fail the isfinite tests below
@@ -1558,7 +1558,7 @@ __device__ __forceinline__ void cwide_node(const float4* __restrict__ wide, uint
         const uint32_t e = min(max((__float_as_uint(need) + 0x7FFFFFu) >> 23, 1u), 180u);
         const float inv_step = __uint_as_float((254u - e) << 23);  // 2^(127 - e)
         org[a] = l * 8.673617379884035e-19f;
-        ex |= (e + 73u) << (8 * a);
+        step[a] = (e + 73u) << 23;  // as a float: step * 2^73
         uint32_t ql = 0, qh = 0;
 #pragma unroll
         for (int c = 0; c < 4; ++c) {
@@ -1579,9 +1579,9 @@ __device__ __forceinline__ void cwide_node(const float4* __restrict__ wide, uint
     }
     if (!ok) atomicOr(bad, 1u);
     uint4* o = out + 4 * static_cast<size_t>(i);
-    o[0] = make_uint4(__float_as_uint(org[0]), __float_as_uint(org[1]), __float_as_uint(org[2]), ex);
+    o[0] = make_uint4(__float_as_uint(org[0]), __float_as_uint(org[1]), __float_as_uint(org[2]), step[0]);
     o[1] = make_uint4(q[0], q[1], q[2], q[3]);
-    o[2] = make_uint4(q[4], q[5], 0u, 0u);
+    o[2] = make_uint4(q[4], q[5], step[1], step[2]);
     o[3] = make_uint4(ref[0], ref[1], ref[2], ref[3]);
 }
 
