@@ -288,7 +288,7 @@ __global__ void __launch_bounds__(BLOCK, kPlocBlocksPerSm) batch_ploc_kernel(Bat
                                                            uint32_t* tickets, unsigned long long* bar, uint32_t max_iters,
                                                            uint32_t* err, uint32_t spin_limit) {
     static_assert(BLOCK >= static_cast<int>(kMaxBatchScenes), "a thread per scene");
-    __shared__ PlocSmem<TILE, BLOCK, MAXR> S;
+    __shared__ PlocTileSmem<TILE, BLOCK, MAXR> S;
     unsigned long long bar_target = 0;  // grid barriers passed x gridDim (thread 0)
     __shared__ uint32_t s_tile_pre[BLOCK];
     __shared__ uint32_t s_n[BLOCK];
@@ -414,23 +414,6 @@ __global__ void __launch_bounds__(256) batch_emit_kernel(const BatchScene* __res
 }
 
 // ------------------------------------------------------------------ launchers
-int batch_ploc_grid() {
-    static int grid = -1;
-    if (grid < 0) {
-        int per_sm = 0, dev = 0, sms = kNumSms, coop = 0;
-        cudaGetDevice(&dev);
-        cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-        cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, dev);
-        if (coop && cudaOccupancyMaxActiveBlocksPerMultiprocessor(
-                        &per_sm, batch_ploc_kernel<kPlocSpan, 256, kPlocMaxRadius>, 256, 0) == cudaSuccess && per_sm > 0)
-            grid = (per_sm < kPlocBlocksPerSm ? per_sm : kPlocBlocksPerSm) * sms;
-        else
-            grid = 0;
-        cudaGetLastError();
-    }
-    return grid;
-}
-
 void launch_batch_box(const crt_triangle* tris, const void* chunks, uint32_t n_chunks, const float* models, void* states,
                       BatchScene* scenes, uint32_t* err, cudaStream_t s) {
     batch_box_kernel<<<n_chunks, 256, 0, s>>>(tris, static_cast<const Chunk*>(chunks), models,
@@ -473,15 +456,16 @@ cudaError_t launch_batch_ploc(BatchScene* scenes, uint32_t n_scenes, uint32_t n_
                               unsigned long long* lookback, uint32_t lb_cap, uint32_t* tickets, uint2* pf,
                               crt_bvh_node* nodes, float4* wide, float4* wide_wt, uint8_t* depth_odd, LeafOut lv,
                               unsigned long long* bar, uint32_t* err, uint32_t spin_limit, cudaStream_t s) {
-    const int grid = batch_ploc_grid(), blocks = batch_cluster_blocks(n_scenes);
+    const void* ploc_fn = reinterpret_cast<const void*>(batch_ploc_kernel<kPlocSpan, 256, kPlocMaxRadius>);
+    static const int grid = cooperative_grid(ploc_fn, kPlocBlocksPerSm);
+    const int blocks = batch_cluster_blocks(n_scenes);
     if (grid <= 0 || blocks <= 0) return cudaErrorNotSupported;
     cudaError_t e = cudaSuccess;
     uint32_t stop_n = static_cast<uint32_t>(blocks * (kClusterTile - 2 * radius)), max_iters = max_n + 1;
     if (max_n > stop_n) {
         void* args[] = {&scenes, &n_scenes, &ca, &cb, &node_box, &node_kids, &it, &radius, &stop_n, &lookback, &lb_cap,
                         &tickets, &bar, &max_iters, &err, &spin_limit};
-        e = cudaLaunchCooperativeKernel(reinterpret_cast<const void*>(batch_ploc_kernel<kPlocSpan, 256, kPlocMaxRadius>),
-                                        dim3(grid), dim3(256), args, 0, s);
+        e = cudaLaunchCooperativeKernel(ploc_fn, dim3(grid), dim3(256), args, 0, s);
         if (e != cudaSuccess) return e;
     }
     const uint32_t inner = n_total - n_scenes;  // internal nodes

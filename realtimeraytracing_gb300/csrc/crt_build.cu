@@ -457,10 +457,10 @@ __global__ void __launch_bounds__(256) leaf_init_kernel(const crt_triangle* __re
 // ================================================ K3: one PLOC iteration
 // For the n live clusters (Morton order, 32-byte records: min.xyz|node id,
 // max.xyz|leaf count) a tile starting at position s with R = radius does:
-//   nearest neighbour of the TILE positions [s-R, s-R+TILE) in [i-R, i+R]
-//     by surface area of the merged box, first strict minimum = lowest j on
-//     ties (bvh.cpp:193-210);
-//   merge decisions for its own ploc_own(R) = TILE-2R positions [s, e):
+//   nearest neighbour of the positions [s - R, e + R) in [i-R, i+R] by surface
+//     area of the merged box, first strict minimum = lowest j on ties
+//     (bvh.cpp:193-210);
+//   merge decisions for its own ploc_own(R) = TILE-3R positions [s, e):
 //     mutual pairs merge at the lower position (bvh.cpp:159-191);
 //   exclusive scan of survivors and compaction (bvh.cpp:125-156), with the
 //     scan across tiles done by decoupled look-back,
@@ -471,11 +471,14 @@ __global__ void __launch_bounds__(256) leaf_init_kernel(const crt_triangle* __re
 // Boxes of positions [s-2R, e+2R) are staged in shared memory as separate
 // min/max coordinate arrays, position s-2R+w at index w; window entries
 // outside [0, n) hold an infinite box (area +inf, never chosen under the strict
-// minimum, as the reference never considers them).  Each thread keeps the
-// boxes of its 4 consecutive positions in registers and walks the 2R+4 boxes
-// around them once, reading two consecutive entries per 8-byte shared load
-// (an even R keeps them aligned), so one load serves up to 8 area
-// evaluations.
+// minimum, as the reference never considers them).
+//
+// PLOC of 16.8 M uniform triangles 6.56 -> 5.09 ms, of 1.31 M 0.75 -> 0.66, by
+// three changes: each pair's area is computed once (ploc_nearest_sym: 6.13 ms),
+// tiles are opened and closed a tile apart (ploc_open: 5.31), and records move in
+// 32-byte accesses, a window's all in flight at once.  A tile's 23.6 k cycles (three
+// blocks an SM) are now: window 2.3, search 8.9, decisions 3.5, look-back 2.5,
+// records 6.4; the search's instructions alone would take about 10.
 //
 // The search compares areas computed from fminf/fmaxf boxes; those differ
 // from the std::min/max boxes only in the sign of a zero, which changes no
@@ -498,14 +501,17 @@ struct __align__(16) PlocSmem {
     static_assert(kWin % 4 == 0, "aligned coordinate arrays");
     float mnx[kWin], mny[kWin], mnz[kWin], mxx[kWin], mxy[kWin], mxz[kWin];
     uint32_t id[kWin], lc[kWin];
-    uint32_t nn[TILE];  // nearest neighbour of position s - R + i
+    __align__(16) uint32_t nn[TILE];  // nearest neighbour of position s - R + i
     unsigned long long wsum[BLOCK / 32];
     unsigned long long prefix;
 };
 
 __device__ __forceinline__ float2 lds2(const float* a) { return *reinterpret_cast<const float2*>(a); }
 
-// Nearest neighbours of this thread's positions q0..q0+3, q0 = s - R + 4t.
+// Nearest neighbours of this thread's positions q0..q0+3, q0 = s - R + 4t (radii
+// without a compiled search, and the cluster kernel).  Each thread keeps the boxes
+// of its 4 positions in registers and walks the 2R+4 boxes around them once,
+// reading two consecutive entries per 8-byte shared load.
 // RC > 0: the radius is the compile-time RC (even); RC == 0:
 // runtime radius R, scalar loads.
 template <int RC, int TILE, int BLOCK, int MAXR>
@@ -600,6 +606,165 @@ __device__ __forceinline__ uint32_t ploc_nearest_at(const PlocSmem<TILE, BLOCK, 
     return static_cast<uint32_t>(bj);
 }
 
+// A tile's shared memory, with the hand-over of ploc_nearest_sym between warps.
+template <int TILE, int BLOCK, int MAXR>
+struct PlocTileSmem : PlocSmem<TILE, BLOCK, MAXR> {
+    static constexpr int kEdges = MAXR / 4 * (MAXR / 4 + 1) / 2;  // of a warp: 1 + 2 + ... groups of four
+    float4 edge_v[BLOCK / 32][kEdges];
+    uint32_t edge_i[BLOCK / 32][kEdges];
+};
+
+// Nearest neighbours of the positions [s - R, e + R) of a tile, each pair's area
+// computed once.  Thread t has the positions q0 .. q0 + 3, q0 = s - 2R + 4t, and
+// walks the groups of four after them as far as R reaches: an area counts for its
+// own position (forward: the candidate is higher) and for the candidate
+// (backward), whose best over this thread's four goes to the thread that owns it,
+// d lanes up, or through shared memory into the next warp.  Ties go to the lowest
+// j: backward over forward, farther backward groups over nearer ones, strict
+// minima in ascending order otherwise.
+//
+// What bounds it: issue slots and the ALU pipe (six minima and maxima and two
+// updates an area, against one update for each of two areas before).
+template <int RC, int TILE, int BLOCK, int MAXR>
+__device__ __forceinline__ void ploc_nearest_sym(PlocTileSmem<TILE, BLOCK, MAXR>& S, int s, int e, int n) {
+    static_assert(RC % 4 == 0 && RC <= MAXR, "whole groups of four");
+    constexpr int D = RC / 4;  // groups after its own that a thread's positions reach
+    const int t = static_cast<int>(threadIdx.x), lane = t & 31, warp = t >> 5;
+    const int q0 = s - 2 * RC + 4 * t, w0 = 4 * t;
+    const float inf = __int_as_float(0x7F800000);
+    float fb[4], bb[4];  // least area forward and backward
+    int fj[4], bj[4];    // its candidate, from q0
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+        fb[i] = bb[i] = inf;
+        fj[i] = bj[i] = i;
+    }
+    const bool live = q0 - 4 * lane < e + RC;  // whole warps: some position is stored (candidates only go up)
+    if (live) {
+        auto four = [&](const float* a, int w, float (&r)[4]) {
+            const float4 v = *reinterpret_cast<const float4*>(a + w);
+            r[0] = v.x; r[1] = v.y; r[2] = v.z; r[3] = v.w;
+        };
+        float anx[4], any[4], anz[4], axx[4], axy[4], axz[4];
+        four(S.mnx, w0, anx); four(S.mny, w0, any); four(S.mnz, w0, anz);
+        four(S.mxx, w0, axx); four(S.mxy, w0, axy); four(S.mxz, w0, axz);
+#pragma unroll
+        for (int k = 1; k < 4; ++k)
+#pragma unroll
+            for (int i = 0; i < k; ++i) {
+                const float dx = fmaxf(axx[i], axx[k]) - fminf(anx[i], anx[k]);
+                const float dy = fmaxf(axy[i], axy[k]) - fminf(any[i], any[k]);
+                const float dz = fmaxf(axz[i], axz[k]) - fminf(anz[i], anz[k]);
+                const float v = 2.0f * (dx * dy + dy * dz + dz * dx);
+                if (v < fb[i]) { fb[i] = v; fj[i] = k; }
+                if (v < bb[k]) { bb[k] = v; bj[k] = i; }
+            }
+#pragma unroll
+        for (int g = 1; g <= D; ++g) {
+            float bnx[4], bny[4], bnz[4], bxx[4], bxy[4], bxz[4], pv[4];
+            four(S.mnx, w0 + 4 * g, bnx); four(S.mny, w0 + 4 * g, bny); four(S.mnz, w0 + 4 * g, bnz);
+            four(S.mxx, w0 + 4 * g, bxx); four(S.mxy, w0 + 4 * g, bxy); four(S.mxz, w0 + 4 * g, bxz);
+            uint32_t pi = 0u;  // the candidates' best among this thread's positions, a byte each
+#pragma unroll
+            for (int u = 0; u < 4; ++u) {
+                pv[u] = inf;
+                uint32_t pu = 0u;
+#pragma unroll
+                for (int i = 0; i < 4; ++i) {
+                    if (4 * g + u - i > RC) continue;
+                    const float dx = fmaxf(axx[i], bxx[u]) - fminf(anx[i], bnx[u]);
+                    const float dy = fmaxf(axy[i], bxy[u]) - fminf(any[i], bny[u]);
+                    const float dz = fmaxf(axz[i], bxz[u]) - fminf(anz[i], bnz[u]);
+                    const float v = 2.0f * (dx * dy + dy * dz + dz * dx);
+                    if (v < fb[i]) { fb[i] = v; fj[i] = 4 * g + u; }
+                    if (v < pv[u]) { pv[u] = v; pu = static_cast<uint32_t>(i) << (8 * u); }
+                }
+                pi |= pu;
+            }
+            const uint32_t ri = __shfl_up_sync(0xFFFFFFFFu, pi, g);
+#pragma unroll
+            for (int u = 0; u < 4; ++u) {
+                const float rv = __shfl_up_sync(0xFFFFFFFFu, pv[u], g);
+                if (lane >= g && rv <= bb[u]) { bb[u] = rv; bj[u] = static_cast<int>(ri >> (8 * u) & 3u) - 4 * g; }
+            }
+            if (lane >= 32 - g) {  // the next warp's lane + g - 32
+                S.edge_v[warp][g * (g - 1) / 2 + lane + g - 32] = make_float4(pv[0], pv[1], pv[2], pv[3]);
+                S.edge_i[warp][g * (g - 1) / 2 + lane + g - 32] = pi;
+            }
+            asm volatile("" ::: "memory");  // the next group's loads stay below this group's work
+        }
+    }
+    __syncthreads();
+    if (!live) return;
+    if (warp > 0)
+        for (int g = lane + 1; g <= D; ++g) {  // groups that lie in the warp before
+            const float4 v = S.edge_v[warp - 1][g * (g - 1) / 2 + lane];
+            const uint32_t ri = S.edge_i[warp - 1][g * (g - 1) / 2 + lane];
+            const float rv[4] = {v.x, v.y, v.z, v.w};
+#pragma unroll
+            for (int u = 0; u < 4; ++u)
+                if (rv[u] <= bb[u]) { bb[u] = rv[u]; bj[u] = static_cast<int>(ri >> (8 * u) & 3u) - 4 * g; }
+        }
+    uint32_t j[4];
+#pragma unroll
+    for (int i = 0; i < 4; ++i) j[i] = static_cast<uint32_t>(q0 + (fb[i] < bb[i] ? fj[i] : (bb[i] < inf ? bj[i] : i)));
+    // four positions from a multiple of four: stored or not together but for the
+    // ends of the array, past which nothing is read
+    if (w0 >= RC && q0 + 3 >= 0 && q0 < min(n, e + RC)) *reinterpret_cast<uint4*>(S.nn + w0 - RC) = make_uint4(j[0], j[1], j[2], j[3]);
+}
+
+// A cluster record or node box, 32 aligned bytes in one access: two 16-byte ones
+// move every sector twice.  Plain accesses: grid_barrier's release and acquire
+// order them between iterations.
+__device__ __forceinline__ void ld_record(const float4* p, float4& a, float4& b) {
+    asm volatile("ld.global.v8.f32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];"
+                 : "=f"(a.x), "=f"(a.y), "=f"(a.z), "=f"(a.w), "=f"(b.x), "=f"(b.y), "=f"(b.z), "=f"(b.w)
+                 : "l"(p)
+                 : "memory");
+}
+__device__ __forceinline__ void st_record(float4* p, const float4& a, const float4& b) {
+    asm volatile("st.global.v8.f32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8};" ::"l"(p), "f"(a.x), "f"(a.y), "f"(a.z), "f"(a.w),
+                 "f"(b.x), "f"(b.y), "f"(b.z), "f"(b.w)
+                 : "memory");
+}
+
+// One warp: (survivors, merges) of the tiles before `tile` (> 0).
+__device__ __forceinline__ void ploc_look_back(uint32_t tile, const unsigned long long* lb_cur, uint32_t* err,
+                                               uint32_t spin_limit, unsigned long long& ev, unsigned long long& em) {
+    const int lane = threadIdx.x & 31;
+    ev = em = 0;
+    // Lane l reads the status word of tile k0 - l (32 predecessors per
+    // round trip, nearest first); the sum runs down to the nearest
+    // inclusive prefix.  (Four words per lane was measured slower:
+    // the nearest prefix is usually a few tiles back.)
+    long long k0 = static_cast<long long>(tile) - 1;
+    SpinBound spin(spin_limit);
+    while (true) {
+        const long long k = k0 - lane;
+        const unsigned long long v = k >= 0 ? ld_relaxed_u64(&lb_cur[k]) : kPlPrefix;
+        const unsigned long long f = v & (3ull << 62);
+        const uint32_t pm = __ballot_sync(0xFFFFFFFFu, f == kPlPrefix);
+        const uint32_t zm = __ballot_sync(0xFFFFFFFFu, f == 0ull);
+        const int stop = pm ? __ffs(pm) - 1 : 31;  // lanes 0..stop are summed
+        const uint32_t upto = stop == 31 ? 0xFFFFFFFFu : ((2u << stop) - 1u);
+        if (zm & upto) {  // a tile before the nearest prefix has not published yet
+            if (!spin.step()) { raise_error(err, kDevTimeout); break; }
+            continue;
+        }
+        unsigned long long cv = lane <= stop ? ((v >> 31) & kPlMask31) : 0ull;
+        unsigned long long cm = lane <= stop ? (v & kPlMask31) : 0ull;
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) {
+            cv += __shfl_xor_sync(0xFFFFFFFFu, cv, o);
+            cm += __shfl_xor_sync(0xFFFFFFFFu, cm, o);
+        }
+        ev += cv;
+        em += cm;
+        if (pm) break;
+        k0 -= 32;
+    }
+}
+
 // One tile of one PLOC iteration (see above).  Reads of data other blocks
 // wrote (the cluster array) bypass L1 (__ldcg), so the same code is correct
 // inside the persistent kernel, where no launch boundary separates iterations.
@@ -611,7 +776,7 @@ __host__ __device__ constexpr uint32_t ploc_own_ipt(int radius) {
     return static_cast<uint32_t>(IPT * BLOCK) - 2u * static_cast<uint32_t>(radius);
 }
 template <int TILE, int BLOCK, int MAXR, int IPT = 4>
-__device__ __forceinline__ void ploc_tile(PlocSmem<TILE, BLOCK, MAXR>& S, uint32_t tile, const uint2 cur, int iter,
+__device__ __forceinline__ void ploc_tile(PlocTileSmem<TILE, BLOCK, MAXR>& S, uint32_t tile, const uint2 cur, int iter,
                                           const float4* __restrict__ cin, float4* __restrict__ cout,
                                           float4* __restrict__ node_box, uint4* __restrict__ node_kids, uint2* it,
                                           uint32_t N, int R, unsigned long long* lb_cur, unsigned long long* lb_next,
@@ -664,9 +829,9 @@ __device__ __forceinline__ void ploc_tile(PlocSmem<TILE, BLOCK, MAXR>& S, uint32
         }
     } else {
         switch (R) {
-            case 8: ploc_nearest<8>(S, s, e, n, R); break;
-            case 16: ploc_nearest<16>(S, s, e, n, R); break;
-            case 32: ploc_nearest<32>(S, s, e, n, R); break;
+            case 8: ploc_nearest_sym<8>(S, s, e, n); break;
+            case 16: ploc_nearest_sym<16>(S, s, e, n); break;
+            case 32: ploc_nearest_sym<32>(S, s, e, n); break;
             default: ploc_nearest<0>(S, s, e, n, R); break;
         }
     }
@@ -715,36 +880,7 @@ __device__ __forceinline__ void ploc_tile(PlocSmem<TILE, BLOCK, MAXR>& S, uint32
             if (lane == 0) st_relaxed_u64(&lb_cur[0], kPlPrefix | (tv << 31) | tm);
         } else {
             if (lane == 0) st_relaxed_u64(&lb_cur[tile], kPlAgg | (tv << 31) | tm);
-            // Lane l reads the status word of tile k0 - l (32 predecessors per
-            // round trip, nearest first); the sum runs down to the nearest
-            // inclusive prefix.  (Four words per lane was measured slower:
-            // the nearest prefix is usually a few tiles back.)
-            long long k0 = static_cast<long long>(tile) - 1;
-            SpinBound spin(spin_limit);
-            while (true) {
-                const long long k = k0 - lane;
-                const unsigned long long v = k >= 0 ? ld_relaxed_u64(&lb_cur[k]) : kPlPrefix;
-                const unsigned long long f = v & (3ull << 62);
-                const uint32_t pm = __ballot_sync(0xFFFFFFFFu, f == kPlPrefix);
-                const uint32_t zm = __ballot_sync(0xFFFFFFFFu, f == 0ull);
-                const int stop = pm ? __ffs(pm) - 1 : 31;  // lanes 0..stop are summed
-                const uint32_t upto = stop == 31 ? 0xFFFFFFFFu : ((2u << stop) - 1u);
-                if (zm & upto) {  // a tile before the nearest prefix has not published yet
-                    if (!spin.step()) { raise_error(err, kDevTimeout); break; }
-                    continue;
-                }
-                unsigned long long cv = lane <= stop ? ((v >> 31) & kPlMask31) : 0ull;
-                unsigned long long cm = lane <= stop ? (v & kPlMask31) : 0ull;
-#pragma unroll
-                for (int o = 16; o > 0; o >>= 1) {
-                    cv += __shfl_xor_sync(0xFFFFFFFFu, cv, o);
-                    cm += __shfl_xor_sync(0xFFFFFFFFu, cm, o);
-                }
-                ev += cv;
-                em += cm;
-                if (pm) break;
-                k0 -= 32;
-            }
+            ploc_look_back(tile, lb_cur, err, spin_limit, ev, em);
             if (lane == 0) st_relaxed_u64(&lb_cur[tile], kPlPrefix | ((ev + tv) << 31) | (em + tm));
         }
         if (lane == 0) {
@@ -789,13 +925,173 @@ __device__ __forceinline__ void ploc_tile(PlocSmem<TILE, BLOCK, MAXR>& S, uint32
     }
 }
 
+// ---- Tiles of an iteration with more tiles than blocks, in two halves.
+// ploc_open: window, search, decisions and the tile's totals, published at once;
+// ploc_close: look-back, then the survivors' records.  A block opens its next tile
+// before it closes the last one, so a tile's predecessors have a whole tile's time
+// to publish: with both halves in one, a third of a tile's time went into waiting
+// for the slowest of the several hundred tiles before it (10.4 k of 31 k cycles).
+// Decisions wait as one word a position; close reads the records again (from L2).
+template <int TILE, int BLOCK, int MAXR>
+struct PlocPipeSmem {
+    static constexpr int kWin = TILE + 2 * MAXR;
+    PlocTileSmem<TILE, BLOCK, MAXR> tile;
+    __align__(16) uint32_t dec[2][TILE];  // place among the tile's survivors | among its merges << 11 | partner - p << 21 | flags
+    unsigned long long prefix;
+    uint32_t ticket;
+};
+constexpr uint32_t kDecKeep = 1u << 27, kDecHead = 1u << 28;
+
+template <int TILE, int BLOCK, int MAXR>
+__device__ __forceinline__ uint32_t ploc_open(PlocPipeSmem<TILE, BLOCK, MAXR>& P, int buf, uint32_t tile, int n,
+                                              const float4* __restrict__ cin, int R, unsigned long long* lb_cur,
+                                              unsigned long long* lb_next) {
+    PlocTileSmem<TILE, BLOCK, MAXR>& S = P.tile;
+    const int own = static_cast<int>(ploc_own(R)), s = static_cast<int>(tile) * own, e = min(n, s + own);
+    const int wbase = s - 2 * R, nbase = s - R;
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    if (threadIdx.x == 0) st_relaxed_u64(&lb_next[tile], 0ull);
+    const float inf = __int_as_float(0x7F800000);
+    {  // every load of the window in flight at once (the last round is a few threads')
+        constexpr int kRounds = (PlocSmem<TILE, BLOCK, MAXR>::kWin + BLOCK - 1) / BLOCK;
+        float4 a[kRounds], b[kRounds];
+        const int first = static_cast<int>(threadIdx.x) + wbase, hi = min(n, e + 2 * R);
+#pragma unroll
+        for (int r = 0; r < kRounds; ++r) {
+            const int p = first + r * BLOCK;
+            if (p >= 0 && p < hi) {
+                ld_record(cin + 2 * static_cast<size_t>(p), a[r], b[r]);
+            } else {
+                a[r] = make_float4(-inf, -inf, -inf, 0.f);
+                b[r] = make_float4(inf, inf, inf, 0.f);
+            }
+        }
+#pragma unroll
+        for (int r = 0; r < kRounds; ++r) {
+            const int w = static_cast<int>(threadIdx.x) + r * BLOCK;
+            if (w >= PlocSmem<TILE, BLOCK, MAXR>::kWin) break;
+            S.mnx[w] = a[r].x; S.mny[w] = a[r].y; S.mnz[w] = a[r].z;
+            S.mxx[w] = b[r].x; S.mxy[w] = b[r].y; S.mxz[w] = b[r].z;
+        }
+    }
+    __syncthreads();
+    switch (R) {
+        case 8: ploc_nearest_sym<8>(S, s, e, n); break;
+        case 16: ploc_nearest_sym<16>(S, s, e, n); break;
+        case 32: ploc_nearest_sym<32>(S, s, e, n); break;
+        default: ploc_nearest<0>(S, s, e, n, R); break;
+    }
+    __syncthreads();
+    // thread t decides positions s + 4t .. s + 4t + 3
+    constexpr int IPT = TILE / BLOCK;
+    uint32_t dec[IPT], nv = 0, nm = 0;
+#pragma unroll
+    for (int q = 0; q < IPT; ++q) {
+        const int p = s + static_cast<int>(threadIdx.x) * IPT + q;
+        dec[q] = 0u;
+        if (p >= e) continue;
+        const int j = static_cast<int>(S.nn[p - nbase]);
+        const bool mutual = (j != p) && (static_cast<int>(S.nn[j - nbase]) == p);
+        if (mutual && p > j) continue;
+        dec[q] = kDecKeep | nv | nm << 11;
+        ++nv;
+        if (mutual) {
+            dec[q] |= kDecHead | static_cast<uint32_t>(j - p) << 21;
+            ++nm;
+        }
+    }
+    const uint32_t packed = nv | nm << 11;
+    uint32_t incl = packed;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+        const uint32_t y = __shfl_up_sync(0xFFFFFFFFu, incl, o);
+        if (lane >= o) incl += y;
+    }
+    if (lane == 31) S.wsum[warp] = incl;
+    __syncthreads();
+    uint32_t before = 0u, total = 0u;  // at most 1,024 | 512: no carry between the two
+#pragma unroll
+    for (int w = 0; w < BLOCK / 32; ++w) {
+        const uint32_t v = static_cast<uint32_t>(S.wsum[w]);
+        if (w < warp) before += v;
+        total += v;
+    }
+    if (threadIdx.x == 0)
+        st_relaxed_u64(&lb_cur[tile], (tile == 0 ? kPlPrefix : kPlAgg) |
+                                          static_cast<unsigned long long>(total & 0x7FFu) << 31 | total >> 11);
+    before += incl - packed;
+#pragma unroll
+    for (int q = 0; q < IPT; ++q) dec[q] = dec[q] ? dec[q] + before : 0u;
+    static_assert(IPT == 4, "one vector a thread");
+    *reinterpret_cast<uint4*>(&P.dec[buf][4 * threadIdx.x]) = make_uint4(dec[0], dec[1], dec[2], dec[3]);
+    return total;
+}
+
+template <int TILE, int BLOCK, int MAXR>
+__device__ __forceinline__ void ploc_close(PlocPipeSmem<TILE, BLOCK, MAXR>& P, int buf, uint32_t tile, uint32_t total,
+                                           const uint2 cur, int iter, const float4* __restrict__ cin,
+                                           float4* __restrict__ cout, float4* __restrict__ node_box,
+                                           uint4* __restrict__ node_kids, uint2* it, uint32_t N, int R,
+                                           unsigned long long* lb_cur, uint32_t* err, uint32_t spin_limit) {
+    constexpr int IPT = TILE / BLOCK;
+    const int n = static_cast<int>(cur.x), own = static_cast<int>(ploc_own(R));
+    const int s = static_cast<int>(tile) * own, e = min(n, s + own);
+    if (threadIdx.x < 32) {
+        const unsigned long long tv = total & 0x7FFu, tm = total >> 11;
+        unsigned long long ev = 0, em = 0;
+        if (tile > 0) {
+            ploc_look_back(tile, lb_cur, err, spin_limit, ev, em);
+            if (threadIdx.x == 0) st_relaxed_u64(&lb_cur[tile], kPlPrefix | ((ev + tv) << 31) | (em + tm));
+        }
+        if (threadIdx.x == 0) {
+            P.prefix = (ev << 32) | em;
+            if (e == n)  // last tile: size and id base of the next iteration
+                it[iter + 1] = make_uint2(static_cast<uint32_t>(ev + tv), cur.y + static_cast<uint32_t>(em + tm));
+        }
+    }
+    __syncthreads();
+    const uint32_t base_v = static_cast<uint32_t>(P.prefix >> 32), base_m = cur.y + static_cast<uint32_t>(P.prefix);
+    // Neighbouring threads take neighbouring positions, one at a time: two or four
+    // positions' records in flight cost registers (16.8 M clusters 5.45 and 6.51 ms
+    // against 5.09; all four during the look-back 6.35).
+#pragma unroll
+    for (int q = 0; q < IPT; ++q) {
+        const int x = q * BLOCK + static_cast<int>(threadIdx.x);
+        const uint32_t d = x < e - s ? P.dec[buf][x] : 0u;
+        if (!d) continue;
+        const uint32_t p = static_cast<uint32_t>(s + x), out_v = base_v + (d & 0x7FFu);
+        const float4* r = cin + 2 * static_cast<size_t>(p);
+        float4 mn, mx;
+        ld_record(r, mn, mx);
+        if (d & kDecHead) {
+            float4 jn, jx, m0, m1;
+            ld_record(r + 2 * (d >> 21 & 0x3Fu), jn, jx);
+            const uint32_t id = base_m + (d >> 11 & 0x3FFu);
+            if (id >= 2 * N - 1 || id < N) { raise_corrupt(err, 2 + (iter << 8), p, id); continue; }
+            // AABB::merge (bvh.cpp:401-413), first argument = lower position
+            m0.x = min_std(mn.x, jn.x); m0.y = min_std(mn.y, jn.y); m0.z = min_std(mn.z, jn.z);
+            m1.x = max_std(mx.x, jx.x); m1.y = max_std(mx.y, jx.y); m1.z = max_std(mx.z, jx.z);
+            m0.w = mn.w;  // left child id
+            m1.w = jn.w;  // right child id
+            st_record(node_box + 2 * static_cast<size_t>(id), m0, m1);
+            const uint32_t lca = __float_as_uint(mx.w), lcb = __float_as_uint(jx.w);
+            // children and their leaf counts, read by the DFS layout
+            node_kids[id - N] = make_uint4(__float_as_uint(mn.w), __float_as_uint(jn.w), lca, lcb);
+            mn = make_float4(m0.x, m0.y, m0.z, __uint_as_float(id));
+            mx = make_float4(m1.x, m1.y, m1.z, __uint_as_float(lca + lcb));
+        }
+        if (out_v >= static_cast<uint32_t>(n)) { raise_corrupt(err, 3 + (iter << 8), p, out_v); continue; }
+        st_record(cout + 2 * static_cast<size_t>(out_v), mn, mx);
+    }
+}
+
 template <int TILE, int BLOCK, int MAXR>
 __global__ void __launch_bounds__(BLOCK) ploc_iteration_kernel(const float4* __restrict__ cin, float4* __restrict__ cout,
                                                                float4* __restrict__ node_box, uint4* __restrict__ node_kids,
                                                                uint2* it, int iter, uint32_t N,
                                                                int R, unsigned long long* lookback, uint32_t* tickets,
                                                                uint32_t n_tiles_cap, uint32_t* err, uint32_t spin_limit) {
-    __shared__ PlocSmem<TILE, BLOCK, MAXR> S;
+    __shared__ PlocTileSmem<TILE, BLOCK, MAXR> S;
     __shared__ uint32_t s_tile;
     const uint2 cur = it[iter];
     const uint32_t n = cur.x;
@@ -1305,20 +1601,73 @@ __global__ void __launch_bounds__(kClusterThreads) ploc_cluster_kernel(const flo
     }
 }
 
+// The iterations of more tiles than one_wave_tiles; iters_out: their number.
 template <int TILE, int BLOCK, int MAXR>
-__global__ void __launch_bounds__(BLOCK, kPlocBlocksPerSm) ploc_persistent_kernel(float4* ca, float4* cb, float4* __restrict__ node_box,
-                                                                uint4* __restrict__ node_kids, uint2* it, uint32_t N,
-                                                                int R, uint32_t stop_n, unsigned long long* lookback,
-                                                                uint32_t* tickets, uint32_t n_tiles_cap,
-                                                                unsigned long long* bar, uint32_t* iters_out,
-                                                                uint32_t* err, uint32_t spin_limit) {
-    __shared__ PlocSmem<TILE, BLOCK, MAXR> S;
-    __shared__ uint32_t s_tile;
+__global__ void __launch_bounds__(BLOCK, kPlocBlocksPerSm) ploc_wide_kernel(float4* ca, float4* cb, float4* __restrict__ node_box,
+                                                           uint4* __restrict__ node_kids, uint2* it, uint32_t N, int R,
+                                                           uint32_t one_wave_tiles, unsigned long long* lookback,
+                                                           uint32_t* tickets, uint32_t n_tiles_cap, unsigned long long* bar,
+                                                           uint32_t* iters_out, uint32_t* err, uint32_t spin_limit) {
+    __shared__ PlocPipeSmem<TILE, BLOCK, MAXR> P;
     unsigned long long bar_target = 0;  // grid barriers passed x gridDim (thread 0)
     int iter = 0;
     for (;; ++iter) {
         const uint2 cur = __ldcg(it + iter);
-        if (cur.x <= 1u) break;
+        const uint32_t n_tiles = (cur.x + ploc_own(R) - 1) / ploc_own(R);
+        if (n_tiles <= one_wave_tiles) break;
+        const float4* cin = (iter & 1) ? cb : ca;
+        float4* cout = (iter & 1) ? ca : cb;
+        unsigned long long* lb_cur = lookback + static_cast<size_t>(iter & 1) * n_tiles_cap;
+        unsigned long long* lb_next = lookback + static_cast<size_t>((iter + 1) & 1) * n_tiles_cap;
+        // A block takes its next ticket when it has opened a tile, and then closes
+        // the tile before.  Tickets follow the order of these starts, and the
+        // smallest unpublished tile's block only waits for smaller ones, so every
+        // look-back wait ends.
+        if (threadIdx.x == 0) P.ticket = atomicAdd(&tickets[iter & 1], 1u);
+        uint32_t open = 0u, open_total = 0u;
+        bool some = false;  // a tile is open
+        for (int buf = 0;; buf ^= 1) {
+            __syncthreads();
+            const uint32_t tile = P.ticket;
+            const bool more = tile < n_tiles;
+            uint32_t total = 0u;
+            if (more) {
+                total = ploc_open(P, buf, tile, static_cast<int>(cur.x), cin, R, lb_cur, lb_next);
+                if (threadIdx.x == 32) {  // not the warp that looks back
+                    P.ticket = atomicAdd(&tickets[iter & 1], 1u);
+                    if (tile == 0) tickets[(iter + 1) & 1] = 0u;
+                }
+            }
+            if (some)
+                ploc_close(P, buf ^ 1, open, open_total, cur, iter, cin, cout, node_box, node_kids, it, N, R, lb_cur, err,
+                           spin_limit);
+            if (!more) break;
+            some = true;
+            open = tile;
+            open_total = total;
+        }
+        if (!grid_barrier(bar, bar_target, err, spin_limit)) return;
+        if (static_cast<uint32_t>(iter) + 1 >= N) { raise_error(err, kDevIterLimit); return; }
+    }
+    if (blockIdx.x == 0 && threadIdx.x == 0) iters_out[0] = static_cast<uint32_t>(iter);
+}
+
+// The iterations of at most a tile a block, down to stop_n clusters.  Two blocks
+// an SM: an iteration is a chain of latencies and its grid barrier, which fewer
+// blocks shorten (65,536 clusters 225 -> 213 us of PLOC, 300,000 379 -> 369).
+// wide_grid: the blocks of ploc_wide_kernel, which counted its barriers in bar too.
+template <int TILE, int BLOCK, int MAXR>
+__global__ void __launch_bounds__(BLOCK, kPlocOneWaveBlocksPerSm) ploc_persistent_kernel(float4* ca, float4* cb, float4* __restrict__ node_box,
+                                                                uint4* __restrict__ node_kids, uint2* it, uint32_t N,
+                                                                int R, uint32_t stop_n, unsigned long long* lookback,
+                                                                uint32_t n_tiles_cap, uint32_t wide_grid,
+                                                                unsigned long long* bar, uint32_t* iters_out,
+                                                                uint32_t* err, uint32_t spin_limit) {
+    __shared__ PlocTileSmem<TILE, BLOCK, MAXR> S;
+    int iter = static_cast<int>(__ldcg(iters_out));
+    unsigned long long bar_target = static_cast<unsigned long long>(iter) * wide_grid;
+    for (;; ++iter) {
+        const uint2 cur = __ldcg(it + iter);
         if (cur.x <= stop_n) break;  // every block reads the same record; the cluster kernel takes over
         const float4* cin = (iter & 1) ? cb : ca;
         float4* cout = (iter & 1) ? ca : cb;
@@ -1327,50 +1676,28 @@ __global__ void __launch_bounds__(BLOCK, kPlocBlocksPerSm) ploc_persistent_kerne
         const uint32_t n_tiles = (cur.x + ploc_own(R) - 1) / ploc_own(R);
         const uint32_t n_t1 = (cur.x + ploc_own_ipt<1, BLOCK>(R) - 1) / ploc_own_ipt<1, BLOCK>(R);
         const uint32_t n_t2 = (cur.x + ploc_own_ipt<2, BLOCK>(R) - 1) / ploc_own_ipt<2, BLOCK>(R);
-        // one (two) positions per thread while those smaller tiles number at
-        // most kPlocSmallTiles1 (kPlocSmallTiles2) per SM and fit the look-back
-        // arrays: the iteration then costs one short tile's latency
-        const uint32_t per_sm = gridDim.x / kPlocBlocksPerSm;
-        const int ipt = (n_t1 <= kPlocSmallTiles1 * per_sm && n_t1 <= n_tiles_cap)   ? 1
-                        : (n_t2 <= kPlocSmallTiles2 * per_sm && n_t2 <= n_tiles_cap) ? 2
-                                                                                      : 4;
-        const bool small = ipt < 4;
-        if (small || n_tiles <= gridDim.x) {
-            // One wave: block b runs tile b (all tiles are co-resident, so
-            // every look-back wait ends), with no ticket round trips.
-            if (blockIdx.x == 0 && threadIdx.x == 0) tickets[(iter + 1) & 1] = 0u;
-            // Every block clears its word of the next iteration's look-back
-            // array: the next iteration may cut its (fewer) clusters into more,
-            // smaller tiles than this one has, and a tile clears only its own
-            // word (the grid barrier below orders these stores before any read).
-            if (threadIdx.x == 0 && blockIdx.x < n_tiles_cap) st_relaxed_u64(&lb_next[blockIdx.x], 0ull);
-            if (ipt == 1) {
-                if (blockIdx.x < n_t1)
-                    ploc_tile<TILE, BLOCK, MAXR, 1>(S, blockIdx.x, cur, iter, cin, cout, node_box, node_kids, it, N, R,
-                                                    lb_cur, lb_next, err, spin_limit);
-            } else if (ipt == 2) {
-                if (blockIdx.x < n_t2)
-                    ploc_tile<TILE, BLOCK, MAXR, 2>(S, blockIdx.x, cur, iter, cin, cout, node_box, node_kids, it, N, R,
-                                                    lb_cur, lb_next, err, spin_limit);
-            } else if (blockIdx.x < n_tiles) {
-                ploc_tile<TILE, BLOCK, MAXR>(S, blockIdx.x, cur, iter, cin, cout, node_box, node_kids, it, N, R, lb_cur,
-                                             lb_next, err, spin_limit);
-            }
-            if (!grid_barrier(bar, bar_target, err, spin_limit)) return;
-            if (static_cast<uint32_t>(iter) + 1 >= N) { raise_error(err, kDevIterLimit); return; }
-            continue;
+        if (n_tiles > gridDim.x) {  // the first kernel stops below that; only corruption gets here
+            if (blockIdx.x == 0 && threadIdx.x == 0) raise_corrupt(err, 15, static_cast<uint32_t>(iter), cur.x);
+            return;
         }
-        // More tiles than blocks: a block takes its next ticket only when it
-        // has finished a tile, so tickets follow completion order and a
-        // tile's look-back finds its predecessors already published.
-        for (;;) {
-            __syncthreads();
-            if (threadIdx.x == 0) s_tile = atomicAdd(&tickets[iter & 1], 1u);
-            __syncthreads();
-            const uint32_t tile = s_tile;
-            if (tile * ploc_own(R) >= cur.x) break;
-            if (tile == 0 && threadIdx.x == 0) tickets[(iter + 1) & 1] = 0u;
-            ploc_tile<TILE, BLOCK, MAXR>(S, tile, cur, iter, cin, cout, node_box, node_kids, it, N, R, lb_cur, lb_next,
+        // One wave: block b runs tile b (all tiles are co-resident, so every
+        // look-back wait ends).  One (two) positions per thread while those smaller
+        // tiles fit the grid and the look-back arrays: the iteration then costs one
+        // short tile's latency.  Every block clears its word of the next iteration's
+        // look-back array: the next iteration may cut its (fewer) clusters into
+        // more, smaller tiles than this one has, and a tile clears only its own
+        // word (the grid barrier below orders these stores before any read).
+        if (threadIdx.x == 0 && blockIdx.x < n_tiles_cap) st_relaxed_u64(&lb_next[blockIdx.x], 0ull);
+        if (n_t1 <= gridDim.x && n_t1 <= n_tiles_cap) {
+            if (blockIdx.x < n_t1)
+                ploc_tile<TILE, BLOCK, MAXR, 1>(S, blockIdx.x, cur, iter, cin, cout, node_box, node_kids, it, N, R, lb_cur,
+                                                lb_next, err, spin_limit);
+        } else if (n_t2 <= gridDim.x && n_t2 <= n_tiles_cap) {
+            if (blockIdx.x < n_t2)
+                ploc_tile<TILE, BLOCK, MAXR, 2>(S, blockIdx.x, cur, iter, cin, cout, node_box, node_kids, it, N, R, lb_cur,
+                                                lb_next, err, spin_limit);
+        } else if (blockIdx.x < n_tiles) {
+            ploc_tile<TILE, BLOCK, MAXR>(S, blockIdx.x, cur, iter, cin, cout, node_box, node_kids, it, N, R, lb_cur, lb_next,
                                          err, spin_limit);
         }
         if (!grid_barrier(bar, bar_target, err, spin_limit)) return;
@@ -1749,22 +2076,15 @@ void launch_layout_emit(const float4* node_box, const uint4* node_kids, const ui
                                                          lv, st, err);
 }
 
-int ploc_persistent_grid() {
-    static int grid = -1;
-    if (grid < 0) {
-        int per_sm = 0, dev = 0, sms = kNumSms, coop = 0;
-        cudaGetDevice(&dev);
-        cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-        cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, dev);
-        if (coop && cudaOccupancyMaxActiveBlocksPerMultiprocessor(
-                        &per_sm, ploc_persistent_kernel<kPlocSpan, 256, kPlocMaxRadius>, 256, 0) == cudaSuccess &&
-            per_sm > 0)
-            grid = (per_sm < kPlocBlocksPerSm ? per_sm : kPlocBlocksPerSm) * sms;
-        else
-            grid = 0;
-        cudaGetLastError();
-    }
-    return grid;
+// Blocks of a cooperative 256-thread launch of f, at most per_sm_max an SM (0: none).
+static int cooperative_grid(const void* f, int per_sm_max) {
+    int per_sm = 0, dev = 0, sms = kNumSms, coop = 0;
+    cudaGetDevice(&dev);
+    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+    cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, dev);
+    if (!coop || cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, f, 256, 0) != cudaSuccess) per_sm = 0;
+    cudaGetLastError();
+    return (per_sm < per_sm_max ? per_sm : per_sm_max) * sms;
 }
 
 // Launch of a PLOC cluster kernel: `clusters` clusters of `blocks` blocks.
@@ -1812,15 +2132,25 @@ cudaError_t launch_ploc_layout(float4* ca, float4* cb, float4* node_box, uint4* 
                                uint2* pf, crt_bvh_node* out, float4* wide, float4* wide_wt, uint8_t* depth_odd,
                                LeafOut lv, const SceneState* st, unsigned long long* bar, uint32_t* iters_out,
                                uint32_t* err, uint32_t spin_limit, cudaEvent_t ploc_done, cudaStream_t s) {
-    const int grid = ploc_persistent_grid(), blocks = ploc_cluster_blocks();
-    if (grid <= 0 || blocks <= 0) return cudaErrorNotSupported;
+    const void* wide_fn = reinterpret_cast<const void*>(ploc_wide_kernel<kPlocSpan, 256, kPlocMaxRadius>);
+    const void* wave_fn = reinterpret_cast<const void*>(ploc_persistent_kernel<kPlocSpan, 256, kPlocMaxRadius>);
+    static const int wide_blocks = cooperative_grid(wide_fn, kPlocBlocksPerSm);
+    static const int wave_blocks = cooperative_grid(wave_fn, kPlocOneWaveBlocksPerSm);
+    const int blocks = ploc_cluster_blocks();
+    if (wide_blocks <= 0 || wave_blocks <= 0 || blocks <= 0) return cudaErrorNotSupported;
     uint32_t stop_n = static_cast<uint32_t>(blocks * (kClusterTile - 2 * radius));
+    uint32_t one_wave = static_cast<uint32_t>(wave_blocks), wide_grid = static_cast<uint32_t>(wide_blocks);
     cudaError_t e = cudaSuccess;
-    if (N > stop_n) {
-        void* args[] = {&ca, &cb, &node_box, &node_kids, &it, &N, &radius, &stop_n, &lookback, &tickets, &n_tiles_cap,
+    if ((N + ploc_own(radius) - 1) / ploc_own(radius) > one_wave) {
+        void* args[] = {&ca, &cb, &node_box, &node_kids, &it, &N, &radius, &one_wave, &lookback, &tickets, &n_tiles_cap,
                         &bar, &iters_out, &err, &spin_limit};
-        e = cudaLaunchCooperativeKernel(reinterpret_cast<const void*>(ploc_persistent_kernel<kPlocSpan, 256, kPlocMaxRadius>),
-                                        dim3(grid), dim3(256), args, 0, s);
+        e = cudaLaunchCooperativeKernel(wide_fn, dim3(wide_grid), dim3(256), args, 0, s);
+        if (e != cudaSuccess) return e;
+    }
+    if (N > stop_n) {
+        void* args[] = {&ca, &cb, &node_box, &node_kids, &it, &N, &radius, &stop_n, &lookback, &n_tiles_cap, &wide_grid,
+                        &bar, &iters_out, &err, &spin_limit};
+        e = cudaLaunchCooperativeKernel(wave_fn, dim3(one_wave), dim3(256), args, 0, s);
         if (e != cudaSuccess) return e;
     }
     ClusterLaunch l(blocks, 1, s);

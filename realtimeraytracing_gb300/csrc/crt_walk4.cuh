@@ -108,7 +108,7 @@ __device__ __forceinline__ bool walk4_setup(Walk4Ray& w, float3 o, float3 d, flo
 // Distance of the plane in byte C of word; SAT: clamped to [0, 1], which is free
 // (distances carry 2^-100, so only negative ones, and NaN, change: to 0).  Steps
 // stored as floats instead of exponent bytes, this clamp and three-operand minima
-// take 17 ALU operations off a visit: 1280x720 frames 838 -> 765 us, 8.4 M bounce
+// take 17 ALU operations off a visit: 1280x720 frames 838 -> 795 us, 8.4 M bounce
 // rays 6.32 -> 6.16 ms (memory latency bounds those).
 template <int C, bool SAT = false>
 __device__ __forceinline__ float walk4_plane(uint32_t word, float a, float b) {

@@ -66,3 +66,17 @@ def test_batches_of_scenes(n_scenes):
         assert batch.scene_info(k)["iterations"] == ref["iterations"]
     batch.free()
     ctx.close()
+
+
+@pytest.mark.parametrize("radius,n", [(16, 304 * 976), (16, 304 * 976 + 1), (8, 304 * 1000 + 1), (32, 304 * 928 + 1),
+                                      (5, 304 * 1009 + 1), (16, 600_001)])
+def test_more_tiles_than_blocks(radius, n):
+    """Iterations of more tiles than the one-wave launch has blocks (two an SM) run
+    opened and closed a tile apart: the largest size without one, one past it for each
+    compiled radius and another, and several tiles a block."""
+    _check(S.uniform_soup(n, seed=n + radius), radius)
+
+
+def test_equal_boxes_over_many_tiles():
+    """Equal boxes across tile and warp boundaries: the lowest position wins ties."""
+    _check(np.repeat(S.uniform_soup(17_000, seed=8), 21, axis=0), 16)
