@@ -230,10 +230,9 @@ __global__ void __launch_bounds__(256) batch_leaf_init_kernel(const crt_triangle
     mx.y = max_std(p0.y, max_std(p1.y, p2.y));
     mx.z = max_std(p0.z, max_std(p1.z, p2.z));
     const size_t nb = 2 * (static_cast<size_t>(sc.node_off) + li);
-    node_box[nb] = make_float4(mn.x, mn.y, mn.z, __uint_as_float(tl));
-    node_box[nb + 1] = make_float4(mx.x, mx.y, mx.z, 0.f);
-    clusters[2 * static_cast<size_t>(i)] = make_float4(mn.x, mn.y, mn.z, __uint_as_float(li));
-    clusters[2 * static_cast<size_t>(i) + 1] = make_float4(mx.x, mx.y, mx.z, __uint_as_float(1u));
+    st_record(node_box + nb, make_float4(mn.x, mn.y, mn.z, __uint_as_float(tl)), make_float4(mx.x, mx.y, mx.z, 0.f));
+    st_record(clusters + 2 * static_cast<size_t>(i), make_float4(mn.x, mn.y, mn.z, __uint_as_float(li)),
+              make_float4(mx.x, mx.y, mx.z, __uint_as_float(1u)));
     // sorted order; the layout moves them into tree order (a one-triangle
     // scene's single leaf is in both orders at once)
     float4* xo = (sc.n_tris == 1 ? xtri : xtri_sorted) + 3 * static_cast<size_t>(i);
