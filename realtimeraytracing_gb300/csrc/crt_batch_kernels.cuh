@@ -272,14 +272,15 @@ __device__ __forceinline__ uint32_t block_exclusive(uint32_t v, uint32_t* s_warp
 // The PLOC iterations of the scenes of more than stop_n live clusters, in
 // lockstep.  Each iteration: every block derives the running scenes' tile counts,
 // takes tiles from one ticket counter, maps a ticket to (scene, tile) and runs the
-// single-scene tile code on that scene's slices.  A grid barrier separates
+// single-scene tile code (ploc_open, ploc_close) on that scene's slices.  A grid barrier separates
 // iterations.  A scene leaves with its iteration count in scenes[].iters once it
 // has stop_n clusters or fewer; batch_cluster_kernel finishes it.  Thread k of
 // every block keeps scene k, and the tile counts are scanned by the whole block:
 // a loop over the scenes in one thread cost 64 dependent steps an iteration.
 // Whole batch builds before and with the three launches below, us: 64 scenes of
-// 1,000-250,000 triangles 2,730 -> 1,663, 16 of 5,000-20,000 886 -> 403, 200 of
-// 100-5,000 1,795 -> 456, 2 of 1-1.5 M 2,493 -> 1,961.
+// 1,000-250,000 triangles 2,730 -> 1,446, 16 of 5,000-20,000 886 -> 394, 200 of
+// 100-5,000 1,795 -> 442, 2 of 1-1.5 M 2,493 -> 1,642 (the first and the last were
+// 1,566 and 1,836 with tiles that wait for their predecessors at once).
 template <int TILE, int BLOCK, int MAXR>
 __global__ void __launch_bounds__(BLOCK, kPlocBlocksPerSm) batch_ploc_kernel(BatchScene* scenes, uint32_t n_scenes, float4* ca, float4* cb,
                                                            float4* node_box, uint4* node_kids, uint2* it, int R,
@@ -287,12 +288,11 @@ __global__ void __launch_bounds__(BLOCK, kPlocBlocksPerSm) batch_ploc_kernel(Bat
                                                            uint32_t* tickets, unsigned long long* bar, uint32_t max_iters,
                                                            uint32_t* err, uint32_t spin_limit) {
     static_assert(BLOCK >= static_cast<int>(kMaxBatchScenes), "a thread per scene");
-    __shared__ PlocTileSmem<TILE, BLOCK, MAXR> S;
+    __shared__ PlocPipeSmem<TILE, BLOCK, MAXR> P;
     unsigned long long bar_target = 0;  // grid barriers passed x gridDim (thread 0)
     __shared__ uint32_t s_tile_pre[BLOCK];
     __shared__ uint32_t s_n[BLOCK];
     __shared__ uint32_t s_warp[BLOCK / 32];
-    __shared__ uint32_t s_tile;
     const uint32_t k = threadIdx.x;
     uint32_t n = k < n_scenes ? scenes[k].n_tris : 0u;  // scene k's live clusters; no longer read once <= stop_n
     const uint32_t it_off = k < n_scenes ? scenes[k].it_off : 0u;
@@ -307,27 +307,46 @@ __global__ void __launch_bounds__(BLOCK, kPlocBlocksPerSm) batch_ploc_kernel(Bat
         s_tile_pre[k] = block_exclusive<BLOCK>(tiles, s_warp, total);
         if (total == 0u) break;  // uniform: every thread has the same total
         if (static_cast<uint32_t>(iter) >= max_iters) { raise_error(err, kDevIterLimit); return; }
-        for (;;) {
+        // as ploc_wide_kernel: a tile is opened before the last one is closed
+        if (threadIdx.x == 0) P.ticket = atomicAdd(&tickets[iter & 1], 1u);
+        uint32_t open = 0u, open_scene = 0u, open_total = 0u;
+        bool some = false;  // a tile is open
+        for (int buf = 0;; buf ^= 1) {
             __syncthreads();
-            if (threadIdx.x == 0) s_tile = atomicAdd(&tickets[iter & 1], 1u);
-            __syncthreads();
-            const uint32_t g = s_tile;
-            if (g >= total) break;
-            if (g == 0 && threadIdx.x == 0) tickets[(iter + 1) & 1] = 0u;
-            uint32_t lo = 0, hi = n_scenes - 1;  // scene whose tile range holds g
-            while (lo < hi) {
-                const uint32_t mid = (lo + hi + 1) >> 1;
-                if (s_tile_pre[mid] <= g) lo = mid; else hi = mid - 1;
+            const uint32_t g = P.ticket;
+            const bool more = g < total;
+            uint32_t lo = 0, tile_total = 0u, tile = 0u;
+            if (more) {
+                uint32_t hi = n_scenes - 1;  // the scene whose tile range holds g
+                while (lo < hi) {
+                    const uint32_t mid = (lo + hi + 1) >> 1;
+                    if (s_tile_pre[mid] <= g) lo = mid; else hi = mid - 1;
+                }
+                tile = g - s_tile_pre[lo];
+                const BatchScene& B = scenes[lo];
+                const float4* cin = ((iter & 1) ? cb : ca) + 2 * static_cast<size_t>(B.tri_off);
+                unsigned long long* lb = lookback + B.lb_off;
+                tile_total = ploc_open(P, buf, tile, static_cast<int>(s_n[lo]), cin, R, lb + static_cast<size_t>(iter & 1) * lb_cap,
+                                       lb + static_cast<size_t>((iter + 1) & 1) * lb_cap);
+                if (threadIdx.x == 32) {  // not the warp that looks back
+                    P.ticket = atomicAdd(&tickets[iter & 1], 1u);
+                    if (g == 0) tickets[(iter + 1) & 1] = 0u;
+                }
             }
-            const uint32_t sc = lo, tile = g - s_tile_pre[sc];
-            const BatchScene B = scenes[sc];
-            const uint2 cur = make_uint2(s_n[sc], __ldcg(it + B.it_off + iter).y);
-            float4* cin = ((iter & 1) ? cb : ca) + 2 * static_cast<size_t>(B.tri_off);
-            float4* cout = ((iter & 1) ? ca : cb) + 2 * static_cast<size_t>(B.tri_off);
-            unsigned long long* lb_cur = lookback + static_cast<size_t>(iter & 1) * lb_cap + B.lb_off;
-            unsigned long long* lb_next = lookback + static_cast<size_t>((iter + 1) & 1) * lb_cap + B.lb_off;
-            ploc_tile<TILE, BLOCK, MAXR>(S, tile, cur, iter, cin, cout, node_box + 2 * static_cast<size_t>(B.node_off),
-                                         node_kids + B.tri_off, it + B.it_off, B.n_tris, R, lb_cur, lb_next, err, spin_limit);
+            if (some) {
+                const BatchScene& B = scenes[open_scene];
+                const uint2 cur = make_uint2(s_n[open_scene], __ldcg(it + B.it_off + iter).y);
+                const float4* cin = ((iter & 1) ? cb : ca) + 2 * static_cast<size_t>(B.tri_off);
+                float4* cout = ((iter & 1) ? ca : cb) + 2 * static_cast<size_t>(B.tri_off);
+                ploc_close(P, buf ^ 1, open, open_total, cur, iter, cin, cout, node_box + 2 * static_cast<size_t>(B.node_off),
+                           node_kids + B.tri_off, it + B.it_off, B.n_tris, R,
+                           lookback + static_cast<size_t>(iter & 1) * lb_cap + B.lb_off, err, spin_limit);
+            }
+            if (!more) break;
+            some = true;
+            open = tile;
+            open_scene = lo;
+            open_total = tile_total;
         }
         if (!grid_barrier(bar, bar_target, err, spin_limit)) return;
     }
