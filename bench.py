@@ -62,7 +62,7 @@ N_BOUNCE = 8 * 1024 * 1024   # --rays: smaller copies of the batch for profilers
 BOUNCE_SEED = 11
 REF_STRIDE = 64        # the reference arm traces rays k % 64, k % 64 + 64, ... in step k
 TRI_WATERTIGHT = 0x2   # crt.h flags, also understood by the oracle
-PROFILE = "trace_pool_kernel_bounce_config3.md"  # ncu summary of the headline's dominant kernel
+PROFILE = "trace_walk4_kernel_bounce.md"  # ncu summary of the headline's dominant kernel
 TRI_REFERENCE = 0x0
 W1, H1 = 1920, 1080    # the icosphere frame
 
@@ -331,9 +331,10 @@ def run_ours(args):
     identical = identical and same(out)
 
     # node fetches and triangle tests per ray
-    ctx.trace(bvh, d_rays, WT | crt.TRACE_STATS, out=out)
+    # counted on the nodes the persistent walk visits (the compressed 4-wide ones)
+    ctx.trace(bvh, d_rays, WT | crt.TRACE_STATS | crt.TRACE_COMPRESSED, out=out)
     f_plain, tt_plain = ctx.last_trace_stats()
-    ctx.trace(bvh, d_rays, LEARNED | crt.TRACE_STATS, out=out)
+    ctx.trace(bvh, d_rays, LEARNED | crt.TRACE_STATS | crt.TRACE_COMPRESSED, out=out)
     f_learned, tt_learned = ctx.last_trace_stats()
     # prediction quality: treelet hit rate on hitting rays
     cls = torch.empty((n,), dtype=torch.int16, device=dev)
@@ -343,7 +344,7 @@ def run_ours(args):
     hit = truth != 127
     hit_rate = float((pc[hit] == truth[hit]).mean()) if hit.any() else 0.0
 
-    # ---- the dominant kernel (trace_pool_kernel in the learned step), timed
+    # ---- the dominant kernel (trace_walk4_kernel in the learned step), timed
     # by the library's CUDA events on its stream around that launch
     k_ms = statistics.mean(k[1] for k in kern)
     order_ms = statistics.mean(k[0] for k in kern)
@@ -440,13 +441,13 @@ def run_ours(args):
                                 "trace kernel over the link), host-timed around the call"},
             "gpu_launches": 6 * args.steps,
             "gpu_launches_note": "per step: infer_kernel (which also writes the order keys and their digit histograms), "
-                                 "4 onesweep_kernel passes, trace_pool_kernel",
-            "roofline": {"kernel": "trace_pool_kernel (learned step: persistent warps over the rays in predicted "
+                                 "4 onesweep_kernel passes, trace_walk4_kernel",
+            "roofline": {"kernel": "trace_walk4_kernel (learned step: persistent warps over the rays in predicted "
                                    "order, closest hit, watertight)",
                          "bound": "hbm", "achieved": round(achieved, 1), "peak": peak, "unit": "GB/s",
                          "frac": round(achieved / peak, 4), "traffic": traffic, "peak_source": peak_kind,
                          "ms_per_launch": round(k_ms, 4), "alg_bytes_per_launch": int(alg_bytes),
-                         "alg_bytes_model": "64 B per node fetched + 48 B per triangle tested + 32 B ray + 16 B hit "
+                         "alg_bytes_model": "64 B per 4-wide node fetched + 48 B per triangle tested + 32 B ray + 16 B hit "
                                             "+ 4 B order index per ray (fetched bytes; most are L1/L2 hits)",
                          "l2_and_issue": {
                              "lts_throughput_pct": read_profile_value(PROFILE, "lts_throughput_pct"),

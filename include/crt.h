@@ -458,7 +458,7 @@ crt_status crt_bounce_rays(crt_ctx* ctx, const crt_bvh* bvh, const crt_ray* prim
  * order (scene s owns tri_counts[s] triangles and ray_counts[s] rays).  Every
  * stage runs as one launch over all scenes (per-scene scene boxes and Morton
  * codes, one radix sort with a final pass that regroups the scenes, all
- * scenes' PLOC iterations in one persistent launch, one trace launch), and
+ * scenes' large PLOC iterations, then their last ones, one trace launch), and
  * crt_batch_run can capture build + trace into a CUDA graph and replay it.
  * Each scene's node array equals crt_build on that scene alone.  Hits carry
  * scene-local triangle indices. */

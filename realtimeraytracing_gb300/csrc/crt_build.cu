@@ -1292,11 +1292,11 @@ __global__ void __launch_bounds__(256) layout_emit_kernel(const float4* __restri
     layout_emit(p, node_box, node_kids, pf, N, dfs, out, wide, wide_wt, depth_odd, lv, st->abs_eps, err);
 }
 
-// ================================== K3+K4 fused: one persistent launch
-// All PLOC iterations, then all layout levels, separated by a grid-wide
-// barrier (co-residency guaranteed by a cooperative launch; every wait is
-// bounded and a timeout ends every block).  Saves the per-iteration launch
-// and the host round trips the multi-launch path needs.
+// ============================ K3 and K4 in a few launches (the default)
+// PLOC iterations separated by a grid-wide barrier (co-residency guaranteed by a
+// cooperative launch; every wait is bounded and a timeout ends every block), the
+// last ones on a cluster, then the layout's two passes.  Saves the per-iteration
+// launch and the host round trips the multi-launch path needs.
 __device__ __forceinline__ bool grid_barrier(unsigned long long* bar, unsigned long long& target, uint32_t* err,
                                              uint32_t spin_limit) {
     // A 64-bit arrival counter that only grows (zeroed before the launch):
