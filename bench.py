@@ -453,8 +453,8 @@ def run_ours(args):
                              "lts_throughput_pct": read_profile_value(PROFILE, "lts_throughput_pct"),
                              "issue_active_pct": read_profile_value(PROFILE, "issue_active_pct"),
                              "threads_per_instruction": read_profile_value(PROFILE, "threads_per_instruction"),
-                             "source": "ncu full set of this kernel on a 1,048,576-ray copy of the workload "
-                                       "(profiles/" + PROFILE + "); the walk is latency-bound, DRAM traffic is "
+                             "source": "ncu sections of this kernel on 1,048,576 bounce rays over the same kind of scene "
+                                       "(profiles/" + PROFILE + "); bound by the ALU pipe and by L2 and HBM latency, DRAM traffic is "
                                        "the 'traffic' bytes"}},
             "rays_sha256": digest(rays_h),
             "reference_sample_hits_sha256": digest(ref_hits),
@@ -662,7 +662,7 @@ def run_frame_experiment(ctx, torch, crt, dev, stream, l2_flush, args):
         "frame_kernel": {"fetched_bytes_gbs": round(alg_bytes / (f_ms * 1e-3) / 1e9, 1),
                          "node_fetches_per_pixel": round(visited / n_rays, 2),
                          "tris_per_pixel": round(tested / n_rays, 2),
-                         "dram_bytes_per_launch": read_profile_value("frame_kernel_config1.md",
+                         "dram_bytes_per_launch": read_profile_value("frame_walk4_kernel_config1.md",
                                                                      "traffic_bytes_per_launch")},
         "primary_trace_node_formats": formats,
         "mesh_upload": mesh,
