@@ -316,6 +316,7 @@ crt_status crt_create(crt_ctx** out, const crt_config* cfg) {
     if (prop.major * 10 + prop.minor != 103)
         return fail(CRT_ERR_UNSUPPORTED, "libcrt is built for sm_103a; device is sm_%d%d", prop.major, prop.minor);
     CRT_CUDA(cudaSetDevice(c.device));
+    crt::build_prepare();
     crt_ctx* x = new crt_ctx();
     x->device = c.device;
     x->cfg = c;

@@ -457,6 +457,11 @@ void launch_batch_leaf_init(const crt_triangle* tris, uint32_t n_total, BatchSce
                                                                  leaf_of_tri, it, nodes, pf, err);
 }
 
+void build_prepare() {
+    ClusterLaunch::allow(reinterpret_cast<const void*>(ploc_cluster_kernel<kPlocMaxRadius>));
+    ClusterLaunch::allow(reinterpret_cast<const void*>(batch_cluster_kernel));
+}
+
 // Blocks of a scene's cluster: the most for which every scene's cluster is
 // resident at once (up to 16; 152 SMs hold 76 clusters of two, 8 of sixteen), so
 // that the scenes' chains of iterations run side by side.

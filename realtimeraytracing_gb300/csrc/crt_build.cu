@@ -2108,11 +2108,16 @@ struct ClusterLaunch {
         c.attrs = &a;
         c.numAttrs = 1;
     }
-    // Allows the kernel f clusters of kClusterBlocks; the clusters of `blocks`
-    // blocks that the device holds at once (0: it cannot run).
-    static int active(const void* f, int blocks) {
+    // Allows the kernel f clusters of kClusterBlocks on the current device (in the
+    // current CUDA context: build_prepare repeats it for every library context).
+    static void allow(const void* f) {
         cudaFuncSetAttribute(f, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
         cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(sizeof(ClusterSmem)));
+        cudaGetLastError();
+    }
+    // The clusters of `blocks` blocks that the device holds at once (0: it cannot run).
+    static int active(const void* f, int blocks) {
+        allow(f);
         ClusterLaunch l(blocks, 1, nullptr);
         int n = 0;
         if (cudaOccupancyMaxActiveClusters(&n, f, &l.c) != cudaSuccess) n = 0;

@@ -234,6 +234,8 @@ size_t ray_order_scratch_bytes(uint32_t n);
 void launch_ray_order(const crt_ray* rays, uint32_t n, const crt_bvh_node* nodes, const BatchScene* scenes,
                       uint32_t n_scenes, uint32_t* order, void* scratch, uint32_t* err, uint32_t spin_limit,
                       cudaStream_t s);
+// Kernel attributes of the builds' cluster kernels, set for the current device.
+void build_prepare();
 // Batched build stages (crt_batch_kernels.cuh).
 size_t batch_box_state_bytes();
 size_t batch_chunk_bytes();
