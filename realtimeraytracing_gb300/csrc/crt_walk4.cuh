@@ -216,9 +216,12 @@ __device__ __forceinline__ void walk4_sts(uint32_t a, uint2 e) {
 // One lane's walk.  cur: the internal node to visit next, or -1 (pop one); pend:
 // a parked leaf.  The stack's newest entries sit in shared memory (a column per
 // thread, so any mix of depths is free of bank conflicts), older ones move to
-// local memory eight at a time.  An entry is (reference, entry distance); its low
-// two distance bits count the siblings pushed just below it, which are farther,
-// so one too-far entry drops them all.
+// local memory eight at a time.  An entry is (reference, entry distance).
+// Closest hit: the low two distance bits count the siblings pushed just below it,
+// which are farther, so one too-far entry drops them all (the count can raise a
+// distance by 3 ulp, far inside the bound's slack of 2^-14).  Any hit: the
+// siblings below are nearer and the bound stays where it was when they were
+// pushed, so entries are taken without another look at their distance.
 struct Walk4Lane {
     static constexpr uint32_t kNoLeaf = 0xFFFFFFFFu;
     const uint4* cw;      // the scene: nodes, leaf triangles, slack
@@ -316,7 +319,7 @@ __device__ __forceinline__ uint32_t walk4_run(Walk4Lane& L, uint32_t s_base, uin
             }
             const uint2 e = walk4_lds(L.top - kRow);
             const bool some = L.top != s_base, full = L.pend != kNoLeaf;
-            const bool near = (ANY ? fabsf(__uint_as_float(e.y)) : __uint_as_float(e.y)) <= L.bound;
+            const bool near = ANY || __uint_as_float(e.y) <= L.bound;
             const bool leaf = static_cast<int>(e.x) < 0;
             blocked = full && (!some || (near && leaf));
             over = !some && !full;
@@ -340,7 +343,7 @@ __device__ __forceinline__ uint32_t walk4_run(Walk4Lane& L, uint32_t s_base, uin
         const uint32_t bm = __ballot_sync(0xFFFFFFFFu, blocked);
         if (__popc(bm) >= FLUSH || !wm) {
             if (L.pend != kNoLeaf) {
-                if ((ANY ? fabsf(L.pend_t) : L.pend_t) <= L.bound) {
+                if (ANY || L.pend_t <= L.bound) {
                     L.template test_leaf<WT>(L.pend);
                     if (COUNT) ++L.tested;
                 }
@@ -379,7 +382,7 @@ __device__ __forceinline__ uint32_t walk4_run(Walk4Lane& L, uint32_t s_base, uin
                 walk4_sts(L.top, make_uint2(n.ref[c], (__float_as_uint(t[c]) & ~3u) | below));
                 if (t[c] < inf) {
                     L.top += kRow;
-                    ++below;
+                    if (!ANY) ++below;
                 }
             }
             // the nearest child is entered; a leaf goes through the stack
