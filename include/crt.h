@@ -244,7 +244,9 @@ crt_status crt_optimize(crt_ctx* ctx, crt_bvh* bvh, uint32_t passes);
  * records in that order, each triangle in exactly one leaf; anything else is
  * CRT_ERR_INVALID_ARG.  Boxes are used as given and must contain their
  * triangles (AABB::buildFromTriangle, bvh.cpp:383-399, makes such boxes); the
- * watertight slack is derived from the root box. */
+ * watertight slack is derived from the root box.  Until a refit, a tree with a
+ * leaf box other than its triangle's, or a child box not inside its parent's,
+ * is traced over the binary nodes whatever the number of rays. */
 crt_status crt_bvh_from_nodes(crt_ctx* ctx, const crt_bvh_node* nodes, uint32_t n_nodes, const crt_triangle* tris,
                               uint32_t n_tris, const crt_mesh_model* models, uint32_t n_models, crt_bvh** out);
 /* The structure check of crt_bvh_from_nodes alone, on the host, without a

@@ -137,6 +137,10 @@ struct crt_bvh {
     mutable bool cwide_ready = false;  // the compressed 4-wide nodes, derived likewise
     uint32_t* cw_bad() const { return reinterpret_cast<uint32_t*>(cwide.as<char>() + 64ull * n); }
     mutable uint64_t frame_pixels = 0;  // pixels of the frames of the current tree
+    // Every leaf's box is its triangle's and lies inside its ancestors', as after a
+    // build or a refit; an imported array may hold others, which the walk over the
+    // compressed nodes does not look at: such a tree is walked on the binary nodes.
+    bool own_boxes = true;
     // Refit topology of the last build (crt_refit, derived on its first call).
     DevBuf refit_link, refit_leaf, refit_dfs, refit_cnt;
     bool refit_ready = false;
@@ -556,6 +560,7 @@ crt_status build_impl(crt_ctx* x, crt_bvh* b, const crt_triangle* tris, uint32_t
     b->frame_pixels = 0;
     b->refit_ready = false;
     b->node_boxes_stale = false;
+    b->own_boxes = true;
     CRT_TRY(b->cwide.reserve(64ull * N + 16));  // derived by the first trace that walks them, which then allocates nothing
     CRT_TRY(b->depth_odd.reserve(N));
     CRT_TRY(b->inv_perm.reserve(4ull * N));
@@ -787,7 +792,7 @@ crt_status finish_walk(crt_ctx* x) {
 // takes 0.035 ns per triangle (73 us at 2.0 M) and a pixel gains 0.05-0.2 ns.
 crt_status frame_walk4(crt_ctx* x, const crt_bvh* b, uint32_t pixels, crt::TraceParams* p) {
     b->frame_pixels += pixels;
-    if (b->n < 2 || (!b->cwide_ready && 4 * b->frame_pixels < b->n)) return CRT_OK;
+    if (b->n < 2 || !b->own_boxes || (!b->cwide_ready && 4 * b->frame_pixels < b->n)) return CRT_OK;
     CRT_TRY(ensure_cwide(x, b));
     p->cwide = b->cwide.as<uint4>();
     p->cw_bad = b->cw_bad();
@@ -824,10 +829,11 @@ crt_status trace_device(crt_ctx* x, const crt_bvh* b, const crt_ray* d_rays, uin
                         bool classes_ready = false, bool wait = false) {
     if (n_rays == 0) return CRT_OK;
     if (flags & CRT_TRACE_WIDE) CRT_TRY(ensure_wide4(x, b));
+    if (!b->own_boxes) flags &= ~CRT_TRACE_COMPRESSED;
     // Large batches over one scene: persistent warps over the compressed nodes;
     // pixels in 8x4 tiles, seeded, 4-wide and counting walks keep one thread per ray.
     const bool pool = !(flags & (CRT_TRACE_WIDE | CRT_TRACE_PER_RAY_THREADS | CRT_TRACE_USE_PREDICTOR | CRT_TRACE_STATS)) &&
-                      !seed_classes && tile_width == 0 && n_rays >= kPoolMinRays && b->n > 1;
+                      !seed_classes && tile_width == 0 && n_rays >= kPoolMinRays && b->n > 1 && b->own_boxes;
     if (pool || (flags & CRT_TRACE_COMPRESSED)) CRT_TRY(ensure_cwide(x, b));
     x->tev_valid = false;
     CRT_CUDA(cudaEventRecord(x->tev[0], x->stream));
@@ -996,6 +1002,7 @@ crt_status crt_refit(crt_ctx* x, crt_bvh* b, const crt_triangle* tris, uint32_t 
     b->cwide_ready = false;
     b->frame_pixels = 0;
     b->node_boxes_stale = N > 1;
+    b->own_boxes = true;
     const crt_status st = x->check_host_error();
     if (st != CRT_OK) {
         b->refit_ready = false;  // derive the topology again next time
@@ -1138,11 +1145,11 @@ crt_status crt_bvh_from_nodes(crt_ctx* x, const crt_bvh_node* nodes, uint32_t n_
         (st = b->wide.reserve(64ull * n_int_alloc)) != CRT_OK || (st = b->wide_wt.reserve(64ull * n_int_alloc)) != CRT_OK ||
         (st = b->cwide.reserve(64ull * N + 16)) != CRT_OK || (st = b->depth_odd.reserve(n_int_alloc)) != CRT_OK || (st = b->inv_perm.reserve(4ull * N)) != CRT_OK)
         return fail_free(st);
-    // staging: idx (n_nodes) | int_pos (N-1) | leaf counts (N-1, uint2) | leaf_pos (N), each part
+    // staging: idx (n_nodes) | int_pos (N-1) | leaf counts (N-1, uint2) | leaf_pos (N) | loose flag, each part
     // starting on a 256-byte boundary (the uint2 loads need 8-byte alignment)
     auto up256 = [](size_t v) { return (v + 255) & ~size_t(255); };
     const size_t o_int = up256(4ull * n_nodes), o_lc = up256(o_int + 4ull * n_int_alloc),
-                 o_leaf = up256(o_lc + 8ull * n_int_alloc), bytes = o_leaf + 4ull * N;
+                 o_leaf = up256(o_lc + 8ull * n_int_alloc), o_loose = up256(o_leaf + 4ull * N), bytes = o_loose + 4;
     if ((st = x->opt_scratch.reserve(bytes)) != CRT_OK) return fail_free(st);
     char* base = x->opt_scratch.as<char>();
     if ((st = stage_model_matrices(x, models, n_models)) != CRT_OK) return fail_free(st);
@@ -1171,12 +1178,17 @@ crt_status crt_bvh_from_nodes(crt_ctx* x, const crt_bvh_node* nodes, uint32_t n_
                        reinterpret_cast<const uint32_t*>(base + o_int), reinterpret_cast<const uint2*>(base + o_lc),
                        reinterpret_cast<const uint32_t*>(base + o_leaf), d_tris, x->models.as<float>(), grow,
                        b->wide.as<float4>(), b->wide_wt.as<float4>(), b->xtri.as<float4>(), b->inv_perm.as<uint32_t>(),
-                       x->err.as<uint32_t>(), s);
-    if (cudaGetLastError() != cudaSuccess) return fail_free(fail(CRT_ERR_CUDA, "crt_bvh_from_nodes: launch failed"));
+                       reinterpret_cast<uint32_t*>(base + o_loose), x->err.as<uint32_t>(), s);
+    // read back in page-locked memory, past the model matrices that may still be on their way
+    uint32_t* h_loose = static_cast<uint32_t*>(x->pinned) + 2 * 64 * 16;
+    if (cudaGetLastError() != cudaSuccess ||
+        cudaMemcpyAsync(h_loose, base + o_loose, 4, cudaMemcpyDeviceToHost, s) != cudaSuccess)
+        return fail_free(fail(CRT_ERR_CUDA, "crt_bvh_from_nodes: launch failed"));
     if ((st = x->check_device_error()) != CRT_OK) return fail_free(st);  // synchronises: the host arrays may go
     b->n = N;
     b->depth_bound = max_depth;
     b->abs_eps = grow;
+    b->own_boxes = *h_loose == 0u;
     b->has_sort = false;
     b->ctx = x;
     *out = b;

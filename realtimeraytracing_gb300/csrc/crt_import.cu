@@ -13,6 +13,11 @@
 //   import_leaves  one thread per leaf (left-to-right order): its triangle
 //                  transformed by its model matrix (glm mat4 * vec4 order, as
 //                  the build's leaf pass) and the triangle -> leaf map.
+// Both set *loose where the array's boxes are not those a build would give it:
+// a leaf's box other than its triangle's, or a child's not inside its parent's.
+// Such a tree's hits are decided by its own boxes, which only the binary walk
+// tests one by one (crt_walk4.cuh re-makes leaf boxes from the triangles and
+// skips the boxes of opened nodes).
 // Compiled with -fmad=false.
 #include <cstdint>
 #include <cuda_runtime.h>
@@ -32,24 +37,30 @@ __global__ void __launch_bounds__(256) import_wide_kernel(const crt_bvh_node* __
                                                           const uint32_t* __restrict__ int_pos,
                                                           const uint2* __restrict__ leaf_counts, uint32_t N, float grow,
                                                           float4* __restrict__ wide, float4* __restrict__ wide_wt,
-                                                          uint32_t* err) {
+                                                          uint32_t* __restrict__ loose, uint32_t* err) {
     const uint32_t k = blockIdx.x * 256 + threadIdx.x;
     if (k + 1 >= N) return;
     const uint32_t d = __ldg(int_pos + k);
     if (d + 1 >= n_nodes) { raise_corrupt(err, 30, k, d); return; }
     const uint4 kd = __ldg(reinterpret_cast<const uint4*>(nodes + d) + 2);
     const uint32_t ch[2] = {kd.y, kd.z};
+    const float4 pmn = __ldg(reinterpret_cast<const float4*>(nodes + d));
+    const float4 pmx = __ldg(reinterpret_cast<const float4*>(nodes + d) + 1);
     float4 cmn[2], cmx[2];
     uint32_t ref[2];
+    bool inside = true;  // a NaN is not inside
 #pragma unroll
     for (int c = 0; c < 2; ++c) {
         if (ch[c] >= n_nodes) { raise_corrupt(err, 30, k, ch[c]); return; }
         const float4* q = reinterpret_cast<const float4*>(nodes + ch[c]);
         cmn[c] = __ldg(q);
         cmx[c] = __ldg(q + 1);
+        inside = inside && pmn.x <= cmn[c].x && pmn.y <= cmn[c].y && pmn.z <= cmn[c].z && cmx[c].x <= pmx.x &&
+                 cmx[c].y <= pmx.y && cmx[c].z <= pmx.z;
         const uint32_t i = __ldg(idx + ch[c]);
         ref[c] = import_is_leaf(nodes, ch[c]) ? (kLeafRef | i) : i;
     }
+    if (!inside) atomicOr(loose, 1u);
     const uint2 lc = __ldg(leaf_counts + k);
     float4* w = wide + 4 * static_cast<size_t>(k);
     w[0] = make_float4(cmn[0].x, cmn[0].y, cmn[0].z, __uint_as_float(ref[0]));
@@ -68,7 +79,7 @@ __global__ void __launch_bounds__(256) import_leaves_kernel(const crt_bvh_node* 
                                                             const crt_triangle* __restrict__ tris,
                                                             const float* __restrict__ models, uint32_t N,
                                                             float4* __restrict__ xtri, uint32_t* __restrict__ leaf_of_tri,
-                                                            uint32_t* err) {
+                                                            uint32_t* __restrict__ loose, uint32_t* err) {
     const uint32_t l = blockIdx.x * 256 + threadIdx.x;
     if (l >= N) return;
     const uint32_t d = __ldg(leaf_pos + l);
@@ -83,18 +94,25 @@ __global__ void __launch_bounds__(256) import_leaves_kernel(const crt_bvh_node* 
     xtri[3 * static_cast<size_t>(l) + 1] = make_float4(p1.x, p1.y, p1.z, __uint_as_float(t.model));
     xtri[3 * static_cast<size_t>(l) + 2] = make_float4(p2.x, p2.y, p2.z, 0.f);
     leaf_of_tri[ti] = l;
+    const float4 mn = __ldg(reinterpret_cast<const float4*>(nodes + d));
+    const float4 mx = __ldg(reinterpret_cast<const float4*>(nodes + d) + 1);
+    const bool own = mn.x == min_std(p0.x, min_std(p1.x, p2.x)) && mn.y == min_std(p0.y, min_std(p1.y, p2.y)) &&
+                     mn.z == min_std(p0.z, min_std(p1.z, p2.z)) && mx.x == max_std(p0.x, max_std(p1.x, p2.x)) &&
+                     mx.y == max_std(p0.y, max_std(p1.y, p2.y)) && mx.z == max_std(p0.z, max_std(p1.z, p2.z));
+    if (!own) atomicOr(loose, 1u);
 }
 
 void launch_import(const crt_bvh_node* nodes, uint32_t N, const uint32_t* idx, const uint32_t* int_pos,
                    const uint2* leaf_counts, const uint32_t* leaf_pos, const crt_triangle* tris, const float* models,
-                   float grow, float4* wide, float4* wide_wt, float4* xtri, uint32_t* leaf_of_tri, uint32_t* err,
-                   cudaStream_t s) {
+                   float grow, float4* wide, float4* wide_wt, float4* xtri, uint32_t* leaf_of_tri,
+                   uint32_t* loose, uint32_t* err, cudaStream_t s) {
     const uint32_t n_nodes = 2 * N - 1;
+    cudaMemsetAsync(loose, 0, 4, s);
     if (N > 1)
         import_wide_kernel<<<(N - 1 + 255) / 256, 256, 0, s>>>(nodes, n_nodes, idx, int_pos, leaf_counts, N, grow, wide,
-                                                               wide_wt, err);
+                                                               wide_wt, loose, err);
     import_leaves_kernel<<<(N + 255) / 256, 256, 0, s>>>(nodes, n_nodes, leaf_pos, tris, models, N, xtri, leaf_of_tri,
-                                                         err);
+                                                         loose, err);
 }
 
 }  // namespace crt
