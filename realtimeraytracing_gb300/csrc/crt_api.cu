@@ -3,6 +3,7 @@
 // trace entry points.  No compute happens on the host: a call that cannot
 // run its kernels returns an error instead of falling back.
 #include <algorithm>
+#include <atomic>
 #include <cmath>
 #include <cstdarg>
 #include <cstdio>
@@ -14,6 +15,7 @@
 #include "crt.h"
 #include "crt_build.cuh"
 #include "crt_common.cuh"
+#include "crt_host.h"
 
 namespace {
 
@@ -132,11 +134,16 @@ struct crt_bvh {
     crt_predictor* predictor = nullptr;
     // The 4-wide traversal nodes are derived on the first CRT_TRACE_WIDE
     // trace after a build, so builds whose trees are never walked 4-wide
-    // neither compute nor store them.
-    mutable bool wide4_ready = false;
-    mutable bool cwide_ready = false;  // the compressed 4-wide nodes, derived likewise
+    // neither compute nor store them.  So are the compressed 4-wide nodes, and
+    // after a refit the node array's boxes below the root, when the array is
+    // read.  Traces of a const tree may run from several contexts at once.
+    struct Derivation {
+        crt::Derived state;
+        cudaEvent_t done = nullptr;  // after the derivation, on the stream it was enqueued on
+    };
+    mutable Derivation wide4_nodes, cwide_nodes, node_boxes;
     uint32_t* cw_bad() const { return reinterpret_cast<uint32_t*>(cwide.as<char>() + 64ull * n); }
-    mutable uint64_t frame_pixels = 0;  // pixels of the frames of the current tree
+    mutable std::atomic<uint64_t> frame_pixels{0};  // pixels of the frames of the current tree
     // Every leaf's box is its triangle's and lies inside its ancestors', as after a
     // build or a refit; an imported array may hold others, which the walk over the
     // compressed nodes does not look at: such a tree is walked on the binary nodes.
@@ -144,9 +151,17 @@ struct crt_bvh {
     // Refit topology of the last build (crt_refit, derived on its first call).
     DevBuf refit_link, refit_leaf, refit_dfs, refit_cnt;
     bool refit_ready = false;
-    // After a refit only the root box of the node array is current; the
-    // others are derived from the traversal nodes when the array is read.
-    mutable bool node_boxes_stale = false;
+    // Since a refit only the root box of the node array is kept current; the
+    // others are derived from the traversal nodes (node_boxes).
+    bool refitted = false;
+    // The tree has changed: what was derived from it no longer holds.
+    void changed(bool by_refit) {
+        wide4_nodes.state.reset();
+        cwide_nodes.state.reset();
+        node_boxes.state.reset();
+        frame_pixels = 0;
+        refitted = by_refit;
+    }
     // Sorted Morton codes and permutation exist (a tree from crt_bvh_from_nodes has none).
     bool has_sort = false;
 };
@@ -188,6 +203,8 @@ struct crt_predictor {
 };
 
 struct crt_ctx {
+    static std::atomic<uint64_t> made;
+    const uint64_t id = ++made;  // never that of another context, past or present
     int device = 0;
     cudaStream_t stream = nullptr;
     crt_config cfg{};
@@ -278,6 +295,7 @@ struct crt_ctx {
         return CRT_OK;
     }
 };
+std::atomic<uint64_t> crt_ctx::made{0};
 
 extern "C" {
 
@@ -555,11 +573,8 @@ crt_status build_impl(crt_ctx* x, crt_bvh* b, const crt_triangle* tris, uint32_t
     CRT_TRY(x->xtri_sorted.reserve(48ull * N));
     CRT_TRY(b->wide.reserve(64ull * N));
     CRT_TRY(b->wide_wt.reserve(64ull * N));
-    b->wide4_ready = false;
-    b->cwide_ready = false;
-    b->frame_pixels = 0;
+    b->changed(false);
     b->refit_ready = false;
-    b->node_boxes_stale = false;
     b->own_boxes = true;
     CRT_TRY(b->cwide.reserve(64ull * N + 16));  // derived by the first trace that walks them, which then allocates nothing
     CRT_TRY(b->depth_odd.reserve(N));
@@ -740,26 +755,44 @@ crt_status check_trace_flags(const crt_bvh* b, uint32_t flags) {
     return CRT_OK;
 }
 
-// Derives the 4-wide traversal nodes of b on x's stream if the last build
-// has not yet done so.
-crt_status ensure_wide4(crt_ctx* x, const crt_bvh* b) {
-    if (b->wide4_ready || b->n <= 1) return CRT_OK;
-    CRT_TRY(b->wide4.reserve(128ull * b->n));
-    crt::launch_wide4(b->wide.as<float4>(), b->depth_odd.as<uint8_t>(), b->n - 1, b->wide4.as<float4>(), x->stream);
-    CRT_CUDA(cudaGetLastError());
-    b->wide4_ready = true;
-    return CRT_OK;
+// Makes what launch() derives from a tree usable on x's stream: enqueued by the
+// first context that needs it, waited for by the others.
+template <class Launch>
+crt_status use_derived(crt_ctx* x, crt_bvh::Derivation& d, Launch launch) {
+    return d.state.use(
+        x->id,
+        [&]() -> crt_status {
+            if (!d.done) CRT_CUDA(cudaEventCreateWithFlags(&d.done, cudaEventDisableTiming));
+            CRT_TRY(launch());
+            CRT_CUDA(cudaGetLastError());
+            CRT_CUDA(cudaEventRecord(d.done, x->stream));
+            return CRT_OK;
+        },
+        [&]() -> crt_status {
+            CRT_CUDA(cudaStreamWaitEvent(x->stream, d.done, 0));
+            return CRT_OK;
+        });
 }
 
-// Derives the compressed 4-wide traversal nodes of b on x's stream if the
-// last build (or refit) has not yet done so; their bad flag follows them.
+// The 4-wide traversal nodes of b's current tree, usable on x's stream.
+crt_status ensure_wide4(crt_ctx* x, const crt_bvh* b) {
+    if (b->n <= 1) return CRT_OK;
+    return use_derived(x, b->wide4_nodes, [&]() -> crt_status {
+        CRT_TRY(b->wide4.reserve(128ull * b->n));
+        crt::launch_wide4(b->wide.as<float4>(), b->depth_odd.as<uint8_t>(), b->n - 1, b->wide4.as<float4>(), x->stream);
+        return CRT_OK;
+    });
+}
+
+// The compressed 4-wide traversal nodes of b's current tree, usable on x's
+// stream; their bad flag follows them.
 crt_status ensure_cwide(crt_ctx* x, const crt_bvh* b) {
-    if (b->cwide_ready || b->n <= 1) return CRT_OK;
-    CRT_TRY(b->cwide.reserve(64ull * b->n + 16));
-    crt::launch_cwide(b->wide.as<float4>(), b->n - 1, b->abs_eps, b->cwide.as<uint4>(), b->cw_bad(), x->stream);
-    CRT_CUDA(cudaGetLastError());
-    b->cwide_ready = true;
-    return CRT_OK;
+    if (b->n <= 1) return CRT_OK;
+    return use_derived(x, b->cwide_nodes, [&]() -> crt_status {
+        CRT_TRY(b->cwide.reserve(64ull * b->n + 16));
+        crt::launch_cwide(b->wide.as<float4>(), b->n - 1, b->abs_eps, b->cwide.as<uint4>(), b->cw_bad(), x->stream);
+        return CRT_OK;
+    });
 }
 
 // Scratch of a persistent walk of n rays: the list of left-over rays lies in
@@ -791,8 +824,8 @@ crt_status finish_walk(crt_ctx* x) {
 // tree have a quarter as many pixels as it has triangles: deriving the nodes
 // takes 0.035 ns per triangle (73 us at 2.0 M) and a pixel gains 0.05-0.2 ns.
 crt_status frame_walk4(crt_ctx* x, const crt_bvh* b, uint32_t pixels, crt::TraceParams* p) {
-    b->frame_pixels += pixels;
-    if (b->n < 2 || !b->own_boxes || (!b->cwide_ready && 4 * b->frame_pixels < b->n)) return CRT_OK;
+    const uint64_t frames = b->frame_pixels += pixels;
+    if (b->n < 2 || !b->own_boxes || (!b->cwide_nodes.state.ready() && 4 * frames < b->n)) return CRT_OK;
     CRT_TRY(ensure_cwide(x, b));
     p->cwide = b->cwide.as<uint4>();
     p->cw_bad = b->cw_bad();
@@ -946,13 +979,13 @@ crt_status crt_rebuild(crt_ctx* x, crt_bvh* b, const crt_triangle* tris, uint32_
 
 // Brings the node array's boxes up to date after a refit (on x's stream).
 static crt_status ensure_node_boxes(crt_ctx* x, const crt_bvh* b) {
-    if (!b->node_boxes_stale) return CRT_OK;
-    x->err_dirty = true;
-    crt::launch_refit_nodes(b->wide.as<float4>(), b->refit_dfs.as<uint32_t>(), b->n,
-                            const_cast<crt_bvh_node*>(b->nodes.as<crt_bvh_node>()), x->err.as<uint32_t>(), x->stream);
-    CRT_CUDA(cudaGetLastError());
-    b->node_boxes_stale = false;
-    return CRT_OK;
+    if (!b->refitted) return CRT_OK;
+    return use_derived(x, b->node_boxes, [&]() -> crt_status {
+        x->err_dirty = true;
+        crt::launch_refit_nodes(b->wide.as<float4>(), b->refit_dfs.as<uint32_t>(), b->n,
+                                const_cast<crt_bvh_node*>(b->nodes.as<crt_bvh_node>()), x->err.as<uint32_t>(), x->stream);
+        return CRT_OK;
+    });
 }
 
 crt_status crt_refit(crt_ctx* x, crt_bvh* b, const crt_triangle* tris, uint32_t n_tris, const crt_mesh_model* models,
@@ -998,10 +1031,7 @@ crt_status crt_refit(crt_ctx* x, crt_bvh* b, const crt_triangle* tris, uint32_t 
     float* h_eps = static_cast<float*>(x->pinned);
     CRT_CUDA(cudaMemcpyAsync(h_eps, &x->refit_state.as<crt::RefitState>()->abs_eps, sizeof(float),
                              cudaMemcpyDeviceToHost, s));
-    b->wide4_ready = false;
-    b->cwide_ready = false;
-    b->frame_pixels = 0;
-    b->node_boxes_stale = N > 1;
+    b->changed(N > 1);
     b->own_boxes = true;
     const crt_status st = x->check_host_error();
     if (st != CRT_OK) {
@@ -1267,11 +1297,8 @@ crt_status crt_optimize(crt_ctx* x, crt_bvh* b, uint32_t passes) {
     crt::launch_layout_emit(box2, kids2, pf, N, dfs, b->nodes.as<crt_bvh_node>(), b->wide.as<float4>(),
                             b->wide_wt.as<float4>(), b->depth_odd.as<uint8_t>(), leaves, st, err, s);
     CRT_CUDA(cudaGetLastError());
-    b->wide4_ready = false;
-    b->cwide_ready = false;
-    b->frame_pixels = 0;
+    b->changed(false);
     b->refit_ready = false;
-    b->node_boxes_stale = false;
     b->depth_bound = H;
     return x->check_device_error();  // also keeps the host staging alive until the copies ran
 }
@@ -1293,6 +1320,8 @@ crt_status crt_bvh_free(crt_bvh* b) {
     b->refit_leaf.release();
     b->refit_dfs.release();
     b->refit_cnt.release();
+    for (crt_bvh::Derivation* d : {&b->wide4_nodes, &b->cwide_nodes, &b->node_boxes})
+        if (d->done) cudaEventDestroy(d->done);
     delete b;
     return CRT_OK;
 }

@@ -1,0 +1,49 @@
+// Host-side rules of libcrt that need neither CUDA nor a GPU, apart so that a
+// plain C++ program can check them.
+#pragma once
+
+#include <cstdint>
+#include <mutex>
+
+namespace crt {
+
+// Something derived from a tree by the first context that needs it and read by
+// every later one.  A tree may be traced from several contexts at once (a host
+// thread and a stream each): the derivation is enqueued once, on the stream of the
+// context that came first, and every other context's stream waits for it before
+// that context reads the result.  A reader never sees a result whose derivation is
+// not yet enqueued, and never runs before it.
+class Derived {
+public:
+    // who: the calling context.  derive() enqueues the derivation and a mark after
+    // it on that context's stream; wait() makes that stream wait for the mark.
+    // Returns what they return: 0, or an error, after which a failed derivation is
+    // left to the next caller.
+    template <class Derive, class Wait>
+    auto use(uint64_t who, Derive derive, Wait wait) -> decltype(derive()) {
+        std::lock_guard<std::mutex> hold(mutex_);
+        if (ready_) return by_ == who ? decltype(derive()){} : wait();
+        const auto status = derive();
+        if (status == decltype(derive()){}) {
+            ready_ = true;
+            by_ = who;
+        }
+        return status;
+    }
+    // The source has changed.  Like the change itself, not beside other uses.
+    void reset() {
+        std::lock_guard<std::mutex> hold(mutex_);
+        ready_ = false;
+    }
+    bool ready() const {
+        std::lock_guard<std::mutex> hold(mutex_);
+        return ready_;
+    }
+
+private:
+    mutable std::mutex mutex_;
+    bool ready_ = false;
+    uint64_t by_ = 0;  // whose stream the derivation is on
+};
+
+}  // namespace crt

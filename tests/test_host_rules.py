@@ -1,0 +1,74 @@
+"""Host-side rules of the library (csrc/crt_host.h), compiled as plain C++ and
+checked without a GPU."""
+import os
+import shutil
+import subprocess
+
+import pytest
+
+ROOT = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
+
+
+def run_cpp(tmp_path, body):
+    gxx = shutil.which("g++")
+    if gxx is None:
+        pytest.skip("no g++")
+    src, exe = tmp_path / "rule.cpp", tmp_path / "rule"
+    src.write_text('''#include "crt_host.h"
+#include <atomic>
+#include <chrono>
+#include <cstdio>
+#include <thread>
+#include <vector>
+#define CHECK(c) do { if (!(c)) { std::printf("line %d: %s\\n", __LINE__, #c); return 1; } } while (0)
+''' + body)
+    subprocess.run([gxx, "-std=c++17", "-O1", "-pthread", "-Wall", "-Werror", "-I",
+                    os.path.join(ROOT, "realtimeraytracing_gb300", "csrc"), str(src), "-o", str(exe)], check=True)
+    r = subprocess.run([str(exe)], capture_output=True, text=True, timeout=60)
+    assert r.returncode == 0, r.stdout
+
+
+def test_derived_data_is_enqueued_once_and_waited_for(tmp_path):
+    """Contexts on threads of their own: one derives, every other one waits for a derivation that is already
+    enqueued, the deriving one does neither again; a failed derivation is left to the next; a reset starts over."""
+    run_cpp(tmp_path, r'''
+enum Status { kOk = 0, kFailed = 3 };
+int main() {
+    for (int round = 0; round < 50; ++round) {
+        crt::Derived d;
+        std::atomic<int> derived{0}, waited{0}, early{0};
+        std::atomic<bool> enqueued{false};
+        std::vector<std::thread> t;
+        for (uint64_t who = 1; who <= 8; ++who)
+            t.emplace_back([&, who] {
+                for (int k = 0; k < 3; ++k) {
+                    bool did = false, saw = false;
+                    const Status s = d.use(who,
+                        [&] { ++derived; did = true; std::this_thread::sleep_for(std::chrono::microseconds(200));
+                              enqueued = true; return kOk; },
+                        [&] { ++waited; saw = true; if (!enqueued) ++early; return kOk; });
+                    if (s != kOk || !enqueued || (did && saw)) ++early;
+                }
+            });
+        for (auto& x : t) x.join();
+        CHECK(derived == 1);
+        CHECK(waited == 3 * 7);
+        CHECK(early == 0);
+        CHECK(d.ready());
+    }
+    crt::Derived d;
+    int derived = 0, waited = 0;
+    auto ok = [&] { ++derived; return kOk; };
+    auto bad = [&] { ++derived; return kFailed; };
+    auto wait = [&] { ++waited; return kFailed; };
+    CHECK(d.use(1, bad, wait) == kFailed && derived == 1 && !d.ready());
+    CHECK(d.use(2, ok, wait) == kOk && derived == 2 && d.ready());
+    CHECK(d.use(2, ok, wait) == kOk && derived == 2 && waited == 0);
+    CHECK(d.use(1, ok, wait) == kFailed && derived == 2 && waited == 1);  // the wait's own error
+    d.reset();
+    CHECK(!d.ready());
+    CHECK(d.use(1, ok, wait) == kOk && derived == 3 && waited == 1);
+    CHECK(d.use(2, ok, wait) == kFailed && waited == 2);
+    return 0;
+}
+''')
