@@ -633,19 +633,20 @@ crt_status build_impl(crt_ctx* x, crt_bvh* b, const crt_triangle* tris, uint32_t
     if (N > 1 && !x->force_multi_launch) {
         unsigned long long* lb = x->ploc_lb.as<unsigned long long>();
         uint32_t* tail = reinterpret_cast<uint32_t*>(lb + 2ull * ploc_tiles);
+        bool enqueued = false;
         const cudaError_t e = crt::launch_ploc_layout(
             x->clus_a.as<float4>(), x->clus_b.as<float4>(), x->node_box.as<float4>(), x->node_kids.as<uint4>(), d_it, N,
             static_cast<int>(x->cfg.ploc_radius), lb, tail, ploc_tiles, x->pos.as<uint2>(), b->nodes.as<crt_bvh_node>(),
             b->wide.as<float4>(), b->wide_wt.as<float4>(), b->depth_odd.as<uint8_t>(), leaves, st,
             reinterpret_cast<unsigned long long*>(tail + 2), tail + 4,
-            err, x->cfg.spin_limit, x->ev[3], s);
+            err, x->cfg.spin_limit, x->ev[3], &enqueued, s);
         if (e == cudaSuccess) {
             CRT_CUDA(cudaMemcpyAsync(h_tail, tail + 4, 4, cudaMemcpyDeviceToHost, s));
             laid_out = true;  // its iteration count is read at the end
-        } else if (e != cudaErrorNotSupported && e != cudaErrorCooperativeLaunchTooLarge) {
-            return fail(CRT_ERR_CUDA, "PLOC launch failed: %s", cudaGetErrorString(e));
         } else {
             cudaGetLastError();
+            if (!crt::may_start_over(e == cudaErrorNotSupported || e == cudaErrorCooperativeLaunchTooLarge, enqueued))
+                return fail(CRT_ERR_CUDA, "PLOC launch failed: %s", cudaGetErrorString(e));
         }
     }
     if (N > 1 && !laid_out) {

@@ -466,13 +466,19 @@ void build_prepare() {
 // resident at once (up to 16; 152 SMs hold 76 clusters of two, 8 of sixteen), so
 // that the scenes' chains of iterations run side by side.
 static int batch_cluster_blocks(uint32_t n_scenes) {
-    static int active[5] = {-1, -1, -1, -1, -1};  // clusters of 1 << i blocks the device holds
-    for (int i = 4; i >= 0; --i) {
-        if (active[i] < 0) active[i] = ClusterLaunch::active(reinterpret_cast<const void*>(batch_cluster_kernel), 1 << i);
+    const std::array<int, 5> active = per_device<std::array<int, 5>>([] {  // clusters of 1 << i blocks the device holds
+        std::array<int, 5> a{};
+        for (int i = 0; i < 5; ++i) a[i] = ClusterLaunch::active(reinterpret_cast<const void*>(batch_cluster_kernel), 1 << i);
+        return a;
+    });
+    for (int i = 4; i >= 0; --i)
         if (active[i] > 0 && (static_cast<uint32_t>(active[i]) >= n_scenes || i == 0)) return 1 << i;
-    }
     return 0;
 }
+
+struct BatchGrids {
+    int ploc = 0, places = 0;
+};
 
 cudaError_t launch_batch_ploc(BatchScene* scenes, uint32_t n_scenes, uint32_t n_total, uint32_t max_n, float4* ca,
                               float4* cb, float4* node_box, uint4* node_kids, uint2* it, int radius,
@@ -480,9 +486,13 @@ cudaError_t launch_batch_ploc(BatchScene* scenes, uint32_t n_scenes, uint32_t n_
                               crt_bvh_node* nodes, float4* wide, float4* wide_wt, uint8_t* depth_odd, LeafOut lv,
                               unsigned long long* bar, uint32_t* err, uint32_t spin_limit, cudaStream_t s) {
     const void* ploc_fn = reinterpret_cast<const void*>(batch_ploc_kernel<kPlocSpan, 256, kPlocMaxRadius>);
-    static const int grid = cooperative_grid(ploc_fn, kPlocBlocksPerSm);
-    const int blocks = batch_cluster_blocks(n_scenes);
-    if (grid <= 0 || blocks <= 0) return cudaErrorNotSupported;
+    const void* places_fn = reinterpret_cast<const void*>(batch_places_kernel<256>);
+    const BatchGrids grids = per_device<BatchGrids>([&] {
+        return BatchGrids{cooperative_grid(ploc_fn, kPlocBlocksPerSm), cooperative_grid(places_fn, kAnyPerSm)};
+    });
+    const int grid = grids.ploc, blocks = batch_cluster_blocks(n_scenes);
+    // a scene's places are laid out by whole blocks: at most inner / share + n_scenes of them, all resident
+    if (grid <= 0 || blocks <= 0 || grids.places <= static_cast<int>(n_scenes)) return cudaErrorNotSupported;
     cudaError_t e = cudaSuccess;
     uint32_t stop_n = static_cast<uint32_t>(blocks * (kClusterTile - 2 * radius)), max_iters = max_n + 1;
     if (max_n > stop_n) {
@@ -497,23 +507,14 @@ cudaError_t launch_batch_ploc(BatchScene* scenes, uint32_t n_scenes, uint32_t n_
     e = cudaLaunchKernelEx(&l.c, batch_cluster_kernel, scenes, static_cast<const float4*>(ca), static_cast<const float4*>(cb),
                            node_box, node_kids, it, radius, err);
     if (e != cudaSuccess) return e;
-    static int place_grid = 0;
-    if (place_grid == 0) {
-        int per_sm = 0;
-        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, batch_places_kernel<256>, 256, 0);
-        place_grid = kNumSms * (per_sm > 0 ? per_sm : 1);
-    }
-    // whole blocks a scene: at most inner / share + n_scenes of them, all resident
-    if (place_grid <= static_cast<int>(n_scenes)) return cudaErrorNotSupported;
-    const uint32_t spread = static_cast<uint32_t>(place_grid) - n_scenes;
+    const uint32_t spread = static_cast<uint32_t>(grids.places) - n_scenes;
     uint32_t share = (inner + spread - 1) / spread;
     share = share > 256 ? share : 256;
     uint32_t* dfs = reinterpret_cast<uint32_t*>(ca);  // node ids by DFS position: the clusters are done with
     const BatchScene* cs = scenes;
     const uint4* ck = node_kids;
     void* args[] = {&cs, &n_scenes, &share, &dfs, &ck, &pf, &err, &spin_limit};
-    e = cudaLaunchCooperativeKernel(reinterpret_cast<const void*>(batch_places_kernel<256>),
-                                    dim3(inner / share + n_scenes), dim3(256), args, 0, s);
+    e = cudaLaunchCooperativeKernel(places_fn, dim3(inner / share + n_scenes), dim3(256), args, 0, s);
     if (e != cudaSuccess) return e;
     const uint32_t slots = n_total + inner;
     batch_emit_kernel<<<(slots + 255) / 256, 256, 0, s>>>(cs, n_scenes, slots, node_box, node_kids, pf, dfs, nodes, wide,

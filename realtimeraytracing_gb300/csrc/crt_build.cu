@@ -4,12 +4,16 @@
 // Reference: srcCommon/scene/geometry/bvh.cpp (CPU, OpenMP) and the DFS
 // flattening in srcOpenGL/scene/scene.cpp:189-208.  Every float result is
 // bit-identical to the reference's (this file is compiled with -fmad=false).
+#include <array>
 #include <cooperative_groups.h>
 #include <cstdint>
 #include <cuda_runtime.h>
+#include <map>
+#include <mutex>
 
 #include "crt_build.cuh"
 #include "crt_common.cuh"
+#include "crt_host.h"
 
 namespace crt {
 
@@ -2082,15 +2086,30 @@ void launch_layout_emit(const float4* node_box, const uint4* node_kids, const ui
                                                          lv, st, err);
 }
 
-// Blocks of a cooperative 256-thread launch of f, at most per_sm_max an SM (0: none).
+// Blocks of a cooperative 256-thread launch of f on the current device, at most
+// per_sm_max an SM (0: none).
 static int cooperative_grid(const void* f, int per_sm_max) {
-    int per_sm = 0, dev = 0, sms = kNumSms, coop = 0;
+    int per_sm = 0, dev = 0, sms = 0, coop = 0;
     cudaGetDevice(&dev);
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
     cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, dev);
     if (!coop || cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, f, 256, 0) != cudaSuccess) per_sm = 0;
     cudaGetLastError();
-    return (per_sm < per_sm_max ? per_sm : per_sm_max) * sms;
+    return resident_blocks(coop != 0, per_sm, per_sm_max, sms);
+}
+constexpr int kAnyPerSm = 1 << 10;
+
+// make()'s result for the current device, made once for each.
+template <class Value, class Make>
+static Value per_device(Make make) {
+    static std::mutex mutex;
+    static std::map<int, Value> made;
+    int dev = 0;
+    cudaGetDevice(&dev);
+    std::lock_guard<std::mutex> hold(mutex);
+    auto at = made.find(dev);
+    if (at == made.end()) at = made.emplace(dev, make()).first;
+    return at->second;
 }
 
 // Launch of a PLOC cluster kernel: `clusters` clusters of `blocks` blocks.
@@ -2126,60 +2145,60 @@ struct ClusterLaunch {
     }
 };
 
-// Blocks of the cluster kernel's cluster on this device (0: it cannot run).
-static int ploc_cluster_blocks() {
-    static int blocks = -1;
-    if (blocks < 0) {
-        int found = 0;
-        for (int b = kClusterBlocks; b >= 8 && found == 0; b /= 2)
-            if (ClusterLaunch::active(reinterpret_cast<const void*>(ploc_cluster_kernel<kPlocMaxRadius>), b) > 0) found = b;
-        blocks = found;
-    }
-    return blocks;
+static const void* const kWideFn = reinterpret_cast<const void*>(ploc_wide_kernel<kPlocSpan, 256, kPlocMaxRadius>);
+static const void* const kWaveFn = reinterpret_cast<const void*>(ploc_persistent_kernel<kPlocSpan, 256, kPlocMaxRadius>);
+static const void* const kPlacesFn = reinterpret_cast<const void*>(layout_places_kernel<256>);
+
+// The grids of launch_ploc_layout on the current device.
+static PlocGrids ploc_grids() {
+    return per_device<PlocGrids>([] {
+        PlocGrids g;
+        g.wide = cooperative_grid(kWideFn, kPlocBlocksPerSm);
+        g.wave = cooperative_grid(kWaveFn, kPlocOneWaveBlocksPerSm);
+        g.places = cooperative_grid(kPlacesFn, kAnyPerSm);
+        for (int b = kClusterBlocks; b >= 8 && g.cluster == 0; b /= 2)
+            if (ClusterLaunch::active(reinterpret_cast<const void*>(ploc_cluster_kernel<kPlocMaxRadius>), b) > 0) g.cluster = b;
+        return g;
+    });
 }
 
 cudaError_t launch_ploc_layout(float4* ca, float4* cb, float4* node_box, uint4* node_kids, uint2* it, uint32_t N,
                                int radius, unsigned long long* lookback, uint32_t* tickets, uint32_t n_tiles_cap,
                                uint2* pf, crt_bvh_node* out, float4* wide, float4* wide_wt, uint8_t* depth_odd,
                                LeafOut lv, const SceneState* st, unsigned long long* bar, uint32_t* iters_out,
-                               uint32_t* err, uint32_t spin_limit, cudaEvent_t ploc_done, cudaStream_t s) {
-    const void* wide_fn = reinterpret_cast<const void*>(ploc_wide_kernel<kPlocSpan, 256, kPlocMaxRadius>);
-    const void* wave_fn = reinterpret_cast<const void*>(ploc_persistent_kernel<kPlocSpan, 256, kPlocMaxRadius>);
-    static const int wide_blocks = cooperative_grid(wide_fn, kPlocBlocksPerSm);
-    static const int wave_blocks = cooperative_grid(wave_fn, kPlocOneWaveBlocksPerSm);
-    const int blocks = ploc_cluster_blocks();
-    if (wide_blocks <= 0 || wave_blocks <= 0 || blocks <= 0) return cudaErrorNotSupported;
-    uint32_t stop_n = static_cast<uint32_t>(blocks * (kClusterTile - 2 * radius));
-    uint32_t one_wave = static_cast<uint32_t>(wave_blocks), wide_grid = static_cast<uint32_t>(wide_blocks);
+                               uint32_t* err, uint32_t spin_limit, cudaEvent_t ploc_done, bool* enqueued,
+                               cudaStream_t s) {
+    *enqueued = false;
+    const PlocGrids grids = ploc_grids();
+    if (!grids.supported()) return cudaErrorNotSupported;
+    uint32_t stop_n = static_cast<uint32_t>(grids.cluster * (kClusterTile - 2 * radius));
+    uint32_t one_wave = static_cast<uint32_t>(grids.wave), wide_grid = static_cast<uint32_t>(grids.wide);
     cudaError_t e = cudaSuccess;
     if ((N + ploc_own(radius) - 1) / ploc_own(radius) > one_wave) {
         void* args[] = {&ca, &cb, &node_box, &node_kids, &it, &N, &radius, &one_wave, &lookback, &tickets, &n_tiles_cap,
                         &bar, &iters_out, &err, &spin_limit};
-        e = cudaLaunchCooperativeKernel(wide_fn, dim3(wide_grid), dim3(256), args, 0, s);
+        e = cudaLaunchCooperativeKernel(kWideFn, dim3(wide_grid), dim3(256), args, 0, s);
         if (e != cudaSuccess) return e;
+        *enqueued = true;
     }
     if (N > stop_n) {
         void* args[] = {&ca, &cb, &node_box, &node_kids, &it, &N, &radius, &stop_n, &lookback, &n_tiles_cap, &wide_grid,
                         &bar, &iters_out, &err, &spin_limit};
-        e = cudaLaunchCooperativeKernel(wave_fn, dim3(one_wave), dim3(256), args, 0, s);
+        e = cudaLaunchCooperativeKernel(kWaveFn, dim3(one_wave), dim3(256), args, 0, s);
         if (e != cudaSuccess) return e;
+        *enqueued = true;
     }
-    ClusterLaunch l(blocks, 1, s);
+    ClusterLaunch l(grids.cluster, 1, s);
     e = cudaLaunchKernelEx(&l.c, ploc_cluster_kernel<kPlocMaxRadius>, static_cast<const float4*>(ca),
                            static_cast<const float4*>(cb), node_box, node_kids, it, N, radius, iters_out, err);
     if (e != cudaSuccess) return e;
+    *enqueued = true;
     cudaEventRecord(ploc_done, s);
-    static int place_grid = 0;
-    if (place_grid == 0) {
-        int per_sm = 0;
-        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, layout_places_kernel<256>, 256, 0);
-        place_grid = kNumSms * (per_sm > 0 ? per_sm : 1);
-    }
     const uint32_t want = (N + 254) / 256;  // N - 1 internal nodes
     uint32_t* dfs = reinterpret_cast<uint32_t*>(ca);
     void* args[] = {&dfs, &node_kids, &N, &pf, &err, &spin_limit};
-    e = cudaLaunchCooperativeKernel(reinterpret_cast<const void*>(layout_places_kernel<256>),
-                                    dim3(want < static_cast<uint32_t>(place_grid) ? want : place_grid), dim3(256), args, 0, s);
+    e = cudaLaunchCooperativeKernel(kPlacesFn, dim3(want < static_cast<uint32_t>(grids.places) ? want : grids.places),
+                                    dim3(256), args, 0, s);
     if (e != cudaSuccess) return e;
     launch_layout_emit(node_box, node_kids, pf, N, dfs, out, wide, wide_wt, depth_odd, lv, st, err, s);
     return cudaGetLastError();

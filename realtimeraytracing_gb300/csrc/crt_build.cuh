@@ -104,12 +104,14 @@ void launch_single_leaf(const float4* node_box, crt_bvh_node* out, LeafOut leave
 // All PLOC iterations (a cooperative launch while the clusters are many, then one
 // thread-block cluster) and the DFS layout; ploc_done is recorded between the two.
 // iters_out[0] (zero before) receives the iteration count.
-// cudaErrorNotSupported when a cooperative or cluster launch is unavailable.
+// cudaErrorNotSupported, with nothing enqueued, when a cooperative or cluster launch
+// is unavailable; *enqueued: whether kernels were, also where a later launch failed.
 cudaError_t launch_ploc_layout(float4* ca, float4* cb, float4* node_box, uint4* node_kids, uint2* it, uint32_t N,
                                int radius, unsigned long long* lookback, uint32_t* tickets, uint32_t n_tiles_cap,
                                uint2* pf, crt_bvh_node* out, float4* wide, float4* wide_wt, uint8_t* depth_odd,
                                LeafOut leaves, const SceneState* st, unsigned long long* bar, uint32_t* iters_out,
-                               uint32_t* err, uint32_t spin_limit, cudaEvent_t ploc_done, cudaStream_t s);
+                               uint32_t* err, uint32_t spin_limit, cudaEvent_t ploc_done, bool* enqueued,
+                               cudaStream_t s);
 
 // Refit (crt_refit.cu).  The slack of the refit tree's root box goes to
 // abs_eps for the host.

@@ -46,4 +46,22 @@ private:
     uint64_t by_ = 0;  // whose stream the derivation is on
 };
 
+// Blocks of a launch whose blocks wait for one another: as many as a device of sms
+// SMs holds at once, per_sm of them an SM (at most per_sm_max); 0: it cannot run.
+constexpr int resident_blocks(bool cooperative, int per_sm, int per_sm_max, int sms) {
+    return !cooperative || per_sm <= 0 || sms <= 0 ? 0 : (per_sm < per_sm_max ? per_sm : per_sm_max) * sms;
+}
+
+// The build's default launches, each with its blocks on the current device.
+struct PlocGrids {
+    int wide = 0, wave = 0, places = 0;  // cooperative launches
+    int cluster = 0;                     // blocks of the thread-block cluster
+    constexpr bool supported() const { return wide > 0 && wave > 0 && places > 0 && cluster > 0; }
+};
+
+// Whether a build whose launch failed may start over on the launch-per-iteration
+// path.  That path reads the first clusters, records and look-back words, so only
+// while no kernel that changes them has been enqueued.
+constexpr bool may_start_over(bool not_supported, bool enqueued) { return not_supported && !enqueued; }
+
 }  // namespace crt

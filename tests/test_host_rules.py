@@ -72,3 +72,28 @@ int main() {
     return 0;
 }
 ''')
+
+
+def test_build_launches_fit_the_device_and_start_over_only_untouched(tmp_path):
+    """Grids whose blocks wait for one another follow the device's SMs (152, or fewer), and a failure after the first
+    launch is a failure: the launch-per-iteration path would read what that launch has overwritten."""
+    run_cpp(tmp_path, r'''
+int main() {
+    for (int sms : {1, 76, 140, 152})
+        for (int per_sm : {1, 2, 3, 8})
+            for (int most : {2, 3, 64}) {
+                const int g = crt::resident_blocks(true, per_sm, most, sms);
+                CHECK(g > 0 && g % sms == 0 && g <= per_sm * sms && g <= most * sms);
+                CHECK(g == per_sm * sms || g == most * sms);
+            }
+    CHECK(crt::resident_blocks(false, 3, 3, 152) == 0);
+    CHECK(crt::resident_blocks(true, 0, 3, 152) == 0);
+    CHECK(crt::resident_blocks(true, 3, 3, 0) == 0);
+    CHECK((crt::PlocGrids{456, 304, 1216, 16}.supported()));
+    CHECK((!crt::PlocGrids{0, 304, 1216, 16}.supported() && !crt::PlocGrids{456, 0, 1216, 16}.supported()));
+    CHECK((!crt::PlocGrids{456, 304, 0, 16}.supported() && !crt::PlocGrids{456, 304, 1216, 0}.supported()));
+    CHECK(crt::may_start_over(true, false));
+    CHECK(!crt::may_start_over(true, true) && !crt::may_start_over(false, false) && !crt::may_start_over(false, true));
+    return 0;
+}
+''')
