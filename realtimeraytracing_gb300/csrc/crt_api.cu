@@ -285,6 +285,8 @@ struct crt_ctx {
     static crt_status describe_error(const uint32_t* ew) {
         const uint32_t e = ew[0];
         if (e & crt::kDevTimeout) return fail(CRT_ERR_DEVICE_TIMEOUT, "a bounded device wait gave up (err=0x%x)", e);
+        if (e & crt::kDevIterLimit)
+            return fail(CRT_ERR_DEVICE_TIMEOUT, "PLOC does not end: clusters whose boxes are not finite (err=0x%x)", e);
         if (e & crt::kDevBadModel) return fail(CRT_ERR_BAD_INPUT, "a triangle references model id >= 64");
         if (e & crt::kDevBadIndex) return fail(CRT_ERR_BAD_INPUT, "a triangle references a vertex past the end");
         if (e & crt::kDevStackOverflow) return fail(CRT_ERR_STACK_OVERFLOW, "a ray overflowed its traversal stack");

@@ -400,6 +400,7 @@ __global__ void __launch_bounds__(BLOCK) batch_places_kernel(const BatchScene* _
         s_mine[2] = blocks;
     }
     __syncthreads();
+    if (build_failed(err)) return;  // as layout_places_kernel
     const BatchScene B = scenes[s_mine[0]];
     const uint32_t N = B.n_tris, stride = s_mine[2] * BLOCK;
     for (uint32_t t = s_mine[1] * BLOCK + threadIdx.x; t + 1 < N; t += stride)
@@ -416,7 +417,7 @@ __global__ void __launch_bounds__(256) batch_emit_kernel(const BatchScene* __res
                                                          float4* __restrict__ wide, float4* __restrict__ wide_wt,
                                                          uint8_t* __restrict__ depth_odd, LeafOut lv, uint32_t* err) {
     const uint32_t q = blockIdx.x * 256 + threadIdx.x;
-    if (q >= n_slots) return;
+    if (q >= n_slots || build_failed(err)) return;
     uint32_t lo = 0, hi = n_scenes - 1;  // node_off: slots before the scene
     while (lo < hi) {
         const uint32_t mid = (lo + hi + 1) >> 1;

@@ -1292,7 +1292,7 @@ __global__ void __launch_bounds__(256) layout_emit_kernel(const float4* __restri
                                                           uint8_t* __restrict__ depth_odd, LeafOut lv,
                                                           const SceneState* __restrict__ st, uint32_t* err) {
     const uint32_t p = blockIdx.x * blockDim.x + threadIdx.x;
-    if (p >= 2 * N - 1) return;
+    if (p >= 2 * N - 1 || build_failed(err)) return;
     layout_emit(p, node_box, node_kids, pf, N, dfs, out, wide, wide_wt, depth_odd, lv, st->abs_eps, err);
 }
 
@@ -1759,6 +1759,7 @@ __global__ void __launch_bounds__(BLOCK) layout_places_kernel(uint32_t* __restri
     // out, waits (bounded) until X's parent has published X's position.  The
     // unfinished node with the largest id never waits (its parent is done), so
     // the co-resident grid always progresses, with no barrier per PLOC level.
+    if (build_failed(err)) return;  // places that no parent hands out: nothing to wait for
     for (uint32_t t = blockIdx.x * BLOCK + threadIdx.x; t + 1 < N; t += gridDim.x * BLOCK)
         if (!layout_place_node(2 * N - 2 - t, t < gridDim.x * BLOCK, dfs, node_kids, N, pf, err, spin_limit)) return;
 }

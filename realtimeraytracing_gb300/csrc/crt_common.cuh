@@ -131,6 +131,13 @@ enum DevError : uint32_t {
 
 __device__ __forceinline__ void raise_error(uint32_t* err, uint32_t code) { atomicOr(err, code); }
 
+// Whether an earlier kernel of a build gave up, so that the records the next one
+// would follow may never have been written (a bad model id leaves them complete).
+// A plain load: a kernel of the same launch may be raising something meanwhile.
+__device__ __forceinline__ bool build_failed(const uint32_t* err) {
+    return (*err & (kDevTimeout | kDevStackOverflow | kDevIterLimit | kDevCorrupt)) != 0u;
+}
+
 // Records the first failed index check: err[1] = site, err[2..3] = values.
 __device__ __forceinline__ void raise_corrupt(uint32_t* err, uint32_t site, uint32_t v0, uint32_t v1) {
     atomicOr(err, static_cast<uint32_t>(kDevCorrupt));
