@@ -226,6 +226,7 @@ struct crt_ctx {
     // they neither clear nor copy one; [4] rays the last persistent trace left over.
     uint32_t* hw = nullptr;
     uint32_t* hw_dev = nullptr;
+    crt::HostErrorWords host_error;
     DevBuf walk_ctr;  // persistent walks' counters (zero between launches)
     // The launch of the rays that the last persistent walk left over, until its
     // number is known (finish_walk).
@@ -256,18 +257,16 @@ struct crt_ctx {
         pinned_cap = bytes;
         return CRT_OK;
     }
-    // Host-visible error word: nothing of this context runs between its calls, so
-    // the host clears it.  It also follows a failed call's kernels here.
-    crt_status begin_host_error() {
-        if (hw[0] == 0u) return CRT_OK;
+    crt_status wait() {
         CRT_CUDA(cudaStreamSynchronize(stream));
-        for (int k = 0; k < 4; ++k) hw[k] = 0u;
         return CRT_OK;
     }
+    crt_status begin_host_error() {
+        return host_error.begin([this] { return wait(); });
+    }
     crt_status check_host_error() {
-        CRT_CUDA(cudaStreamSynchronize(stream));
-        const uint32_t ew[4] = {hw[0], hw[1], hw[2], hw[3]};
-        for (int k = 0; k < 4; ++k) hw[k] = 0u;
+        uint32_t ew[4];
+        CRT_TRY(host_error.end([this] { return wait(); }, ew));
         return describe_error(ew);
     }
     crt_status begin_device_error() {
@@ -367,6 +366,7 @@ crt_status crt_create(crt_ctx** out, const crt_config* cfg) {
                         cudaHostGetDevicePointer(reinterpret_cast<void**>(&x->hw_dev), x->hw, 0) != cudaSuccess))
         s = fail(CRT_ERR_CUDA, "host-visible words");
     if (s == CRT_OK) std::memset(x->hw, 0, 64);
+    x->host_error.words = x->hw;
     if (s == CRT_OK) {
         crt::SceneState init{};
         for (int a = 0; a < 3; ++a) { init.key_max[a] = 0ull; init.key_min[a] = ~0ull; }

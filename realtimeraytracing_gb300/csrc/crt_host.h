@@ -46,6 +46,41 @@ private:
     uint64_t by_ = 0;  // whose stream the derivation is on
 };
 
+// Four page-locked words that a context's kernels raise errors in, so that its
+// calls neither clear nor copy a device word.  begin() before a call enqueues its
+// kernels, end() once it has; sync() waits for the context's stream and returns 0 or
+// an error.  A call that returns between the two leaves kernels behind that may
+// still raise something: the next begin() waits for them, so that no call reports
+// another's error.
+class HostErrorWords {
+public:
+    template <class Sync>
+    auto begin(Sync sync) -> decltype(sync()) {
+        if (open_) {
+            const auto status = sync();
+            if (status != decltype(sync()){}) return status;
+        }
+        clear();
+        open_ = true;
+        return {};
+    }
+    template <class Sync>
+    auto end(Sync sync, uint32_t out[4]) -> decltype(sync()) {
+        const auto status = sync();
+        if (status != decltype(sync()){}) return status;
+        for (int k = 0; k < 4; ++k) out[k] = words[k];
+        open_ = false;
+        return {};
+    }
+    volatile uint32_t* words = nullptr;
+
+private:
+    void clear() {
+        for (int k = 0; k < 4; ++k) words[k] = 0u;
+    }
+    bool open_ = false;
+};
+
 // Blocks of a launch whose blocks wait for one another: as many as a device of sms
 // SMs holds at once, per_sm of them an SM (at most per_sm_max); 0: it cannot run.
 constexpr int resident_blocks(bool cooperative, int per_sm, int per_sm_max, int sms) {

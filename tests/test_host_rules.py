@@ -97,3 +97,35 @@ int main() {
     return 0;
 }
 ''')
+
+
+def test_an_abandoned_calls_error_is_not_the_next_calls(tmp_path):
+    """A call returns early while its kernels run; one of them raises an error afterwards.  The next call waits for
+    them before it clears the words, and reports its own errors only."""
+    run_cpp(tmp_path, r'''
+enum Status { kOk = 0, kFailed = 3 };
+int main() {
+    uint32_t w[4] = {9, 9, 9, 9}, out[4];
+    std::vector<uint32_t> queue;  // words that kernels in flight will raise
+    int waits = 0;
+    auto sync = [&] { ++waits; for (uint32_t e : queue) w[0] |= e; queue.clear(); return kOk; };
+    auto dead = [&] { return kFailed; };
+    crt::HostErrorWords e;
+    e.words = w;
+    CHECK(e.begin(sync) == kOk && waits == 0 && w[0] == 0 && w[3] == 0);
+    CHECK(e.end(sync, out) == kOk && waits == 1 && out[0] == 0);
+    CHECK(e.begin(sync) == kOk && waits == 1);  // nothing is in flight between calls: no wait
+    queue.push_back(4);
+    CHECK(e.end(sync, out) == kOk && out[0] == 4);
+    CHECK(e.begin(sync) == kOk && waits == 2 && w[0] == 0);
+    queue.push_back(16);  // and the call returns without end()
+    CHECK(e.begin(sync) == kOk && waits == 3 && queue.empty() && w[0] == 0);
+    queue.push_back(1);
+    CHECK(e.end(sync, out) == kOk && out[0] == 1);
+    CHECK(e.begin(sync) == kOk && e.end(dead, out) == kFailed);  // not known to be over: the next call waits
+    CHECK(e.begin(dead) == kFailed);
+    waits = 0;
+    CHECK(e.begin(sync) == kOk && waits == 1);
+    return 0;
+}
+''')
