@@ -227,7 +227,7 @@ struct crt_ctx {
     uint32_t* hw = nullptr;
     uint32_t* hw_dev = nullptr;
     crt::HostErrorWords host_error;
-    DevBuf walk_ctr;  // persistent walks' counters (zero between launches)
+    DevBuf walk;  // persistent walks' scratch (crt::WalkScratch; counters zero between launches)
     // The launch of the rays that the last persistent walk left over, until its
     // number is known (finish_walk).
     std::function<void(uint32_t)> left_over;
@@ -360,8 +360,8 @@ crt_status crt_create(crt_ctx** out, const crt_config* cfg) {
     if (s == CRT_OK) s = x->cam.reserve(sizeof(crt_camera));
     if (s == CRT_OK) s = x->trace_stats.reserve(16);
     if (s == CRT_OK) s = x->pinned_reserve(1 << 16);
-    if (s == CRT_OK) s = x->walk_ctr.reserve(16);
-    if (s == CRT_OK && (cudaMemset(x->walk_ctr.p, 0, 16) != cudaSuccess ||
+    if (s == CRT_OK) s = x->walk.reserve(crt::kWalkScratchBytes);
+    if (s == CRT_OK && (cudaMemset(x->walk.p, 0, 16) != cudaSuccess ||
                         cudaHostAlloc(reinterpret_cast<void**>(&x->hw), 64, cudaHostAllocMapped) != cudaSuccess ||
                         cudaHostGetDevicePointer(reinterpret_cast<void**>(&x->hw_dev), x->hw, 0) != cudaSuccess))
         s = fail(CRT_ERR_CUDA, "host-visible words");
@@ -392,7 +392,7 @@ crt_status crt_destroy(crt_ctx* x) {
                       &x->ray_order, &x->ray_order_scratch, &x->shade_models, &x->shade_materials,
                       &x->shade_rays, &x->shade_hits, &x->image, &x->refit_state, &x->xtri_sorted,
                       &x->mesh_vertices, &x->mesh_indices, &x->mesh_out, &x->probe_flag, &x->step_in,
-                      &x->step_out, &x->walk_ctr};
+                      &x->step_out, &x->walk};
     for (DevBuf* b : bufs) b->release();
     if (x->hw) cudaFreeHost(x->hw);
     for (auto& e : x->ev)
@@ -798,16 +798,6 @@ crt_status ensure_cwide(crt_ctx* x, const crt_bvh* b) {
     });
 }
 
-// Scratch of a persistent walk of n rays: the list of left-over rays lies in
-// build scratch, idle between builds.
-crt_status walk_scratch(crt_ctx* x, uint32_t n, bool wait, crt::WalkScratch* w) {
-    CRT_TRY(x->node_box.reserve(4ull * n));
-    w->ctr = x->walk_ctr.as<uint32_t>();
-    w->left = x->node_box.as<uint32_t>();
-    w->host_left = wait ? x->hw_dev + 4 : nullptr;
-    return CRT_OK;
-}
-
 // Waits for a persistent walk issued with host_left and launches the rays it
 // left over.
 crt_status finish_walk(crt_ctx* x) {
@@ -838,10 +828,14 @@ crt_status frame_walk4(crt_ctx* x, const crt_bvh* b, uint32_t pixels, crt::Trace
 // A one-launch frame, and the pixels it leaves to the binary walk.
 crt_status frame_launch(crt_ctx* x, const crt::TraceParams& p, const crt_camera* cam, uint32_t width, uint32_t height,
                         const float* light, crt_hit* hits_shadow, uint32_t flags, const crt::ShadeParams* sp) {
-    crt::WalkScratch ws;
-    if (p.cwide) CRT_TRY(walk_scratch(x, p.n_rays, true, &ws));
+    const crt::WalkScratch ws(x->walk.p, x->hw_dev + 4);
+    crt::TraceParams q = p;
     auto launch = [&](uint32_t left) {
-        crt::launch_frame(p, cam, width, height, 0, height, light, hits_shadow, flags,
+        if (left > crt::kWalkLeft) {  // the whole image on the binary nodes
+            q.cwide = nullptr;
+            if (q.stats) cudaMemsetAsync(q.stats, 0, 16, x->stream);
+        }
+        crt::launch_frame(q, cam, width, height, 0, height, light, hits_shadow, flags,
                           static_cast<int>(x->cfg.trace_block), sp, ws, left, x->stream);
     };
     launch(0);
@@ -940,15 +934,14 @@ crt_status trace_device(crt_ctx* x, const crt_bvh* b, const crt_ray* d_rays, uin
     const bool deep = (b->depth_bound + 2 > 64) || (3 * ((b->depth_bound + 2) / 2) + 3 > 96);
     const uint32_t launch_flags =
         (flags & (CRT_TRACE_ANY | CRT_TRI_WATERTIGHT | CRT_TRACE_WIDE | CRT_TRACE_COMPRESSED)) | (deep ? (1u << 16) : 0u);
-    crt::WalkScratch ws;
-    if (pool) CRT_TRY(walk_scratch(x, n_rays, wait, &ws));
+    const crt::WalkScratch ws(x->walk.p, wait ? x->hw_dev + 4 : nullptr);
     CRT_CUDA(cudaEventRecord(x->tev[1], x->stream));
     if (pool) crt::launch_trace_pool(p, launch_flags, ws, x->stream);
     else crt::launch_trace(p, launch_flags, static_cast<int>(x->cfg.trace_block), x->stream);
     CRT_CUDA(cudaGetLastError());
     CRT_CUDA(cudaEventRecord(x->tev[2], x->stream));
     x->tev_valid = true;
-    if (ws.host_left)
+    if (pool && wait)
         x->left_over = [=](uint32_t n) {
             crt::launch_trace_left(p, launch_flags, ws, n, x->stream);
             cudaEventRecord(x->tev[2], x->stream);
@@ -1955,7 +1948,7 @@ struct crt_batch {
     bool cwide_ready = false;
     bool g_cwide = false;                 // the captured graph derives them
     uint32_t* cw_bad() const { return reinterpret_cast<uint32_t*>(cwide.as<char>() + 64ull * n_tris); }
-    DevBuf walk_ctr;                      // the persistent trace's counters (zero between launches)
+    DevBuf walk;                          // the persistent trace's scratch (crt::WalkScratch; counters zero between launches)
     bool models_set = false;
     cudaGraphExec_t graph = nullptr;
     const void* g_tris = nullptr;
@@ -2051,7 +2044,7 @@ crt_status batch_trace_enqueue(crt_ctx* x, crt_batch* bt, const crt_ray* rays, u
         p.cw_bad = bt->cw_bad();
         crt::launch_trace_batch_pool(p, bt->scenes.as<crt::BatchScene>(), bt->n_scenes,
                                      flags & (CRT_TRACE_ANY | CRT_TRI_WATERTIGHT), deep,
-                                     crt::WalkScratch{bt->walk_ctr.as<uint32_t>(), bt->node_box.as<uint32_t>(), nullptr}, s);
+                                     crt::WalkScratch(bt->walk.p, nullptr), s);
     } else
         crt::launch_trace_batch(p, bt->scenes.as<crt::BatchScene>(), bt->n_scenes, bt->n_rays,
                                 flags & (CRT_TRACE_ANY | CRT_TRI_WATERTIGHT), static_cast<int>(bt->cfg.trace_block), deep,
@@ -2221,9 +2214,8 @@ crt_status crt_batch_create(crt_ctx* x, const uint32_t* tri_counts, const uint32
                       &bt->inv_perm})
         R(*b, 4ull * N);
     R(bt->node_kids, 16ull * N);
-    // node_box also holds the trace's left-over rays: it is build scratch, idle between builds
-    R(bt->node_box, std::max<size_t>(32ull * (2ull * N), 4ull * bt->ray_cap));
-    R(bt->walk_ctr, 16);
+    R(bt->node_box, 32ull * (2ull * N));
+    R(bt->walk, crt::kWalkScratchBytes);
     R(bt->cwide, 64ull * N + 16);
     R(bt->pf, 8ull * N);
     R(bt->clus_a, 32ull * N);
@@ -2244,7 +2236,7 @@ crt_status crt_batch_create(crt_ctx* x, const uint32_t* tri_counts, const uint32
     seg[n_scenes] = N;
     bt->tri_off = seg;
     st = CRT_OK;
-    if (cudaMemset(bt->walk_ctr.p, 0, 16) != cudaSuccess ||
+    if (cudaMemset(bt->walk.p, 0, 16) != cudaSuccess ||
         cudaMemcpy(bt->scenes.p, hs.data(), sizeof(crt::BatchScene) * n_scenes, cudaMemcpyHostToDevice) != cudaSuccess ||
         cudaMemcpy(bt->seg_off.p, seg.data(), 4ull * seg.size(), cudaMemcpyHostToDevice) != cudaSuccess ||
         cudaMemcpy(bt->seg_hist.p, segh.data(), 4ull * 256, cudaMemcpyHostToDevice) != cudaSuccess ||
@@ -2270,7 +2262,7 @@ crt_status crt_batch_free(crt_batch* bt) {
                       &bt->codes_a, &bt->codes_b, &bt->vals_a, &bt->vals_b, &bt->codes, &bt->perm_global,
                       &bt->perm_local, &bt->node_box, &bt->node_kids, &bt->pf, &bt->clus_a, &bt->clus_b, &bt->it,
                       &bt->ploc_lb, &bt->hist, &bt->sort_lb, &bt->nodes, &bt->wide, &bt->wide_wt, &bt->depth_odd, &bt->xtri, &bt->ray_order, &bt->ray_order_scratch,
-                      &bt->inv_perm, &bt->xtri_sorted, &bt->cwide, &bt->walk_ctr};
+                      &bt->inv_perm, &bt->xtri_sorted, &bt->cwide, &bt->walk};
     for (DevBuf* b : bufs) b->release();
     delete bt;
     return CRT_OK;

@@ -163,17 +163,25 @@ struct TraceParams {
 };
 void launch_trace(const TraceParams& p, uint32_t flags, int block, cudaStream_t s);
 // Scratch of a persistent walk over the compressed nodes: 16 bytes of counters,
-// zero before its first use and again after each launch, room for the index of
-// every ray, and optionally a page-locked word for the number of rays left to the
-// binary walk.  With it the caller waits for the launch and then launches the
-// left-over rays itself; without, they are launched right away.
+// zero before its first use and again after each launch, the list of the rays left
+// to the binary walk, and optionally a page-locked word for their number.  With it
+// the caller waits for the launch and then launches the left-over rays itself;
+// without, they are launched right away.  The list holds kWalkLeft rays and is
+// reserved once, with the context or the batch: usually it stays empty, and a
+// launch that would leave more gives up, after which all its rays are walked on the
+// binary nodes in their order.
+constexpr uint32_t kWalkLeft = 65536;
+constexpr size_t kWalkScratchBytes = 16 + 4 * static_cast<size_t>(kWalkLeft);
 struct WalkScratch {
     uint32_t* ctr = nullptr;
     uint32_t* left = nullptr;
     uint32_t* host_left = nullptr;
+    WalkScratch() = default;
+    WalkScratch(void* scratch, uint32_t* host) : ctr(static_cast<uint32_t*>(scratch)), left(ctr + 4), host_left(host) {}
 };
 // Many rays by persistent warps that refill finished lanes from a ray counter;
-// compressed nodes, no seeding, rays in caller order or p.order.
+// compressed nodes, no seeding, rays in caller order or p.order.  launch_trace_left:
+// the n rays such a launch left over (all of them above kWalkLeft).
 void launch_trace_pool(const TraceParams& p, uint32_t flags, const WalkScratch& w, cudaStream_t s);
 void launch_trace_left(const TraceParams& p, uint32_t flags, const WalkScratch& w, uint32_t n, cudaStream_t s);
 
@@ -199,7 +207,7 @@ void launch_shade(const TraceParams& p, const ShadeParams& sp, cudaStream_t s);
 // any hit into hits_shadow, and with shade, their texels into shade->image,
 // in one launch (p.tile_width: width for 8x4 pixel tiles, or 0).  With p.cwide
 // over the compressed nodes (w with host_left); left != 0: the pixels such a
-// launch left over.
+// launch left over, at most kWalkLeft.
 void launch_frame(const TraceParams& p, const crt_camera* cam, uint32_t width, uint32_t height, uint32_t y0,
                   uint32_t rows, const float* light, crt_hit* hits_shadow, uint32_t flags, int block,
                   const ShadeParams* shade, const WalkScratch& w, uint32_t left, cudaStream_t s);

@@ -230,11 +230,12 @@ __global__ void __launch_bounds__(kWalk4Block, kWalk4Blocks)
             redo = redo || L.redo;
             if (valid && !redo) reinterpret_cast<uint4*>(f.hits_shadow)[i] = L.hit();
         }
-        if (valid && redo) left[atomicAdd(&ctr->left, 1u)] = i;
+        walk4_leave(ctr, left, valid && redo, i, tiles);
         uint32_t next = tiles;
         if (tiles > warps) {
-            if (lane == 0) next = warps + atomicAdd(&ctr->taken, 1u);
+            if (lane == 0) next = atomicAdd(&ctr->taken, 1u);
             next = __shfl_sync(0xFFFFFFFFu, next, 0);
+            next = next < tiles - warps ? next + warps : tiles;
         }
         tile = next;
     }
@@ -248,7 +249,7 @@ __global__ void __launch_bounds__(kWalk4Block, kWalk4Blocks)
 template <bool WT, int STACK, bool SHADE>
 __global__ void __launch_bounds__(kWalk4Block)
     frame_left_kernel(TraceParams p, FrameParams f, ShadeParams sp, uint32_t n, const uint32_t* __restrict__ left) {
-    n = min(n, p.n_rays);
+    n = min(n, kWalkLeft);
     for (uint32_t k = blockIdx.x * kWalk4Block + threadIdx.x; k < n; k += gridDim.x * kWalk4Block) {
         const uint32_t i = left[k];
         if (i >= p.n_rays) raise_corrupt(p.err, 7, k, i);

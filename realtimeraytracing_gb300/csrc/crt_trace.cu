@@ -216,7 +216,8 @@ static void launch_walk4_t(const TraceParams& p, bool deep, const WalkScratch& w
         if (w.host_left) return;
     }
     const uint32_t* count = left == 0 ? &ctr->last_left : nullptr;
-    const uint32_t few = std::min(left == 0 ? want : (left + kWalk4Block - 1) / kWalk4Block, static_cast<uint32_t>(kNumSms * 16));
+    const uint32_t items = left == 0 || left > kWalkLeft ? p.n_rays : left;
+    const uint32_t few = std::min((items - 1) / kWalk4Block + 1, static_cast<uint32_t>(kNumSms * 16));
     if (deep) walk4_left_kernel<ANY, WT, 1024, BATCH><<<few, kWalk4Block, 0, s>>>(p, count, left, w.left, scenes, n_scenes);
     else walk4_left_kernel<ANY, WT, 64, BATCH><<<few, kWalk4Block, 0, s>>>(p, count, left, w.left, scenes, n_scenes);
 }

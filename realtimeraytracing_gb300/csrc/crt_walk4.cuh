@@ -396,12 +396,31 @@ __device__ __forceinline__ uint32_t walk4_run(Walk4Lane& L, uint32_t s_base, uin
 
 // A persistent walk's counters in device memory.  The launch's last block zeroes
 // them for the next one (no clear in between) and hands the number of rays left
-// over to the device (last_left) and, where given, to page-locked host memory,
-// so that a caller that waits for the launch anyway starts walk4_left_kernel only
-// when there are any.
+// over (above kWalkLeft they are not all on the list) to the device, last_left, and
+// where given to page-locked host memory, so that a caller that waits for the
+// launch anyway starts walk4_left_kernel only when there are any.
 struct Walk4Counters {
     uint32_t taken, left, blocks, last_left;
 };
+// Puts item i of the lanes with redo on the list of what is left to the binary
+// walk (whole warps; one atomic each).  Once the list overflows the launch's result
+// is not used: limit, the number of items to take, goes into the counter, and every
+// warp finds nothing more to take.
+__device__ __forceinline__ void walk4_leave(Walk4Counters* ctr, uint32_t* __restrict__ left, bool redo, uint32_t i,
+                                            uint32_t limit) {
+    const uint32_t m = __ballot_sync(0xFFFFFFFFu, redo);
+    if (!m) return;
+    const uint32_t lane = threadIdx.x & 31u, cnt = static_cast<uint32_t>(__popc(m));
+    const int leader = __ffs(m) - 1;
+    uint32_t base = 0;
+    if (lane == static_cast<uint32_t>(leader)) {
+        base = atomicAdd(&ctr->left, cnt);
+        if (base + cnt > kWalkLeft) atomicMax(&ctr->taken, limit);
+    }
+    base = __shfl_sync(0xFFFFFFFFu, base, leader);
+    const uint32_t k = base + static_cast<uint32_t>(__popc(m & ((1u << lane) - 1u)));
+    if (redo && k < kWalkLeft) left[k] = i;
+}
 __device__ __forceinline__ void walk4_finish(Walk4Counters* ctr, uint32_t* host_left) {
     __syncthreads();
     if (threadIdx.x != 0) return;
@@ -488,9 +507,10 @@ __global__ void __launch_bounds__(kWalk4Block, kWalk4Blocks)
         if (i == kIdle && !pool_left) i = kDone;
         if (__all_sync(0xFFFFFFFFu, i == kDone)) break;
         const uint32_t om = walk4_run<ANY, WT, kWalk4Flush>(L, s_base, st, pool_left ? kWalk4Refill : 32);
-        if ((om >> lane & 1u) && i < kDone) {
-            if (L.redo) left[atomicAdd(&ctr->left, 1u)] = i;
-            else reinterpret_cast<uint4*>(p.hits)[i] = L.hit();
+        const bool done = (om >> lane & 1u) && i < kDone;
+        walk4_leave(ctr, left, done && L.redo, i, p.n_rays);
+        if (done) {
+            if (!L.redo) reinterpret_cast<uint4*>(p.hits)[i] = L.hit();
             i = kIdle;
         }
     }
@@ -498,15 +518,19 @@ __global__ void __launch_bounds__(kWalk4Block, kWalk4Blocks)
 }
 
 // The binary walk of the rays a trace_walk4_kernel launch left over (few or none):
-// n of them, or as many as *count says.
+// n of them, or as many as *count says; all rays if they are more than the list
+// holds.
 template <bool ANY, bool WT, int STACK, bool BATCH>
 __global__ void __launch_bounds__(kWalk4Block)
     walk4_left_kernel(const TraceParams p, const uint32_t* __restrict__ count, uint32_t n,
                       const uint32_t* __restrict__ left, const BatchScene* __restrict__ scenes, uint32_t n_scenes) {
-    n = min(count ? *count : n, p.n_rays);
-    for (uint32_t k = blockIdx.x * kWalk4Block + threadIdx.x; k < n; k += gridDim.x * kWalk4Block) {
-        const uint32_t i = left[k];
-        if (i >= p.n_rays) { raise_corrupt(p.err, 7, k, i); continue; }
+    if (count) n = *count;
+    const bool all = n > kWalkLeft;
+    const uint64_t total = all ? p.n_rays : n;
+    for (uint64_t k = static_cast<uint64_t>(blockIdx.x) * kWalk4Block + threadIdx.x; k < total;
+         k += static_cast<uint64_t>(gridDim.x) * kWalk4Block) {
+        const uint32_t i = !all ? left[k] : p.order ? __ldg(p.order + k) : static_cast<uint32_t>(k);
+        if (i >= p.n_rays) { raise_corrupt(p.err, 7, static_cast<uint32_t>(k), i); continue; }
         TraceParams q = p;
         if (BATCH) {
             uint32_t lo = 0, hi = n_scenes - 1;
