@@ -131,8 +131,9 @@ typedef struct crt_camera {
                                        layout stays the export format.  Traces of >= 65,536 rays and
                                        frames take them without the flag */
 #define CRT_TRACE_PER_RAY_THREADS 0x100u /* crt_trace of >= 65,536 rays normally runs on persistent warps
-                                       over the compressed nodes whose lanes take a new ray as soon as
-                                       theirs is done; this flag keeps one thread per ray for its whole
+                                       over the compressed nodes (closest hits of rays and scenes those
+                                       cannot take: over the binary nodes) whose lanes take a new ray as
+                                       soon as theirs is done; this flag keeps one thread per ray for its whole
                                        walk of the binary nodes instead (same hits) */
 
 typedef struct crt_config {

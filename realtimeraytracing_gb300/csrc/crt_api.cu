@@ -154,12 +154,16 @@ struct crt_bvh {
     // Since a refit only the root box of the node array is kept current; the
     // others are derived from the traversal nodes (node_boxes).
     bool refitted = false;
+    // A box of the current tree's compressed nodes could not be quantised (a launch
+    // over them has said so): the walk over them would leave every ray over.
+    mutable std::atomic<bool> unquantised{false};
     // The tree has changed: what was derived from it no longer holds.
     void changed(bool by_refit) {
         wide4_nodes.state.reset();
         cwide_nodes.state.reset();
         node_boxes.state.reset();
         frame_pixels = 0;
+        unquantised = false;
         refitted = by_refit;
     }
     // Sorted Morton codes and permutation exist (a tree from crt_bvh_from_nodes has none).
@@ -361,7 +365,7 @@ crt_status crt_create(crt_ctx** out, const crt_config* cfg) {
     if (s == CRT_OK) s = x->trace_stats.reserve(16);
     if (s == CRT_OK) s = x->pinned_reserve(1 << 16);
     if (s == CRT_OK) s = x->walk.reserve(crt::kWalkScratchBytes);
-    if (s == CRT_OK && (cudaMemset(x->walk.p, 0, 16) != cudaSuccess ||
+    if (s == CRT_OK && (cudaMemset(x->walk.p, 0, crt::kWalkCounterBytes) != cudaSuccess ||
                         cudaHostAlloc(reinterpret_cast<void**>(&x->hw), 64, cudaHostAllocMapped) != cudaSuccess ||
                         cudaHostGetDevicePointer(reinterpret_cast<void**>(&x->hw_dev), x->hw, 0) != cudaSuccess))
         s = fail(CRT_ERR_CUDA, "host-visible words");
@@ -798,14 +802,20 @@ crt_status ensure_cwide(crt_ctx* x, const crt_bvh* b) {
     });
 }
 
-// Waits for a persistent walk issued with host_left and launches the rays it
+// Whether the walk over b's compressed nodes can take rays at all, as far as known.
+bool walk4_usable(const crt_bvh* b) {
+    return b->n > 1 && b->own_boxes && !b->unquantised && crt::walk4_scene(b->abs_eps);
+}
+
+// Waits for a persistent walk over b issued with host_left and launches the rays it
 // left over.
-crt_status finish_walk(crt_ctx* x) {
+crt_status finish_walk(crt_ctx* x, const crt_bvh* b) {
     if (!x->left_over) return CRT_OK;
     auto launch = std::move(x->left_over);
     x->left_over = nullptr;
     CRT_CUDA(cudaStreamSynchronize(x->stream));
     const uint32_t n = reinterpret_cast<volatile uint32_t*>(x->hw)[4];
+    if (reinterpret_cast<volatile uint32_t*>(x->hw)[5] != 0u) b->unquantised = true;
     if (n != 0) {
         launch(n);
         CRT_CUDA(cudaGetLastError());
@@ -816,9 +826,11 @@ crt_status finish_walk(crt_ctx* x) {
 // One-launch frames walk the compressed nodes once the frames of the current
 // tree have a quarter as many pixels as it has triangles: deriving the nodes
 // takes 0.035 ns per triangle (73 us at 2.0 M) and a pixel gains 0.05-0.2 ns.
-crt_status frame_walk4(crt_ctx* x, const crt_bvh* b, uint32_t pixels, crt::TraceParams* p) {
+// cam: in host memory, or null where its position is not known here.
+crt_status frame_walk4(crt_ctx* x, const crt_bvh* b, const crt_camera* cam, uint32_t pixels, crt::TraceParams* p) {
+    if (!walk4_usable(b) || (cam && !crt::walk4_camera(cam->eye, b->abs_eps))) return CRT_OK;
     const uint64_t frames = b->frame_pixels += pixels;
-    if (b->n < 2 || !b->own_boxes || (!b->cwide_nodes.state.ready() && 4 * frames < b->n)) return CRT_OK;
+    if (!b->cwide_nodes.state.ready() && 4 * frames < b->n) return CRT_OK;
     CRT_TRY(ensure_cwide(x, b));
     p->cwide = b->cwide.as<uint4>();
     p->cw_bad = b->cw_bad();
@@ -826,7 +838,7 @@ crt_status frame_walk4(crt_ctx* x, const crt_bvh* b, uint32_t pixels, crt::Trace
 }
 
 // A one-launch frame, and the pixels it leaves to the binary walk.
-crt_status frame_launch(crt_ctx* x, const crt::TraceParams& p, const crt_camera* cam, uint32_t width, uint32_t height,
+crt_status frame_launch(crt_ctx* x, const crt_bvh* b, const crt::TraceParams& p, const crt_camera* cam, uint32_t width, uint32_t height,
                         const float* light, crt_hit* hits_shadow, uint32_t flags, const crt::ShadeParams* sp) {
     const crt::WalkScratch ws(x->walk.p, x->hw_dev + 4);
     crt::TraceParams q = p;
@@ -842,7 +854,7 @@ crt_status frame_launch(crt_ctx* x, const crt::TraceParams& p, const crt_camera*
     CRT_CUDA(cudaGetLastError());
     if (!p.cwide) return CRT_OK;
     x->left_over = launch;
-    return finish_walk(x);
+    return finish_walk(x, b);
 }
 
 // Enqueues one traversal launch on device-resident rays/hits (no sync).
@@ -860,10 +872,13 @@ crt_status trace_device(crt_ctx* x, const crt_bvh* b, const crt_ray* d_rays, uin
     if (n_rays == 0) return CRT_OK;
     if (flags & CRT_TRACE_WIDE) CRT_TRY(ensure_wide4(x, b));
     if (!b->own_boxes) flags &= ~CRT_TRACE_COMPRESSED;
-    // Large batches over one scene: persistent warps over the compressed nodes;
-    // pixels in 8x4 tiles, seeded, 4-wide and counting walks keep one thread per ray.
-    const bool pool = !(flags & (CRT_TRACE_WIDE | CRT_TRACE_PER_RAY_THREADS | CRT_TRACE_USE_PREDICTOR | CRT_TRACE_STATS)) &&
-                      !seed_classes && tile_width == 0 && n_rays >= kPoolMinRays && b->n > 1 && b->own_boxes;
+    // Large batches over one scene: persistent warps, over the compressed nodes where
+    // those take its rays (closest hits over the binary nodes otherwise); pixels in
+    // 8x4 tiles, seeded, 4-wide and counting walks keep one thread per ray.
+    const bool large = !(flags & (CRT_TRACE_WIDE | CRT_TRACE_PER_RAY_THREADS | CRT_TRACE_USE_PREDICTOR | CRT_TRACE_STATS)) &&
+                       !seed_classes && tile_width == 0 && n_rays >= kPoolMinRays && b->n > 1;
+    const bool pool = large && walk4_usable(b);
+    const bool binary_pool = large && !pool && !(flags & (CRT_TRACE_ANY | CRT_TRACE_COMPRESSED));
     if (pool || (flags & CRT_TRACE_COMPRESSED)) CRT_TRY(ensure_cwide(x, b));
     x->tev_valid = false;
     CRT_CUDA(cudaEventRecord(x->tev[0], x->stream));
@@ -937,13 +952,17 @@ crt_status trace_device(crt_ctx* x, const crt_bvh* b, const crt_ray* d_rays, uin
     const crt::WalkScratch ws(x->walk.p, wait ? x->hw_dev + 4 : nullptr);
     CRT_CUDA(cudaEventRecord(x->tev[1], x->stream));
     if (pool) crt::launch_trace_pool(p, launch_flags, ws, x->stream);
+    else if (binary_pool) crt::launch_trace_binary_pool(p, launch_flags, ws, x->stream);
     else crt::launch_trace(p, launch_flags, static_cast<int>(x->cfg.trace_block), x->stream);
     CRT_CUDA(cudaGetLastError());
     CRT_CUDA(cudaEventRecord(x->tev[2], x->stream));
     x->tev_valid = true;
     if (pool && wait)
         x->left_over = [=](uint32_t n) {
-            crt::launch_trace_left(p, launch_flags, ws, n, x->stream);
+            if (n == crt::kWalkAll && (flags & CRT_TRACE_ANY))
+                crt::launch_trace(p, launch_flags & ~CRT_TRACE_COMPRESSED, static_cast<int>(x->cfg.trace_block), x->stream);
+            else
+                crt::launch_trace_left(p, launch_flags, ws, n, x->stream);
             cudaEventRecord(x->tev[2], x->stream);
         };
     return CRT_OK;
@@ -1499,7 +1518,7 @@ crt_status crt_trace(crt_ctx* x, const crt_bvh* b, const crt_ray* rays, uint32_t
         d_hits = x->hits_out.as<crt_hit>();
     }
     CRT_TRY(trace_device(x, b, d_rays, n_rays, flags, d_hits, nullptr, 0, classes_ready, true));
-    CRT_TRY(finish_walk(x));
+    CRT_TRY(finish_walk(x, b));
     if (!dev_out) CRT_CUDA(cudaMemcpyAsync(hits, d_hits, sizeof(crt_hit) * n_rays, cudaMemcpyDeviceToHost, x->stream));
     CRT_TRY(x->check_host_error());
     if (flags & CRT_TRACE_STATS)
@@ -1607,7 +1626,7 @@ crt_status crt_trace_frame(crt_ctx* x, const crt_bvh* b, const crt_camera* cam, 
         p.abs_eps = b->abs_eps;
         p.err = x->hw_dev;
         p.tile_width = tw;
-        CRT_TRY(frame_walk4(x, b, n, &p));
+        CRT_TRY(frame_walk4(x, b, d_cam == cam ? nullptr : cam, n, &p));
         if (flags & CRT_TRACE_STATS) {
             CRT_CUDA(cudaMemsetAsync(x->trace_stats.p, 0, 16, x->stream));
             p.stats = x->trace_stats.as<unsigned long long>();
@@ -1617,7 +1636,7 @@ crt_status crt_trace_frame(crt_ctx* x, const crt_bvh* b, const crt_camera* cam, 
         // One launch for the whole image.  Splitting it into row bands whose
         // hits are copied out on a second stream while the next band runs was
         // measured slower at every band count (2, 4, 8) on GB300.
-        CRT_TRY(frame_launch(x, p, d_cam, width, height, light, d_hs, kflags, nullptr));
+        CRT_TRY(frame_launch(x, b, p, d_cam, width, height, light, d_hs, kflags, nullptr));
         if (!dev_p)
             CRT_CUDA(cudaMemcpyAsync(hits_primary, d_hp, sizeof(crt_hit) * static_cast<size_t>(n), cudaMemcpyDeviceToHost,
                                      x->stream));
@@ -2236,7 +2255,7 @@ crt_status crt_batch_create(crt_ctx* x, const uint32_t* tri_counts, const uint32
     seg[n_scenes] = N;
     bt->tri_off = seg;
     st = CRT_OK;
-    if (cudaMemset(bt->walk.p, 0, 16) != cudaSuccess ||
+    if (cudaMemset(bt->walk.p, 0, crt::kWalkCounterBytes) != cudaSuccess ||
         cudaMemcpy(bt->scenes.p, hs.data(), sizeof(crt::BatchScene) * n_scenes, cudaMemcpyHostToDevice) != cudaSuccess ||
         cudaMemcpy(bt->seg_off.p, seg.data(), 4ull * seg.size(), cudaMemcpyHostToDevice) != cudaSuccess ||
         cudaMemcpy(bt->seg_hist.p, segh.data(), 4ull * 256, cudaMemcpyHostToDevice) != cudaSuccess ||
@@ -2665,14 +2684,14 @@ crt_status crt_render_frame(crt_ctx* x, const crt_bvh* b, const crt_camera* cam,
         crt::TraceParams p = bvh_params(x, b, flags);
         p.n_rays = n;
         p.tile_width = tw;
-        CRT_TRY(frame_walk4(x, b, n, &p));
+        CRT_TRY(frame_walk4(x, b, d_cam == cam ? nullptr : cam, n, &p));
         if (flags & CRT_TRACE_STATS) {
             CRT_CUDA(cudaMemsetAsync(x->trace_stats.p, 0, 16, x->stream));
             p.stats = x->trace_stats.as<unsigned long long>();
         }
         const bool deep = b->depth_bound + 2 > 64;
         const uint32_t kflags = (flags & CRT_TRI_WATERTIGHT) | (deep ? (1u << 16) : 0u);
-        CRT_TRY(frame_launch(x, p, d_cam, width, height, nullptr, nullptr, kflags, &sp));
+        CRT_TRY(frame_launch(x, b, p, d_cam, width, height, nullptr, nullptr, kflags, &sp));
     } else {
         CRT_TRY(x->frame_rays.reserve(sizeof(crt_ray) * static_cast<size_t>(n)));
         CRT_TRY(x->frame_hits.reserve(sizeof(crt_hit) * static_cast<size_t>(n)));

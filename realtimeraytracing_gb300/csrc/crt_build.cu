@@ -1874,7 +1874,7 @@ __device__ __forceinline__ void cwide_node(const float4* __restrict__ wide, uint
             if (k == best) { mn[k] = g0; mx[k] = g1; ref[k] = __float_as_uint(g0.w); }
         mn[c] = g2; mx[c] = g3; ref[c] = __float_as_uint(g1.w);
     }
-    bool ok = abs_eps >= 8.673617379884035e-19f && abs_eps <= 1073741824.f;  // a range of 2^-40 .. 2^50
+    bool ok = walk4_scene(abs_eps);
 #pragma unroll
     for (int c = 0; c < 4; ++c)  // the walk follows references unchecked
         ok = ok && (ref[c] == kNoChild || ((ref[c] & kLeafRef) ? (ref[c] & ~kLeafRef) <= n_internal : ref[c] < n_internal));

@@ -162,28 +162,31 @@ struct TraceParams {
     const uint32_t* order = nullptr;
 };
 void launch_trace(const TraceParams& p, uint32_t flags, int block, cudaStream_t s);
-// Scratch of a persistent walk over the compressed nodes: 16 bytes of counters,
-// zero before its first use and again after each launch, the list of the rays left
-// to the binary walk, and optionally a page-locked word for their number.  With it
-// the caller waits for the launch and then launches the left-over rays itself;
-// without, they are launched right away.  The list holds kWalkLeft rays and is
-// reserved once, with the context or the batch: usually it stays empty, and a
-// launch that would leave more gives up, after which all its rays are walked on the
-// binary nodes in their order.
-constexpr uint32_t kWalkLeft = 65536;
-constexpr size_t kWalkScratchBytes = 16 + 4 * static_cast<size_t>(kWalkLeft);
+// Scratch of a persistent walk over the compressed nodes: its counters, zero before
+// its first use and again after each launch, the list of the rays left to the binary
+// walk, and optionally two page-locked words for their number and the nodes' bad
+// flag.  With them the caller waits for the launch and then launches the left-over
+// rays itself; without, they are launched right away.  The list holds kWalkLeft rays
+// and is reserved once, with the context or the batch: usually it stays empty.  Where
+// more are left, all rays are looked through for marked ones; where most are, and for
+// a frame's pixels, all are walked on the binary nodes (a number of kWalkAll).
+constexpr uint32_t kWalkLeft = 65536, kWalkAll = 0xFFFFFFFFu;
+constexpr size_t kWalkCounterBytes = 32, kWalkScratchBytes = kWalkCounterBytes + 4 * static_cast<size_t>(kWalkLeft);
 struct WalkScratch {
     uint32_t* ctr = nullptr;
     uint32_t* left = nullptr;
     uint32_t* host_left = nullptr;
     WalkScratch() = default;
-    WalkScratch(void* scratch, uint32_t* host) : ctr(static_cast<uint32_t*>(scratch)), left(ctr + 4), host_left(host) {}
+    WalkScratch(void* scratch, uint32_t* host) : ctr(static_cast<uint32_t*>(scratch)), left(ctr + kWalkCounterBytes / 4), host_left(host) {}
 };
 // Many rays by persistent warps that refill finished lanes from a ray counter;
 // compressed nodes, no seeding, rays in caller order or p.order.  launch_trace_left:
-// the n rays such a launch left over (all of them above kWalkLeft).
+// the n rays such a launch left over.
 void launch_trace_pool(const TraceParams& p, uint32_t flags, const WalkScratch& w, cudaStream_t s);
 void launch_trace_left(const TraceParams& p, uint32_t flags, const WalkScratch& w, uint32_t n, cudaStream_t s);
+// The closest hits of many rays by persistent warps over the binary nodes, in caller
+// order or p.order (w: its counters).
+void launch_trace_binary_pool(const TraceParams& p, uint32_t flags, const WalkScratch& w, cudaStream_t s);
 
 // Shading (getColor + imageStore) inputs; the BVH, leaf records and error
 // word come from the TraceParams it runs with.

@@ -230,7 +230,7 @@ __global__ void __launch_bounds__(kWalk4Block, kWalk4Blocks)
             redo = redo || L.redo;
             if (valid && !redo) reinterpret_cast<uint4*>(f.hits_shadow)[i] = L.hit();
         }
-        walk4_leave(ctr, left, valid && redo, i, tiles);
+        walk4_leave<false>(ctr, left, valid && redo, i, tiles);
         uint32_t next = tiles;
         if (tiles > warps) {
             if (lane == 0) next = atomicAdd(&ctr->taken, 1u);
@@ -243,7 +243,7 @@ __global__ void __launch_bounds__(kWalk4Block, kWalk4Blocks)
         atomicAdd(p.stats + 0, static_cast<unsigned long long>(L.fetched));
         atomicAdd(p.stats + 1, static_cast<unsigned long long>(L.tested));
     }
-    walk4_finish(ctr, host_left);
+    walk4_finish(ctr, host_left, p.cw_bad);
 }
 
 template <bool WT, int STACK, bool SHADE>

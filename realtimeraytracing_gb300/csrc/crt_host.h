@@ -1,9 +1,16 @@
 // Host-side rules of libcrt that need neither CUDA nor a GPU, apart so that a
-// plain C++ program can check them.
+// plain C++ program can check them (what kernels use too is CRT_HOST_DEVICE).
 #pragma once
 
+#include <cmath>
 #include <cstdint>
 #include <mutex>
+
+#ifdef __CUDACC__
+#define CRT_HOST_DEVICE __host__ __device__
+#else
+#define CRT_HOST_DEVICE
+#endif
 
 namespace crt {
 
@@ -98,5 +105,21 @@ struct PlocGrids {
 // path.  That path reads the first clusters, records and look-back words, so only
 // while no kernel that changes them has been enqueued.
 constexpr bool may_start_over(bool not_supported, bool enqueued) { return not_supported && !enqueued; }
+
+// What the walk over the compressed nodes takes (crt_walk4.cuh), as far as the host
+// can tell before a launch; each of these refuses every ray of a scene or an image,
+// which then goes to the binary nodes at once instead of by way of the left-over
+// list.  A scene's range (its largest coordinate or extent) is abs_eps * 2^20.
+// Nodes are quantised for ranges of 2^-40 .. 2^50:
+CRT_HOST_DEVICE constexpr bool walk4_scene(float abs_eps) {
+    return abs_eps >= 8.673617379884035e-19f && abs_eps <= 1073741824.f;
+}
+// Camera rays: origins within 8 ranges, ranges within 2^20 of the unit directions
+// (whose largest component is at least 0.57).
+inline bool walk4_camera(const float eye[3], float abs_eps) {
+    const float range = abs_eps * 1048576.f;
+    return std::fabs(eye[0]) <= 8.f * range && std::fabs(eye[1]) <= 8.f * range && std::fabs(eye[2]) <= 8.f * range &&
+           range <= 1048576.f && range * 1048576.f >= 0.5f;
+}
 
 }  // namespace crt

@@ -8,6 +8,7 @@
 
 #include "crt_build.cuh"
 #include "crt_common.cuh"
+#include "crt_pool.cuh"
 #include "crt_traverse.cuh"
 #include "crt_walk4.cuh"
 
@@ -199,6 +200,28 @@ static void launch_trace_t(const TraceParams& p, int block, bool deep, bool seed
     else launch_trace_b<ANY, WT, 128>(p, deep, seed, walk, s);
 }
 
+// trace_pool_kernel over the n rays left over (*count of them, if given), or over all
+// rays (kWalkAll).
+template <bool WT, int STACK, bool BATCH>
+static void launch_pool_s(const TraceParams& p, const WalkScratch& w, const uint32_t* count, uint32_t n,
+                          const BatchScene* scenes, uint32_t n_scenes, cudaStream_t s) {
+    static const uint32_t grid = [] {
+        int per_sm = 0;
+        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, trace_pool_kernel<WT, STACK, BATCH>, kWalk4Block, 0);
+        return static_cast<uint32_t>(kNumSms * (per_sm > 0 ? per_sm : 1));
+    }();
+    const uint32_t items = count || n > kWalkLeft ? p.n_rays : n;
+    trace_pool_kernel<WT, STACK, BATCH><<<std::min((items - 1) / kWalk4Block + 1, grid), kWalk4Block, 0, s>>>(
+        p, reinterpret_cast<Walk4Counters*>(w.ctr), count, n, w.left, scenes, n_scenes);
+}
+
+template <bool WT, bool BATCH>
+static void launch_pool(const TraceParams& p, bool deep, const WalkScratch& w, const uint32_t* count, uint32_t n,
+                        const BatchScene* scenes, uint32_t n_scenes, cudaStream_t s) {
+    if (deep) launch_pool_s<WT, 1024, BATCH>(p, w, count, n, scenes, n_scenes, s);
+    else launch_pool_s<WT, 64, BATCH>(p, w, count, n, scenes, n_scenes, s);
+}
+
 template <bool ANY, bool WT, bool BATCH>
 static void launch_walk4_t(const TraceParams& p, bool deep, const WalkScratch& w, uint32_t left, const BatchScene* scenes,
                            uint32_t n_scenes, cudaStream_t s) {
@@ -216,8 +239,14 @@ static void launch_walk4_t(const TraceParams& p, bool deep, const WalkScratch& w
         if (w.host_left) return;
     }
     const uint32_t* count = left == 0 ? &ctr->last_left : nullptr;
+    if (!ANY) {
+        launch_pool<WT, BATCH>(p, deep, w, count, left, scenes, n_scenes, s);
+        return;
+    }
+    // a thread an item where their number is known
     const uint32_t items = left == 0 || left > kWalkLeft ? p.n_rays : left;
-    const uint32_t few = std::min((items - 1) / kWalk4Block + 1, static_cast<uint32_t>(kNumSms * 16));
+    const uint32_t full = (items - 1) / kWalk4Block + 1;
+    const uint32_t few = left == 0 ? std::min(full, static_cast<uint32_t>(kNumSms * 16)) : full;
     if (deep) walk4_left_kernel<ANY, WT, 1024, BATCH><<<few, kWalk4Block, 0, s>>>(p, count, left, w.left, scenes, n_scenes);
     else walk4_left_kernel<ANY, WT, 64, BATCH><<<few, kWalk4Block, 0, s>>>(p, count, left, w.left, scenes, n_scenes);
 }
@@ -238,6 +267,13 @@ void launch_trace_pool(const TraceParams& p, uint32_t flags, const WalkScratch& 
 
 void launch_trace_left(const TraceParams& p, uint32_t flags, const WalkScratch& w, uint32_t n, cudaStream_t s) {
     if (n != 0) launch_walk4<false>(p, flags, (flags >> 16) != 0, w, n, nullptr, 0, s);
+}
+
+void launch_trace_binary_pool(const TraceParams& p, uint32_t flags, const WalkScratch& w, cudaStream_t s) {
+    if (p.n_rays == 0) return;
+    const bool deep = (flags >> 16) != 0;
+    if (flags & CRT_TRI_WATERTIGHT) launch_pool<true, false>(p, deep, w, nullptr, kWalkAll, nullptr, 0, s);
+    else launch_pool<false, false>(p, deep, w, nullptr, kWalkAll, nullptr, 0, s);
 }
 
 void launch_trace_batch_pool(const TraceParams& p, const BatchScene* scenes, uint32_t n_scenes, uint32_t flags,

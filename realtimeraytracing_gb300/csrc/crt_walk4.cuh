@@ -396,18 +396,26 @@ __device__ __forceinline__ uint32_t walk4_run(Walk4Lane& L, uint32_t s_base, uin
 
 // A persistent walk's counters in device memory.  The launch's last block zeroes
 // them for the next one (no clear in between) and hands the number of rays left
-// over (above kWalkLeft they are not all on the list) to the device, last_left, and
-// where given to page-locked host memory, so that a caller that waits for the
-// launch anyway starts walk4_left_kernel only when there are any.
+// over (above kWalkLeft they are not all on the list; kWalkAll: it gave up) to the
+// device, last_left, and where given to page-locked host memory, with the nodes' bad
+// flag after it, so that a caller that waits for the launch anyway starts the kernel
+// for them only when there are any, and knows a scene that cannot be quantised from
+// then on.
 struct Walk4Counters {
-    uint32_t taken, left, blocks, last_left;
+    uint32_t taken, left, blocks, last_left, gave_up, pad[3];
 };
+static_assert(sizeof(Walk4Counters) == kWalkCounterBytes, "walk scratch");
+
 // Puts item i of the lanes with redo on the list of what is left to the binary
-// walk (whole warps; one atomic each).  Once the list overflows the launch's result
-// is not used: limit, the number of items to take, goes into the counter, and every
-// warp finds nothing more to take.
+// walk (whole warps; one atomic each).  An overflowing list makes a launch give up
+// where what it took so far is little use: at once (MARKS false), or where 9 in 16 of
+// the rays taken were left over (4.2 M rays over 4.19 M triangles, all, 3/4, 1/2 and
+// 1/16 of them from far away: 5.9, 6.2, 5.4, 3.9 ms; on the binary nodes from the
+// start 5.9, 5.8, 5.7, 5.6).  The counter then gets the number of items to take, so that every
+// warp finds nothing more to take, and all items are walked on the binary nodes.
+template <bool MARKS>
 __device__ __forceinline__ void walk4_leave(Walk4Counters* ctr, uint32_t* __restrict__ left, bool redo, uint32_t i,
-                                            uint32_t limit) {
+                                            uint32_t items) {
     const uint32_t m = __ballot_sync(0xFFFFFFFFu, redo);
     if (!m) return;
     const uint32_t lane = threadIdx.x & 31u, cnt = static_cast<uint32_t>(__popc(m));
@@ -415,22 +423,43 @@ __device__ __forceinline__ void walk4_leave(Walk4Counters* ctr, uint32_t* __rest
     uint32_t base = 0;
     if (lane == static_cast<uint32_t>(leader)) {
         base = atomicAdd(&ctr->left, cnt);
-        if (base + cnt > kWalkLeft) atomicMax(&ctr->taken, limit);
+        if (base >= kWalkLeft) {
+            const uint32_t taken = *reinterpret_cast<volatile uint32_t*>(&ctr->taken);
+            if (!MARKS || (base >= taken / 2u + taken / 16u && taken < items)) {
+                atomicMax(&ctr->taken, items);
+                *reinterpret_cast<volatile uint32_t*>(&ctr->gave_up) = 1u;
+            }
+        }
     }
     base = __shfl_sync(0xFFFFFFFFu, base, leader);
     const uint32_t k = base + static_cast<uint32_t>(__popc(m & ((1u << lane) - 1u)));
     if (redo && k < kWalkLeft) left[k] = i;
 }
-__device__ __forceinline__ void walk4_finish(Walk4Counters* ctr, uint32_t* host_left) {
+
+// The hit record of a ray that was left over, until the binary walk writes its hit
+// (a miss otherwise has a distance of 0): where the rays left are more than the list
+// holds, these marks are what names them.
+constexpr uint32_t kLeftMark = 0x7FFFFFFFu;
+__device__ __forceinline__ uint4 left_mark() { return make_uint4(CRT_MISS, kLeftMark, 0u, 0u); }
+__device__ __forceinline__ bool left_marked(const crt_hit* hits, uint32_t i) {
+    const uint2 h = *reinterpret_cast<const uint2*>(hits + i);
+    return h.x == CRT_MISS && h.y == kLeftMark;
+}
+
+__device__ __forceinline__ void walk4_finish(Walk4Counters* ctr, uint32_t* host_left, const uint32_t* bad) {
     __syncthreads();
     if (threadIdx.x != 0) return;
     __threadfence();
     if (atomicInc(&ctr->blocks, gridDim.x - 1) != gridDim.x - 1) return;
     __threadfence();
-    const uint32_t n = atomicExch(&ctr->left, 0u);
+    const uint32_t listed = atomicExch(&ctr->left, 0u);
+    const uint32_t n = atomicExch(&ctr->gave_up, 0u) != 0u ? kWalkAll : listed;
     ctr->taken = 0u;
     ctr->last_left = n;
-    if (host_left) *reinterpret_cast<volatile uint32_t*>(host_left) = n;
+    if (host_left) {
+        reinterpret_cast<volatile uint32_t*>(host_left)[0] = n;
+        reinterpret_cast<volatile uint32_t*>(host_left)[1] = *bad;
+    }
 }
 
 // Persistent warps over a ray pool, one ray per lane; lanes whose ray is done take
@@ -449,7 +478,7 @@ __device__ __forceinline__ void walk4_finish(Walk4Counters* ctr, uint32_t* host_
 // 0.36 without).
 //
 // Rays the compressed walk cannot take (walk4_setup, unquantised scenes, one-leaf
-// trees, walks deeper than the stack) go to the list `left` for walk4_left_kernel.
+// trees, walks deeper than the stack) go to the list `left` and are marked.
 // ctr (Walk4Counters, zero between launches): the rays taken and left.
 template <bool ANY, bool WT, bool BATCH>
 __global__ void __launch_bounds__(kWalk4Block, kWalk4Blocks)
@@ -508,18 +537,18 @@ __global__ void __launch_bounds__(kWalk4Block, kWalk4Blocks)
         if (__all_sync(0xFFFFFFFFu, i == kDone)) break;
         const uint32_t om = walk4_run<ANY, WT, kWalk4Flush>(L, s_base, st, pool_left ? kWalk4Refill : 32);
         const bool done = (om >> lane & 1u) && i < kDone;
-        walk4_leave(ctr, left, done && L.redo, i, p.n_rays);
+        walk4_leave<true>(ctr, left, done && L.redo, i, p.n_rays);
         if (done) {
-            if (!L.redo) reinterpret_cast<uint4*>(p.hits)[i] = L.hit();
+            reinterpret_cast<uint4*>(p.hits)[i] = L.redo ? left_mark() : L.hit();
             i = kIdle;
         }
     }
-    walk4_finish(ctr, host_left);
+    walk4_finish(ctr, host_left, p.cw_bad);
 }
 
-// The binary walk of the rays a trace_walk4_kernel launch left over (few or none):
-// n of them, or as many as *count says; all rays if they are more than the list
-// holds.
+// The binary walk of the any-hit rays a trace_walk4_kernel launch left over, a thread
+// each: n of them, or as many as *count says; where they are more than the list holds,
+// all rays are looked at for marks (kWalkAll: all are walked).  Closest hits: trace_pool_kernel (crt_pool.cuh).
 template <bool ANY, bool WT, int STACK, bool BATCH>
 __global__ void __launch_bounds__(kWalk4Block)
     walk4_left_kernel(const TraceParams p, const uint32_t* __restrict__ count, uint32_t n,
@@ -531,6 +560,7 @@ __global__ void __launch_bounds__(kWalk4Block)
          k += static_cast<uint64_t>(gridDim.x) * kWalk4Block) {
         const uint32_t i = !all ? left[k] : p.order ? __ldg(p.order + k) : static_cast<uint32_t>(k);
         if (i >= p.n_rays) { raise_corrupt(p.err, 7, static_cast<uint32_t>(k), i); continue; }
+        if (all && n != kWalkAll && !left_marked(p.hits, i)) continue;
         TraceParams q = p;
         if (BATCH) {
             uint32_t lo = 0, hi = n_scenes - 1;

@@ -1,8 +1,9 @@
 """Rays and pixels that the walk over the compressed nodes leaves to the binary
 walk: their list is reserved with the context or the batch, so a first call
-allocates nothing however many rays there are to a triangle, and a launch that
-would leave more than the list holds (65,536) walks all its rays on the binary
-nodes.  None, one, about as many as fit, and all of the rays are left over, in
+allocates nothing however many rays there are to a triangle; more rays than the
+list holds (65,536) are found by their marks, and a launch that leaves most of its
+rays gives up and walks all on the binary nodes.  None, one, about as many as fit,
+three quarters and all of the rays are left over, in
 caller and sorted order, by traces, frames and batches; hits against one thread
 per ray on the binary nodes, bit for bit."""
 import numpy as np
@@ -28,7 +29,7 @@ def far_rays(n, n_far, seed):
 
 
 @pytest.mark.parametrize("flags", [crt.TRI_WATERTIGHT, crt.TRI_REFERENCE, crt.TRI_WATERTIGHT | crt.TRACE_ANY])
-@pytest.mark.parametrize("n_far", [0, 1, LISTED - 1, LISTED, LISTED + 1, N_RAYS])
+@pytest.mark.parametrize("n_far", [0, 1, LISTED - 1, LISTED, LISTED + 1, 150001, N_RAYS])
 def test_any_number_left_over(ctx, n_far, flags):
     tris = S.uniform_soup(3000, seed=61)
     bvh = ctx.build(tris, models=S.identity_models(1))
@@ -57,7 +58,7 @@ def test_frames_from_near_and_far(ctx, w, h, z):
 
 
 @pytest.mark.parametrize("flags", [crt.TRI_WATERTIGHT, crt.TRI_WATERTIGHT | crt.TRACE_ANY])
-@pytest.mark.parametrize("n_far", [1, LISTED, LISTED + 1, N_RAYS])
+@pytest.mark.parametrize("n_far", [1, LISTED, LISTED + 1, 150001, N_RAYS])
 def test_batches(ctx, n_far, flags):
     torch = pytest.importorskip("torch")
     tris = [S.uniform_soup(n, seed=n) for n in (700, 1, 3001)]

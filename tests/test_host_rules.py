@@ -129,3 +129,36 @@ int main() {
     return 0;
 }
 ''')
+
+
+def test_scenes_and_cameras_the_compressed_walk_refuses(tmp_path):
+    """The bounds, from both sides; what is not a number is refused."""
+    run_cpp(tmp_path, r'''
+#include <limits>
+int main() {
+    const float inf = std::numeric_limits<float>::infinity(), nan = std::nanf("");
+    const float lo = std::ldexp(1.f, -60), hi = std::ldexp(1.f, 30);
+    CHECK(crt::walk4_scene(lo) && crt::walk4_scene(hi) && crt::walk4_scene(1e-6f));
+    CHECK(!crt::walk4_scene(std::nextafter(lo, 0.f)) && !crt::walk4_scene(std::nextafter(hi, inf)));
+    CHECK(!crt::walk4_scene(inf) && !crt::walk4_scene(nan) && !crt::walk4_scene(0.f));
+    const float eps = std::ldexp(3.f, -20);  // a scene of range 3
+    for (int a = 0; a < 3; ++a)
+        for (float sign : {1.f, -1.f}) {
+            float e[3] = {0.5f, 0.5f, -1.5f};
+            CHECK(crt::walk4_camera(e, eps));
+            e[a] = sign * 24.f;
+            CHECK(crt::walk4_camera(e, eps));
+            e[a] = sign * std::nextafter(24.f, inf);
+            CHECK(!crt::walk4_camera(e, eps));
+            e[a] = sign * inf;
+            CHECK(!crt::walk4_camera(e, eps));
+            e[a] = nan;
+            CHECK(!crt::walk4_camera(e, eps));
+        }
+    const float o[3] = {0.f, 0.f, 0.f};
+    CHECK(crt::walk4_camera(o, 1.f) && !crt::walk4_camera(o, std::nextafter(1.f, inf)));  // range 2^20
+    CHECK(crt::walk4_camera(o, std::ldexp(1.f, -41)) && !crt::walk4_camera(o, std::nextafter(std::ldexp(1.f, -41), 0.f)));
+    CHECK(!crt::walk4_camera(o, nan) && !crt::walk4_camera(o, inf));
+    return 0;
+}
+''')
