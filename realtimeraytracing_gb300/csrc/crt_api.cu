@@ -1963,7 +1963,7 @@ struct crt_batch {
     DevBuf node_box, node_kids, pf, clus_a, clus_b, it, ploc_lb, hist, sort_lb;
     DevBuf nodes, wide, wide_wt, depth_odd, xtri, xtri_sorted, inv_perm;
     DevBuf ray_order, ray_order_scratch;  // CRT_TRACE_SORT_RAYS
-    DevBuf cwide;                         // compressed 4-wide nodes (and their bad flag) of the scenes' current trees
+    DevBuf cwide;                         // compressed 4-wide nodes of the scenes' current trees, and a bad flag a scene
     bool cwide_ready = false;
     bool g_cwide = false;                 // the captured graph derives them
     uint32_t* cw_bad() const { return reinterpret_cast<uint32_t*>(cwide.as<char>() + 64ull * n_tris); }
@@ -2235,7 +2235,7 @@ crt_status crt_batch_create(crt_ctx* x, const uint32_t* tri_counts, const uint32
     R(bt->node_kids, 16ull * N);
     R(bt->node_box, 32ull * (2ull * N));
     R(bt->walk, crt::kWalkScratchBytes);
-    R(bt->cwide, 64ull * N + 16);
+    R(bt->cwide, 64ull * N + 4ull * n_scenes);
     R(bt->pf, 8ull * N);
     R(bt->clus_a, 32ull * N);
     R(bt->clus_b, 32ull * N);

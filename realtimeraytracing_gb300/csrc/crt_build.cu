@@ -1943,7 +1943,7 @@ __global__ void __launch_bounds__(256) cwide_batch_kernel(const float4* __restri
     const uint32_t i = j - sc.tri_off;
     if (i + 1 >= sc.n_tris) return;
     const size_t base = 4 * static_cast<size_t>(sc.wide_off);
-    cwide_node(wide + base, i, sc.n_tris - 1, sc.abs_eps, cwide + base, bad);
+    cwide_node(wide + base, i, sc.n_tris - 1, sc.abs_eps, cwide + base, bad + lo);
 }
 
 void launch_cwide(const float4* wide, uint32_t n_internal, float abs_eps, uint4* cwide, uint32_t* bad, cudaStream_t s) {
@@ -1954,7 +1954,7 @@ void launch_cwide(const float4* wide, uint32_t n_internal, float abs_eps, uint4*
 
 void launch_cwide_batch(const float4* wide, const BatchScene* scenes, uint32_t n_scenes, uint32_t n_total, uint4* cwide,
                         uint32_t* bad, cudaStream_t s) {
-    cudaMemsetAsync(bad, 0, 4, s);
+    cudaMemsetAsync(bad, 0, 4ull * n_scenes, s);
     cwide_batch_kernel<<<(n_total + 255) / 256, 256, 0, s>>>(wide, scenes, n_scenes, n_total, cwide, bad);
 }
 

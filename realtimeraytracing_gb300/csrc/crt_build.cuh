@@ -143,7 +143,8 @@ struct TraceParams {
                              // traces: boxes already grown by abs_eps)
     const float4* wide4;     // 128-B 4-wide traversal nodes (even-depth internal nodes)
     const uint4* cwide = nullptr;  // 64-B compressed 4-wide traversal nodes (same indices)
-    const uint32_t* cw_bad = nullptr;  // nonzero: some box of cwide could not be quantised (walk the binary nodes)
+    const uint32_t* cw_bad = nullptr;  // nonzero: some box of cwide could not be quantised (walk the binary nodes);
+                                       // one flag, or one a scene of a batch
     const float4* xtri;      // 3 float4 per leaf (tree order): transformed p0 | tri id, p1 | model id, p2
     const crt_ray* rays;
     crt_hit* hits;
@@ -234,7 +235,7 @@ struct BatchScene {
 static_assert(sizeof(BatchScene) == 48, "batch scene record");
 void launch_trace_batch(const TraceParams& p, const BatchScene* scenes, uint32_t n_scenes, uint32_t n_rays,
                         uint32_t flags, int block, bool deep, cudaStream_t s);
-// The same nodes for every scene of a batch of n_total triangles.
+// The same nodes for every scene of a batch of n_total triangles; bad: a flag a scene.
 void launch_cwide_batch(const float4* wide, const struct BatchScene* scenes, uint32_t n_scenes, uint32_t n_total,
                         uint4* cwide, uint32_t* bad, cudaStream_t s);
 // The persistent ray pool over a batch: no seeding; p holds the batch's node

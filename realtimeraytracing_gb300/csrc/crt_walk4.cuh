@@ -494,14 +494,13 @@ __global__ void __launch_bounds__(kWalk4Block, kWalk4Blocks)
     }
     const uint32_t lane = threadIdx.x & 31u;
     const uint32_t s_base = static_cast<uint32_t>(__cvta_generic_to_shared(&s_st[1][threadIdx.x]));
-    const bool quantised = __ldg(p.cw_bad) == 0u;
     uint2 st[kWalk4Local];
     Walk4Lane L{};
     L.cw = p.cwide;
     L.xtri = p.xtri;
     L.abs_eps = p.abs_eps;
     L.stop(s_base);
-    bool walkable = quantised && p.n_nodes > 2;
+    bool walkable = !BATCH && __ldg(p.cw_bad) == 0u && p.n_nodes > 2;
     uint32_t i = kIdle;
     bool pool_left = true;
     while (true) {
@@ -521,11 +520,12 @@ __global__ void __launch_bounds__(kWalk4Block, kWalk4Blocks)
                     i = kIdle;
                 } else {
                     if (BATCH) {
-                        const BatchScene bs = scenes[batch_scene_of(s_ray_off, n_scenes, i)];
+                        const uint32_t k_scene = batch_scene_of(s_ray_off, n_scenes, i);
+                        const BatchScene bs = scenes[k_scene];
                         L.cw = p.cwide + 4 * static_cast<size_t>(bs.wide_off);
                         L.xtri = p.xtri + 3 * static_cast<size_t>(bs.tri_off);
                         L.abs_eps = bs.abs_eps;
-                        walkable = quantised && bs.n_tris > 1;
+                        walkable = __ldg(p.cw_bad + k_scene) == 0u && bs.n_tris > 1;
                     }
                     const float4 r0 = __ldg(reinterpret_cast<const float4*>(p.rays + i));
                     const float4 r1 = __ldg(reinterpret_cast<const float4*>(p.rays + i) + 1);
