@@ -409,10 +409,12 @@ static_assert(sizeof(Walk4Counters) == kWalkCounterBytes, "walk scratch");
 // Puts item i of the lanes with redo on the list of what is left to the binary
 // walk (whole warps; one atomic each).  An overflowing list makes a launch give up
 // where what it took so far is little use: at once (MARKS false), or where 9 in 16 of
-// the rays taken were left over (4.2 M rays over 4.19 M triangles, all, 3/4, 1/2 and
-// 1/16 of them from far away: 5.9, 6.2, 5.4, 3.9 ms; on the binary nodes from the
-// start 5.9, 5.8, 5.7, 5.6).  The counter then gets the number of items to take, so that every
-// warp finds nothing more to take, and all items are walked on the binary nodes.
+// the first quarter of the rays were left over.  4.2 M rays over 4.19 M triangles,
+// 1/64, 1/16, 1/4, 1/2, 3/4 and all of them from far away, in runs of neighbours: 3.4,
+// 3.9, 4.3, 5.4, 6.2, 5.9 ms (every other one: 6.2); on the binary nodes from the
+// start 5.6 to 5.9.  Giving up from 7 in 16 on costs the half 0.8 ms, later than the
+// first quarter up to 2 ms.  On giving up the counter gets the number of items to
+// take, so that every warp finds nothing more to take.
 template <bool MARKS>
 __device__ __forceinline__ void walk4_leave(Walk4Counters* ctr, uint32_t* __restrict__ left, bool redo, uint32_t i,
                                             uint32_t items) {
@@ -425,7 +427,7 @@ __device__ __forceinline__ void walk4_leave(Walk4Counters* ctr, uint32_t* __rest
         base = atomicAdd(&ctr->left, cnt);
         if (base >= kWalkLeft) {
             const uint32_t taken = *reinterpret_cast<volatile uint32_t*>(&ctr->taken);
-            if (!MARKS || (base >= taken / 2u + taken / 16u && taken < items)) {
+            if (!MARKS || (base >= taken / 2u + taken / 16u && taken < items / 4u)) {
                 atomicMax(&ctr->taken, items);
                 *reinterpret_cast<volatile uint32_t*>(&ctr->gave_up) = 1u;
             }
