@@ -44,29 +44,21 @@ crt_status fail(crt_status s, const char* fmt, ...) {
         if (s_ != CRT_OK) return s_;   \
     } while (0)
 
-struct DevBuf {
-    void* p = nullptr;
-    size_t cap = 0;
+struct CudaMemory {
+    static void* alloc(size_t bytes) {
+        void* p = nullptr;
+        if (cudaMalloc(&p, bytes) == cudaSuccess) return p;
+        cudaGetLastError();  // a refused allocation is reported where it is an error
+        return nullptr;
+    }
+    static void free(void* p) { cudaFree(p); }
+};
+
+struct DevBuf : crt::GrowingBuffer<CudaMemory> {
     crt_status reserve(size_t bytes) {
-        if (bytes <= cap) return CRT_OK;
-        if (p) cudaFree(p);
-        p = nullptr;
-        cap = 0;
-        const size_t want = bytes + bytes / 8 + 256;
-        cudaError_t e = cudaMalloc(&p, want);
-        if (e != cudaSuccess) {
-            p = nullptr;
-            return fail(CRT_ERR_OOM, "cudaMalloc(%zu) failed: %s", want, cudaGetErrorString(e));
-        }
-        cap = want;
+        if (!try_reserve(bytes)) return fail(CRT_ERR_OOM, "cudaMalloc(%zu) failed: out of memory", wanted(bytes));
         return CRT_OK;
     }
-    void release() {
-        if (p) cudaFree(p);
-        p = nullptr;
-        cap = 0;
-    }
-    template <class T> T* as() const { return static_cast<T*>(p); }
 };
 
 bool is_device_ptr(const void* ptr) {
@@ -142,6 +134,7 @@ struct crt_bvh {
         cudaEvent_t done = nullptr;  // after the derivation, on the stream it was enqueued on
     };
     mutable Derivation wide4_nodes, cwide_nodes, node_boxes;
+    static size_t cwide_bytes(uint32_t n) { return 64ull * n + 16; }
     uint32_t* cw_bad() const { return reinterpret_cast<uint32_t*>(cwide.as<char>() + 64ull * n); }
     mutable std::atomic<uint64_t> frame_pixels{0};  // pixels of the frames of the current tree
     // Every leaf's box is its triangle's and lies inside its ancestors', as after a
@@ -157,6 +150,7 @@ struct crt_bvh {
     // A box of the current tree's compressed nodes could not be quantised (a launch
     // over them has said so): the walk over them would leave every ray over.
     mutable std::atomic<bool> unquantised{false};
+    mutable std::atomic<bool> no_cwide{false};  // no memory for them
     // The tree has changed: what was derived from it no longer holds.
     void changed(bool by_refit) {
         wide4_nodes.state.reset();
@@ -164,6 +158,7 @@ struct crt_bvh {
         node_boxes.state.reset();
         frame_pixels = 0;
         unquantised = false;
+        no_cwide = false;
         refitted = by_refit;
     }
     // Sorted Morton codes and permutation exist (a tree from crt_bvh_from_nodes has none).
@@ -582,11 +577,13 @@ crt_status build_impl(crt_ctx* x, crt_bvh* b, const crt_triangle* tris, uint32_t
     b->changed(false);
     b->refit_ready = false;
     b->own_boxes = true;
-    CRT_TRY(b->cwide.reserve(64ull * N + 16));  // derived by the first trace that walks them, which then allocates nothing
     CRT_TRY(b->depth_odd.reserve(N));
     CRT_TRY(b->inv_perm.reserve(4ull * N));
     CRT_TRY(b->codes.reserve(4ull * N));
     CRT_TRY(b->perm.reserve(4ull * N));
+    // the compressed nodes, so that the first trace that derives them allocates
+    // nothing; where memory is short the tree does without (walk4_ready)
+    b->cwide.try_reserve(b->cwide_bytes(N));
 
     CRT_TRY(stage_model_matrices(x, models, n_models));
     const float* d_models = x->models.as<float>();
@@ -796,7 +793,7 @@ crt_status ensure_wide4(crt_ctx* x, const crt_bvh* b) {
 crt_status ensure_cwide(crt_ctx* x, const crt_bvh* b) {
     if (b->n <= 1) return CRT_OK;
     return use_derived(x, b->cwide_nodes, [&]() -> crt_status {
-        CRT_TRY(b->cwide.reserve(64ull * b->n + 16));
+        CRT_TRY(b->cwide.reserve(b->cwide_bytes(b->n)));
         crt::launch_cwide(b->wide.as<float4>(), b->n - 1, b->abs_eps, b->cwide.as<uint4>(), b->cw_bad(), x->stream);
         return CRT_OK;
     });
@@ -804,7 +801,18 @@ crt_status ensure_cwide(crt_ctx* x, const crt_bvh* b) {
 
 // Whether the walk over b's compressed nodes can take rays at all, as far as known.
 bool walk4_usable(const crt_bvh* b) {
-    return b->n > 1 && b->own_boxes && !b->unquantised && crt::walk4_scene(b->abs_eps);
+    return b->n > 1 && b->own_boxes && !b->unquantised && !b->no_cwide && crt::walk4_scene(b->abs_eps);
+}
+
+// The same with the nodes derived; a tree that there is no memory for them for is
+// walked on its binary nodes (until it changes).
+crt_status walk4_ready(crt_ctx* x, const crt_bvh* b, bool* ready) {
+    *ready = false;
+    const crt_status st = ensure_cwide(x, b);
+    if (st == CRT_ERR_OOM) b->no_cwide = true;
+    else if (st != CRT_OK) return st;
+    *ready = st == CRT_OK;
+    return CRT_OK;
 }
 
 // Waits for a persistent walk over b issued with host_left and launches the rays it
@@ -831,7 +839,9 @@ crt_status frame_walk4(crt_ctx* x, const crt_bvh* b, const crt_camera* cam, uint
     if (!walk4_usable(b) || (cam && !crt::walk4_camera(cam->eye, b->abs_eps))) return CRT_OK;
     const uint64_t frames = b->frame_pixels += pixels;
     if (!b->cwide_nodes.state.ready() && 4 * frames < b->n) return CRT_OK;
-    CRT_TRY(ensure_cwide(x, b));
+    bool ready;
+    CRT_TRY(walk4_ready(x, b, &ready));
+    if (!ready) return CRT_OK;
     p->cwide = b->cwide.as<uint4>();
     p->cw_bad = b->cw_bad();
     return CRT_OK;
@@ -877,9 +887,10 @@ crt_status trace_device(crt_ctx* x, const crt_bvh* b, const crt_ray* d_rays, uin
     // 8x4 tiles, seeded, 4-wide and counting walks keep one thread per ray.
     const bool large = !(flags & (CRT_TRACE_WIDE | CRT_TRACE_PER_RAY_THREADS | CRT_TRACE_USE_PREDICTOR | CRT_TRACE_STATS)) &&
                        !seed_classes && tile_width == 0 && n_rays >= kPoolMinRays && b->n > 1;
-    const bool pool = large && walk4_usable(b);
+    bool pool = large && walk4_usable(b);
+    if (flags & CRT_TRACE_COMPRESSED) CRT_TRY(ensure_cwide(x, b));
+    else if (pool) CRT_TRY(walk4_ready(x, b, &pool));
     const bool binary_pool = large && !pool && !(flags & (CRT_TRACE_ANY | CRT_TRACE_COMPRESSED));
-    if (pool || (flags & CRT_TRACE_COMPRESSED)) CRT_TRY(ensure_cwide(x, b));
     x->tev_valid = false;
     CRT_CUDA(cudaEventRecord(x->tev[0], x->stream));
     crt::TraceParams p{};
@@ -1188,7 +1199,7 @@ crt_status crt_bvh_from_nodes(crt_ctx* x, const crt_bvh_node* nodes, uint32_t n_
     crt_status st = CRT_OK;
     if ((st = b->nodes.reserve(sizeof(crt_bvh_node) * n_nodes)) != CRT_OK || (st = b->xtri.reserve(48ull * N)) != CRT_OK ||
         (st = b->wide.reserve(64ull * n_int_alloc)) != CRT_OK || (st = b->wide_wt.reserve(64ull * n_int_alloc)) != CRT_OK ||
-        (st = b->cwide.reserve(64ull * N + 16)) != CRT_OK || (st = b->depth_odd.reserve(n_int_alloc)) != CRT_OK || (st = b->inv_perm.reserve(4ull * N)) != CRT_OK)
+        (st = b->depth_odd.reserve(n_int_alloc)) != CRT_OK || (st = b->inv_perm.reserve(4ull * N)) != CRT_OK)
         return fail_free(st);
     // staging: idx (n_nodes) | int_pos (N-1) | leaf counts (N-1, uint2) | leaf_pos (N) | loose flag, each part
     // starting on a 256-byte boundary (the uint2 loads need 8-byte alignment)
@@ -1197,6 +1208,7 @@ crt_status crt_bvh_from_nodes(crt_ctx* x, const crt_bvh_node* nodes, uint32_t n_
                  o_leaf = up256(o_lc + 8ull * n_int_alloc), o_loose = up256(o_leaf + 4ull * N), bytes = o_loose + 4;
     if ((st = x->opt_scratch.reserve(bytes)) != CRT_OK) return fail_free(st);
     char* base = x->opt_scratch.as<char>();
+    b->cwide.try_reserve(b->cwide_bytes(N));  // as a build does
     if ((st = stage_model_matrices(x, models, n_models)) != CRT_OK) return fail_free(st);
     const crt_triangle* d_tris = tris;
     if (!is_device_ptr(tris)) {
@@ -2054,7 +2066,8 @@ crt_status batch_trace_enqueue(crt_ctx* x, crt_batch* bt, const crt_ray* rays, u
     }
     // large batches: the persistent ray pool, each lane walking its ray's scene
     // (as trace_device does for one scene)
-    if (batch_pool(bt, flags)) {
+    const crt::WalkScratch ws(bt->walk.p, nullptr);
+    if (batch_pool(bt, flags) && bt->cwide.p) {
         if (!bt->cwide_ready)
             crt::launch_cwide_batch(bt->wide.as<float4>(), bt->scenes.as<crt::BatchScene>(), bt->n_scenes, bt->n_tris,
                                     bt->cwide.as<uint4>(), bt->cw_bad(), s);
@@ -2062,9 +2075,10 @@ crt_status batch_trace_enqueue(crt_ctx* x, crt_batch* bt, const crt_ray* rays, u
         p.cwide = bt->cwide.as<uint4>();
         p.cw_bad = bt->cw_bad();
         crt::launch_trace_batch_pool(p, bt->scenes.as<crt::BatchScene>(), bt->n_scenes,
-                                     flags & (CRT_TRACE_ANY | CRT_TRI_WATERTIGHT), deep,
-                                     crt::WalkScratch(bt->walk.p, nullptr), s);
-    } else
+                                     flags & (CRT_TRACE_ANY | CRT_TRI_WATERTIGHT), deep, ws, s);
+    } else if (batch_pool(bt, flags) && !(flags & CRT_TRACE_ANY))
+        crt::launch_trace_batch_binary_pool(p, bt->scenes.as<crt::BatchScene>(), bt->n_scenes, flags, deep, ws, s);
+    else
         crt::launch_trace_batch(p, bt->scenes.as<crt::BatchScene>(), bt->n_scenes, bt->n_rays,
                                 flags & (CRT_TRACE_ANY | CRT_TRI_WATERTIGHT), static_cast<int>(bt->cfg.trace_block), deep,
                                 s);
@@ -2235,7 +2249,6 @@ crt_status crt_batch_create(crt_ctx* x, const uint32_t* tri_counts, const uint32
     R(bt->node_kids, 16ull * N);
     R(bt->node_box, 32ull * (2ull * N));
     R(bt->walk, crt::kWalkScratchBytes);
-    R(bt->cwide, 64ull * N + 4ull * n_scenes);
     R(bt->pf, 8ull * N);
     R(bt->clus_a, 32ull * N);
     R(bt->clus_b, 32ull * N);
@@ -2250,6 +2263,7 @@ crt_status crt_batch_create(crt_ctx* x, const uint32_t* tri_counts, const uint32
     R(bt->xtri, 48ull * N);
     R(bt->xtri_sorted, 48ull * N);
     if (st != CRT_OK) { crt_batch_free(bt); return st; }
+    bt->cwide.try_reserve(64ull * N + 4ull * n_scenes);  // without them its traces walk the binary nodes
     std::vector<uint32_t> seg(n_scenes + 1), segh(256, 0);
     for (uint32_t k = 0; k < n_scenes; ++k) { seg[k] = hs[k].tri_off; segh[k] = hs[k].n_tris; }
     seg[n_scenes] = N;

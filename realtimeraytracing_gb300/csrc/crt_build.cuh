@@ -242,6 +242,9 @@ void launch_cwide_batch(const float4* wide, const struct BatchScene* scenes, uin
 // arrays and p.n_rays the batch's ray count.
 void launch_trace_batch_pool(const TraceParams& p, const BatchScene* scenes, uint32_t n_scenes, uint32_t flags,
                              bool deep, const WalkScratch& w, cudaStream_t s);
+// launch_trace_binary_pool over a batch.
+void launch_trace_batch_binary_pool(const TraceParams& p, const BatchScene* scenes, uint32_t n_scenes, uint32_t flags,
+                                    bool deep, const WalkScratch& w, cudaStream_t s);
 // CRT_TRACE_SORT_RAYS: order[k] = k-th ray by coherence key (origin cell,
 // direction; with scenes, scene first).  scratch: ray_order_scratch_bytes(n).
 size_t ray_order_scratch_bytes(uint32_t n);

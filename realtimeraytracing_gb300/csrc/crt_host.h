@@ -3,6 +3,7 @@
 #pragma once
 
 #include <cmath>
+#include <cstddef>
 #include <cstdint>
 #include <mutex>
 
@@ -51,6 +52,30 @@ private:
     mutable std::mutex mutex_;
     bool ready_ = false;
     uint64_t by_ = 0;  // whose stream the derivation is on
+};
+
+// A device allocation that only grows, by Memory::alloc(size) (null: refused) and
+// Memory::free(p).  Growing drops the contents; a refused one leaves it empty.
+template <class Memory>
+struct GrowingBuffer {
+    void* p = nullptr;
+    size_t cap = 0;
+    // For what a call can do without: refusing it is no error.
+    bool try_reserve(size_t bytes) {
+        if (bytes <= cap) return true;
+        release();
+        const size_t want = wanted(bytes);
+        p = Memory::alloc(want);
+        cap = p ? want : 0;
+        return p != nullptr;
+    }
+    void release() {
+        if (p) Memory::free(p);
+        p = nullptr;
+        cap = 0;
+    }
+    static constexpr size_t wanted(size_t bytes) { return bytes + bytes / 8 + 256; }
+    template <class T> T* as() const { return static_cast<T*>(p); }
 };
 
 // Four page-locked words that a context's kernels raise errors in, so that its

@@ -276,6 +276,13 @@ void launch_trace_binary_pool(const TraceParams& p, uint32_t flags, const WalkSc
     else launch_pool<false, false>(p, deep, w, nullptr, kWalkAll, nullptr, 0, s);
 }
 
+void launch_trace_batch_binary_pool(const TraceParams& p, const BatchScene* scenes, uint32_t n_scenes, uint32_t flags,
+                                    bool deep, const WalkScratch& w, cudaStream_t s) {
+    if (p.n_rays == 0 || n_scenes == 0) return;
+    if (flags & CRT_TRI_WATERTIGHT) launch_pool<true, true>(p, deep, w, nullptr, kWalkAll, scenes, n_scenes, s);
+    else launch_pool<false, true>(p, deep, w, nullptr, kWalkAll, scenes, n_scenes, s);
+}
+
 void launch_trace_batch_pool(const TraceParams& p, const BatchScene* scenes, uint32_t n_scenes, uint32_t flags,
                              bool deep, const WalkScratch& w, cudaStream_t s) {
     if (p.n_rays != 0 && n_scenes != 0) launch_walk4<true>(p, flags, deep, w, 0, scenes, n_scenes, s);

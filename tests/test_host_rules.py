@@ -18,6 +18,7 @@ def run_cpp(tmp_path, body):
 #include <atomic>
 #include <chrono>
 #include <cstdio>
+#include <cstdlib>
 #include <thread>
 #include <vector>
 #define CHECK(c) do { if (!(c)) { std::printf("line %d: %s\\n", __LINE__, #c); return 1; } } while (0)
@@ -159,6 +160,43 @@ int main() {
     CHECK(crt::walk4_camera(o, 1.f) && !crt::walk4_camera(o, std::nextafter(1.f, inf)));  // range 2^20
     CHECK(crt::walk4_camera(o, std::ldexp(1.f, -41)) && !crt::walk4_camera(o, std::nextafter(std::ldexp(1.f, -41), 0.f)));
     CHECK(!crt::walk4_camera(o, nan) && !crt::walk4_camera(o, inf));
+    return 0;
+}
+''')
+
+
+def test_memory_a_call_can_do_without(tmp_path):
+    """A refused optional buffer is no error, stays empty and takes nothing from what was reserved before it; it is
+    there once memory is; growing frees before it allocates."""
+    run_cpp(tmp_path, r'''
+static size_t g_free = 0, g_live = 0;
+struct Budget {
+    static void* alloc(size_t n) {
+        if (n > g_free) return nullptr;
+        size_t* p = static_cast<size_t*>(std::malloc(sizeof(size_t)));
+        *p = n;
+        g_free -= n;
+        ++g_live;
+        return p;
+    }
+    static void free(void* p) { g_free += *static_cast<size_t*>(p); --g_live; std::free(p); }
+};
+using Buf = crt::GrowingBuffer<Budget>;
+int main() {
+    const size_t tree = Buf::wanted(1000), nodes = Buf::wanted(640);
+    g_free = tree + nodes - 1;  // a build that just fits, without the optional nodes
+    Buf a, b;
+    CHECK(a.try_reserve(1000) && a.cap == tree);
+    CHECK(!b.try_reserve(640) && b.p == nullptr && b.cap == 0 && g_live == 1);
+    CHECK(a.p && a.try_reserve(1000) && g_live == 1);  // held, and not allocated again
+    g_free += 1;
+    CHECK(b.try_reserve(640) && b.p && g_free == 0);
+    void* old = b.p;
+    CHECK(b.try_reserve(b.cap) && b.p == old);
+    a.release();
+    CHECK(b.try_reserve(1000) && g_live == 1);  // out of what it and a gave back
+    CHECK(!b.try_reserve(100000) && b.p == nullptr && g_live == 0 && g_free == tree + nodes);
+    b.release();
     return 0;
 }
 ''')
