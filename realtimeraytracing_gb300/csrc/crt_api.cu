@@ -136,7 +136,8 @@ struct crt_bvh {
     mutable Derivation wide4_nodes, cwide_nodes, node_boxes;
     static size_t cwide_bytes(uint32_t n) { return 64ull * n + 16; }
     uint32_t* cw_bad() const { return reinterpret_cast<uint32_t*>(cwide.as<char>() + 64ull * n); }
-    mutable std::atomic<uint64_t> frame_pixels{0};  // pixels of the frames of the current tree
+    // what the current tree's frames and large traces have asked for (crt::Walk4Demand)
+    mutable std::atomic<uint64_t> frame_demand{0}, trace_demand{0};
     // Every leaf's box is its triangle's and lies inside its ancestors', as after a
     // build or a refit; an imported array may hold others, which the walk over the
     // compressed nodes does not look at: such a tree is walked on the binary nodes.
@@ -156,7 +157,8 @@ struct crt_bvh {
         wide4_nodes.state.reset();
         cwide_nodes.state.reset();
         node_boxes.state.reset();
-        frame_pixels = 0;
+        frame_demand = 0;
+        trace_demand = 0;
         unquantised = false;
         no_cwide = false;
         refitted = by_refit;
@@ -831,14 +833,12 @@ crt_status finish_walk(crt_ctx* x, const crt_bvh* b) {
     return CRT_OK;
 }
 
-// One-launch frames walk the compressed nodes once the frames of the current
-// tree have a quarter as many pixels as it has triangles: deriving the nodes
-// takes 0.035 ns per triangle (73 us at 2.0 M) and a pixel gains 0.05-0.2 ns.
+// One-launch frames walk the compressed nodes once the tree's frames pay for them.
 // cam: in host memory, or null where its position is not known here.
 crt_status frame_walk4(crt_ctx* x, const crt_bvh* b, const crt_camera* cam, uint32_t pixels, crt::TraceParams* p) {
     if (!walk4_usable(b) || (cam && !crt::walk4_camera(cam->eye, b->abs_eps))) return CRT_OK;
-    const uint64_t frames = b->frame_pixels += pixels;
-    if (!b->cwide_nodes.state.ready() && 4 * frames < b->n) return CRT_OK;
+    const uint64_t asked = b->frame_demand += crt::Walk4Demand::pixels(pixels);
+    if (!crt::walk4_pays(asked, b->n) && !b->cwide_nodes.state.ready()) return CRT_OK;
     bool ready;
     CRT_TRY(walk4_ready(x, b, &ready));
     if (!ready) return CRT_OK;
@@ -868,8 +868,9 @@ crt_status frame_launch(crt_ctx* x, const crt_bvh* b, const crt::TraceParams& p,
 }
 
 // Enqueues one traversal launch on device-resident rays/hits (no sync).
-constexpr uint32_t kPoolMinRays = 65536;  // below this a launch of one thread per ray fills the GPU as well
-                                          // (measured sides at the kernel, crt_walk4.cuh)
+// Below this a launch of one thread per ray fills the GPU as well; 65,536 rays over
+// 0.26, 2.0 and 4.2 M triangles: 239, 300 and 328 us, one thread a ray 346, 402, 558.
+constexpr uint32_t kPoolMinRays = 65536;
 constexpr uint32_t kChunkedCopyMinRays = 1u << 20;  // crt_trace: smaller host batches copy in one piece
 
 // classes_ready: the predictor's classes of these rays are already in its
@@ -888,8 +889,13 @@ crt_status trace_device(crt_ctx* x, const crt_bvh* b, const crt_ray* d_rays, uin
     const bool large = !(flags & (CRT_TRACE_WIDE | CRT_TRACE_PER_RAY_THREADS | CRT_TRACE_USE_PREDICTOR | CRT_TRACE_STATS)) &&
                        !seed_classes && tile_width == 0 && n_rays >= kPoolMinRays && b->n > 1;
     bool pool = large && walk4_usable(b);
-    if (flags & CRT_TRACE_COMPRESSED) CRT_TRY(ensure_cwide(x, b));
-    else if (pool) CRT_TRY(walk4_ready(x, b, &pool));
+    if (flags & CRT_TRACE_COMPRESSED) {
+        CRT_TRY(ensure_cwide(x, b));
+    } else if (pool) {
+        const uint64_t asked = (flags & CRT_TRACE_ANY) ? crt::Walk4Demand::any(n_rays) : crt::Walk4Demand::closest(n_rays);
+        pool = crt::walk4_pays(b->trace_demand += asked, b->n) || b->cwide_nodes.state.ready();
+        if (pool) CRT_TRY(walk4_ready(x, b, &pool));
+    }
     const bool binary_pool = large && !pool && !(flags & (CRT_TRACE_ANY | CRT_TRACE_COMPRESSED));
     x->tev_valid = false;
     CRT_CUDA(cudaEventRecord(x->tev[0], x->stream));
@@ -1977,6 +1983,7 @@ struct crt_batch {
     DevBuf ray_order, ray_order_scratch;  // CRT_TRACE_SORT_RAYS
     DevBuf cwide;                         // compressed 4-wide nodes of the scenes' current trees, and a bad flag a scene
     bool cwide_ready = false;
+    uint64_t trace_demand = 0;            // what those trees' traces have asked for (crt::Walk4Demand)
     bool g_cwide = false;                 // the captured graph derives them
     uint32_t* cw_bad() const { return reinterpret_cast<uint32_t*>(cwide.as<char>() + 64ull * n_tris); }
     DevBuf walk;                          // the persistent trace's scratch (crt::WalkScratch; counters zero between launches)
@@ -2067,7 +2074,12 @@ crt_status batch_trace_enqueue(crt_ctx* x, crt_batch* bt, const crt_ray* rays, u
     // large batches: the persistent ray pool, each lane walking its ray's scene
     // (as trace_device does for one scene)
     const crt::WalkScratch ws(bt->walk.p, nullptr);
-    if (batch_pool(bt, flags) && bt->cwide.p) {
+    bool walk4 = batch_pool(bt, flags) && bt->cwide.p;
+    if (walk4) {
+        bt->trace_demand += (flags & CRT_TRACE_ANY) ? crt::Walk4Demand::any(bt->n_rays) : crt::Walk4Demand::closest(bt->n_rays);
+        walk4 = bt->cwide_ready || crt::walk4_pays(bt->trace_demand, bt->n_tris);
+    }
+    if (walk4) {
         if (!bt->cwide_ready)
             crt::launch_cwide_batch(bt->wide.as<float4>(), bt->scenes.as<crt::BatchScene>(), bt->n_scenes, bt->n_tris,
                                     bt->cwide.as<uint4>(), bt->cw_bad(), s);
@@ -2106,6 +2118,7 @@ crt_status batch_enqueue(crt_ctx* x, crt_batch* bt, const crt_triangle* tris, co
     const size_t lb_words = static_cast<size_t>(tiles) * 256 + 1;  // per pass (room for 256-digit scene pass)
     uint32_t* err = bt->err.as<uint32_t>();
     bt->cwide_ready = false;
+    bt->trace_demand = 0;
     CRT_CUDA(cudaMemsetAsync(bt->err.p, 0, 16, s));
     CRT_CUDA(cudaMemsetAsync(bt->states.p, 0, crt::batch_box_state_bytes() * bt->n_scenes, s));
     CRT_CUDA(cudaMemsetAsync(bt->hist.p, 0, 4ull * passes * radix, s));

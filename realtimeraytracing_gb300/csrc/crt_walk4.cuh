@@ -475,9 +475,7 @@ __device__ __forceinline__ void walk4_finish(Walk4Counters* ctr, uint32_t* host_
 // triangles 12.7 -> 6.5 ms in caller order (660 -> 1290 Mrays/s), 12.2 -> 7.1
 // in predicted order with its inference and sort; 1.5 M sorted rays over 0.3 M
 // triangles 1.60 -> 1.04 ms.  Any hit, one thread per ray before: 4.2 M rays
-// 6.70 -> 2.69 ms.  Deriving the nodes takes 75 us at 4.19 M triangles, less
-// than the 65,536 rays of the smallest launch gain (0.53 -> 0.43 ms with it,
-// 0.36 without).
+// 6.70 -> 2.69 ms.  Walk4Demand (crt_host.h) says when deriving the nodes pays.
 //
 // Rays the compressed walk cannot take (walk4_setup, unquantised scenes, one-leaf
 // trees, walks deeper than the stack) go to the list `left` and are marked.

@@ -200,3 +200,17 @@ int main() {
     return 0;
 }
 ''')
+
+
+def test_rays_that_pay_for_the_compressed_nodes(tmp_path):
+    run_cpp(tmp_path, r'''
+using D = crt::Walk4Demand;
+int main() {
+    CHECK(crt::walk4_pays(D::closest(65536), 4194304) && !crt::walk4_pays(D::closest(65536), 4194305));
+    CHECK(crt::walk4_pays(D::any(65536), 1048576) && !crt::walk4_pays(D::any(65536), 1048577));
+    CHECK(crt::walk4_pays(D::pixels(262144), 1048576) && !crt::walk4_pays(D::pixels(262143), 1048576));
+    CHECK(!crt::walk4_pays(3 * D::closest(65536), 16777216) && crt::walk4_pays(4 * D::closest(65536), 16777216));
+    CHECK(crt::walk4_pays(D::closest(0xFFFFFFFFull), 0xFFFFFFFFu));  // no overflow at the largest calls
+    return 0;
+}
+''')
