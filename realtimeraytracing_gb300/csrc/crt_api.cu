@@ -887,7 +887,7 @@ crt_status trace_device(crt_ctx* x, const crt_bvh* b, const crt_ray* d_rays, uin
     // those take its rays (closest hits over the binary nodes otherwise); pixels in
     // 8x4 tiles, seeded, 4-wide and counting walks keep one thread per ray.
     const bool large = !(flags & (CRT_TRACE_WIDE | CRT_TRACE_PER_RAY_THREADS | CRT_TRACE_USE_PREDICTOR | CRT_TRACE_STATS)) &&
-                       !seed_classes && tile_width == 0 && n_rays >= kPoolMinRays && b->n > 1;
+                       !seed_classes && tile_width == 0 && n_rays >= kPoolMinRays && n_rays <= crt::kMostPoolItems && b->n > 1;
     bool pool = large && walk4_usable(b);
     if (flags & CRT_TRACE_COMPRESSED) {
         CRT_TRY(ensure_cwide(x, b));

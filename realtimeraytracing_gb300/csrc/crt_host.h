@@ -147,6 +147,14 @@ inline bool walk4_camera(const float eye[3], float abs_eps) {
            range <= 1048576.f && range * 1048576.f >= 0.5f;
 }
 
+// Tiles of `size` items that n items make, for every n that fits.
+CRT_HOST_DEVICE constexpr uint32_t tiles_of(uint32_t n, uint32_t size) { return n / size + (n % size != 0u ? 1u : 0u); }
+
+// Persistent warps take items from a 32-bit counter, which ends up past their number
+// by at most 32 a resident warp (152 SMs of 64 warps): above this bound it could come
+// round to 0 and hand them out again.
+constexpr uint32_t kMostPoolItems = 0xFFF00000u;
+
 // When the rays traced over a tree of n triangles pay for deriving its compressed
 // nodes, which takes 0.035 ns a triangle and 30 us: until then they are walked on the
 // binary nodes.  Rays count from the tree's last change on, so a tree that is traced

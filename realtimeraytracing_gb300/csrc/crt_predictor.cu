@@ -23,6 +23,7 @@
 
 #include "crt_build.cuh"
 #include "crt_common.cuh"
+#include "crt_host.h"
 #include "crt_predictor.cuh"
 #include "crt_tc.cuh"
 
@@ -497,7 +498,9 @@ __global__ void __launch_bounds__(kTrainThreads) train_kernel(PredictorDev P, co
     constexpr uint32_t cW3 = 256, cW2 = 320, cW1 = 384;
     float db3 = 0.f, db2 = 0.f, db1 = 0.f, loss = 0.f;
     bool first = true, ok = true;
-    for (uint32_t tile = blockIdx.x; tile * 128u < n_samples; tile += gridDim.x) {
+    // whole tiles are counted: their first samples would wrap past 2^32 for the largest calls
+    const uint32_t tiles = tiles_of(n_samples, 128u);
+    for (uint32_t tile = blockIdx.x; tile < tiles; tile += gridDim.x) {
         ok = false;  // until the tile's last MMA wait has succeeded
         const uint32_t s = tile * 128u + row;
         const uint64_t ri = static_cast<uint64_t>(s) * stride + offset;
@@ -1156,7 +1159,7 @@ cudaError_t pred_train_step(const PredictorDev& P, const crt_bvh_node* nodes, co
         if (e != cudaSuccess) return e;
         attr = true;
     }
-    const uint32_t tiles = (n_samples + 127) / 128;
+    const uint32_t tiles = tiles_of(n_samples, 128u);
     if (tiles == 0) return cudaSuccess;
     const uint32_t grid = tiles < static_cast<uint32_t>(kNumSms) ? tiles : static_cast<uint32_t>(kNumSms);
     pred::train_kernel<<<grid, pred::kTrainThreads, pred::kTrainSmem, s>>>(P, nodes, rays, n_rays, hits, targets, n_samples, stride,

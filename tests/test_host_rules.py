@@ -214,3 +214,22 @@ int main() {
     return 0;
 }
 ''')
+
+
+def test_counting_up_to_the_largest_calls(tmp_path):
+    """A persistent grid's tiles end for every 32-bit number of samples, and its ray counter never comes round."""
+    run_cpp(tmp_path, r'''
+int main() {
+    CHECK(crt::tiles_of(0, 128) == 0 && crt::tiles_of(1, 128) == 1 && crt::tiles_of(128, 128) == 1 && crt::tiles_of(129, 128) == 2);
+    for (uint32_t n : {0xFFFFFFFFu, 0xFFFFFF81u, 0xFFFFFF80u, 0xFFFFB400u, 0x80000001u}) {
+        const uint32_t tiles = crt::tiles_of(n, 128);
+        CHECK(128ull * tiles >= n && 128ull * (tiles - 1) < n);
+        uint64_t steps = 0;
+        uint32_t last = 0;
+        for (uint32_t tile = 151; tile < tiles; tile += 152, ++steps) { CHECK(tile >= last); last = tile; }
+        CHECK(steps == (tiles - 151 + 151) / 152);
+    }
+    CHECK(static_cast<uint64_t>(crt::kMostPoolItems) + 32ull * 152 * 64 < (1ull << 32));
+    return 0;
+}
+''')
