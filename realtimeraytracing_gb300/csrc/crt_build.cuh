@@ -169,8 +169,8 @@ void launch_trace(const TraceParams& p, uint32_t flags, int block, cudaStream_t 
 // flag.  With them the caller waits for the launch and then launches the left-over
 // rays itself; without, they are launched right away.  The list holds kWalkLeft rays
 // and is reserved once, with the context or the batch: usually it stays empty.  Where
-// more are left, all rays are looked through for marked ones; where most are, and for
-// a frame's pixels, all are walked on the binary nodes (a number of kWalkAll).
+// more are left, all rays are looked through for marked ones; where most are (a number
+// of kWalkAll), and for a frame's pixels, all are walked on the binary nodes.
 constexpr uint32_t kWalkLeft = 65536, kWalkAll = 0xFFFFFFFFu;
 constexpr size_t kWalkCounterBytes = 32, kWalkScratchBytes = kWalkCounterBytes + 4 * static_cast<size_t>(kWalkLeft);
 struct WalkScratch {

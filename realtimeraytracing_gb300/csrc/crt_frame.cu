@@ -230,12 +230,14 @@ __global__ void __launch_bounds__(kWalk4Block, kWalk4Blocks)
             redo = redo || L.redo;
             if (valid && !redo) reinterpret_cast<uint4*>(f.hits_shadow)[i] = L.hit();
         }
-        walk4_leave<false>(ctr, left, valid && redo, i, tiles);
+        if (valid && redo) {  // past the list the host does the whole image again
+            const uint32_t k = atomicAdd(&ctr->left, 1u);
+            if (k < kWalkLeft) left[k] = i;
+        }
         uint32_t next = tiles;
         if (tiles > warps) {
-            if (lane == 0) next = atomicAdd(&ctr->taken, 1u);
+            if (lane == 0) next = warps + atomicAdd(&ctr->taken, 1u);
             next = __shfl_sync(0xFFFFFFFFu, next, 0);
-            next = next < tiles - warps ? next + warps : tiles;
         }
         tile = next;
     }

@@ -406,36 +406,25 @@ struct Walk4Counters {
 };
 static_assert(sizeof(Walk4Counters) == kWalkCounterBytes, "walk scratch");
 
-// Puts item i of the lanes with redo on the list of what is left to the binary
-// walk (whole warps; one atomic each).  An overflowing list makes a launch give up
-// where what it took so far is little use: at once (MARKS false), or where 9 in 16 of
-// the first quarter of the rays were left over.  4.2 M rays over 4.19 M triangles,
-// 1/64, 1/16, 1/4, 1/2, 3/4 and all of them from far away, in runs of neighbours: 3.4,
-// 3.9, 4.3, 5.4, 6.2, 5.9 ms (every other one: 6.2); on the binary nodes from the
-// start 5.6 to 5.9.  Giving up from 7 in 16 on costs the half 0.8 ms, later than the
-// first quarter up to 2 ms.  On giving up the counter gets the number of items to
-// take, so that every warp finds nothing more to take.
-template <bool MARKS>
-__device__ __forceinline__ void walk4_leave(Walk4Counters* ctr, uint32_t* __restrict__ left, bool redo, uint32_t i,
-                                            uint32_t items) {
-    const uint32_t m = __ballot_sync(0xFFFFFFFFu, redo);
-    if (!m) return;
-    const uint32_t lane = threadIdx.x & 31u, cnt = static_cast<uint32_t>(__popc(m));
-    const int leader = __ffs(m) - 1;
-    uint32_t base = 0;
-    if (lane == static_cast<uint32_t>(leader)) {
-        base = atomicAdd(&ctr->left, cnt);
-        if (base >= kWalkLeft) {
-            const uint32_t taken = *reinterpret_cast<volatile uint32_t*>(&ctr->taken);
-            if (!MARKS || (base >= taken / 2u + taken / 16u && taken < items / 4u)) {
-                atomicMax(&ctr->taken, items);
-                *reinterpret_cast<volatile uint32_t*>(&ctr->gave_up) = 1u;
-            }
-        }
+// Puts ray i on the list of what is left to the binary walk (the compiler makes it
+// one atomic a warp).  An overflowing list makes a launch give up where what it took
+// so far is little use, where 9 in 16 of the first quarter of the rays were left over.
+// 4.2 M rays over 4.19 M triangles, 1/64, 1/16, 1/4, 1/2, 3/4 and all of them from far
+// away, in runs of neighbours: 3.4, 3.9, 4.3, 5.4, 6.2, 5.9 ms (every other one: 6.2);
+// on the binary nodes from the start 5.6 to 5.9.  Giving up from 7 in 16 on costs the
+// half 0.8 ms, later than the first quarter up to 2 ms.  On giving up the counter gets
+// the number of rays, so that every warp finds nothing more to take.
+__device__ __forceinline__ void walk4_leave(Walk4Counters* ctr, uint32_t* __restrict__ left, uint32_t i, uint32_t n_rays) {
+    const uint32_t k = atomicAdd(&ctr->left, 1u);
+    if (k < kWalkLeft) {
+        left[k] = i;
+        return;
     }
-    base = __shfl_sync(0xFFFFFFFFu, base, leader);
-    const uint32_t k = base + static_cast<uint32_t>(__popc(m & ((1u << lane) - 1u)));
-    if (redo && k < kWalkLeft) left[k] = i;
+    const uint32_t taken = *reinterpret_cast<volatile uint32_t*>(&ctr->taken);
+    if (k >= taken / 2u + taken / 16u && taken < n_rays / 4u) {
+        atomicMax(&ctr->taken, n_rays);
+        *reinterpret_cast<volatile uint32_t*>(&ctr->gave_up) = 1u;
+    }
 }
 
 // The hit record of a ray that was left over, until the binary walk writes its hit
@@ -454,14 +443,14 @@ __device__ __forceinline__ void walk4_finish(Walk4Counters* ctr, uint32_t* host_
     __threadfence();
     if (atomicInc(&ctr->blocks, gridDim.x - 1) != gridDim.x - 1) return;
     __threadfence();
-    const uint32_t listed = atomicExch(&ctr->left, 0u);
-    const uint32_t n = atomicExch(&ctr->gave_up, 0u) != 0u ? kWalkAll : listed;
-    ctr->taken = 0u;
+    // every other block is done with the counters: three loads in flight at once
+    const uint32_t listed = ld_relaxed_u32(&ctr->left), gave_up = ld_relaxed_u32(&ctr->gave_up);
+    const uint32_t unquantised = host_left ? __ldg(bad) : 0u;
+    const uint32_t n = gave_up != 0u ? kWalkAll : listed;
+    if (host_left)  // both words in one store
+        *reinterpret_cast<volatile unsigned long long*>(host_left) = static_cast<unsigned long long>(unquantised) << 32 | n;
+    ctr->taken = ctr->left = ctr->gave_up = 0u;
     ctr->last_left = n;
-    if (host_left) {
-        reinterpret_cast<volatile uint32_t*>(host_left)[0] = n;
-        reinterpret_cast<volatile uint32_t*>(host_left)[1] = *bad;
-    }
 }
 
 // Persistent warps over a ray pool, one ray per lane; lanes whose ray is done take
@@ -487,9 +476,14 @@ __global__ void __launch_bounds__(kWalk4Block, kWalk4Blocks)
     constexpr uint32_t kIdle = 0xFFFFFFFFu, kDone = 0xFFFFFFFEu;
     __shared__ uint2 s_st[kWalk4Shared + 1][kWalk4Block];  // row 0 is read (and ignored) below an empty stack
     __shared__ uint32_t s_ray_off[BATCH ? kMaxBatchScenes + 1 : 1];
+    __shared__ uint32_t s_bad[BATCH ? kMaxBatchScenes / 32 : 1];  // a bit a scene: unquantised, or one leaf
     if (BATCH) {
         for (uint32_t k = threadIdx.x; k <= n_scenes; k += kWalk4Block)
             s_ray_off[k] = k < n_scenes ? scenes[k].ray_off : scenes[n_scenes - 1].ray_off + scenes[n_scenes - 1].n_rays;
+        for (uint32_t k = threadIdx.x; k < kMaxBatchScenes; k += kWalk4Block) {
+            const uint32_t m = __ballot_sync(0xFFFFFFFFu, k < n_scenes && (__ldg(p.cw_bad + k) != 0u || scenes[k].n_tris < 2u));
+            if ((k & 31u) == 0u) s_bad[k >> 5] = m;
+        }
         __syncthreads();
     }
     const uint32_t lane = threadIdx.x & 31u;
@@ -525,7 +519,7 @@ __global__ void __launch_bounds__(kWalk4Block, kWalk4Blocks)
                         L.cw = p.cwide + 4 * static_cast<size_t>(bs.wide_off);
                         L.xtri = p.xtri + 3 * static_cast<size_t>(bs.tri_off);
                         L.abs_eps = bs.abs_eps;
-                        walkable = __ldg(p.cw_bad + k_scene) == 0u && bs.n_tris > 1;
+                        walkable = (s_bad[k_scene >> 5] >> (k_scene & 31u) & 1u) == 0u;
                     }
                     const float4 r0 = __ldg(reinterpret_cast<const float4*>(p.rays + i));
                     const float4 r1 = __ldg(reinterpret_cast<const float4*>(p.rays + i) + 1);
@@ -537,9 +531,13 @@ __global__ void __launch_bounds__(kWalk4Block, kWalk4Blocks)
         if (__all_sync(0xFFFFFFFFu, i == kDone)) break;
         const uint32_t om = walk4_run<ANY, WT, kWalk4Flush>(L, s_base, st, pool_left ? kWalk4Refill : 32);
         const bool done = (om >> lane & 1u) && i < kDone;
-        walk4_leave<true>(ctr, left, done && L.redo, i, p.n_rays);
         if (done) {
-            reinterpret_cast<uint4*>(p.hits)[i] = L.redo ? left_mark() : L.hit();
+            uint4 h = L.hit();
+            if (L.redo) {
+                walk4_leave(ctr, left, i, p.n_rays);
+                h = left_mark();
+            }
+            reinterpret_cast<uint4*>(p.hits)[i] = h;
             i = kIdle;
         }
     }
