@@ -62,7 +62,6 @@ N_BOUNCE = 8 * 1024 * 1024   # --rays: smaller copies of the batch for profilers
 BOUNCE_SEED = 11
 REF_STRIDE = 64        # the reference arm traces rays k % 64, k % 64 + 64, ... in step k
 TRI_WATERTIGHT = 0x2   # crt.h flags, also understood by the oracle
-PROFILE = "trace_walk4_kernel_bounce.md"  # ncu summary of the headline's dominant kernel
 TRI_REFERENCE = 0x0
 W1, H1 = 1920, 1080    # the icosphere frame
 
@@ -76,17 +75,13 @@ def load_peaks():
         return 6800.0, "fallback"
 
 
-def read_profile_value(name, key):
-    """A number from a committed ncu summary (a line 'key: value ...')."""
-    path = os.path.join(ROOT, "profiles", name)
+def kernel_counters(kernel):
+    """The ncu counters of a kernel that the JSON line quotes (profiles/counters.json)."""
     try:
-        with open(path) as f:
-            for line in f:
-                if line.strip().startswith(key + ":"):
-                    return float(line.split(":", 1)[1].split()[0])
-    except (OSError, ValueError):
-        pass
-    return None
+        with open(os.path.join(ROOT, "profiles", "counters.json")) as f:
+            return json.load(f)[kernel]
+    except (OSError, ValueError, KeyError):
+        return {}
 
 
 def digest(a) -> str:
@@ -351,7 +346,8 @@ def run_ours(args):
     alg_bytes = 64.0 * f_learned + 48.0 * tt_learned + (32.0 + 16.0 + 4.0) * n  # nodes, triangles, ray, hit, order
     peak, peak_kind = load_peaks()
     achieved = alg_bytes / (k_ms * 1e-3) / 1e9
-    traffic = read_profile_value(PROFILE, "traffic_bytes_per_launch")
+    counters = kernel_counters("trace_walk4_kernel")
+    traffic = counters.get("dram_bytes_per_launch")
 
     # ---- end to end through the public API: host rays in, host hits out
     rays_pin = torch.from_numpy(rays_h).pin_memory()
@@ -444,18 +440,15 @@ def run_ours(args):
                                  "4 onesweep_kernel passes, trace_walk4_kernel",
             "roofline": {"kernel": "trace_walk4_kernel (learned step: persistent warps over the rays in predicted "
                                    "order, closest hit, watertight)",
-                         "bound": "hbm", "achieved": round(achieved, 1), "peak": peak, "unit": "GB/s",
-                         "frac": round(achieved / peak, 4), "traffic": traffic, "peak_source": peak_kind,
+                         "bound": "alu and cache-miss latency", "achieved": round(achieved, 1), "peak": peak, "unit": "GB/s",
+                         "frac": round(achieved / peak, 4),
+                         "frac_is": "fetched bytes, most of them L1/L2 hits, against the HBM copy rate; not what bounds it",
+                         "traffic": traffic, "peak_source": peak_kind,
+                         "dram_frac": round(traffic / (k_ms * 1e-3) / 1e9 / peak, 4) if traffic else None,
                          "ms_per_launch": round(k_ms, 4), "alg_bytes_per_launch": int(alg_bytes),
                          "alg_bytes_model": "64 B per 4-wide node fetched + 48 B per triangle tested + 32 B ray + 16 B hit "
-                                            "+ 4 B order index per ray (fetched bytes; most are L1/L2 hits)",
-                         "l2_and_issue": {
-                             "lts_throughput_pct": read_profile_value(PROFILE, "lts_throughput_pct"),
-                             "issue_active_pct": read_profile_value(PROFILE, "issue_active_pct"),
-                             "threads_per_instruction": read_profile_value(PROFILE, "threads_per_instruction"),
-                             "source": "ncu sections of this kernel on 1,048,576 bounce rays over the same kind of scene "
-                                       "(profiles/" + PROFILE + "); bound by the ALU pipe and by L2 and HBM latency, DRAM traffic is "
-                                       "the 'traffic' bytes"}},
+                                            "+ 4 B order index per ray",
+                         "counters": counters},
             "rays_sha256": digest(rays_h),
             "reference_sample_hits_sha256": digest(ref_hits),
             "reference_sample_hits": int((ref_hits[:, 0].view(np.uint32) != 0xFFFFFFFF).sum()),
@@ -662,8 +655,7 @@ def run_frame_experiment(ctx, torch, crt, dev, stream, l2_flush, args):
         "frame_kernel": {"fetched_bytes_gbs": round(alg_bytes / (f_ms * 1e-3) / 1e9, 1),
                          "node_fetches_per_pixel": round(visited / n_rays, 2),
                          "tris_per_pixel": round(tested / n_rays, 2),
-                         "dram_bytes_per_launch": read_profile_value("frame_walk4_kernel_config1.md",
-                                                                     "traffic_bytes_per_launch")},
+                         "dram_bytes_per_launch": kernel_counters("frame_walk4_kernel").get("dram_bytes_per_launch")},
         "primary_trace_node_formats": formats,
         "mesh_upload": mesh,
         "imported_tree": imported,

@@ -24,7 +24,9 @@
  *   - Errors come back as crt_status; crt_last_error_string() describes the
  *     last failure on the calling thread.  Nothing here calls exit().
  *   - One context per host thread.  A context owns its device buffers; a
- *     crt_bvh owns the node array until crt_bvh_free.
+ *     crt_bvh owns the node array until crt_bvh_free.  Several contexts may
+ *     trace one crt_bvh at once (without a predictor's flags); a call that
+ *     changes it needs it to itself.
  */
 #ifndef CRT_H
 #define CRT_H
@@ -129,7 +131,7 @@ typedef struct crt_camera {
 #define CRT_TRACE_COMPRESSED  0x80u /* walk 64-byte compressed 4-wide nodes: 8-bit child boxes rounded
                                        outward, exact leaf boxes re-checked (same hits); the reference
                                        layout stays the export format.  Traces of >= 65,536 rays and
-                                       frames take them without the flag */
+                                       frames take them without the flag once they pay for deriving them */
 #define CRT_TRACE_PER_RAY_THREADS 0x100u /* crt_trace of >= 65,536 rays normally runs on persistent warps
                                        over the compressed nodes (closest hits of rays and scenes those
                                        cannot take: over the binary nodes) whose lanes take a new ray as

@@ -1829,10 +1829,10 @@ __global__ void __launch_bounds__(256) wide4_kernel(const float4* __restrict__ w
 // into its own two.  Every step is rounded outward by directed float rounding:
 // the child's box grown by g = 4 * abs_eps, the origin the least corner, the
 // step the least power of two with 255 of them covering the node's extent.
-// Any node may be entered, so every rank gets a record (64 B read in order, at
-// most two more gathered from L2, 64 B written per node); opening by area
-// fills the slots better than taking the grandchildren (which leave a slot
-// empty beside every leaf) and visits fewer nodes.
+// Every rank gets a record, also those a walk never enters because they were opened
+// away (64 B read in order, at most two more gathered from L2, 64 B written per node);
+// opening by area fills the slots better than taking the grandchildren (which leave a
+// slot empty beside every leaf) and visits fewer nodes.
 __device__ __forceinline__ float half_area(float4 mn, float4 mx) {
     const float x = mx.x - mn.x, y = mx.y - mn.y, z = mx.z - mn.z;
     return x * y + y * z + z * x;

@@ -1,9 +1,10 @@
 // The 64-byte compressed 4-wide nodes and the persistent closest-hit / any-hit
 // walk over them (crt_trace.cu).  Compiled with -fmad=false.
 //
-// Record of binary internal node i (any node can be entered, so the array is
-// indexed by the binary rank): its subtree's top opened twice, the internal
-// child of largest area first, so up to four children.
+// Record of binary internal node i: its subtree's top opened twice, the internal
+// child of largest area first, so up to four children.  The array is indexed by the
+// binary rank; a walk enters at rank 0 and follows references, so the records of
+// ranks that were opened away lie between those it reads.
 //   words 0-2   origin (minimum corner over the children) * 2^-60
 //   words 3, 10, 11  step * 2^73 per axis (a power of two)
 //   words 4-9   8-bit steps of the children's planes: min x, y, z, max x, y, z;
@@ -33,9 +34,12 @@
 // inside is rejected too, but for leaves flat in the ray's own plane, whose
 // triangles the shader's predicate rejects (a = 0): the tested leaves that can
 // hit are still those whose own box passes.
-// Rays outside that range (far origins, extreme scales, negative tmin), scenes
-// whose boxes cannot be quantised and walks that outgrow their stack take the
-// binary walk (trace_one), one call per ray.
+// That holds for trees whose leaf boxes are their triangles' and whose children lie
+// inside their parents, as builds and refits make them; other imported trees keep to
+// the binary nodes (crt_import.cu).  Rays outside that range (far origins, extreme
+// scales, negative tmin), scenes whose boxes cannot be quantised and walks that
+// outgrow their stack are left to the binary walk: closest hits to trace_pool_kernel
+// (crt_pool.cuh), any hits and pixels to a thread each.
 #pragma once
 
 #include <cstdint>
@@ -108,8 +112,8 @@ __device__ __forceinline__ bool walk4_setup(Walk4Ray& w, float3 o, float3 d, flo
 // Distance of the plane in byte C of word; SAT: clamped to [0, 1], which is free
 // (distances carry 2^-100, so only negative ones, and NaN, change: to 0).  Steps
 // stored as floats instead of exponent bytes, this clamp and three-operand minima
-// take 17 ALU operations off a visit: 1280x720 frames 838 -> 795 us, 8.4 M bounce
-// rays 6.32 -> 6.16 ms (memory latency bounds those).
+// take 17 ALU operations off a visit: 1920x1080 frames with shadow rays over 1.31 M
+// triangles 838 -> 795 us, 8.4 M bounce rays 6.32 -> 6.16 ms (memory latency bounds those).
 template <int C, bool SAT = false>
 __device__ __forceinline__ float walk4_plane(uint32_t word, float a, float b) {
     // byte C of word to bits 16-23, zeros elsewhere
