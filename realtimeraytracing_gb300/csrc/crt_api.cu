@@ -848,8 +848,9 @@ crt_status frame_walk4(crt_ctx* x, const crt_bvh* b, const crt_camera* cam, uint
 }
 
 // A one-launch frame, and the pixels it leaves to the binary walk.
-crt_status frame_launch(crt_ctx* x, const crt_bvh* b, const crt::TraceParams& p, const crt_camera* cam, uint32_t width, uint32_t height,
-                        const float* light, crt_hit* hits_shadow, uint32_t flags, const crt::ShadeParams* sp) {
+crt_status frame_launch(crt_ctx* x, const crt_bvh* b, const crt::TraceParams& p, const crt_camera* cam, uint32_t width,
+                        uint32_t height, const float* light, crt_hit* hits_shadow, uint32_t flags,
+                        const crt::ShadeParams* sp) {
     const crt::WalkScratch ws(x->walk.p, x->hw_dev + 4);
     crt::TraceParams q = p;
     auto launch = [&](uint32_t left) {
@@ -867,12 +868,12 @@ crt_status frame_launch(crt_ctx* x, const crt_bvh* b, const crt::TraceParams& p,
     return finish_walk(x, b);
 }
 
-// Enqueues one traversal launch on device-resident rays/hits (no sync).
 // Below this a launch of one thread per ray fills the GPU as well; 65,536 rays over
 // 0.26, 2.0 and 4.2 M triangles: 239, 300 and 328 us, one thread a ray 346, 402, 558.
 constexpr uint32_t kPoolMinRays = 65536;
 constexpr uint32_t kChunkedCopyMinRays = 1u << 20;  // crt_trace: smaller host batches copy in one piece
 
+// Enqueues one traversal launch on device-resident rays/hits (no sync).
 // classes_ready: the predictor's classes of these rays are already in its
 // class buffer, and with CRT_TRACE_PREDICTOR_ORDER their order keys in its
 // order scratch (crt_trace's chunked copy ran the inference per chunk).
@@ -886,8 +887,9 @@ crt_status trace_device(crt_ctx* x, const crt_bvh* b, const crt_ray* d_rays, uin
     // Large batches over one scene: persistent warps, over the compressed nodes where
     // those take its rays (closest hits over the binary nodes otherwise); pixels in
     // 8x4 tiles, seeded, 4-wide and counting walks keep one thread per ray.
-    const bool large = !(flags & (CRT_TRACE_WIDE | CRT_TRACE_PER_RAY_THREADS | CRT_TRACE_USE_PREDICTOR | CRT_TRACE_STATS)) &&
-                       !seed_classes && tile_width == 0 && n_rays >= kPoolMinRays && n_rays <= crt::kMostPoolItems && b->n > 1;
+    constexpr uint32_t kOneThread = CRT_TRACE_WIDE | CRT_TRACE_PER_RAY_THREADS | CRT_TRACE_USE_PREDICTOR | CRT_TRACE_STATS;
+    const bool large = !(flags & kOneThread) && !seed_classes && tile_width == 0 && n_rays >= kPoolMinRays &&
+                       n_rays <= crt::kMostPoolItems && b->n > 1;
     bool pool = large && walk4_usable(b);
     if (flags & CRT_TRACE_COMPRESSED) {
         CRT_TRY(ensure_cwide(x, b));
@@ -1986,7 +1988,7 @@ struct crt_batch {
     uint64_t trace_demand = 0;            // what those trees' traces have asked for (crt::Walk4Demand)
     bool g_cwide = false;                 // the captured graph derives them
     uint32_t* cw_bad() const { return reinterpret_cast<uint32_t*>(cwide.as<char>() + 64ull * n_tris); }
-    DevBuf walk;                          // the persistent trace's scratch (crt::WalkScratch; counters zero between launches)
+    DevBuf walk;                          // the persistent trace's scratch (crt::WalkScratch)
     bool models_set = false;
     cudaGraphExec_t graph = nullptr;
     const void* g_tris = nullptr;
@@ -2076,7 +2078,8 @@ crt_status batch_trace_enqueue(crt_ctx* x, crt_batch* bt, const crt_ray* rays, u
     const crt::WalkScratch ws(bt->walk.p, nullptr);
     bool walk4 = batch_pool(bt, flags) && bt->cwide.p;
     if (walk4) {
-        bt->trace_demand += (flags & CRT_TRACE_ANY) ? crt::Walk4Demand::any(bt->n_rays) : crt::Walk4Demand::closest(bt->n_rays);
+        const uint64_t rays_now = bt->n_rays;
+        bt->trace_demand += (flags & CRT_TRACE_ANY) ? crt::Walk4Demand::any(rays_now) : crt::Walk4Demand::closest(rays_now);
         walk4 = bt->cwide_ready || crt::walk4_pays(bt->trace_demand, bt->n_tris);
     }
     if (walk4) {

@@ -178,7 +178,8 @@ struct WalkScratch {
     uint32_t* left = nullptr;
     uint32_t* host_left = nullptr;
     WalkScratch() = default;
-    WalkScratch(void* scratch, uint32_t* host) : ctr(static_cast<uint32_t*>(scratch)), left(ctr + kWalkCounterBytes / 4), host_left(host) {}
+    WalkScratch(void* scratch, uint32_t* host)
+        : ctr(static_cast<uint32_t*>(scratch)), left(ctr + kWalkCounterBytes / 4), host_left(host) {}
 };
 // Many rays by persistent warps that refill finished lanes from a ray counter;
 // compressed nodes, no seeding, rays in caller order or p.order.  launch_trace_left:
